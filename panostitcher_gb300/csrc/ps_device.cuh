@@ -13,7 +13,7 @@
 //   C[j]   short4 collapsed result of level j >= 1 (resultPyr after
 //          normalise + collapse); |value| < 3300 so int16 is exact.
 //   maps   float2 dst->src map, stored tile-compact for the level-0 tiles
-//          that a camera covers (512 pixels per 32x16 tile, row-major in the tile).
+//          that a camera covers (512 pixels per 32x16 tile, in 16x2 blocks).
 // Work is described by item lists built at prepare time from the pyramids'
 // supports, so no kernel touches canvas area a camera cannot influence.
 #pragma once
@@ -30,6 +30,13 @@ constexpr int kRemapTW = 32, kRemapTH = 16;    // level-0 remap tile (two pixels
 constexpr int kDownTW = 32, kDownTH = 16;      // pyrDown output tile (two pixels per thread)
 constexpr int kBlendTW = 64, kBlendTH = 16;    // blend tile (a 2x2 pixel block per thread)
 constexpr int kThreads = 256;
+
+// Pixel i of a remap tile (its map, its linear weight): the tile is 16 blocks
+// of 16x2 pixels, two across and eight down, a warp's 32 pixels each.  The
+// frame's texels under a 16x2 block lie on fewer lines than under a 32x1 row,
+// whose image in the frame is tilted.
+__host__ __device__ constexpr int mapTileX(int i) { return (i >> 5 & 1) * 16 + (i & 15); }
+__host__ __device__ constexpr int mapTileY(int i) { return (i >> 6) * 2 + (i >> 4 & 1); }
 
 struct LevelDev {
     int w, h;            // level size
@@ -149,17 +156,6 @@ struct Segment {
     const RigDev* rig;
     const FrameDev* frame;
     int count, prefix;
-};
-
-// A level-0 pixel whose fp32 remap lies near a rounding tie, listed by the
-// remap for its exact recompute: everything the recompute needs without
-// looking the tile up again.
-struct RemapTie {
-    const FrameDev* frame;
-    const RigDev* rig;
-    float mx, my;    // the map value
-    uint32_t pixel;  // y * pitch + x in the camera's level-0 plane
-    int cam;
 };
 
 #ifdef __CUDACC__

@@ -170,7 +170,7 @@ struct LaunchShape {
     int tailHalf = 1;              // the tail blends levels above 0 in 64x8 half tiles
     int ctasPerSm[3] = {0, 0, 0};  // k_remap, k_pyrdown, k_blend; 0 = as many as fit
     int smallBlendMaxItems = 0;    // blend levels above 0 with at most this many tiles run in k_blend_small
-    int remapDefer = 1;            // near-tie remap pixels recomputed by k_remap_fix (1) or inside k_remap (0)
+    int remapDefer = 1;            // kept for its callers: both values run the same launch
     bool operator==(const LaunchShape& o) const
     {
         return tailMaxItems == o.tailMaxItems && tailCluster == o.tailCluster && tailHalf == o.tailHalf &&
@@ -184,18 +184,16 @@ struct LaunchShape {
 // perSm > 0 caps the CTAs per SM of the one-wave persistent grid; counter
 // (remap and blend) is a zeroed int through which the launch hands out its
 // work items
-// defer: near-tie pixels go on the list (tieCount, ties) for launchRemapFix;
-// otherwise k_remap recomputes them itself.  srcFmt: the format of every
-// source of the launch (PS_FMT_BGR32 selects the specialised kernel), or 0
-// when they differ
-cudaError_t launchRemap(const Segment* segs, int nsegs, int total, int perSm, int* counter, int* tieCount,
-                        RemapTie* ties, bool defer, int srcFmt, cudaStream_t st);
-// the pixels k_remap listed as lying near a rounding tie, recomputed exactly;
-// ties has room for kRemapTiesPerTile entries per remap tile of the launch,
-// and tieCount is a zeroed int
-cudaError_t launchRemapFix(const Segment* segs, int nsegs, int total, const int* tieCount, const RemapTie* ties,
-                           cudaStream_t st);
-constexpr int kRemapTiesPerTile = 2;
+// srcFmt: the format of every source of the launch as remapSourceFormat
+// gives it, or 0 when they differ; maps: every rig of the launch has resident
+// maps
+cudaError_t launchRemap(const Segment* segs, int nsegs, int total, int perSm, int* counter, int srcFmt, bool maps,
+                        cudaStream_t st);
+// The format k_remap, k_linear and k_reproject16s may be specialised for: the
+// frame's own, or 0 (the general kernel) for frames of one column or row,
+// where the clamped left taps of the specialised ones would not exist, and for
+// pitches of 4 GB or more, which their 32-bit row step cannot hold.
+int remapSourceFormat(int fmt, int sw, int sh, long long pitch);
 cudaError_t launchPyrDown(const Segment* segs, int nsegs, int total, int perSm, cudaStream_t st);
 // counter: a zeroed int the launch hands its tiles out through
 // Accesses the checked build's kernels refused since the last reset
@@ -218,7 +216,7 @@ cudaError_t launchTail(const Segment* segs, int nsegs, int cluster, cudaStream_t
 int residentCtasPerSm(int kind);
 int tailClusterMax();
 // linear-blend mode: LinearItems of every segment; maxCams sizes the LUT stage
-cudaError_t launchLinear(const Segment* segs, int nsegs, int total, int maxCams, cudaStream_t st);
+cudaError_t launchLinear(const Segment* segs, int nsegs, int total, int maxCams, int srcFmt, cudaStream_t st);
 
 // ---- camera parameter files (ps_params.cpp) ----------------------------------------
 // loadPhotoParams for PTGui .pts files; empty when the file holds no usable

@@ -4,8 +4,6 @@
 // work lists:
 //   k_remap        level 0: LUT gain + bilinear remap of every covered tile,
 //                  written as uchar4 G0 (cudaTransform + cudaReprojectTo16S);
-//   k_remap_fix    (launch shapes that defer them) the near-tie pixels the
-//                  remap listed, recomputed with the double sequence;
 //   k_pyrdown      levels 1..L: masked 5x5 decimation G_j -> G_{j+1}
 //                  (pyrDown16SC4To16SC4 with alpha scale);
 //   k_blend        levels L..0: for every canvas tile, the Laplacian of each
@@ -29,7 +27,6 @@
 
 namespace ps {
 
-__constant__ int c_k5[5] = {1, 4, 6, 4, 1};
 
 // ---- the checked build ---------------------------------------------------------
 // Compiled with -DPS_CHECK_BOUNDS (libpanostitch_checked.so), every global
@@ -97,10 +94,17 @@ __device__ __forceinline__ long long cBytes(const LevelDev& L) { return (long lo
 // arithmetic follows the double-precision CPU bilinear (source/Warp/
 // ZReproject.cpp:101-130): weights from the float map coordinates, taps
 // (x0,y0) (x1,y0) (x0,y1) (x1,y1) with x1 and y1 clamped to the frame, the
-// result rounded half to even.  The fast path computes in fp32 (absolute
-// error < 1.3e-4 for values <= 255); a result within 2e-4 of a rounding tie
-// is recomputed with the reference's exact sequence of IEEE double
-// operations, so the stored byte equals the double-precision one.
+// result rounded half to even.
+//
+// The fast path is fixed point.  A weight is W = w * 2^24, read out of the
+// mantissa of 1 + w, with an error below 2^-23 (one fma rounded at 2^-24,
+// and 1 - fx rounded at 2^-25 where the coordinate is below 1); the weight of
+// (x0,y0) is 2^24 minus the other three, so constant areas are exact.  A
+// channel is then four 32-bit multiply-adds of table bytes by weights, exact in
+// 32 bits: no byte-to-float step per tap, and the rounded byte is the top byte
+// of the sum, packed by two PRMTs.  The sum's error is below 255 * 4 * 2^-24 =
+// 6.1e-5; a sum within 2^-13 of a rounding tie (0.07% of the pixels) goes to
+// remapExact.
 // ============================================================================
 __device__ __forceinline__ uint32_t loadTexel(const uint8_t* row, int x, int fmt, const uint8_t* base, long long bytes)
 {
@@ -128,71 +132,163 @@ __device__ __noinline__ int bilinearExact(double x, double y, int x0, int y0, in
 // its low mantissa bits.
 __device__ __forceinline__ float byteToFloat(uint32_t b) { return __int_as_float(0x4B000000u | b) - 8388608.f; }
 
-// The remap of one pixel: the texel fetch and the LUT + bilinear finish.
-struct RemapTap {
-    uint32_t t00, t01, t10, t11;  // texels (x0,y0) (x1,y0) (x0,y1) (x1,y1)
-    float fx, fy;                 // fractional coordinates
-    int x0, y0;                   // -1: the map is invalid here
+// The camera frame a pixel samples.
+struct RemapSrc {
+    const uint8_t* base;
+    long long pitch;
+    int fmt, sw, sh;
 };
 
-// Integer parts use a float addition at 2^23 scale (round toward zero: the
-// floor of a non-negative coordinate), which keeps the conversion unit out
-// of the inner loop.
-__device__ __forceinline__ void remapFetch(float2 m, const uint8_t* base, long long pitch, int fmt, int sw, int sh,
-                                           RemapTap& p)
+// The byte the reference's double sequence gives, for a pixel the fast path
+// could not decide (its map is valid).  A coordinate of 1 or more has a
+// fraction of at most 23 bits, so the weights are integers over 2^46 and the
+// sum is exact in 64 bits; the double sequence is within 7 * 2^-46 of it, so
+// where the sum is farther than 2^-40 from a tie its rounding is the same.
+// The double sequence itself (FP64 runs at 1/64 rate here: 60 such operations
+// a pixel were most of the old recompute's cost) is left for the sums nearer
+// than that and for coordinates below 1 with a longer fraction.
+__device__ __noinline__ uint32_t remapExact(float2 m, RemapSrc src, const uint8_t* lut)
 {
-    p.x0 = -1;
-    if (!(m.x >= 0.f && m.y >= 0.f && m.x < (float)sw && m.y < (float)sh)) return;
-    const float tx = __fadd_rz(m.x, 8388608.f), ty = __fadd_rz(m.y, 8388608.f);  // 2^23 + floor
-    const int x0 = __float_as_int(tx) - 0x4B000000, y0 = __float_as_int(ty) - 0x4B000000;
+    const uint8_t* base = src.base;
+    const long long pitch = src.pitch;
+    const int fmt = src.fmt, sw = src.sw, sh = src.sh;
+    const int x0 = (int)m.x, y0 = (int)m.y;
     const int x1 = min(x0 + 1, sw - 1), y1 = min(y0 + 1, sh - 1);
     const uint8_t* r0 = base + (size_t)y0 * pitch;
     const uint8_t* r1 = base + (size_t)y1 * pitch;
     const long long bytes = pitch * sh;
-    p.t00 = loadTexel(r0, x0, fmt, base, bytes);
-    p.t01 = loadTexel(r0, x1, fmt, base, bytes);
-    p.t10 = loadTexel(r1, x0, fmt, base, bytes);
-    p.t11 = loadTexel(r1, x1, fmt, base, bytes);
-    p.fx = m.x - (tx - 8388608.f);  // exact
-    p.fy = m.y - (ty - 8388608.f);
-    p.x0 = x0;
-    p.y0 = y0;
-}
-
-// Returns B | G << 8 | R << 16 (0 where the map is invalid).
-// The fp32 result of a pixel's three channels.  Where a channel lies within
-// 2e-4 of a rounding tie, fp32 cannot decide the byte: with exact, that
-// channel is recomputed with the reference's double sequence; without,
-// nearTie is set and the caller has the pixel recomputed (k_remap_fix).
-template <bool kExact>
-__device__ __forceinline__ uint32_t remapFinish(const RemapTap& p, float2 m, const uint8_t* lut, bool& nearTie)
-{
-    if (p.x0 < 0) return 0;
-    const float gx = 1.f - p.fx, gy = 1.f - p.fy;
-    const float w00 = gx * gy, w01 = p.fx * gy, w10 = gx * p.fy, w11 = p.fx * p.fy;
+    const uint32_t t00 = loadTexel(r0, x0, fmt, base, bytes), t01 = loadTexel(r0, x1, fmt, base, bytes);
+    const uint32_t t10 = loadTexel(r1, x0, fmt, base, bytes), t11 = loadTexel(r1, x1, fmt, base, bytes);
+    const float qx = (m.x - (float)x0) * 8388608.f, qy = (m.y - (float)y0) * 8388608.f;  // both exact
+    const uint32_t ix = (uint32_t)qx, iy = (uint32_t)qy;
+    const bool fixed = (float)ix == qx && (float)iy == qy;
+    const uint64_t one = 8388608u;
+    const uint64_t w11 = (uint64_t)ix * iy, w01 = (uint64_t)ix * (one - iy), w10 = (one - ix) * iy;
+    const uint64_t w00 = (one - ix) * (one - iy);
     uint32_t out = 0;
-#pragma unroll
+#pragma unroll 1
     for (int c = 0; c < 3; c++) {
-        const uint32_t sel = 0x4440u | (uint32_t)c;  // byte c, zero-extended
-        const int p00 = lut[c * 256 + __byte_perm(p.t00, 0, sel)];
-        const int p01 = lut[c * 256 + __byte_perm(p.t01, 0, sel)];
-        const int p10 = lut[c * 256 + __byte_perm(p.t10, 0, sel)];
-        const int p11 = lut[c * 256 + __byte_perm(p.t11, 0, sel)];
-        const float r = fmaf(byteToFloat(p11), w11,
-                             fmaf(byteToFloat(p10), w10, fmaf(byteToFloat(p01), w01, byteToFloat(p00) * w00)));
-        // r lies in [-1e-4, 255 + 1e-4]; 1.5 * 2^23 + r rounds r to the
-        // nearest integer, ties to even, in the low mantissa bits
-        const float t = r + 12582912.f;
-        int v = __float_as_int(t) - 0x4B400000;
-        const bool tie = fabsf(r - (t - 12582912.f)) > 0.4998f;  // within 2e-4 of a tie
-        if (kExact) {
-            if (tie) v = bilinearExact((double)m.x, (double)m.y, p.x0, p.y0, p00, p01, p10, p11);
-        } else {
-            nearTie |= tie;
-        }
-        out |= (uint32_t)v << (8 * c);
+        const int s = 8 * c;
+        const uint8_t* t = lut + c * 256;
+        const int p00 = t[(t00 >> s) & 0xFF], p01 = t[(t01 >> s) & 0xFF];
+        const int p10 = t[(t10 >> s) & 0xFF], p11 = t[(t11 >> s) & 0xFF];
+        const uint64_t sum = p00 * w00 + p01 * w01 + p10 * w10 + p11 * w11 + (1ull << 45);  // + 1/2
+        uint32_t v = (uint32_t)(sum >> 46);
+        const uint64_t frac = sum & ((1ull << 46) - 1);  // 0 at a tie
+        if (!fixed || ((frac + 64) & ((1ull << 46) - 1)) <= 128)
+            v = (uint32_t)bilinearExact((double)m.x, (double)m.y, x0, y0, p00, p01, p10, p11);
+        out |= v << s;
     }
     return out;
+}
+
+// The remap of one pixel: the texel fetch and the LUT + bilinear finish.
+struct RemapTap {
+    uint32_t t00, t01, t10, t11;  // texels (x0,y0) (x1,y0) (x0,y1) (x1,y1)
+    float fx, fy;                 // fractional coordinates
+    bool valid;                   // false: the map is invalid here
+};
+
+// The texel pair (x, y), (x + 1, y) of a BGR24 row: its six bytes start at any
+// alignment, so they are cut out of the two or (offset 3) three aligned words
+// that hold them.  Every word read holds at least one of the six bytes.  The
+// byte loads this replaced (twelve a pixel) kept L1 at 63% of its rate: the
+// remap of 2 x 960x960 to 2048x1024 took 53 us.
+__device__ __forceinline__ void loadPair24(const uint8_t* p, uint32_t& a, uint32_t& b, const uint8_t* base,
+                                           long long bytes)
+{
+    a = b = 0;
+    if (!insideRange(p, 6, base, bytes)) return;
+    const uint32_t o = (uint32_t)reinterpret_cast<uintptr_t>(p) & 3u;
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(p - o);
+    const uint32_t w0 = __ldg(q), w1 = __ldg(q + 1), w2 = o == 3 ? __ldg(q + 2) : 0u;
+    a = __byte_perm(w0, w1, 0x3210u + 0x1111u * o);
+    b = o == 3 ? __byte_perm(w1, w2, 0x5432u) : __byte_perm(w0, w1, 0x0543u + 0x0111u * o);
+}
+
+// Integer parts use a float addition at 2^23 scale (round toward zero: the
+// floor of a non-negative coordinate, an integer of 2^31 or more for any other
+// value), which keeps the conversion unit out of the inner loop.  kFmt fixes
+// the format at compile time (see remapSourceFormat) or leaves everything to
+// the frame (0).  With kFmt the left tap is clamped to the frame's last but one
+// column (row), the fraction then becoming 1, which is the same sample: both
+// columns and both rows are then at fixed distances, and an invalid pixel
+// fetches some texel of the frame, to be dropped by the finish.
+template <int kFmt>
+__device__ __forceinline__ void remapFetch(float2 m, const RemapSrc& S, RemapTap& p)
+{
+    const long long bytes = S.pitch * S.sh;
+    if constexpr (kFmt != 0) {
+        const uint32_t x = __float_as_uint(__fadd_rz(m.x, 8388608.f)) - 0x4B000000u;
+        const uint32_t y = __float_as_uint(__fadd_rz(m.y, 8388608.f)) - 0x4B000000u;
+        p.valid = x < (uint32_t)S.sw && y < (uint32_t)S.sh;
+        const uint32_t x0 = min(x, (uint32_t)S.sw - 2u), y0 = min(y, (uint32_t)S.sh - 2u);
+        p.fx = fminf(m.x - (__uint_as_float(x0 + 0x4B000000u) - 8388608.f), 1.f);  // exact
+        p.fy = fminf(m.y - (__uint_as_float(y0 + 0x4B000000u) - 8388608.f), 1.f);
+        const uint32_t pitch = (uint32_t)S.pitch;
+        const uint8_t* r0 = S.base + (uint64_t)y0 * pitch;
+        if constexpr (kFmt == PS_FMT_BGR32) {
+            const uint32_t* q0 = reinterpret_cast<const uint32_t*>(r0) + x0;
+            const uint32_t* q1 = reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(q0) + pitch);
+            p.t00 = ldChecked(q0, S.base, bytes);
+            p.t01 = ldChecked(q0 + 1, S.base, bytes);
+            p.t10 = ldChecked(q1, S.base, bytes);
+            p.t11 = ldChecked(q1 + 1, S.base, bytes);
+        } else {
+            const uint8_t* q0 = r0 + 3 * x0;
+            loadPair24(q0, p.t00, p.t01, S.base, bytes);
+            loadPair24(q0 + pitch, p.t10, p.t11, S.base, bytes);
+        }
+    } else {
+        p.valid = m.x >= 0.f && m.y >= 0.f && m.x < (float)S.sw && m.y < (float)S.sh;
+        const float mx = p.valid ? m.x : 0.f, my = p.valid ? m.y : 0.f;
+        const float tx = __fadd_rz(mx, 8388608.f), ty = __fadd_rz(my, 8388608.f);
+        const int x0 = __float_as_int(tx) - 0x4B000000, y0 = __float_as_int(ty) - 0x4B000000;
+        const int x1 = min(x0 + 1, S.sw - 1), y1 = min(y0 + 1, S.sh - 1);
+        const uint8_t* r0 = S.base + (size_t)y0 * S.pitch;
+        const uint8_t* r1 = S.base + (size_t)y1 * S.pitch;
+        p.t00 = loadTexel(r0, x0, S.fmt, S.base, bytes);
+        p.t01 = loadTexel(r0, x1, S.fmt, S.base, bytes);
+        p.t10 = loadTexel(r1, x0, S.fmt, S.base, bytes);
+        p.t11 = loadTexel(r1, x1, S.fmt, S.base, bytes);
+        p.fx = mx - (tx - 8388608.f);
+        p.fy = my - (ty - 8388608.f);
+    }
+}
+
+// w * 2^24 of a weight in [0, 1]: 1 + w has w * 2^23 in its mantissa.
+__device__ __forceinline__ uint32_t fixedWeight(float a, float b)
+{
+    return 2u * __float_as_uint(fmaf(a, b, 1.f)) - 0x7F000000u;
+}
+
+// A LUT in shared memory on a 256-byte boundary, so that one PRMT puts a
+// texel's byte c into the low byte of the table's address.
+__device__ __forceinline__ uint32_t lutEntry(uint32_t lutAddr, uint32_t texel, int c)
+{
+    return static_cast<const uint8_t*>(__cvta_shared_to_generic(__byte_perm(texel, lutAddr, 0x7650u + c)))[c * 256];
+}
+
+// Returns B | G << 8 | R << 16 (0 where the map is invalid); nearTie: the
+// pixel needs remapExact.  lutAddr: the camera's LUT (lutEntry).
+__device__ __forceinline__ uint32_t remapFinish(const RemapTap& p, uint32_t lutAddr, bool& nearTie)
+{
+    const float gx = 1.f - p.fx, gy = 1.f - p.fy;
+    const uint32_t w01 = fixedWeight(p.fx, gy), w10 = fixedWeight(gx, p.fy), w11 = fixedWeight(p.fx, p.fy);
+    const uint32_t w00 = 0x1000000u - (w01 + w10 + w11);
+    uint32_t r[3];
+    nearTie = false;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const uint32_t p00 = lutEntry(lutAddr, p.t00, c), p01 = lutEntry(lutAddr, p.t01, c);
+        const uint32_t p10 = lutEntry(lutAddr, p.t10, c), p11 = lutEntry(lutAddr, p.t11, c);
+        r[c] = p00 * w00 + p01 * w01 + p10 * w10 + p11 * w11 + 0x800000u;  // + 1/2
+        // the fraction (24 bits, moved to the top) within 2^-13 of zero
+        nearTie |= (r[c] << 8) + (2048u << 8) < (4096u << 8);
+    }
+    nearTie = nearTie && p.valid;
+    // the top bytes of the three sums
+    return __byte_perm(__byte_perm(r[0], r[1], 0x0073), r[2], 0x0710) & (p.valid ? 0x00FFFFFFu : 0u);
 }
 
 // Map-free remap: the source coordinate of canvas pixel (cx, cy) in fp32,
@@ -252,228 +348,229 @@ __device__ __forceinline__ float2 mapFreeValue(const RemapParamF& m, uint32_t co
                        fminf(fmaxf(v.y, 0.f), __int_as_float(__float_as_int((float)sh) - 1)));
 }
 
-// The remap of one pixel, exact (kExact) or fp32 with the near-tie flag.
-template <bool kExact = true>
-__device__ __forceinline__ uint32_t remapPixel(float2 m, const uint8_t* base, long long pitch, int fmt, int sw,
-                                               int sh, const uint8_t* lut, bool& nearTie)
-{
-    RemapTap p;
-    remapFetch(m, base, pitch, fmt, sw, sh, p);
-    return remapFinish<kExact>(p, m, lut, nearTie);
-}
-
-__device__ __forceinline__ uint32_t remapPixel(float2 m, const uint8_t* base, long long pitch, int fmt, int sw,
-                                               int sh, const uint8_t* lut)
-{
-    bool unused = false;
-    return remapPixel<true>(m, base, pitch, fmt, sw, sh, lut, unused);
-}
-
-// Level-0 remap over the covered 32x16 tiles of every camera; each thread
-// remaps two pixels (rows ly and ly + 8) so two independent gathers are in
-// flight; the tile's map is 512 consecutive float2.  A CTA walks a
-// contiguous run of items (camera-major, so the camera rarely changes): the
-// camera's constants and LUT are reloaded only when it does, and the next
-// item's map is loaded before the current item's gathers.
-struct RemapSeg {
-    const RemapItem* items;
-    int prefix, end;
-    const RigDev* R;
-    const FrameDev* F;
-};
-
-__device__ __forceinline__ RemapSeg remapSeg(const Segment* segs, int nsegs, int s, int total)
-{
-    const Segment& sg = segs[s];
-    return {static_cast<const RemapItem*>(sg.items), sg.prefix, s + 1 < nsegs ? segs[s + 1].prefix : total, sg.rig,
-            sg.frame};
-}
-
-// Items are handed out in chunks of kRemapChunk through `counter` (zero at
-// launch); the next chunk is fetched one chunk ahead, so the next item and
-// its map are always known before the current item is gathered.
-constexpr int kRemapChunk = 8;
-
-// The map value of pixel (lx, row) of a remap tile: from the resident maps,
-// or, map-free, from the coverage bits (the FP64 coverage of prepare) and the
-// fp32 geometry.
-__device__ __forceinline__ float2 remapMapValue(const RigDev& R, const RemapItem& itm, int lx, int row)
+// The map value of pixel i of a remap tile (mapTileX, mapTileY): from the
+// resident map at `map`, or, map-free, from the tile's coverage words there
+// (the FP64 coverage of prepare) and the fp32 geometry.
+template <bool kMaps>
+__device__ __forceinline__ float2 remapMapValue(const void* map, const RigDev& R, const RemapItem& itm, int i)
 {
     const long long tiles = R.numRemapItems;
-    if (R.maps) {
-        const float2* mt = R.maps + (size_t)itm.mapTile * (kRemapTW * kRemapTH) + row * kRemapTW + lx;
-        return ldChecked(mt, R.maps, tiles * kRemapTW * kRemapTH * (long long)sizeof(float2));
+    if (kMaps || R.maps)
+        return ldChecked(static_cast<const float2*>(map) + i, R.maps,
+                         tiles * kRemapTW * kRemapTH * (long long)sizeof(float2));
+    const int lx = mapTileX(i), ly = mapTileY(i);
+    const uint32_t bits = ldChecked(static_cast<const uint32_t*>(map) + ly, R.covTiles, tiles * kRemapTH * 4);
+    return mapFreeValue(R.camsF[itm.cam], bits, lx, itm.tx * kRemapTW + lx, itm.ty * kRemapTH + ly, R.srcW, R.srcH);
+}
+
+// Level-0 remap over the covered 32x16 tiles of every camera.  The launch is
+// bound by L1's rate on the gathers (four texels and twelve table bytes a
+// pixel: its data pipe is 66% busy, its tags more) and by their latency, so
+// everything is arranged for warps that never wait for each other: a consumer
+// warp takes 16x2 blocks of a chunk's tiles, one pixel a lane, and all it needs
+// besides its map values lies in shared memory or registers.  (A warp's taps
+// fall on 4.3 - 8.3 lines of the frame with 16x2 blocks, 5.6 - 13 with 32x1
+// rows.)  A producer warp hands the tiles out: it takes a run of tiles from the
+// launch's counter and resolves them to chunks (one camera's tiles, its frame,
+// its LUT) in a ring that it fills ahead of the consumers.  Runs shrink
+// towards the end of the launch (a share of what is left), so the CTAs finish
+// together.
+// The rare pixels near a rounding tie are only marked (a ballot kept by the
+// lane of the block's number) and recomputed by remapExact after the chunk: a
+// call or a second code path inside the loop costs every pixel its registers.
+// Measured (events around the launch): 6 x 1920x1080 to 4096x2048 57.5 us, and
+// 69 + 14 us before (float sums, whole CTAs per tile, the near-tie pixels in a
+// second launch); 8 x 3840x2160 to 7680x3840 197 us, before 263 + 19 us; one
+// 1920x960 BGR24 frame to 2048x1024 29 us, before 54 + 14 us.  Four CTAs of 56
+// registers: more warps spill (9 consumers: 62 us, 11 at 40 registers: 68 us),
+// texels fetched one block ahead cost registers too (73 us).
+constexpr int kRemapWarps = 8;                         // consumer warps
+constexpr int kRemapThreads = (kRemapWarps + 1) * 32;  // + the producer warp
+constexpr int kRemapRun = 8;                           // most tiles of a chunk
+constexpr int kRemapCtas = 4;                          // CTAs per SM: 36 warps of 56 registers
+constexpr int kRemapRing = 4;                          // chunks
+constexpr int kRemapBlocks = kRemapTW * kRemapTH / 32;  // 16x2 blocks of a tile
+static_assert((kRemapRun * kRemapBlocks + kRemapWarps - 1) / kRemapWarps <= 32, "a lane per block of a warp's chunk");
+
+// A tile of a chunk, resolved: its map (map-free: its coverage words), its
+// first pixel in the camera's level-0 plane (a 128-byte boundary) and, in that
+// address's low bits, the number of its rows inside the canvas.
+struct alignas(16) RemapTile {
+    const void* map;
+    uint64_t g;
+};
+__device__ __forceinline__ uint32_t* remapPixelAt(const RemapTile& t, uint32_t off)
+{
+    return reinterpret_cast<uint32_t*>(t.g & ~31ull) + off;
+}
+
+struct RemapChunk {
+    RemapSrc src;
+    const RigDev* R;
+    int n, gpitch;        // n: tiles, 0 ends the launch
+    RemapTile tile[kRemapRun];
+    RemapItem item[kRemapRun];
+    alignas(256) uint8_t lut[3 * 256];
+};
+
+// The producer warp's state: the run of tiles it has taken.
+struct RemapRun {
+    int it, end, pos, seg;
+};
+
+// The next chunk (all lanes of the producer warp); false after the last one.
+__device__ __forceinline__ bool remapProduce(RemapRun& r, RemapChunk& c, const Segment* segs, int nsegs, int total,
+                                             int* counter)
+{
+    const int lane = threadIdx.x & 31;
+    if (r.it >= r.end) {  // a new run: a quarter of a CTA's share of what is left
+        const int want = max(1, min(kRemapRun, (total - r.pos) / (4 * (int)gridDim.x)));
+        int v = 0;
+        if (lane == 0) v = atomicAdd(counter, want);
+        r.it = r.pos = __shfl_sync(0xffffffffu, v, 0);
+        r.end = min(r.it + want, total);
     }
-    const uint32_t* cw = R.covTiles + (size_t)itm.mapTile * kRemapTH;
-    const uint32_t bits = ldChecked(cw + row, R.covTiles, tiles * kRemapTH * 4);
-    return mapFreeValue(R.camsF[itm.cam], bits, lx, itm.tx * kRemapTW + lx, itm.ty * kRemapTH + row, R.srcW,
-                        R.srcH);
-}
-
-// The exact pixel: the reference's double sequence where fp32 lies near a
-// tie; the camera's LUT is read from global memory.
-__device__ __forceinline__ void remapFixPixel(const FrameDev& F, const RigDev& R, float2 m, uint32_t pixel, int cam)
-{
-    const uint32_t pitch = (uint32_t)R.lv[0].pitch;
-    if (pixel % pitch >= (uint32_t)R.W || pixel / pitch >= (uint32_t)R.H) return;  // a tile's part off the canvas
-    const uint32_t v = remapPixel(m, F.src[cam], F.srcPitch[cam], F.srcFmt, R.srcW, R.srcH, F.luts + cam * 768);
-    uint32_t* g = reinterpret_cast<uint32_t*>(R.lv[0].G) + (size_t)cam * R.lv[0].camStride + pixel;
-    if (inside(g, R.lv[0].G, gBytes(R, R.lv[0]))) *g = v;
-}
-
-// The rare pixels whose fp32 remap lies near a rounding tie (about 0.1% of
-// them) get the reference's double sequence.  Inline (kDefer false), the
-// check with its out-of-line double call costs every pixel (a quarter of the
-// kernel's instructions; keeping the double sequence inline spills).
-// Deferred, a warp appends such pixels to the launch's list (tieCount, ties:
-// room for tieCap entries, one atomic per warp) and k_remap_fix recomputes
-// them before anything reads level 0: the remap is faster, and the short
-// extra launch costs latency only when nothing else is in flight.  kFmt
-// fixes the sources' format at compile time (PS_FMT_BGR32, the common
-// case, saves the per-texel format test) or leaves it to the frame (0).
-template <bool kDefer, int kFmt>
-__global__ void __launch_bounds__(kThreads, 4) k_remap(const Segment* __restrict__ segs, int nsegs, int total,
-                                                       int* __restrict__ counter, int* __restrict__ tieCount,
-                                                       RemapTie* __restrict__ ties, int tieCap)
-{
-    __shared__ uint8_t lut[3 * 256];
-    __shared__ int s_grab;
-    auto grab = [&] {  // all threads together
-        __syncthreads();
-        if (threadIdx.x == 0) s_grab = atomicAdd(counter, kRemapChunk);
-        __syncthreads();
-        return s_grab;
-    };
-    const int lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
-    // The hand-out counter, items, descriptors and maps are written before
-    // the launch sequence, not by a kernel: the first chunk and its map are
-    // fetched while the previous kernel finishes.
-    int it = grab(), end = 0, nextBegin = total, s = 0;
-    RemapSeg cur{};
+    if (r.it >= total) {
+        if (lane == 0) c.n = 0;
+        return false;
+    }
+    r.seg = findSegment(segs, nsegs, r.it, r.seg);
+    const Segment& sg = segs[r.seg];
+    const int last = min(r.end, sg.prefix + sg.count);  // the run's tiles in this segment
     RemapItem item{};
-    float2 m0{}, m1{};
-    if (it < total) {
-        end = min(it + kRemapChunk, total);
-        nextBegin = grab();
-        s = findSegment(segs, nsegs, it, 0);
-        cur = remapSeg(segs, nsegs, s, total);
-        item = cur.items[it - cur.prefix];
-        m0 = remapMapValue(*cur.R, item, lx, ly);
-        m1 = remapMapValue(*cur.R, item, lx, ly + 8);
+    if (r.it + lane < last) item = static_cast<const RemapItem*>(sg.items)[r.it - sg.prefix + lane];
+    const int cam = __shfl_sync(0xffffffffu, (int)item.cam, 0);
+    const uint32_t other = __ballot_sync(0xffffffffu, r.it + lane >= last || item.cam != cam);
+    const int n = other ? __ffs(other) - 1 : 32;  // the leading tiles of that camera
+    const FrameDev& F = *sg.frame;
+    const RigDev& R = *sg.rig;
+    const LevelDev& L = R.lv[0];
+    if (lane < n) {
+        c.item[lane] = item;
+        c.tile[lane] = {R.maps ? static_cast<const void*>(R.maps + (size_t)item.mapTile * (kRemapTW * kRemapTH))
+                               : static_cast<const void*>(R.covTiles + (size_t)item.mapTile * kRemapTH),
+                        reinterpret_cast<uint64_t>(reinterpret_cast<uint32_t*>(L.G) + (size_t)cam * L.camStride +
+                                                   (size_t)item.ty * kRemapTH * L.pitch + item.tx * kRemapTW) +
+                            (uint32_t)min(kRemapTH, R.H - item.ty * kRemapTH)};
     }
-    waitPrevGrid();
-    allowNextGrid();
-    if (it >= total) return;
-    // constants of the loaded camera
-    int camSeg = -1, cam = -1;
-    const FrameDev* camF = nullptr;  // the frame and rig of the loaded camera
-    const RigDev* camR = nullptr;
-    const uint8_t* base = nullptr;
-    long long pitch = 0;
-    int fmt = 0, sw = 0, sh = 0, W = 0, H = 0, gpitch = 0;
-    uint32_t* G = nullptr;
-    const void* gLo = nullptr;  // the level-0 buffer of the camera's rig and its extent (checked build)
-    long long gExt = 0;
-    for (;;) {
-        if (item.cam != cam || s != camSeg) {  // uniform across the block
-            const FrameDev& F = *cur.F;
-            const RigDev& R = *cur.R;
-            cam = item.cam;
-            camSeg = s;
-            camF = &F;
-            camR = &R;
-            base = F.src[cam];
-            pitch = F.srcPitch[cam];
-            fmt = F.srcFmt;
-            sw = R.srcW;
-            sh = R.srcH;
-            W = R.W;
-            H = R.H;
-            gpitch = R.lv[0].pitch;
-            G = reinterpret_cast<uint32_t*>(R.lv[0].G) + (size_t)cam * R.lv[0].camStride;
-            gLo = R.lv[0].G;
-            gExt = gBytes(R, R.lv[0]);
-            __syncthreads();
-            const uint8_t* src = F.luts + cam * 768;
-            for (int k = threadIdx.x; k < 768; k += kThreads) lut[k] = __ldg(src + k);
-            __syncthreads();
-        }
-        // the next item (the rest of this chunk, else the next chunk's first) and its map
-        const int nit = it + 1 < end ? it + 1 : (nextBegin < total ? nextBegin : -1);
-        RemapItem nitem = item;
-        float2 n0 = m0, n1 = m1;
-        if (nit >= 0) {
-            if (nit >= cur.end) {
-                s = findSegment(segs, nsegs, nit, s);
-                cur = remapSeg(segs, nsegs, s, total);
-            }
-            nitem = cur.items[nit - cur.prefix];
-            n0 = remapMapValue(*cur.R, nitem, lx, ly);
-            n1 = remapMapValue(*cur.R, nitem, lx, ly + 8);
-        }
-        bool tie0 = false, tie1 = false;
-        const uint32_t v0 = remapPixel<!kDefer>(m0, base, pitch, kFmt ? kFmt : fmt, sw, sh, lut, tie0);
-        const uint32_t v1 = remapPixel<!kDefer>(m1, base, pitch, kFmt ? kFmt : fmt, sw, sh, lut, tie1);
-        const int x = item.tx * kRemapTW + lx, y0 = item.ty * kRemapTH + ly, y1 = y0 + 8;
-        if (kDefer) {
-            const uint32_t b0 = __ballot_sync(0xffffffffu, tie0), b1 = __ballot_sync(0xffffffffu, tie1);
-            if (b0 | b1) {  // the warp's near-tie pixels, one atomic for the warp
-                int e = 0;
-                if (lx == 0) e = atomicAdd(tieCount, __popc(b0) + __popc(b1));
-                e = __shfl_sync(0xffffffffu, e, 0);
-                const uint32_t below = (1u << lx) - 1u;
-                const int e0 = e + __popc(b0 & below), e1 = e + __popc(b0) + __popc(b1 & below);
-                if (tie0 && e0 < tieCap) ties[e0] = {camF, camR, m0.x, m0.y, (uint32_t)((size_t)y0 * gpitch + x), cam};
-                if (tie1 && e1 < tieCap) ties[e1] = {camF, camR, m1.x, m1.y, (uint32_t)((size_t)y1 * gpitch + x), cam};
-            }
-        }
-        if (x < W) {
-            if (y0 < H && inside(G + (size_t)y0 * gpitch + x, gLo, gExt)) G[(size_t)y0 * gpitch + x] = v0;
-            if (y1 < H && inside(G + (size_t)y1 * gpitch + x, gLo, gExt)) G[(size_t)y1 * gpitch + x] = v1;
-        }
-        if (nit < 0) break;
-        if (it + 1 >= end) {  // into the next chunk; fetch the one after it
-            end = min(nextBegin + kRemapChunk, total);
-            nextBegin = grab();
-        }
-        it = nit;
-        item = nitem;
-        m0 = n0;
-        m1 = n1;
+    const uint4* t = reinterpret_cast<const uint4*>(F.luts + cam * 768);
+    for (int k = lane; k < 48; k += 32) reinterpret_cast<uint4*>(c.lut)[k] = __ldg(t + k);
+    if (lane == 0) {
+        c.src = {F.src[cam], F.srcPitch[cam], F.srcFmt, R.srcW, R.srcH};
+        c.R = &R;
+        c.n = n;
+        c.gpitch = L.pitch;
     }
+    r.it += n;
+    return true;
 }
 
-// The exact recompute of the pixels k_remap put on the launch's list
-// (ties[0 .. *tieCount)), one thread per entry.  An entry carries its frame,
-// rig, map value and pixel, so the recompute is a short chain of loads.
-// Most frames list none.  A list that overflowed (more than tieCap entries)
-// has every pixel of the launch recomputed, tile by tile.
-__global__ void __launch_bounds__(kThreads) k_remap_fix(const Segment* __restrict__ segs, int nsegs, int total,
-                                                        const int* __restrict__ tieCount,
-                                                        const RemapTie* __restrict__ ties, int tieCap)
+// A wait of the launch ran out: every frame of it is flagged.
+__device__ __forceinline__ void flagTimeout(const Segment* segs, int nsegs)
 {
-    waitPrevGrid();
-    allowNextGrid();
-    const int listed = __ldcg(tieCount);
-    const long long stride = (long long)gridDim.x * kThreads;
-    const long long first = blockIdx.x * (long long)kThreads + threadIdx.x;
-    if (listed <= tieCap) {
-        for (long long e = first; e < listed; e += stride) {
-            const RemapTie t = ties[e];
-            remapFixPixel(*t.frame, *t.rig, make_float2(t.mx, t.my), t.pixel, t.cam);
+    for (int k = 0; k < nsegs; k++)
+        if (segs[k].frame->status) atomicOr(segs[k].frame->status, 4);
+}
+
+template <int kFmt, bool kMaps>
+__global__ void __launch_bounds__(kRemapThreads, kRemapCtas) k_remap(const Segment* __restrict__ segs, int nsegs,
+                                                                        int total, int* __restrict__ counter)
+{
+    __shared__ RemapChunk s_chunk[kRemapRing];
+    __shared__ uint64_t full[kRemapRing], empty[kRemapRing];
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0)
+        for (int k = 0; k < kRemapRing; k++) {
+            mbarInit(&full[k], 1);
+            mbarInit(&empty[k], kRemapWarps);
         }
+    __syncthreads();
+    if (threadIdx.x >= kRemapWarps * 32) {
+        // The hand-out counter, items, descriptors and LUTs are written before
+        // the launch sequence, not by a kernel: the first chunks are resolved
+        // while the previous kernel finishes.
+        RemapRun r{0, 0, 0, 0};
+        bool more = true;
+        for (int k = 0; more; k++) {
+            const int s = k % kRemapRing;
+            if (k >= kRemapRing && !mbarWait(&empty[s], (k / kRemapRing - 1) & 1)) {
+                if (lane == 0) flagTimeout(segs, nsegs);
+                break;
+            }
+            more = remapProduce(r, s_chunk[s], segs, nsegs, total, counter);
+            __syncwarp();
+            if (lane == 0) mbarArrive(&full[s]);
+        }
+        waitPrevGrid();
+        allowNextGrid();
         return;
     }
-    for (long long e = first; e < (long long)total * kThreads * 2; e += stride) {  // the list overflowed
-        const int it = (int)(e / (kThreads * 2)), t = (int)(e % (kThreads * 2)) >> 1, half = (int)(e & 1);
-        const int s = findSegment(segs, nsegs, it, 0);
-        const RemapSeg cur = remapSeg(segs, nsegs, s, total);
-        const RemapItem item = cur.items[it - cur.prefix];
-        const int lx = t & 31, row = (t >> 5) + half * 8;
-        const int x = item.tx * kRemapTW + lx, y = item.ty * kRemapTH + row;
-        if (x < cur.R->W && y < cur.R->H)
-            remapFixPixel(*cur.F, *cur.R, remapMapValue(*cur.R, item, lx, row),
-                          (uint32_t)((size_t)y * cur.R->lv[0].pitch + x), item.cam);
+    const int warp = threadIdx.x >> 5;
+    bool waited = false;
+    for (int k = 0;; k++) {
+        const int s = k % kRemapRing;
+        if (!mbarWait(&full[s], (k / kRemapRing) & 1)) {
+            if (lane == 0) flagTimeout(segs, nsegs);
+            break;
+        }
+        const RemapChunk& c = s_chunk[s];
+        const int blocks = c.n * kRemapBlocks;
+        if (blocks == 0) break;
+        // registers for what every block of the chunk needs: the compiler
+        // would read shared memory again after each store
+        const RemapSrc src = c.src;
+        const int gpitch = c.gpitch;
+        const RigDev* const R = c.R;
+        const uint32_t lutAddr = smemAddr(c.lut);
+        auto mapAt = [&](int b) {
+            return remapMapValue<kMaps>(c.tile[b / kRemapBlocks].map, *R, c.item[b / kRemapBlocks],
+                                        b % kRemapBlocks * 32 + lane);
+        };
+        int b = warp;
+        float2 m{};
+        if (b < blocks) m = mapAt(b);
+        if (!waited) {
+            waitPrevGrid();
+            allowNextGrid();
+            waited = true;
+        }
+        uint32_t ties = 0;  // lane q: the near-tie pixels of the warp's q-th block
+        for (int q = 0; b < blocks; q++) {
+            float2 nm = m;
+            if (b + kRemapWarps < blocks) nm = mapAt(b + kRemapWarps);
+            RemapTap p;
+            remapFetch<kFmt>(m, src, p);
+            bool tie;
+            const uint32_t v = remapFinish(p, lutAddr, tie);
+            // pixels beyond the canvas are invalid in the map: the columns
+            // inside the plane's row pitch keep their zeros
+            const int i = b % kRemapBlocks * 32 + lane;
+            const RemapTile t = c.tile[b / kRemapBlocks];
+            uint32_t* g = remapPixelAt(t, (uint32_t)(mapTileY(i) * gpitch + mapTileX(i)));
+            if (mapTileY(i) < (int)(t.g & 31u) && inside(g, R->lv[0].G, gBytes(*R, R->lv[0]))) *g = v;
+            const uint32_t near = __ballot_sync(0xffffffffu, tie);
+            if (lane == q) ties = near;
+            b += kRemapWarps;
+            m = nm;
+        }
+        for (uint32_t any = __ballot_sync(0xffffffffu, ties != 0); any; any &= any - 1) {
+            const int q = __ffs(any) - 1;
+            if (__shfl_sync(0xffffffffu, ties, q) >> lane & 1u) {
+                const int e = warp + q * kRemapWarps, i = e % kRemapBlocks * 32 + lane;
+                const RemapTile te = c.tile[e / kRemapBlocks];
+                uint32_t* g = remapPixelAt(te, (uint32_t)(mapTileY(i) * gpitch + mapTileX(i)));
+                const float2 me = remapMapValue<kMaps>(te.map, *R, c.item[e / kRemapBlocks], i);
+                const uint32_t v = remapExact(me, c.src, c.lut);
+                if (inside(g, R->lv[0].G, gBytes(*R, R->lv[0]))) *g = v;
+            }
+            __syncwarp();
+        }
+        __syncwarp();
+        if (lane == 0) mbarArrive(&empty[s]);  // this warp is done with the chunk
+    }
+    if (!waited) {
+        waitPrevGrid();
+        allowNextGrid();
     }
 }
 
@@ -484,9 +581,8 @@ __global__ void __launch_bounds__(kThreads) k_remap_fix(const Segment* __restric
 // in fp32 with one rounded product and one rounded sum per camera
 // (reprojectWeightedAccumulateTo32F, source/Warp/ZReproject.cpp:606-633),
 // then convertTo(CV_8U): round half to even, saturate.  One 32x16 canvas
-// tile per item (all tiles are items, so uncovered tiles are written 0);
-// each thread two pixels (rows ly and ly + 8).  The LUTs of all cameras of
-// the current rig are staged in shared memory.
+// tile per item (all tiles are items, so uncovered tiles are written 0).  The
+// LUTs of all cameras of the current rig are staged in shared memory.
 // ============================================================================
 __device__ __forceinline__ void storeBgr(const FrameDev& F, int x, int y, int H, uint32_t v)
 {
@@ -511,71 +607,154 @@ __device__ __forceinline__ uint32_t roundSaturate3(const float* a)
     return v;
 }
 
-__global__ void __launch_bounds__(kThreads) k_linear(const Segment* __restrict__ segs, int nsegs, int total)
+// A CTA takes runs of four consecutive tiles and one pixel a thread (16x2 block
+// per warp); the map, weight and camera of the next (tile, camera) pair are
+// loaded before the current one's texels, the launch being bound by the latency
+// of that chain and by L1.  6 x 1920x1080 to 4096x2048: 109 us before (32x1
+// rows, two pixels a thread, no look-ahead, FP64 near ties), 87.5 us now; three
+// CTAs of 40 registers spill (135 us).
+constexpr int kLinearThreads = kRemapTW * kRemapTH;
+constexpr int kLinearCtas = 2;  // CTAs per SM
+constexpr int kLinearRun = 4;  // consecutive tiles of a CTA's step
+
+template <int kFmt>
+__global__ void __launch_bounds__(kLinearThreads, kLinearCtas) k_linear(const Segment* __restrict__ segs, int nsegs,
+                                                                           int total)
 {
-    extern __shared__ uint8_t luts[];  // 768 bytes per camera of the current rig
-    const int lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
+    extern __shared__ __align__(256) uint8_t luts[];  // 768 bytes per camera of the current rig
+    const int lx = mapTileX(threadIdx.x), ly = mapTileY(threadIdx.x);
     int s = 0, loaded = -1;
     waitPrevGrid();
     allowNextGrid();
-    for (int it = blockIdx.x; it < total; it += gridDim.x) {  // uniform across the CTA
-        s = findSegment(segs, nsegs, it, s);
-        const Segment& sg = segs[s];
-        const RigDev& R = *sg.rig;
-        const FrameDev& F = *sg.frame;
-        if (s != loaded) {
-            __syncthreads();
-            for (int k = threadIdx.x; k < R.n * 768; k += kThreads) luts[k] = __ldg(F.luts + k);
-            __syncthreads();
-            loaded = s;
-        }
-        const LinearItem item = static_cast<const LinearItem*>(sg.items)[it - sg.prefix];
-        float a0[3] = {0.f, 0.f, 0.f}, a1[3] = {0.f, 0.f, 0.f};
-        for (uint32_t q = 0; q < item.count; q++) {
-            const RemapItem ri = R.remapItems[item.first + q];
-            const size_t base = (size_t)ri.mapTile * (kRemapTW * kRemapTH) + threadIdx.x;
-            const long long tilePx = (long long)R.numRemapItems * kRemapTW * kRemapTH;
-            const float2 m0 = ldChecked(R.maps + base, R.maps, tilePx * 8);
-            const float2 m1 = ldChecked(R.maps + base + kThreads, R.maps, tilePx * 8);
-            const float w0 = ldChecked(R.linWeights + base, R.linWeights, tilePx * 4);
-            const float w1 = ldChecked(R.linWeights + base + kThreads, R.linWeights, tilePx * 4);
-            const uint8_t* src = F.src[ri.cam];
-            const long long pitch = F.srcPitch[ri.cam];
-            const uint8_t* lut = luts + ri.cam * 768;
-            const uint32_t v0 = remapPixel(m0, src, pitch, F.srcFmt, R.srcW, R.srcH, lut);
-            const uint32_t v1 = remapPixel(m1, src, pitch, F.srcFmt, R.srcW, R.srcH, lut);
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                a0[c] = __fadd_rn(a0[c], __fmul_rn(byteToFloat((v0 >> (8 * c)) & 0xFF), w0));
-                a1[c] = __fadd_rn(a1[c], __fmul_rn(byteToFloat((v1 >> (8 * c)) & 0xFF), w1));
+    for (int run = blockIdx.x * kLinearRun; run < total; run += gridDim.x * kLinearRun) {
+        for (int it = run, end; it < min(run + kLinearRun, total); it = end) {  // the run's tiles, segment by segment
+            s = findSegment(segs, nsegs, it, s);
+            const Segment& sg = segs[s];
+            end = min(min(run + kLinearRun, total), sg.prefix + sg.count);
+            const RigDev& R = *sg.rig;
+            const FrameDev& F = *sg.frame;
+            if (s != loaded) {
+                __syncthreads();
+                for (int k = threadIdx.x; k < R.n * 768; k += kLinearThreads) luts[k] = __ldg(F.luts + k);
+                __syncthreads();
+                loaded = s;
             }
-        }
-        const int x = item.tx * kRemapTW + lx, y0 = item.ty * kRemapTH + ly, y1 = y0 + 8;
-        if (x < R.W) {
-            if (y0 < R.H) storeBgr(F, x, y0, R.H, roundSaturate3(a0));
-            if (y1 < R.H) storeBgr(F, x, y1, R.H, roundSaturate3(a1));
+            const uint32_t lutAddr = smemAddr(luts);
+            const LinearItem* items = static_cast<const LinearItem*>(sg.items) + (it - sg.prefix);
+            const long long tilePx = (long long)R.numRemapItems * kRemapTW * kRemapTH;
+            // The tiles' cameras are consecutive remap items (a remap item's
+            // tile number is its index), so the next one's map, weight and
+            // camera are loaded before the current one's texels.
+            float2 m = make_float2(-1.f, -1.f);
+            float w = 0.f;
+            int cam = 0;
+            const uint32_t last = items[end - it - 1].first + items[end - it - 1].count;
+            auto load = [&](uint32_t e, float2& mv, float& wv, int& cv) {
+                const size_t base = (size_t)e * (kRemapTW * kRemapTH) + threadIdx.x;
+                mv = ldChecked(R.maps + base, R.maps, tilePx * 8);
+                wv = ldChecked(R.linWeights + base, R.linWeights, tilePx * 4);
+                cv = R.remapItems[e].cam;
+            };
+            auto add = [&](float* a, uint32_t v, float wv) {
+#pragma unroll
+                for (int c = 0; c < 3; c++) a[c] = __fadd_rn(a[c], __fmul_rn(byteToFloat((v >> (8 * c)) & 0xFF), wv));
+            };
+            uint32_t e = items[0].first;
+            if (e < last) load(e, m, w, cam);
+            for (int k = 0; k < end - it; k++) {
+                const LinearItem item = items[k];
+                float a[3] = {0.f, 0.f, 0.f};
+                bool ties = false;
+                for (const uint32_t stop = item.first + item.count; e < stop; e++) {
+                    float2 nm = m;
+                    float nw = w;
+                    int ncam = cam;
+                    if (e + 1 < last) load(e + 1, nm, nw, ncam);
+                    const RemapSrc src{F.src[cam], F.srcPitch[cam], F.srcFmt, R.srcW, R.srcH};
+                    RemapTap p;
+                    remapFetch<kFmt>(m, src, p);
+                    bool tie;
+                    const uint32_t v = remapFinish(p, lutAddr + cam * 768, tie);
+                    ties |= tie;
+                    add(a, v, w);
+                    m = nm;
+                    w = nw;
+                    cam = ncam;
+                }
+                if (ties) {  // near a rounding tie in some camera: the pixel again, exactly
+                    a[0] = a[1] = a[2] = 0.f;
+                    for (uint32_t q = item.first; q < item.first + item.count; q++) {
+                        float2 qm;
+                        float qw;
+                        int qcam;
+                        load(q, qm, qw, qcam);
+                        const RemapSrc src{F.src[qcam], F.srcPitch[qcam], F.srcFmt, R.srcW, R.srcH};
+                        const bool valid = qm.x >= 0.f && qm.y >= 0.f && qm.x < (float)src.sw && qm.y < (float)src.sh;
+                        add(a, valid ? remapExact(qm, src, luts + qcam * 768) : 0u, qw);
+                    }
+                }
+                const int x = item.tx * kRemapTW + lx, y = item.ty * kRemapTH + ly;
+                if (x < R.W && y < R.H) storeBgr(F, x, y, R.H, roundSaturate3(a));
+            }
         }
     }
 }
 
 // Standalone cudaReprojectTo16S with an optional LUT: full-canvas maps,
-// int16x4 output (B, G, R, 0).
-__global__ void __launch_bounds__(kThreads) k_reproject16s(const uint8_t* __restrict__ src, long long srcPitch,
-                                                           int sw, int sh, int fmt, const float* __restrict__ xmap,
+// int16x4 output (B, G, R, 0).  A CTA takes a 64x16 tile, a warp four 16x2
+// blocks of it whose map values are all loaded first, so that one round trip to
+// memory serves 128 pixels; a block no pixel of which is valid (most of a
+// canvas, for one camera) fetches nothing.  Near-tie pixels are recomputed at
+// the end, which keeps the call out of the blocks' code.  4096x2048 from
+// 1920x1080: 53.8 us before (one pixel a thread, FP64 behind a
+// test per channel), 29.2 us now.
+constexpr int kReprojectBlocks = 4;
+
+template <int kFmt>
+__global__ void __launch_bounds__(kThreads) k_reproject16s(RemapSrc src, const float* __restrict__ xmap,
                                                            const float* __restrict__ ymap, long long mapPitch,
                                                            int W, int H, const uint8_t* __restrict__ glut,
                                                            short4* dst, long long dstPitch)
 {
-    __shared__ uint8_t lut[3 * 256];
+    __shared__ __align__(256) uint8_t lut[3 * 256];
+    const int lane = threadIdx.x & 31;
+    const int x = blockIdx.x * 16 * kReprojectBlocks + (lane & 15), y = blockIdx.y * 16 + (threadIdx.x >> 5) * 2 + (lane >> 4);
+    float2 m[kReprojectBlocks];
+    if (y < H) {
+        const float* xr = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(xmap) + (size_t)y * mapPitch);
+        const float* yr = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(ymap) + (size_t)y * mapPitch);
+#pragma unroll
+        for (int k = 0; k < kReprojectBlocks; k++)
+            m[k] = x + 16 * k < W ? make_float2(__ldg(xr + x + 16 * k), __ldg(yr + x + 16 * k)) : make_float2(-1.f, -1.f);
+    }
     for (int k = threadIdx.x; k < 768; k += kThreads) lut[k] = glut ? glut[k] : (uint8_t)(k & 255);
     __syncthreads();
-    const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
-    if (x >= W || y >= H) return;
-    const float2 m = make_float2(reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(xmap) + y * mapPitch)[x],
-                                 reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(ymap) + y * mapPitch)[x]);
-    const uint32_t v = remapPixel(m, src, srcPitch, fmt, sw, sh, lut);
-    reinterpret_cast<short4*>(reinterpret_cast<uint8_t*>(dst) + y * dstPitch)[x] =
-        make_short4((short)(v & 0xFF), (short)((v >> 8) & 0xFF), (short)((v >> 16) & 0xFF), 0);
+    if (y >= H) return;
+    const uint32_t lanes = __activemask();  // the warp's lanes inside the canvas
+    short4* row = reinterpret_cast<short4*>(reinterpret_cast<uint8_t*>(dst) + (size_t)y * dstPitch) + x;
+    auto store = [&](int k, uint32_t v) {
+        row[16 * k] = make_short4((short)(v & 0xFF), (short)((v >> 8) & 0xFF), (short)((v >> 16) & 0xFF), 0);
+    };
+    uint32_t ties = 0;
+#pragma unroll
+    for (int k = 0; k < kReprojectBlocks; k++) {
+        uint32_t v = 0;
+        if (__any_sync(lanes, m[k].x >= 0.f)) {
+            RemapTap p;
+            bool tie;
+            remapFetch<kFmt>(m[k], src, p);
+            v = remapFinish(p, smemAddr(lut), tie);
+            if (tie) ties |= 1u << k;
+        }
+        if (x + 16 * k < W) store(k, v);
+    }
+#pragma unroll 1
+    for (; ties; ties &= ties - 1) {
+        const int k = __ffs(ties) - 1;
+        const float* xr = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(xmap) + (size_t)y * mapPitch);
+        const float* yr = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(ymap) + (size_t)y * mapPitch);
+        store(k, remapExact(make_float2(xr[x + 16 * k], yr[x + 16 * k]), src, lut));
+    }
 }
 
 // ============================================================================
@@ -2116,56 +2295,37 @@ int residentCtasPerSm(int kind)
 {
     switch (kind) {
     case 0:
-        return std::min(std::min(residentPerSm<k_remap<true, 0>>(kThreads), residentPerSm<k_remap<false, 0>>(kThreads)),
-                        std::min(residentPerSm<k_remap<true, PS_FMT_BGR32>>(kThreads),
-                                 residentPerSm<k_remap<false, PS_FMT_BGR32>>(kThreads)));
+        return std::min({residentPerSm<k_remap<0, true>>(kRemapThreads), residentPerSm<k_remap<PS_FMT_BGR24, true>>(kRemapThreads),
+                         residentPerSm<k_remap<PS_FMT_BGR32, true>>(kRemapThreads)});
     case 1: return residentPerSm<k_pyrdown>(kThreads);
     case 2: return residentPerSm<k_blend>(kBlendThreads);
     default: return 1;
     }
 }
 
-// Entries the launch's tie list has room for.
-static int tieListCap(int total)
+int remapSourceFormat(int fmt, int sw, int sh, long long pitch)
 {
-#ifdef PS_CHECK_BOUNDS
-    // the checked build's tests may lower it (0: k_remap_fix takes its overflow path)
-    static const int perTile = [] {
-        const char* v = std::getenv("PS_CHECKED_TIE_LIST_PER_TILE");
-        return v ? std::max(0, std::min(std::atoi(v), kRemapTiesPerTile)) : kRemapTiesPerTile;
-    }();
-    return perTile * total;
-#else
-    return kRemapTiesPerTile * total;
-#endif
+    constexpr int kMost = 1 << 22;
+    return sw >= 2 && sh >= 2 && sw <= kMost && sh <= kMost && pitch >= 0 && pitch < (1LL << 32) ? fmt : 0;
 }
 
-template <bool kDefer, int kFmt>
-static cudaError_t launchRemapAs(const Segment* segs, int nsegs, int total, int perSm, int* counter, int* tieCount,
-                                 RemapTie* ties, cudaStream_t st)
+template <int kFmt, bool kMaps>
+static cudaError_t launchRemapAs(const Segment* segs, int nsegs, int total, int perSm, int* counter, cudaStream_t st)
 {
-    return launchPdl(k_remap<kDefer, kFmt>, gridFor(total, residentPerSm<k_remap<kDefer, kFmt>>(kThreads), perSm),
-                     kThreads, st, segs, nsegs, total, counter, tieCount, ties, kDefer ? tieListCap(total) : 0);
+    return launchPdl(k_remap<kFmt, kMaps>, gridFor(total, residentPerSm<k_remap<kFmt, kMaps>>(kRemapThreads), perSm),
+                     kRemapThreads, st, segs, nsegs, total, counter);
 }
 
-cudaError_t launchRemap(const Segment* segs, int nsegs, int total, int perSm, int* counter, int* tieCount,
-                        RemapTie* ties, bool defer, int srcFmt, cudaStream_t st)
+cudaError_t launchRemap(const Segment* segs, int nsegs, int total, int perSm, int* counter, int srcFmt, bool maps,
+                        cudaStream_t st)
 {
     if (total <= 0) return cudaSuccess;
-    const bool bgr32 = srcFmt == PS_FMT_BGR32;
-    if (defer)
-        return bgr32 ? launchRemapAs<true, PS_FMT_BGR32>(segs, nsegs, total, perSm, counter, tieCount, ties, st)
-                     : launchRemapAs<true, 0>(segs, nsegs, total, perSm, counter, tieCount, ties, st);
-    return bgr32 ? launchRemapAs<false, PS_FMT_BGR32>(segs, nsegs, total, perSm, counter, tieCount, ties, st)
-                 : launchRemapAs<false, 0>(segs, nsegs, total, perSm, counter, tieCount, ties, st);
-}
-
-cudaError_t launchRemapFix(const Segment* segs, int nsegs, int total, const int* tieCount, const RemapTie* ties,
-                           cudaStream_t st)
-{
-    if (total <= 0) return cudaSuccess;
-    return launchPdl(k_remap_fix, 2 * smCount(), kThreads, st, segs, nsegs, total, tieCount, ties,
-                     tieListCap(total));
+    if (!maps) return launchRemapAs<0, false>(segs, nsegs, total, perSm, counter, st);
+    switch (srcFmt) {
+    case PS_FMT_BGR32: return launchRemapAs<PS_FMT_BGR32, true>(segs, nsegs, total, perSm, counter, st);
+    case PS_FMT_BGR24: return launchRemapAs<PS_FMT_BGR24, true>(segs, nsegs, total, perSm, counter, st);
+    default: return launchRemapAs<0, true>(segs, nsegs, total, perSm, counter, st);
+    }
 }
 
 cudaError_t launchPyrDown(const Segment* segs, int nsegs, int total, int perSm, cudaStream_t st)
@@ -2175,12 +2335,12 @@ cudaError_t launchPyrDown(const Segment* segs, int nsegs, int total, int perSm, 
                      total);
 }
 
-cudaError_t launchLinear(const Segment* segs, int nsegs, int total, int maxCams, cudaStream_t st)
+template <int kFmt>
+static cudaError_t launchLinearAs(const Segment* segs, int nsegs, int total, int maxCams, cudaStream_t st)
 {
-    if (total <= 0) return cudaSuccess;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(gridFor(total, residentPerSm<k_linear>(kThreads, (size_t)PS_MAX_CAMS * 768)));
-    cfg.blockDim = dim3(kThreads);
+    cfg.gridDim = dim3(gridFor(total, residentPerSm<k_linear<kFmt>>(kLinearThreads, (size_t)PS_MAX_CAMS * 768)));
+    cfg.blockDim = dim3(kLinearThreads);
     cfg.dynamicSmemBytes = (size_t)maxCams * 768;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -2188,7 +2348,17 @@ cudaError_t launchLinear(const Segment* segs, int nsegs, int total, int maxCams,
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_linear, segs, nsegs, total);
+    return cudaLaunchKernelEx(&cfg, k_linear<kFmt>, segs, nsegs, total);
+}
+
+cudaError_t launchLinear(const Segment* segs, int nsegs, int total, int maxCams, int srcFmt, cudaStream_t st)
+{
+    if (total <= 0) return cudaSuccess;
+    switch (srcFmt) {
+    case PS_FMT_BGR32: return launchLinearAs<PS_FMT_BGR32>(segs, nsegs, total, maxCams, st);
+    case PS_FMT_BGR24: return launchLinearAs<PS_FMT_BGR24>(segs, nsegs, total, maxCams, st);
+    default: return launchLinearAs<0>(segs, nsegs, total, maxCams, st);
+    }
 }
 
 cudaError_t launchBlend(const Segment* segs, int nsegs, int total, int perSm, int* counter, int probePolls,
@@ -2314,9 +2484,18 @@ cudaError_t launchReprojectTo16S(const uint8_t* src, long long srcPitch, int src
                                  const float* xmap, const float* ymap, long long mapPitch, int dstW, int dstH,
                                  const uint8_t* lut, int16_t* dst, long long dstPitch, cudaStream_t st)
 {
-    dim3 grid((dstW + 31) / 32, (dstH + 7) / 8);
-    k_reproject16s<<<grid, kThreads, 0, st>>>(src, srcPitch, srcW, srcH, srcFmt, xmap, ymap, mapPitch, dstW, dstH,
-                                              lut, reinterpret_cast<short4*>(dst), dstPitch);
+    dim3 grid((dstW + 16 * kReprojectBlocks - 1) / (16 * kReprojectBlocks), (dstH + 15) / 16);
+    const RemapSrc S{src, srcPitch, srcFmt, srcW, srcH};
+    short4* const d = reinterpret_cast<short4*>(dst);
+    switch (remapSourceFormat(srcFmt, srcW, srcH, srcPitch)) {
+    case PS_FMT_BGR32:
+        k_reproject16s<PS_FMT_BGR32><<<grid, kThreads, 0, st>>>(S, xmap, ymap, mapPitch, dstW, dstH, lut, d, dstPitch);
+        break;
+    case PS_FMT_BGR24:
+        k_reproject16s<PS_FMT_BGR24><<<grid, kThreads, 0, st>>>(S, xmap, ymap, mapPitch, dstW, dstH, lut, d, dstPitch);
+        break;
+    default: k_reproject16s<0><<<grid, kThreads, 0, st>>>(S, xmap, ymap, mapPitch, dstW, dstH, lut, d, dstPitch);
+    }
     return cudaGetLastError();
 }
 

@@ -568,7 +568,7 @@ __global__ void k_compact_maps(const float* __restrict__ xmap, const float* __re
                                long long maskStride, const RemapItem* __restrict__ items, float2* maps)
 {
     const RemapItem it = items[blockIdx.x];
-    const int x = it.tx * kRemapTW + (threadIdx.x & 31), y = it.ty * kRemapTH + (threadIdx.x >> 5);
+    const int x = it.tx * kRemapTW + mapTileX(threadIdx.x), y = it.ty * kRemapTH + mapTileY(threadIdx.x);
     float2 v = make_float2(-1.f, -1.f);
     if (x < W && y < H) {
         const size_t i = (size_t)it.cam * maskStride + (size_t)y * W + x;
@@ -706,7 +706,7 @@ __global__ void k_compact_weights(const float* __restrict__ w, int W, int H, lon
                                   const RemapItem* __restrict__ items, float* out)
 {
     const RemapItem it = items[blockIdx.x];
-    const int x = it.tx * kRemapTW + (threadIdx.x & 31), y = it.ty * kRemapTH + (threadIdx.x >> 5);
+    const int x = it.tx * kRemapTW + mapTileX(threadIdx.x), y = it.ty * kRemapTH + mapTileY(threadIdx.x);
     out[(size_t)it.mapTile * (kRemapTW * kRemapTH) + threadIdx.x] =
         (x < W && y < H) ? w[(size_t)it.cam * npx + (size_t)y * W + x] : 0.f;
 }

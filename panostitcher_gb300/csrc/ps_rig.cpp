@@ -221,9 +221,7 @@ static long long listBytes(int W, int H, int n, int L, int slots)
         w = (w + 1) / 2;
         h = (h + 1) / 2;
     }
-    // remap items and each state slot's tie list
-    return b + (long long)divUp(W, kRemapTW) * divUp(H, kRemapTH) * n *
-                   (sizeof(RemapItem) + sizeof(RemapTie) * kRemapTiesPerTile * slots);
+    return b + (long long)divUp(W, kRemapTW) * divUp(H, kRemapTH) * n * sizeof(RemapItem);
 }
 
 long long Rig::estimateBlenderBytes(int W, int H, int n, int maxLevels, int slots)
@@ -1069,7 +1067,7 @@ void Rig::exportState(int what, int cam, int level, void* host, long long bytes)
         for (const RemapItem& it : hRemap_) {
             if (it.cam != cam) continue;
             for (int k = 0; k < kRemapTW * kRemapTH; k++) {
-                const int x = it.tx * kRemapTW + (k % kRemapTW), y = it.ty * kRemapTH + (k / kRemapTW);
+                const int x = it.tx * kRemapTW + mapTileX(k), y = it.ty * kRemapTH + mapTileY(k);
                 if (x < W_ && y < H_) {
                     const float2 v = m[(size_t)it.mapTile * kRemapTW * kRemapTH + k];
                     out[(size_t)y * W_ + x] = what == 0 ? v.x : v.y;
@@ -1096,7 +1094,7 @@ void Rig::exportState(int what, int cam, int level, void* host, long long bytes)
         for (const RemapItem& it : hRemap_) {
             if (it.cam != cam) continue;
             for (int k = 0; k < kRemapTW * kRemapTH; k++) {
-                const int x = it.tx * kRemapTW + (k % kRemapTW), y = it.ty * kRemapTH + (k / kRemapTW);
+                const int x = it.tx * kRemapTW + mapTileX(k), y = it.ty * kRemapTH + mapTileY(k);
                 if (x < W_ && y < H_) out[(size_t)y * W_ + x] = w[(size_t)it.mapTile * kRemapTW * kRemapTH + k];
             }
         }
@@ -1337,8 +1335,8 @@ void Plan::bind(const std::vector<Rig*>& rigs)
     };
     tailCluster_ = widest([](const LaunchShape& s) { return s.tailCluster; });
     for (int k = 0; k < 3; k++) perSm_[k] = widest([k](const LaunchShape& s) { return s.ctasPerSm[k]; });
-    remapDefer_ = false;  // deferred when any rig of the launch asks for it
-    for (Rig* r : rigs) remapDefer_ = remapDefer_ || r->shape().remapDefer;
+    maps_ = true;
+    for (Rig* r : rigs) maps_ = maps_ && !r->mapFree();
     probe_ = 0;
     for (Rig* r : rigs) probe_ = std::max(probe_, r->waitProbe());
     auto addStep = [&](int kind, const std::vector<std::pair<int, std::pair<const void*, int>>>& parts, int step) {
@@ -1366,14 +1364,6 @@ void Plan::bind(const std::vector<Rig*>& rigs)
     for (int r = 0; r < nr; r++)
         if (!rigs[r]->linear()) parts.push_back({r, {rigs[r]->remapItems(), rigs[r]->numRemapItems()}});
     addStep(0, parts, 0);
-    int remapTotal = 0;
-    if (remapDefer_ && !steps_.empty() && steps_.back().kind == 0) {  // its exact recompute, same segments
-        Step f = steps_.back();
-        f.kind = 7;
-        f.bytes = 0;
-        remapTotal = f.total;
-        steps_.push_back(f);
-    }
     for (int J = 1; J <= maxL; J++) {
         parts.clear();
         for (int r = 0; r < nr; r++)
@@ -1416,19 +1406,15 @@ void Plan::bind(const std::vector<Rig*>& rigs)
         for (size_t k = before; k < steps_.size(); k++) steps_[k].early = s > 0;
     }
     // one work counter per step after the segments, zeroed in every run's staged copy
-    // and the remap's tie count after them
     counterOff_ = (segOff_ + segs_.size() * sizeof(Segment) + 15) / 16 * 16;
-    const size_t need = counterOff_ + (steps_.size() + 1) * sizeof(int);
+    const size_t need = counterOff_ + steps_.size() * sizeof(int);
     for (IoSlot& sl : io_)
         if (need > sl.dArgs.bytes()) {
             const size_t cap = need + need / 2;
             sl.dArgs.alloc(cap);
             sl.stage.alloc(cap);
         }
-    stageBytes_ = counterOff_ + (steps_.size() + 1) * sizeof(int);
-    for (IoSlot& sl : io_)
-        if ((size_t)remapTotal * kRemapTiesPerTile * sizeof(RemapTie) > sl.ties.bytes())
-            sl.ties.alloc((size_t)remapTotal * kRemapTiesPerTile * sizeof(RemapTie));
+    stageBytes_ = need;
 }
 
 Plan::~Plan()
@@ -1464,24 +1450,20 @@ void Plan::launchAll(const IoSlot& slot, cudaStream_t st, int srcFmt, Profiler* 
         const Step& s = steps_[si];
         const Segment* p = segs + s.segOff;
         static const char* const kRangeName[] = {"ps.remap", "ps.pyrdown", "ps.blend", "ps.tail",
-                                                 "ps.linear", "ps.cvt", "ps.blend_small", "ps.remap_fix"};
-        NvtxRange range(kRangeName[s.kind >= 0 && s.kind <= 7 ? s.kind : 5]);
+                                                 "ps.linear", "ps.cvt", "ps.blend_small"};
+        NvtxRange range(kRangeName[s.kind >= 0 && s.kind <= 6 ? s.kind : 5]);
         cudaEvent_t a = nullptr, b = nullptr;
         if (prof) {
             a = prof->event();
             b = prof->event();
             PS_CUDA(cudaEventRecord(a, st));
         }
-        int* tieCount = counters + steps_.size();  // the remap's count of listed near-tie pixels
-        if (s.kind == 0)
-            PS_CUDA(launchRemap(p, s.nsegs, s.total, perSm_[0], counters + si, tieCount, slot.ties.as<RemapTie>(),
-                                remapDefer_, srcFmt, st));
-        else if (s.kind == 7) PS_CUDA(launchRemapFix(p, s.nsegs, s.total, tieCount, slot.ties.as<RemapTie>(), st));
+        if (s.kind == 0) PS_CUDA(launchRemap(p, s.nsegs, s.total, perSm_[0], counters + si, srcFmt, maps_, st));
         else if (s.kind == 1) PS_CUDA(launchPyrDown(p, s.nsegs, s.total, perSm_[1], st));
         else if (s.kind == 2) PS_CUDA(launchBlend(p, s.nsegs, s.total, perSm_[2], counters + si, probe_, s.early, st));
         else if (s.kind == 3) PS_CUDA(launchTail(p, s.nsegs, tailCluster_, st));
         else if (s.kind == 6) PS_CUDA(launchBlendSmall(p, s.nsegs, s.total, s.early, st));
-        else PS_CUDA(launchLinear(p, s.nsegs, s.total, maxCams_, st));
+        else PS_CUDA(launchLinear(p, s.nsegs, s.total, maxCams_, srcFmt, st));
         if (prof) {
             PS_CUDA(cudaEventRecord(b, st));
             prof->record(s.kind, s.level, s.bytes, a, b);
@@ -1537,7 +1519,7 @@ void Plan::run(const std::vector<FrameInput>& in, cudaStream_t st, bool useGraph
     uint8_t* dArgs = S.dArgs.as<uint8_t>();
     std::vector<YuvFrames> cvt;  // decoder frames converted into the slots' BGR32 staging
     double cvtBytes = 0;
-    int srcFmt = -1;  // the format all rigs' sources share, else 0
+    int srcFmt = -1;  // the format all rigs' sources share and the remap may be specialised for, else 0
     for (size_t r = 0; r < rigs_.size(); r++) {
         Rig* rig = rigs_[r];
         const FrameInput& f = in[r];
@@ -1668,7 +1650,10 @@ void Plan::run(const std::vector<FrameInput>& in, cudaStream_t st, bool useGraph
             fd.outFmt = d.format;
         }
         fd.status = rig->statusWord();
-        srcFmt = srcFmt < 0 || srcFmt == fd.srcFmt ? fd.srcFmt : 0;
+        long long widest = 0;
+        for (int i = 0; i < n; i++) widest = std::max(widest, fd.srcPitch[i]);
+        const int fmt = remapSourceFormat(fd.srcFmt, rig->srcW(), rig->srcH(), widest);
+        srcFmt = srcFmt < 0 || srcFmt == fmt ? fmt : 0;
         std::memcpy(stage + sizeof(FrameDev) * r, &fd, sizeof fd);
     }
     if (!segs_.empty()) {
@@ -1680,7 +1665,7 @@ void Plan::run(const std::vector<FrameInput>& in, cudaStream_t st, bool useGraph
             sg[k].rig = rigs_[segRig_[k]]->deviceDesc(rs[segRig_[k]]);
         }
     }
-    std::memset(stage + counterOff_, 0, (steps_.size() + 1) * sizeof(int));
+    std::memset(stage + counterOff_, 0, steps_.size() * sizeof(int));
     PS_CUDA(cudaMemcpyAsync(dArgs, stage, stageBytes_, cudaMemcpyHostToDevice, sIn_));
     PS_CUDA(cudaEventRecord(S.argsCopied, sIn_));
 
@@ -1702,7 +1687,6 @@ void Plan::run(const std::vector<FrameInput>& in, cudaStream_t st, bool useGraph
             prof->record(5, 0, cvtBytes / cvt.size(), a, b);
         }
     }
-    srcFmt = srcFmt == PS_FMT_BGR32 ? PS_FMT_BGR32 : 0;  // the formats the remap is specialised for
     if (useGraph) {
         if (S.graph && S.graphFmt != srcFmt) {  // re-record for the other format, after the slot's last run
             if (S.used) PS_CUDA(cudaEventSynchronize(S.computed));

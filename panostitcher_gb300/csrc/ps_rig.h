@@ -271,8 +271,7 @@ public:
 
 private:
     struct Step {
-        int kind;  // 0 remap, 1 pyrDown, 2 blend, 3 tail, 4 linear-blend render, 6 few-tile blend,
-                   // 7 the exact recompute of the remap tiles near rounding ties
+        int kind;  // 0 remap, 1 pyrDown, 2 blend, 3 tail, 4 linear-blend render, 6 few-tile blend
         int segOff, nsegs, total;
         int level;      // level of the first rig in the step
         double bytes;   // algorithmic bytes of the step (all rigs)
@@ -283,13 +282,12 @@ private:
     struct IoSlot {
         DevBuf dArgs;   // [FrameDev x nr][LUTs][Segment x nseg]
         HostBuf stage;  // pinned staging copy of dArgs
-        DevBuf ties;    // the remap's list of near-tie pixels for k_remap_fix
         cudaGraphExec_t graph = nullptr;
         int graphFmt = 0;  // the sources' format the graph's remap was specialised for (0: any)
         cudaEvent_t argsCopied = nullptr, computed = nullptr, downloaded = nullptr;
         bool used = false;
     };
-    // srcFmt: the format every source of the run shares (0: mixed)
+    // srcFmt: the format the run's remap is specialised for (0: none)
     void launchAll(const IoSlot& slot, cudaStream_t st, int srcFmt, Profiler* prof = nullptr);
     void dropGraph();
     void ensureStreams();
@@ -304,7 +302,7 @@ private:
     size_t segOff_ = 0, counterOff_ = 0, stageBytes_ = 0;
     int maxCams_ = 0;
     int tailCluster_ = 0, perSm_[3] = {0, 0, 0};  // launch widths (from the rigs' shapes)
-    bool remapDefer_ = true;                      // k_remap lists near-tie pixels for k_remap_fix
+    bool maps_ = true;                             // every rig has resident maps
     int probe_ = 0;                                // wait probe of k_blend (Rig::setWaitProbe)
     IoSlot io_[Rig::kIoSlots];
     int nextIo_ = 0;

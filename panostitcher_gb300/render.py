@@ -291,7 +291,7 @@ class CudaPanoramaRender2:
         check(lib().ps_render_profile(self._h, int(bool(enabled))))
 
     KERNELS = {0: "k_remap", 1: "k_pyrdown", 2: "k_blend", 3: "k_tail", 4: "k_linear", 5: "k_yuv_to_bgr32",
-               6: "k_blend_small", 7: "k_remap_fix"}
+               6: "k_blend_small"}
 
     def profile_read(self, kind: int, level: int = -1):
         """(launches, total_ms, algorithmic_bytes) of finished profiled launches."""
