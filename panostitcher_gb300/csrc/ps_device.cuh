@@ -181,13 +181,25 @@ __device__ __forceinline__ void itemRange(int total, int& begin, int& end)
 // ---- borders: source/CudaAccel/CudaUtil.cuh:6-98 ------------------------------
 // Vertical reflect-101 (BrdColReflect101) and horizontal wrap (BrdRowWrap),
 // restated with the reference's exact index formulas.
+// The divisions are for levels smaller than a filter's reach; they are a
+// hundred cycles each, and the few-tile levels map every row and column.
 __device__ __forceinline__ int rowLow(int y, int H) { return abs(y) % H; }
 __device__ __forceinline__ int rowHigh(int y, int H) { int last = H - 1; return abs(last - abs(last - y)) % H; }
 __device__ __forceinline__ int colLow(int x, int W) { return x >= 0 ? x : x - ((x - W + 1) / W) * W; }
 __device__ __forceinline__ int colHigh(int x, int W) { return x < W ? x : x % W; }
 // any row index of a pyramid tile -> the row the reference reads
-__device__ __forceinline__ int rowMap(int y, int H) { return y < 0 ? rowLow(y, H) : (y >= H ? rowHigh(y, H) : y); }
-__device__ __forceinline__ int colMap(int x, int W) { return x < 0 ? colLow(x, W) : (x >= W ? colHigh(x, W) : x); }
+__device__ __forceinline__ int rowMap(int y, int H)
+{
+    const int r = y < 0 ? -y : (y >= H ? 2 * (H - 1) - y : y);  // one reflection
+    if ((unsigned)r < (unsigned)H) return r;
+    return y < 0 ? rowLow(y, H) : rowHigh(y, H);
+}
+__device__ __forceinline__ int colMap(int x, int W)
+{
+    const int c = x < 0 ? x + W : (x >= W ? x - W : x);  // one turn
+    if ((unsigned)c < (unsigned)W) return c;
+    return x < 0 ? colLow(x, W) : colHigh(x, W);
+}
 
 // C truncating division a / d given rcp = __frcp_rn(d), exact for |a| < 2^24
 // (exact in fp32), 1 <= d < 2^16 and |a| / d < 2^21: the fp32 quotient then

@@ -1029,25 +1029,29 @@ constexpr int kConsumers = kThreads;          // 8 warps
 constexpr int kBlendThreads = kConsumers + 32;  // + the producer warp
 
 // One unit's shared-memory stage: NC cameras of one tile (k_blend stages
-// two cameras per unit in a ring; the tail kernel stages up to eight at once).
+// two cameras per unit in a ring; the kernels of the few-tile levels stage up
+// to eight at once, of a half tile).
 // Every camera's part starts on a 128-byte boundary, as the bulk tensor
 // copies into it require: the footprint of a camera is kFH rows of kFpW
 // words (a dense box), padded to kFpCam words.
-template <int NC>
+// ROWS: the rows of the tile it holds, all or one half's.
+template <int NC, int ROWS = kBlendTH>
 struct alignas(128) BlendStageT {
-    static constexpr int kCams = NC;
-    static constexpr int kFpCam = (kFH * kFpW + 31) / 32 * 32;
-    uint32_t gj[NC][kBlendTH][kBlendTW];  // G_j, uchar4
-    uint16_t w[NC][kBlendTH][kBlendTW];   // weights
-    uint32_t fpw[NC][kFpCam];             // G_{j+1} footprint: row r, column c at [r * kFpW + c]
-    uint2 cf[kFH][kCfW];                  // C_{j+1} footprint (short4 bits)
+    static constexpr int kCams = NC, kRows = ROWS, kFpRows = ROWS / 2 + 2;
+    static constexpr int kFpCam = (kFpRows * kFpW + 31) / 32 * 32;
+    uint32_t gj[NC][ROWS][kBlendTW];  // G_j, uchar4
+    uint16_t w[NC][ROWS][kBlendTW];   // weights
+    uint32_t fpw[NC][kFpCam];         // G_{j+1} footprint: row r, column c at [r * kFpW + c]
+    uint2 cf[kFpRows][kCfW];          // C_{j+1} footprint (short4 bits)
 };
 using BlendStage = BlendStageT<kCamsPerUnit>;
 static_assert(offsetof(BlendStage, w) % 128 == 0 && offsetof(BlendStage, fpw) % 128 == 0 &&
                   offsetof(BlendStage, cf) % 128 == 0 && sizeof(BlendStage::gj[0]) % 128 == 0 &&
                   sizeof(BlendStage::w[0]) % 128 == 0 && sizeof(BlendStage::fpw[0]) % 128 == 0,
               "every bulk tensor copy destination starts on a 128-byte boundary");
-constexpr int kTailCamsPerUnit = 8;
+constexpr int kHalfRows = kBlendTH / 2;
+using HalfStage = BlendStageT<8, kHalfRows>;  // half tiles of the few-tile levels
+using WholeStage = BlendStageT<4>;            // whole tiles in the tail kernel
 
 // What the consumers need of a unit besides its stage: the level geometry
 // and the frame's output, resolved once per unit (in k_blend by the
@@ -1070,8 +1074,9 @@ __device__ __forceinline__ void fillGeo(UnitGeo& g, const RigDev& R, const Frame
     g.pitch = Lj.pitch;
     g.full = R.full;
     g.hasUp = j < R.L;
-    g.outFmt = F.outFmt;
     g.C = Lj.C;
+    if (j > 0) return;  // the frame's output is level 0's
+    g.outFmt = F.outFmt;
     g.um = R.unionMask;
     g.out = F.out;
     g.outU = F.outU;
@@ -1199,15 +1204,11 @@ struct BlendAcc {
 // tail kernel).  Threads 0..kConsumers-1; the caller synchronises.
 // fRow / fCol: footprint index tables (kFH / kFW ints) filled here; sync is
 // the barrier over the calling threads.
-// half >= 0 stages only what computeUnitRows reads for that 64x8 half:
-// its eight rows and footprint rows 4*half .. 4*half+5.
 template <bool kFresh, class Stage, class Sync>
 __device__ __forceinline__ void stageUnitDirect(Stage& S, const RigDev& R, const uint4& raw, int chunk, int* fRow,
-                                                int* fCol, Sync sync, int half = -1)
+                                                int* fCol, Sync sync)
 {
-    const int lx = (threadIdx.x & 31) * 2;
-    const int ly = half < 0 ? (threadIdx.x >> 5) * 2 : 8 * half + (threadIdx.x >> 5);
-    const int rowsPerThread = half < 0 ? 2 : 1;
+    const int lx = (threadIdx.x & 31) * 2, ly = (threadIdx.x >> 5) * 2;
     const int j = raw.x & 0xFF, camCnt = (raw.x >> 16) & 0xFF;
     const int tx = raw.y & 0xFFFF, ty = raw.y >> 16;
     const LevelDev& Lj = R.lv[j];
@@ -1221,7 +1222,7 @@ __device__ __forceinline__ void stageUnitDirect(Stage& S, const RigDev& R, const
     const int fx0 = tx * (kBlendTW / 2) - 1, fy0 = ty * (kBlendTH / 2) - 1;
     for (int q = 0; q < nc; q++) {
         const int cam = tileCam(raw, R.camLists, c0 + q);
-        for (int r = 0; r < rowsPerThread; r++) {
+        for (int r = 0; r < 2; r++) {
             uint2 g = make_uint2(0, 0);
             uint32_t w = 0;
             if (y + r < Lj.h) {  // columns up to the pitch are allocated (and zero beyond the width)
@@ -1239,11 +1240,10 @@ __device__ __forceinline__ void stageUnitDirect(Stage& S, const RigDev& R, const
         if (threadIdx.x < kFH) fRow[threadIdx.x] = rowMap(fy0 + (int)threadIdx.x, Lu.h);
         else if (threadIdx.x < kFH + kFW) fCol[threadIdx.x - kFH] = colMap(fx0 + (int)threadIdx.x - kFH, Lu.w);
         sync();
-        const int rb = half < 0 ? 0 : 4 * half, nr = half < 0 ? kFH : 6;
-        const int elems = nr * kFW;
+        constexpr int elems = kFH * kFW;
         for (int k = threadIdx.x; k < nc * elems; k += kConsumers) {
             const int q = k / elems, e = k - q * elems;
-            const int r = rb + e / kFW, c = e % kFW;
+            const int r = e / kFW, c = e % kFW;
             const int cam = tileCam(raw, R.camLists, c0 + q);
             const uint32_t* gp = reinterpret_cast<const uint32_t*>(Lu.G) + (size_t)cam * Lu.camStride +
                                  (size_t)fRow[r] * Lu.pitch + fCol[c];
@@ -1251,122 +1251,107 @@ __device__ __forceinline__ void stageUnitDirect(Stage& S, const RigDev& R, const
         }
         if (last)
             for (int k = threadIdx.x; k < elems; k += kConsumers) {
-                const int r = rb + k / kFW, c = k % kFW;
+                const int r = k / kFW, c = k % kFW;
                 const uint2* cp = reinterpret_cast<const uint2*>(Lu.C + (size_t)fRow[r] * Lu.pitch + fCol[c]);
                 S.cf[r][c + 1] = inside(cp, Lu.C, cBytes(Lu)) ? ldLevel<kFresh>(cp) : make_uint2(0, 0);
             }
     }
 }
 
-// The same staging for the tail kernel and k_blend_small, where one unit's
-// staging is most of a small level's critical path, so it is kept short in
-// instructions and round trips:
-//   - every load of the unit is issued into registers before any is stored,
-//     so the loads are in flight together;
-//   - the footprint rows (G_{j+1} of each camera, then C_{j+1}) are spread
-//     over the warps row by row: a row's index mapping is worked out once per
-//     row, a lane's two columns once per unit (columns fx0 + lane and, for
-//     lanes 0 and 1, fx0 + 32 + lane).
-// Threads 0..kConsumers-1; the caller synchronises before the stage is read.
-// doG: the cameras' G_j rows, weights and G_{j+1} footprints; doC: the
-// C_{j+1} footprint (the only part the previous blend launch writes, so the
-// rest may be staged before the wait for it).
-template <bool kFresh, class Stage>
-__device__ __forceinline__ void stageUnitRows(Stage& S, const RigDev& R, const uint4& raw, int chunk, int half,
-                                              bool doG = true, bool doC = true)
+// The half-tile staging of the few-tile levels, where one unit's staging is
+// most of a level's critical path: 16-byte loads of whole rows, the footprint
+// element by element with the reference's index mapping, in little code (a level's kernel runs its code once, so every
+// line of it is fetched from L2).  A unit is eight rows (8 * half ..) of a tile
+// and up to eight of its cameras.  Threads 0..kConsumers-1; the caller
+// synchronises before the stage is read.
+//
+// stageHalfG: the cameras' G_j rows, weights and G_{j+1} footprints.
+// stageHalfC: the C_{j+1} footprint, with a tile's last unit -- the only part
+// the level above's blend writes, so the rest may be staged before it.
+static_assert(HalfStage::kFpRows * kFW <= kConsumers, "a footprint element a thread");
+
+// Element (r, c) of a half tile's footprint in a plane of level Lu.  Elements
+// that no pixel of level Lj needs (the tile reaches beyond the level) map to 0.
+__device__ __forceinline__ size_t halfFpOffset(const LevelDev& Lu, const LevelDev& Lj, int tx, int ty, int half, int r,
+                                               int c)
 {
-    constexpr int NC = Stage::kCams;
-    constexpr int kWarps = kConsumers / 32;
-    constexpr int kGRows = (NC * kFH + kWarps - 1) / kWarps;  // footprint rows of G_{j+1} per warp
-    constexpr int kCRows = (kFH + kWarps - 1) / kWarps;       // footprint rows of C_{j+1} per warp
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    const int lx = lane * 2;
-    const int ly = half < 0 ? wp * 2 : 8 * half + wp;
-    const int rowsPerThread = half < 0 ? 2 : 1;
+    const int x = tx * kBlendTW, y = ty * kBlendTH + kHalfRows * half;
+    if (c > (Lj.w - x + 1) / 2 + 1 || r > (Lj.h - y + 1) / 2 + 1) return 0;
+    return (size_t)rowMap(y / 2 - 1 + r, Lu.h) * Lu.pitch + colMap(x / 2 - 1 + c, Lu.w);
+}
+
+template <bool kFresh>
+__device__ __forceinline__ void stageHalfG(HalfStage& S, const RigDev& R, const uint4& raw, int chunk, int half)
+{
+    constexpr int NC = HalfStage::kCams;
     const int j = raw.x & 0xFF, camCnt = (raw.x >> 16) & 0xFF;
     const int tx = raw.y & 0xFFFF, ty = raw.y >> 16;
     const LevelDev& Lj = R.lv[j];
-    const bool hasUp = j < R.L;
-    const LevelDev& Lu = R.lv[hasUp ? j + 1 : j];
-    const int x = tx * kBlendTW + lx, y = ty * kBlendTH + ly;
-    const int c0 = chunk * NC;
-    const int nc = max(0, min(NC, camCnt - c0));
-    const bool last = chunk == unitChunks<NC>(raw) - 1;
-    const int fx0 = tx * (kBlendTW / 2) - 1, fy0 = ty * (kBlendTH / 2) - 1;
-    const int rb = half < 0 ? 0 : 4 * half, nr = half < 0 ? kFH : 6;
-    const int colA = colMap(fx0 + lane, Lu.w);
-    const bool hasB = lane < kFW - 32;
-    const int colB = hasB ? colMap(fx0 + 32 + lane, Lu.w) : 0;
-    uint2 gv[NC][2];
-    uint32_t wv[NC][2];
-    uint32_t fa[kGRows], fb[kGRows];
-    uint2 ca[kCRows], cb[kCRows];
+    const int c0 = chunk * NC, nc = max(0, min(NC, camCnt - c0));
+    const int t = threadIdx.x;
+    auto camAt = [&](int q) { return (size_t)tileCam(raw, R.camLists, c0 + q); };
+    // every load of the unit before any store: G_j rows (two cameras a pass),
+    // weights (four cameras a pass; columns up to the pitch are allocated, and
+    // zero beyond the width), and one footprint element of every camera, whose
+    // index mapping is thus worked out once
+    uint4 g[NC / 2], w[NC / 4];
+    uint32_t f[NC];
+    const int gc = (t & 15) * 4, gr = t >> 4 & 7, gy = ty * kBlendTH + kHalfRows * half + gr;
+    const int wc = (t & 7) * 8, wr = t >> 3 & 7, wy = ty * kBlendTH + kHalfRows * half + wr;
+    const int fr = t / kFW, fc = t % kFW;
+    const bool hasF = j < R.L && fr < HalfStage::kFpRows;
+    const LevelDev& Lu = R.lv[j < R.L ? j + 1 : j];
+    const size_t fo = hasF ? halfFpOffset(Lu, Lj, tx, ty, half, fr, fc) : 0;
 #pragma unroll
     for (int q = 0; q < NC; q++) {
-        const int cam = q < nc ? tileCam(raw, R.camLists, c0 + q) : 0;
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            gv[q][r] = make_uint2(0, 0);
-            wv[q][r] = 0;
-            if (doG && q < nc && r < rowsPerThread && y + r < Lj.h) {  // columns up to the pitch are allocated
-                const size_t o = (size_t)cam * Lj.camStride + (size_t)(y + r) * Lj.pitch + x;
-                const uint2* gp = reinterpret_cast<const uint2*>(Lj.G + o);
-                const uint32_t* wp2 = reinterpret_cast<const uint32_t*>(Lj.Wt + o);
-                if (inside(gp, Lj.G, gBytes(R, Lj))) gv[q][r] = ldLevel<kFresh>(gp);
-                if (inside(wp2, Lj.Wt, wBytes(R, Lj))) wv[q][r] = __ldg(wp2);
-            }
+        f[q] = 0;
+        if (q < nc && hasF) {
+            const uint32_t* p = reinterpret_cast<const uint32_t*>(Lu.G) + camAt(q) * Lu.camStride + fo;
+            if (inside(p, Lu.G, gBytes(R, Lu))) f[q] = ldLevel<kFresh>(p);
         }
     }
-    const int gTasks = hasUp && doG ? nc * nr : 0;
 #pragma unroll
-    for (int i = 0; i < kGRows; i++) {
-        const int t = wp + i * kWarps;  // row task: camera t / nr, footprint row rb + t % nr
-        fa[i] = fb[i] = 0;
-        if (t < gTasks) {
-            const int q = t / nr, r = rb + (t - q * nr);
-            const uint32_t* row = reinterpret_cast<const uint32_t*>(Lu.G) +
-                                  (size_t)tileCam(raw, R.camLists, c0 + q) * Lu.camStride +
-                                  (size_t)rowMap(fy0 + r, Lu.h) * Lu.pitch;
-            if (inside(row + colA, Lu.G, gBytes(R, Lu))) fa[i] = ldLevel<kFresh>(row + colA);
-            if (hasB && inside(row + colB, Lu.G, gBytes(R, Lu))) fb[i] = ldLevel<kFresh>(row + colB);
+    for (int i = 0; i < NC / 2; i++) {
+        const int q = (t >> 7) + 2 * i;
+        g[i] = make_uint4(0, 0, 0, 0);
+        if (q < nc && gy < Lj.h) {
+            const uint4* p = reinterpret_cast<const uint4*>(Lj.G + camAt(q) * Lj.camStride + (size_t)gy * Lj.pitch +
+                                                            tx * kBlendTW + gc);
+            if (inside(p, Lj.G, gBytes(R, Lj))) g[i] = ldLevel<kFresh>(p);
         }
     }
-    const int cTasks = hasUp && last && doC ? nr : 0;
 #pragma unroll
-    for (int i = 0; i < kCRows; i++) {
-        const int t = wp + i * kWarps;
-        ca[i] = cb[i] = make_uint2(0, 0);
-        if (t < cTasks) {
-            const uint2* row = reinterpret_cast<const uint2*>(Lu.C + (size_t)rowMap(fy0 + rb + t, Lu.h) * Lu.pitch);
-            if (inside(row + colA, Lu.C, cBytes(Lu))) ca[i] = ldLevel<kFresh>(row + colA);
-            if (hasB && inside(row + colB, Lu.C, cBytes(Lu))) cb[i] = ldLevel<kFresh>(row + colB);
+    for (int i = 0; i < NC / 4; i++) {
+        const int q = (t >> 6) + 4 * i;
+        w[i] = make_uint4(0, 0, 0, 0);
+        if (q < nc && wy < Lj.h) {
+            const uint4* p = reinterpret_cast<const uint4*>(Lj.Wt + camAt(q) * Lj.camStride + (size_t)wy * Lj.pitch +
+                                                            tx * kBlendTW + wc);
+            if (inside(p, Lj.Wt, wBytes(R, Lj))) w[i] = __ldg(p);
         }
     }
 #pragma unroll
     for (int q = 0; q < NC; q++)
+        if (q < nc && hasF) S.fpw[q][fr * kFpW + fc + 3] = f[q];
 #pragma unroll
-        for (int r = 0; r < 2; r++)
-            if (doG && q < nc && r < rowsPerThread) {
-                *reinterpret_cast<uint2*>(&S.gj[q][ly + r][lx]) = gv[q][r];
-                *reinterpret_cast<uint32_t*>(&S.w[q][ly + r][lx]) = wv[q][r];
-            }
+    for (int i = 0; i < NC / 2; i++)
+        if ((t >> 7) + 2 * i < nc) *reinterpret_cast<uint4*>(&S.gj[(t >> 7) + 2 * i][gr][gc]) = g[i];
 #pragma unroll
-    for (int i = 0; i < kGRows; i++) {
-        const int t = wp + i * kWarps;
-        if (t < gTasks) {
-            const int q = t / nr, r = rb + (t - q * nr);
-            S.fpw[q][r * kFpW + lane + 3] = fa[i];
-            if (hasB) S.fpw[q][r * kFpW + 32 + lane + 3] = fb[i];
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < kCRows; i++) {
-        const int t = wp + i * kWarps;
-        if (t < cTasks) {
-            S.cf[rb + t][lane + 1] = ca[i];
-            if (hasB) S.cf[rb + t][32 + lane + 1] = cb[i];
-        }
-    }
+    for (int i = 0; i < NC / 4; i++)
+        if ((t >> 6) + 4 * i < nc) *reinterpret_cast<uint4*>(&S.w[(t >> 6) + 4 * i][wr][wc]) = w[i];
+}
+
+template <bool kFresh>
+__device__ __forceinline__ void stageHalfC(HalfStage& S, const RigDev& R, const uint4& raw, int chunk, int half)
+{
+    const int j = raw.x & 0xFF;
+    const int tx = raw.y & 0xFFFF, ty = raw.y >> 16;
+    if (j >= R.L || chunk != unitChunks<HalfStage::kCams>(raw) - 1) return;
+    const LevelDev& Lu = R.lv[j + 1];
+    const int r = threadIdx.x / kFW, c = threadIdx.x % kFW;
+    if (r >= HalfStage::kFpRows) return;
+    const uint2* p = reinterpret_cast<const uint2*>(Lu.C + halfFpOffset(Lu, R.lv[j], tx, ty, half, r, c));
+    S.cf[r][c + 1] = inside(p, Lu.C, cBytes(Lu)) ? ldLevel<kFresh>(p) : make_uint2(0, 0);
 }
 
 // Accumulate one unit from its stage; at a tile's last unit normalise,
@@ -1606,12 +1591,10 @@ struct PairAcc {
     int wsum0, wsum1;
 };
 
-template <class Stage>
-__device__ __forceinline__ void computeUnitRows(const Stage& S, const UnitGeo& G, const uint4& raw, int chunk,
+__device__ __forceinline__ void computeUnitRows(const HalfStage& S, const UnitGeo& G, const uint4& raw, int chunk,
                                                 PairAcc& acc, int half)
 {
-    const int lx = (threadIdx.x & 31) * 2, lr = threadIdx.x >> 5;  // row in the half tile
-    const int ly = 8 * half + lr;                                    // row in the tile
+    const int lx = (threadIdx.x & 31) * 2, ly = threadIdx.x >> 5;  // row in the half tile
     // vertical taps: even rows footprint rows ly/2 .. ly/2+2 (1 6 1), odd rows
     // (ly+1)/2 .. (ly+1)/2+1 (4 4); footprint columns lx/2 .. lx/2+2 as in computeUnit
     const bool evenRow = (ly & 1) == 0;
@@ -1620,8 +1603,8 @@ __device__ __forceinline__ void computeUnitRows(const Stage& S, const UnitGeo& G
     const int j = raw.x & 0xFF, camCnt = (raw.x >> 16) & 0xFF;
     const int tx = raw.y & 0xFFFF, ty = raw.y >> 16;
     const bool hasUp = G.hasUp != 0;
-    const int x = tx * kBlendTW + lx, y = ty * kBlendTH + ly;
-    constexpr int NC = Stage::kCams;
+    const int x = tx * kBlendTW + lx, y = ty * kBlendTH + kHalfRows * half + ly;
+    constexpr int NC = HalfStage::kCams;
     const int c0 = chunk * NC;
     const int nc = max(0, min(NC, camCnt - c0));
     const bool first = chunk == 0, last = chunk == unitChunks<NC>(raw) - 1;
@@ -1629,6 +1612,7 @@ __device__ __forceinline__ void computeUnitRows(const Stage& S, const UnitGeo& G
         acc.r0[0] = acc.r0[1] = acc.r0[2] = acc.r1[0] = acc.r1[1] = acc.r1[2] = 0;
         acc.wsum0 = acc.wsum1 = 0;
     }
+#pragma unroll 2
     for (int q = 0; q < nc; q++) {
         uint32_t u0lo = 0, u0hi = 0, u1lo = 0, u1hi = 0;
         if (hasUp) {
@@ -1956,60 +1940,107 @@ __global__ void __launch_bounds__(kBlendThreads, 4) k_blend(const Segment* __res
 // CTAs, with a cluster barrier (release / acquire, so the level's global
 // writes are visible to the whole cluster) between levels.  These levels
 // hold few tiles, so separate launches would cost mostly launch latency.
+// A level is a chain of latencies: its data from L2 (0.7 us), the arithmetic
+// (1 - 2 us, two warps a scheduler), the barrier (0.5 us of release, 0.4 us of
+// wait).  Descriptors and first items wait in shared memory, a level's G part
+// is staged during the barrier above it, no division maps an index.  Seven
+// levels of 6 x 1920x1080 to 4096x2048 take 25 us, 46 us before that; the nine
+// of a 256x128 canvas 24 us, 36 us before.
 // ============================================================================
 constexpr int kTailCluster = 8;       // portable cluster size
 constexpr int kTailClusterWide = 16;  // used when the GPU can co-schedule it
 
-__device__ __forceinline__ void clusterSync()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void clusterArrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void clusterWait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-union TailSmem {
-    DownSmem down;
-    BlendStageT<kTailCamsPerUnit> blend;
+// The rig's descriptor and the CTA's first item of every level are copied to
+// shared memory while the launch before finishes, so that a level's chain is
+// one round trip to L2 (its data), the arithmetic, the stores and the barrier.
+struct TailSmem {
+    RigDev rig;
+    DownItem down[PS_MAX_LEVELS + 1];
+    uint4 blend[PS_MAX_LEVELS + 1];
+    int fRow[kFH], fCol[kFW];
+    union Stage {
+        DownSmem down;
+        HalfStage half[2];
+        WholeStage whole;
+    };
+    alignas(128) unsigned char stage[sizeof(Stage)];
 };
+static_assert(sizeof(RigDev) % 4 == 0 && sizeof(DownItem) % 4 == 0 && sizeof(BlendItem) == 16, "copied word by word");
 
 __global__ void __launch_bounds__(kThreads) k_tail(const Segment* __restrict__ segs, int nsegs, int cluster)
 {
     extern __shared__ __align__(128) uint8_t tailSmem[];  // a TailSmem (dynamic: above the 48 KB static limit)
     TailSmem& sm = *reinterpret_cast<TailSmem*>(tailSmem);
-    
+    TailSmem::Stage& st = *reinterpret_cast<TailSmem::Stage*>(sm.stage);
     const int rig = blockIdx.x / cluster, rank = blockIdx.x % cluster;
-    initMagic(sm.down.magic);
+    const Segment& sg = segs[min(rig, nsegs - 1)];  // the grid is nsegs clusters
+    const RigDev& R = sm.rig;
+    for (int k = threadIdx.x; k < (int)sizeof(RigDev) / 4; k += kThreads)
+        reinterpret_cast<uint32_t*>(&sm.rig)[k] = __ldg(reinterpret_cast<const uint32_t*>(sg.rig) + k);
+    initMagic(st.down.magic);
+    __syncthreads();
+    // blend levels above 0 (with tailHalf) go as half tiles with two pixels
+    // per thread, so the few tiles of these levels keep twice the CTAs and all
+    // warps busy; otherwise whole tiles, 2x2 blocks
+    auto parts = [&](int j) { return j > 0 && R.tailHalf ? 2 : 1; };
+    if (threadIdx.x <= R.L) {
+        const int j = threadIdx.x;
+        if (j >= R.tailDown && rank < R.downCnt[j]) sm.down[j] = R.downItems[R.downOff[j] + rank];
+        if (j >= R.tailBlend && rank < parts(j) * R.blendCnt[j])
+            sm.blend[j] = *reinterpret_cast<const uint4*>(R.blendItems + R.blendOff[j] + rank / parts(j));
+    }
+    __syncthreads();
     waitPrevGrid();
     allowNextGrid();
-    if (rig >= nsegs) return;  // never: the grid is nsegs clusters
-    __syncthreads();  // the magic table
-    const Segment& sg = segs[rig];
-    const RigDev& R = *sg.rig;
     for (int J = R.tailDown; J <= R.L; J++) {
-        const DownItem* items = R.downItems + R.downOff[J];
-        for (int k = rank; k < R.downCnt[J]; k += cluster) pyrDownTile<true>(R, items[k], sm.down);
-        clusterSync();
+        for (int k = rank; k < R.downCnt[J]; k += cluster)
+            pyrDownTile<true>(R, k == rank ? sm.down[J] : R.downItems[R.downOff[J] + k], st.down);
+        clusterArrive();
+        clusterWait();
     }
     BlendAcc acc;
     PairAcc pacc;
+    // With half tiles, the level's first unit is staged but for its C_{j+1}
+    // footprint while the CTA waits for the level above (two buffers in turn).
+    auto stageAhead = [&](int j) {
+        if (j >= R.tailBlend && parts(j) == 2 && rank < 2 * R.blendCnt[j])
+            stageHalfG<true>(st.half[j & 1], R, sm.blend[j], 0, rank & 1);
+    };
+    __syncthreads();  // the stages overlay the pyrDown's shared memory
+    stageAhead(R.L);
     for (int j = R.L; j >= R.tailBlend; j--) {
         const BlendItem* items = R.blendItems + R.blendOff[j];
         UnitGeo geo;
         fillGeo(geo, R, *sg.frame, j);
-        // levels above 0 (with tailHalf): half tiles with two pixels per
-        // thread, so the few tiles of these levels keep twice the CTAs and
-        // all warps busy; otherwise whole tiles, 2x2 blocks
-        const int parts = j > 0 && R.tailHalf ? 2 : 1;
-        for (int k = rank; k < parts * R.blendCnt[j]; k += cluster) {
-            const uint4 raw = *reinterpret_cast<const uint4*>(items + k / parts);
-            const bool active = !((raw.x & 0xFF) == 0 && ((raw.x >> 8) & 0xFF) == 0);
-            for (int chunk = 0; chunk < unitChunks<kTailCamsPerUnit>(raw); chunk++) {
-                __syncthreads();  // readers of the previous unit are done
-                if (active) stageUnitRows<true>(sm.blend, R, raw, chunk, parts == 2 ? (k & 1) : -1);
-                __syncthreads();
-                if (parts == 2) computeUnitRows(sm.blend, geo, raw, chunk, pacc, k & 1);
-                else computeUnit(sm.blend, geo, raw, chunk, false, acc);
+        for (int k = rank; k < parts(j) * R.blendCnt[j]; k += cluster) {
+            const uint4 raw = k == rank ? sm.blend[j] : *reinterpret_cast<const uint4*>(items + k / parts(j));
+            if (parts(j) == 2) {
+                HalfStage& h = st.half[j & 1];
+                for (int chunk = 0; chunk < unitChunks<HalfStage::kCams>(raw); chunk++) {
+                    if (k != rank || chunk > 0) {
+                        __syncthreads();  // readers of the previous unit are done
+                        stageHalfG<true>(h, R, raw, chunk, k & 1);
+                    }
+                    stageHalfC<true>(h, R, raw, chunk, k & 1);
+                    __syncthreads();
+                    computeUnitRows(h, geo, raw, chunk, pacc, k & 1);
+                }
+            } else {
+                const bool active = !(j == 0 && ((raw.x >> 8) & 0xFF) == 0);
+                for (int chunk = 0; chunk < unitChunks<WholeStage::kCams>(raw); chunk++) {
+                    __syncthreads();
+                    if (active) stageUnitDirect<true>(st.whole, R, raw, chunk, sm.fRow, sm.fCol, [] { __syncthreads(); });
+                    __syncthreads();
+                    computeUnit(st.whole, geo, raw, chunk, false, acc);
+                }
             }
         }
-        clusterSync();
+        clusterArrive();
+        stageAhead(j - 1);
+        clusterWait();
     }
 }
 
@@ -2021,13 +2052,10 @@ __global__ void __launch_bounds__(kThreads) k_tail(const Segment* __restrict__ s
 // a chain of load-and-compute rounds that these levels cannot hide behind
 // other tiles; here each CTA has one short chain and all its warps busy.
 // ============================================================================
-using SmallStage = BlendStageT<kTailCamsPerUnit>;
-
 __global__ void __launch_bounds__(kThreads) k_blend_small(const Segment* __restrict__ segs, int nsegs, int total,
                                                           int early)
 {
-    extern __shared__ __align__(128) uint8_t smallSmem[];  // a SmallStage (dynamic: above the 48 KB static limit)
-    SmallStage& st = *reinterpret_cast<SmallStage*>(smallSmem);
+    __shared__ HalfStage st;
 
     // Items and descriptors are written before the launch sequence, not by
     // a kernel: the first item's are read while the previous kernel finishes.
@@ -2044,7 +2072,7 @@ __global__ void __launch_bounds__(kThreads) k_blend_small(const Segment* __restr
         s = findSegment(segs, nsegs, first, s);
         raw = __ldg(static_cast<const uint4*>(segs[s].items) + ((first - segs[s].prefix) >> 1));
         fillGeo(geo, *segs[s].rig, *segs[s].frame, raw.x & 0xFF);
-        if (pre) stageUnitRows<true>(st, *segs[s].rig, raw, 0, (first - segs[s].prefix) & 1, true, false);
+        if (pre) stageHalfG<true>(st, *segs[s].rig, raw, 0, (first - segs[s].prefix) & 1);
     }
     waitPrevGrid();
     allowNextGrid();
@@ -2058,10 +2086,11 @@ __global__ void __launch_bounds__(kThreads) k_blend_small(const Segment* __restr
         const Segment& sg = segs[s];
         const RigDev& R = *sg.rig;
         const int half = (it - sg.prefix) & 1;
-        for (int chunk = 0; chunk < unitChunks<kTailCamsPerUnit>(raw); chunk++) {
+        for (int chunk = 0; chunk < unitChunks<HalfStage::kCams>(raw); chunk++) {
             __syncthreads();  // readers of the previous unit are done
-            const bool staged = pre && it == first && chunk == 0;  // G part staged before the wait
-            stageUnitRows<false>(st, R, raw, chunk, half, !staged, true);
+            // the first unit's G part was staged before the wait
+            if (!(pre && it == first && chunk == 0)) stageHalfG<false>(st, R, raw, chunk, half);
+            stageHalfC<false>(st, R, raw, chunk, half);
             __syncthreads();
             computeUnitRows(st, geo, raw, chunk, acc, half);
         }
@@ -2372,21 +2401,8 @@ cudaError_t launchBlend(const Segment* segs, int nsegs, int total, int perSm, in
 cudaError_t launchBlendSmall(const Segment* segs, int nsegs, int total, bool early, cudaStream_t st)
 {
     if (total <= 0) return cudaSuccess;
-    static const int perSm = [] {  // the attribute is set before any launch can see perSm
-        cudaFuncSetAttribute(k_blend_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallStage));
-        return residentPerSm<k_blend_small>(kThreads, sizeof(SmallStage));
-    }();
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(gridFor(total, perSm));
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = sizeof(SmallStage);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_blend_small, segs, nsegs, total, (int)early);
+    return launchPdl(k_blend_small, gridFor(total, residentPerSm<k_blend_small>(kThreads)), kThreads, st, segs, nsegs,
+                     total, (int)early);
 }
 
 int tailClusterMax()
