@@ -11,9 +11,9 @@
  * Every entry point returns an int status (PS_OK or a PS_E* code) and never
  * throws; ps_last_error() returns the thread-local message of the last
  * failure.  Work is ordered on the caller's CUDA stream (NULL = the legacy
- * default stream): the renders run on their own streams, and the caller's
- * stream waits for each call's completion; no entry point synchronises the
- * stream unless it says so.  A ps_render is not thread-safe; distinct
+ * default stream): the renders run on it or on their own streams, and the
+ * caller's stream waits for each call's completion; no entry point
+ * synchronises the stream unless it says so.  A ps_render is not thread-safe; distinct
  * renders may be used from different threads.  A render records its launch
  * sequence as a CUDA graph with stream capture (on its first frames, after
  * prepare or a launch-shape change, and throughout ps_render_autotune);
@@ -143,7 +143,8 @@ int ps_render_prepare_with_seams(ps_render* r, const ps_photo_param* params, int
    reference logs a warning and skips the correction).  dst: a dst_w x dst_h
    BGR32 or BGR24 image, host or device.  Host src / dst are copied inside
    the call (pinned memory keeps the copies asynchronous); device src / dst
-   are read / written in place.  The work runs on the render's own copy-in,
+   are read / written in place.  With device src and dst alone the work
+   runs on the caller's stream; else it runs on the render's own copy-in,
    compute and copy-out streams, and the caller's stream waits for its
    completion.  A render keeps a set of per-frame state per frame in flight
    (ps_render_set_frames_in_flight; eight by default), so that many calls

@@ -1294,6 +1294,8 @@ void Plan::quiesce()
         if (st) PS_CUDA(cudaStreamSynchronize(st));
     for (cudaStream_t st : sComp_)
         if (st) PS_CUDA(cudaStreamSynchronize(st));
+    for (IoSlot& sl : io_)  // runs on the callers' streams
+        if (sl.used) PS_CUDA(cudaEventSynchronize(sl.computed));
 }
 
 void Plan::bind(const std::vector<Rig*>& rigs)
@@ -1423,6 +1425,8 @@ Plan::~Plan()
         if (st) cudaStreamSynchronize(st);
     for (cudaStream_t st : sComp_)
         if (st) cudaStreamSynchronize(st);
+    for (IoSlot& sl : io_)
+        if (sl.used && cudaEventSynchronize(sl.computed) != cudaSuccess) cudaGetLastError();
     dropGraph();
     for (cudaStream_t st : {sIn_, sOut_, capStream_})
         if (st) cudaStreamDestroy(st);
@@ -1473,12 +1477,26 @@ void Plan::launchAll(const IoSlot& slot, cudaStream_t st, int srcFmt, Profiler* 
 
 static int bytesPerPixel(int fmt) { return fmt == PS_FMT_BGR24 ? 3 : 4; }
 
+// Whether a stream is being captured (an error, such as the legacy stream's
+// while another thread captures, counts as yes).
+static bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &c) == cudaSuccess) return c != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 // One run: copy-in (host frames, the staged arguments), compute (one stream
 // per slot), copy-out (host canvases).  Runs take the kIoSlots slots of
 // arguments and rig state in turn and wait only for the previous run on the
 // same slot, so with host buffers on both sides consecutive runs overlap.
 // With any device input or output the run also waits for the caller's
 // stream.  The caller's stream waits for the run's completion.
+// A run with device buffers alone (direct) has nothing to copy but its
+// arguments, which need not wait for the caller: its kernels go to the caller's
+// stream itself.  Between two frames on one stream the detour over the plan's
+// streams was 14 - 16 us of waiting for events and a copy; now it is 3 us.
 void Plan::run(const std::vector<FrameInput>& in, cudaStream_t st, bool useGraph, Profiler* prof)
 {
     NvtxRange range("ps.run");
@@ -1488,31 +1506,31 @@ void Plan::run(const std::vector<FrameInput>& in, cudaStream_t st, bool useGraph
     ensureStreams();
     const int si = nextIo_;
     IoSlot& S = io_[si];
-    bool hostOnly = true;
+    bool hostOnly = true, direct = true;
+    auto buffer = [&](int location) { (location == PS_MEM_HOST ? direct : hostOnly) = false; };
     for (const FrameInput& f : in) {
         Rig* rig = rigs_[&f - in.data()];
         if (f.psrc) {
             rig->ensurePlanar();  // before any work of this run is queued
-            for (int i = 0; i < rig->numImages(); i++)
-                if (f.psrc[i].location != PS_MEM_HOST) hostOnly = false;
+            for (int i = 0; i < rig->numImages(); i++) buffer(f.psrc[i].location);
         } else if (!f.src) {
             hostOnly = false;  // level 0 written on the caller's stream
         } else {
-            for (int i = 0; i < rig->numImages(); i++)
-                if (f.src[i].location != PS_MEM_HOST) hostOnly = false;
+            for (int i = 0; i < rig->numImages(); i++) buffer(f.src[i].location);
         }
-        if ((f.ydst ? f.ydst->location : f.dst->location) != PS_MEM_HOST) hostOnly = false;
+        buffer(f.ydst ? f.ydst->location : f.dst->location);
     }
+    direct = direct && !capturing(st);
     if (S.used) PS_CUDA(cudaEventSynchronize(S.argsCopied));  // the slot's pinned stage is free again
-    PS_CUDA(cudaEventRecord(callerEv_, st));
+    if (!direct) PS_CUDA(cudaEventRecord(callerEv_, st));
     // each rig's state slot (pyramids, I/O staging); without sources it is
     // the slot imagesToLevel0 just filled (peekSlot)
     std::vector<int> rs(rigs_.size());
     for (size_t r = 0; r < rigs_.size(); r++) rs[r] = rigs_[r]->acquireSlot();
-    cudaStream_t comp = sComp_[si];
+    cudaStream_t comp = direct ? st : sComp_[si];
 
     // ---- copy-in: after the previous kernels on the rigs' slots (inputs, pyramids) and on this args slot
-    if (!hostOnly) PS_CUDA(cudaStreamWaitEvent(sIn_, callerEv_, 0));
+    if (!direct && !hostOnly) PS_CUDA(cudaStreamWaitEvent(sIn_, callerEv_, 0));
     if (S.used) PS_CUDA(cudaStreamWaitEvent(sIn_, S.computed, 0));
     for (size_t r = 0; r < rigs_.size(); r++) PS_CUDA(cudaStreamWaitEvent(sIn_, rigs_[r]->slotComputed(rs[r]), 0));
     uint8_t* stage = S.stage.as<uint8_t>();
@@ -1669,11 +1687,13 @@ void Plan::run(const std::vector<FrameInput>& in, cudaStream_t st, bool useGraph
     PS_CUDA(cudaMemcpyAsync(dArgs, stage, stageBytes_, cudaMemcpyHostToDevice, sIn_));
     PS_CUDA(cudaEventRecord(S.argsCopied, sIn_));
 
-    // ---- compute: one stream per args slot, so two runs' kernels can overlap
+    // ---- compute: one stream per args slot (or the caller's), so two runs' kernels can overlap
     PS_CUDA(cudaStreamWaitEvent(comp, S.argsCopied, 0));
-    if (!hostOnly) PS_CUDA(cudaStreamWaitEvent(comp, callerEv_, 0));
-    for (size_t r = 0; r < rigs_.size(); r++)  // the output staging has been read out
-        PS_CUDA(cudaStreamWaitEvent(comp, rigs_[r]->slotDownloaded(rs[r]), 0));
+    if (!direct) {
+        if (!hostOnly) PS_CUDA(cudaStreamWaitEvent(comp, callerEv_, 0));
+        for (size_t r = 0; r < rigs_.size(); r++)  // the output staging has been read out
+            PS_CUDA(cudaStreamWaitEvent(comp, rigs_[r]->slotDownloaded(rs[r]), 0));
+    }
     for (const YuvFrames& y : cvt) {
         cudaEvent_t a = nullptr, b = nullptr;
         if (prof) {
@@ -1715,6 +1735,9 @@ void Plan::run(const std::vector<FrameInput>& in, cudaStream_t st, bool useGraph
     }
     PS_CUDA(cudaEventRecord(S.computed, comp));
     for (size_t r = 0; r < rigs_.size(); r++) PS_CUDA(cudaEventRecord(rigs_[r]->slotComputed(rs[r]), comp));
+    S.used = true;
+    nextIo_ = (si + 1) % Rig::kIoSlots;
+    if (direct) return;  // nothing to download, and the caller's stream is behind the kernels
 
     // ---- copy-out
     PS_CUDA(cudaStreamWaitEvent(sOut_, S.computed, 0));
@@ -1746,8 +1769,6 @@ void Plan::run(const std::vector<FrameInput>& in, cudaStream_t st, bool useGraph
     PS_CUDA(cudaEventRecord(S.downloaded, sOut_));
     for (size_t r = 0; r < rigs_.size(); r++) PS_CUDA(cudaEventRecord(rigs_[r]->slotDownloaded(rs[r]), sOut_));
     PS_CUDA(cudaStreamWaitEvent(st, S.downloaded, 0));
-    S.used = true;
-    nextIo_ = (si + 1) % Rig::kIoSlots;
 }
 
 }  // namespace ps
