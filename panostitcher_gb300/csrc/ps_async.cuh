@@ -11,7 +11,7 @@
 
 namespace ps {
 
-constexpr long long kMaxPolls = 1LL << 24;
+constexpr int kMaxPolls = 1 << 24;
 
 __device__ __forceinline__ uint32_t smemAddr(const void* p)
 {
@@ -48,22 +48,11 @@ __device__ __forceinline__ bool mbarTryWait(uint64_t* bar, uint32_t parity)
 }
 
 // Bounded wait for the phase with the given parity to complete.
-__device__ __forceinline__ bool mbarWait(uint64_t* bar, uint32_t parity, long long maxPolls = kMaxPolls)
+__device__ __forceinline__ bool mbarWait(uint64_t* bar, uint32_t parity, int maxPolls = kMaxPolls)
 {
-    for (long long i = 0; i < maxPolls; i++)
+    for (int i = 0; i < maxPolls; i++)
         if (mbarTryWait(bar, parity)) return true;
     return false;
-}
-
-// Global -> shared bulk copy completing on an mbarrier.  dst, src and bytes
-// must be multiples of 16.
-__device__ __forceinline__ void bulkCopy(void* dst, const void* src, uint32_t bytes, uint64_t* bar)
-{
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smemAddr(dst)),
-        "l"(src), "r"(bytes), "r"(smemAddr(bar))
-        : "memory");
 }
 
 // Bulk tensor copies (TMA, tile mode, no swizzle) of one box of a 3-D or

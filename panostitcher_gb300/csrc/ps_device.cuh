@@ -10,8 +10,9 @@
 //   Wt[j]  uint16 seam-weight pyramid (weightPyrs, 0..256), same pitch as G.
 //   Am[j]  uint16 alpha divisor m = alphaPyr / 256 (alphaPyrs is always a
 //          multiple of 256 because its level source is 0/256), level >= 1.
-//   C[j]   short4 collapsed result of level j >= 1 (resultPyr after
-//          normalise + collapse); |value| < 3300 so int16 is exact.
+//   C[j]   collapsed result of level j >= 1 (resultPyr after normalise +
+//          collapse), four int16 a pixel: B, R, G, each + kCBias, and 0;
+//          |value| < 8700, so int16 is exact.
 //   maps   float2 dst->src map, stored tile-compact for the level-0 tiles
 //          that a camera covers (512 pixels per 32x16 tile, in 16x2 blocks).
 // Work is described by item lists built at prepare time from the pyramids'
@@ -30,6 +31,7 @@ constexpr int kRemapTW = 32, kRemapTH = 16;    // level-0 remap tile (two pixels
 constexpr int kDownTW = 32, kDownTH = 16;      // pyrDown output tile (two pixels per thread)
 constexpr int kBlendTW = 64, kBlendTH = 16;    // blend tile (a 2x2 pixel block per thread)
 constexpr int kThreads = 256;
+constexpr int kCBias = 256;  // of the collapsed levels' values
 
 // Pixel i of a remap tile (its map, its linear weight): the tile is 16 blocks
 // of 16x2 pixels, two across and eight down, a warp's 32 pixels each.  The

@@ -31,11 +31,11 @@ namespace ps {
 // ---- the checked build ---------------------------------------------------------
 // Compiled with -DPS_CHECK_BOUNDS (libpanostitch_checked.so), every global
 // access of the stitch kernels is checked against the extent of the buffer
-// it belongs to.  An access outside is not made -- a load reads 0, a store
-// is dropped, a bulk copy reads from the buffer's start instead, so its
-// byte count still completes its barrier -- and the device-wide violation
-// counter goes up (ps_debug_bounds_violations).  Nothing traps.  In the
-// normal build every check is a constant true.
+// it belongs to.  An access outside is not made -- a load reads 0, a store is
+// dropped -- and the device-wide violation counter goes up
+// (ps_debug_bounds_violations).  Nothing traps.  k_blend's units are then all
+// staged by checked loads instead of tensor copies (which the hardware
+// bounds).  In the normal build every check is a constant true.
 #ifdef PS_CHECK_BOUNDS
 __device__ unsigned long long g_boundsViolations;
 #endif
@@ -72,15 +72,6 @@ template <class T>
 __device__ __forceinline__ T ldChecked(const T* p, const void* base, long long bytes)
 {
     return inside(p, base, bytes) ? __ldg(p) : T{};
-}
-
-// A bulk copy whose source range is checked: outside its buffer it copies
-// from the buffer's start instead, so the barrier still receives its bytes.
-__device__ __forceinline__ void bulkCopyChecked(void* dst, const void* src, uint32_t bytes, uint64_t* bar,
-                                                const void* base, long long ext)
-{
-    if (!insideRange(src, bytes, base, ext)) src = base;
-    bulkCopy(dst, src, bytes, bar);
 }
 
 // Extents of a rig's buffers.
@@ -1008,15 +999,21 @@ __global__ void __launch_bounds__(kThreads, 5) k_pyrdown(const Segment* __restri
 // block at (2*(t%32), 2*(t/32)), so the zero-inserted upsample's three
 // footprint rows serve both of its rows and the YUV chroma of the block is
 // its own.  Work flows through a 2-stage shared-memory ring of "units" (a
-// tile and up to two of its cameras).  A
-// dedicated producer warp stages each unit with bulk asynchronous copies of
-// whole rows -- the cameras' G_j and weight rows, their G_{j+1} footprint
-// rows and, with a tile's last unit, the C_{j+1} footprint rows -- completing
-// on the stage's "full" mbarrier; the eight consumer warps compute from
-// shared memory and release the stage on its "empty" mbarrier.  Tiles whose
-// footprints cross the canvas border (horizontal wrap, vertical
-// reflect-101) are staged by the consumers with the reference's index
-// mapping.
+// tile and up to two of its cameras).  A dedicated producer warp stages each
+// unit with bulk tensor copies -- per camera the G_j tile, its weights (not
+// for uniform tiles) and its G_{j+1} footprint, and with a tile's last unit
+// the C_{j+1} footprint -- completing on the stage's "full" mbarrier; the
+// eight consumer warps compute from shared memory and release the stage on its
+// "empty" mbarrier.  Tiles whose footprints cross the canvas border
+// (horizontal wrap, vertical reflect-101) are staged by the consumers with the
+// reference's index mapping.
+//
+// Level 0 of 6 x 1920x1080 to 4096x2048: 37 us, 42 before the uniform tiles'
+// packed path and the runs (24.4 M instead of 32.0 M warp instructions); of 8 x
+// 3840x2160 to 7680x3840: 80 us, 100 before.  Left: a unit's arithmetic (2300
+// cycles of eight warps a scheduler) and the producer's work on the next one
+// (2300 cycles too) take turns waiting for each other; a 4-stage ring, a
+// 3-stage one and one lane doing the producer's work measured no shorter.
 // ============================================================================
 constexpr int kFW = kBlendTW / 2 + 2;  // 34: footprint columns fx0 .. fx0+33
 constexpr int kFH = kBlendTH / 2 + 2;  // 10: footprint rows    fy0 .. fy0+9
@@ -1026,6 +1023,11 @@ constexpr int kFpW = 40;   // staged footprint row: columns fx0-3 .. fx0+36 (16-
 constexpr int kCfW = 36;   // staged collapse footprint row: columns fx0-1 .. fx0+34
 constexpr int kMaxSmemSegs = 64;
 constexpr int kConsumers = kThreads;          // 8 warps
+// Tiles the producer takes at a time: a kBlendShare'th of a CTA's part of what
+// is left, at most kBlendRun.  One at a time, the atomic's round trip and the
+// descriptor's load per tile held the consumers up (7680x3840 level 0: 94 us,
+// 84 with runs of 4); larger shares leave CTAs unequal at the end.
+constexpr int kBlendRun = 4, kBlendShare = 4;
 constexpr int kBlendThreads = kConsumers + 32;  // + the producer warp
 
 // One unit's shared-memory stage: NC cameras of one tile (k_blend stages
@@ -1088,7 +1090,8 @@ __device__ __forceinline__ void fillGeo(UnitGeo& g, const RigDev& R, const Frame
 
 struct UnitInfo {
     uint4 raw;
-    int seg, chunk, valid, staged;  // staged: copies issued by the producer
+    int chunk, valid, staged;  // staged: copies issued by the producer
+    int seg;                   // the segment geo was filled in for
     UnitGeo geo;
 };
 
@@ -1354,205 +1357,138 @@ __device__ __forceinline__ void stageHalfC(HalfStage& S, const RigDev& R, const 
     S.cf[r][c + 1] = inside(p, Lu.C, cBytes(Lu)) ? ldLevel<kFresh>(p) : make_uint2(0, 0);
 }
 
-// Accumulate one unit from its stage; at a tile's last unit normalise,
-// collapse and store.  Threads 0..kConsumers-1.  staged: the unit came from
-// the bulk copies (weights absent for uniform tiles).
-//
+// ---- the zero-inserted upsample of a 2x2 block ----------------------------------
 // Thread (lane, warp) owns rows ly = 2*warp, ly + 1 and columns lx = 2*lane,
-// lx + 1 of the tile.  The zero-inserted upsample (weights 1 6 1 for an even
-// output row / column, 4 4 for an odd one) reads footprint rows warp ..
-// warp+2 (even row: all three; odd row: the last two) and columns lane ..
-// lane+2 the same way.
-__device__ __forceinline__ void upsample2x2(const uint32_t* g, int pitchW, uint32_t* ulo, uint32_t* uhi)
+// lx + 1 of the tile.  The upsample (weights 1 6 1 for an even output row or
+// column, 4 4 for an odd one, over 64) reads footprint rows warp .. warp+2
+// (even row: all three; odd row: the last two) and columns lane .. lane+2 the
+// same way.  Words hold two channels in 16-bit lanes.  The common factors 4
+// and 16 of the odd rows and columns are left out and taken off the final
+// shift: (4x + 32) >> 6 = (x + 8) >> 4, (16x + 32) >> 6 = (x + 2) >> 2.
+struct ColumnSums {
+    uint32_t e, o;  // even row: a + 6 b + c; odd row: b + c
+};
+__device__ __forceinline__ ColumnSums columnSums(uint32_t a, uint32_t b, uint32_t c) { return {a + 6 * b + c, b + c}; }
+
+// The block's four values, rounded and shifted; one: a 1 in every lane in use.
+// Lane sums are at most 64 * 1023 + 32, so nothing carries between lanes; the
+// shifts move bits from the upper lane into the lower, which the caller masks.
+__device__ __forceinline__ void upsampleBlock(const ColumnSums* s, uint32_t one, uint32_t* out)
 {
-    uint32_t elo[3], ehi[3], olo[3], ohi[3];
+    out[0] = (s[0].e + s[2].e + 32 * one + 6 * s[1].e) >> 6;
+    out[1] = (s[1].e + s[2].e + 8 * one) >> 4;
+    out[2] = (s[0].o + s[2].o + 8 * one + 6 * s[1].o) >> 4;
+    out[3] = (s[1].o + s[2].o + 2 * one) >> 2;
+}
+
+// U = pyrUp(G_{j+1}) of the block from the camera's footprint g (row pitch
+// kFpW): B | R << 16 in lo, G in hi, 0..255 each.
+__device__ __forceinline__ void upsampleG(const uint32_t* g, uint32_t* lo, uint32_t* hi)
+{
+    ColumnSums sl[3], sh[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        const uint2 a = unpackBytes(g[k]), b = unpackBytes(g[pitchW + k]), c = unpackBytes(g[2 * pitchW + k]);
-        elo[k] = a.x + 6 * b.x + c.x;
-        ehi[k] = a.y + 6 * b.y + c.y;
-        olo[k] = 4 * (b.x + c.x);
-        ohi[k] = 4 * (b.y + c.y);
+        const uint32_t a = g[k], b = g[kFpW + k], c = g[2 * kFpW + k];
+        sl[k] = columnSums(__byte_perm(a, 0, 0x4240), __byte_perm(b, 0, 0x4240), __byte_perm(c, 0, 0x4240));
+        sh[k] = columnSums(__byte_perm(a, 0, 0x4341), __byte_perm(b, 0, 0x4341), __byte_perm(c, 0, 0x4341));
     }
-    ulo[0] = elo[0] + 6 * elo[1] + elo[2];
-    uhi[0] = ehi[0] + 6 * ehi[1] + ehi[2];
-    ulo[1] = 4 * (elo[1] + elo[2]);
-    uhi[1] = 4 * (ehi[1] + ehi[2]);
-    ulo[2] = olo[0] + 6 * olo[1] + olo[2];
-    uhi[2] = ohi[0] + 6 * ohi[1] + ohi[2];
-    ulo[3] = 4 * (olo[1] + olo[2]);
-    uhi[3] = 4 * (ohi[1] + ohi[2]);
+    upsampleBlock(sl, 0x00010001u, lo);
+    upsampleBlock(sh, 1u, hi);  // the fourth channel is 0
+#pragma unroll
+    for (int p = 0; p < 4; p++) lo[p] &= 0x00FF00FFu;
 }
 
-// The Laplacian L = G - ((U + 32) >> 6) of one pixel, B and R in the two
-// 16-bit lanes of one word, each biased by 256: lanes hold 256 + L in
-// 1..511, so neither the lane sums nor the subtraction carry or borrow
-// across lanes (U is at most 64 * 255).  G is returned unbiased.
-struct Lap {
-    uint32_t br;  // (256 + L_B) | (256 + L_R) << 16
-    int g;        // L_G
+// ---- the collapsed levels C_j ---------------------------------------------------
+// A pixel is two words, B | R << 16 and G, each lane the value + kCBias.  |C| <
+// 8700 (see ps_device.cuh), so a lane is a signed 16-bit number; nearly always
+// C lies in -256 .. 767, where the lanes are 0..1023 and the upsample runs two
+// channels per word (cInRange).
+__device__ __forceinline__ uint2 packC(int b, int g, int r)
+{
+    return make_uint2((uint32_t)(uint16_t)(b + kCBias) | ((uint32_t)(uint16_t)(r + kCBias) << 16),
+                      (uint32_t)(uint16_t)(g + kCBias));
+}
+
+// The thread's nine footprint pixels of C_{j+1}.
+struct CFootprint {
+    uint2 v[3][3];  // [row][column]
 };
-
-__device__ __forceinline__ Lap laplacian(uint32_t gpx, uint32_t ulo, uint32_t uhi)
+__device__ __forceinline__ CFootprint loadC(const uint2* cf)
 {
-    const uint32_t ubr = ((ulo + 0x00200020u) >> 6) & 0x03FF03FFu;  // round(U) of B and R, per lane
-    Lap l;
-    l.br = __byte_perm(gpx, 0, 0x4240) + 0x01000100u - ubr;         // G's B and R bytes into the lanes
-    l.g = (int)__byte_perm(gpx, 0, 0x4441) - (int)(((uhi & 0xFFFFu) + 32u) >> 6);
-    return l;
+    CFootprint f;
+#pragma unroll
+    for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) f.v[r][k] = cf[r * kCfW + k];
+    return f;
 }
-
-template <class Stage>
-__device__ __forceinline__ void computeUnit(const Stage& S, const UnitGeo& G, const uint4& raw, int chunk,
-                                            bool staged, BlendAcc& acc)
+__device__ __forceinline__ bool cInRange(const CFootprint& f)
 {
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    const int lx = 2 * lane, ly = 2 * wp;
-    const int j = raw.x & 0xFF, cls = (raw.x >> 8) & 0xFF, camCnt = (raw.x >> 16) & 0xFF;
-    const bool uni = ((raw.x >> 24) & kTileUniform) != 0;
-    const int tx = raw.y & 0xFFFF, ty = raw.y >> 16;
-    const bool hasUp = G.hasUp != 0;
-    const int x = tx * kBlendTW + lx, y = ty * kBlendTH + ly;
-    const bool active = !(j == 0 && cls == 0);
-    constexpr int NC = Stage::kCams;
-    const int c0 = chunk * NC;
-    const int nc = max(0, min(NC, camCnt - c0));
-    const bool first = chunk == 0, last = chunk == unitChunks<NC>(raw) - 1;
-    const bool fast = uni && staged;  // weights were not staged
-    if (first) {
+    uint32_t any = 0;
 #pragma unroll
-        for (int p = 0; p < 4; p++) {
-            acc.r[p][0] = acc.r[p][1] = acc.r[p][2] = 0;
-            acc.wsum[p] = 0;
-        }
+    for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) any |= f.v[r][k].x | f.v[r][k].y;
+    return (any & 0xFC00FC00u) == 0;
+}
+// pyrUp(C_{j+1}) of the block, biased by kCBias: B | R << 16 in lo, G in hi.
+__device__ __forceinline__ void upsampleC(const CFootprint& f, uint32_t* lo, uint32_t* hi)
+{
+    ColumnSums sl[3], sh[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        sl[k] = columnSums(f.v[0][k].x, f.v[1][k].x, f.v[2][k].x);
+        sh[k] = columnSums(f.v[0][k].y, f.v[1][k].y, f.v[2][k].y);
     }
-    if (active) {
-        for (int q = 0; q < nc; q++) {
-            uint32_t ulo[4] = {0, 0, 0, 0}, uhi[4] = {0, 0, 0, 0};
-            if (hasUp) upsample2x2(&S.fpw[q][wp * kFpW + 3 + lane], kFpW, ulo, uhi);
-            const uint2 gt = *reinterpret_cast<const uint2*>(&S.gj[q][ly][lx]);
-            const uint2 gb = *reinterpret_cast<const uint2*>(&S.gj[q][ly + 1][lx]);
-            const uint32_t gp[4] = {gt.x, gt.y, gb.x, gb.y};
-            uint32_t wq[2] = {0, 0};
-            if (!fast) {
-                wq[0] = *reinterpret_cast<const uint32_t*>(&S.w[q][ly][lx]);
-                wq[1] = *reinterpret_cast<const uint32_t*>(&S.w[q][ly + 1][lx]);
-            }
+    upsampleBlock(sl, 0x00010001u, lo);
+    upsampleBlock(sh, 1u, hi);
 #pragma unroll
-            for (int p = 0; p < 4; p++) {
-                const Lap l = laplacian(gp[p], ulo[p], uhi[p]);
-                if (fast) {
-                    acc.r[p][0] = (int)(l.br & 0xFFFFu) - 256;
-                    acc.r[p][1] = l.g;
-                    acc.r[p][2] = (int)(l.br >> 16) - 256;
-                } else {
-                    // B and R accumulate w * (256 + L); the 256 * sum(w) comes off at normalisation
-                    const int w = (int)((wq[p >> 1] >> (16 * (p & 1))) & 0xFFFFu);
-                    acc.r[p][0] += w * (int)(l.br & 0xFFFFu);
-                    acc.r[p][1] += w * l.g;
-                    acc.r[p][2] += w * (int)(l.br >> 16);
-                    acc.wsum[p] += w;
-                }
-            }
-        }
-    }
-    if (!last) return;
-    if (!fast) {
+    for (int p = 0; p < 4; p++) lo[p] &= 0x03FF03FFu;
+}
+// The same for any values, added to n[p] = (B, G, R).
+__device__ __forceinline__ void addUpsampledC(const CFootprint& f, int (*n)[3])
+{
 #pragma unroll
-        for (int p = 0; p < 4; p++) {
-            acc.r[p][0] -= acc.wsum[p] << 8;
-            acc.r[p][2] -= acc.wsum[p] << 8;
-        }
-    }
-    int n[4][3];
-    if (fast) {
-#pragma unroll
-        for (int p = 0; p < 4; p++)
-#pragma unroll
-            for (int c = 0; c < 3; c++) n[p][c] = acc.r[p][c];
-    } else if (G.full) {
-#pragma unroll
-        for (int p = 0; p < 4; p++)
-#pragma unroll
-            for (int c = 0; c < 3; c++) n[p][c] = (acc.r[p][c] + 128) >> 8;
-    } else if (j == 0 && __all_sync(0xffffffffu, ((acc.wsum[0] | acc.wsum[1] | acc.wsum[2] | acc.wsum[3]) & ~256) == 0)) {
-        // Level-0 weights are the 0/256 seam masks.  Where each pixel's sum is 0 or 256 (one camera at
-        // most: always, unless custom masks overlap), R = 256 L exactly, and R / W truncated is the shift.
-#pragma unroll
-        for (int p = 0; p < 4; p++)
-#pragma unroll
-            for (int c = 0; c < 3; c++) n[p][c] = acc.r[p][c] >> 8;
-    } else {
-#pragma unroll
-        for (int p = 0; p < 4; p++) {
-            const int d = acc.wsum[p] ? acc.wsum[p] : 1;
-            const float inv = __frcp_rn((float)d);
-#pragma unroll
-            for (int c = 0; c < 3; c++) n[p][c] = divTrunc(acc.r[p][c], d, inv);
-        }
-    }
-    // collapse: + pyrUp32(C_{j+1})
-    if (hasUp && active) {
-        const uint2* cf = &S.cf[wp][1 + lane];
-        int e[3][3], o[3][3];  // vertical sums per footprint column, even / odd row
+    for (int ch = 0; ch < 3; ch++) {
+        int e[3], o[3];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
-            const uint2 a = cf[k], b = cf[kCfW + k], c = cf[2 * kCfW + k];
-            const int av[3] = {(short)(a.x & 0xFFFF), (short)(a.x >> 16), (short)(a.y & 0xFFFF)};
-            const int bv[3] = {(short)(b.x & 0xFFFF), (short)(b.x >> 16), (short)(b.y & 0xFFFF)};
-            const int cv[3] = {(short)(c.x & 0xFFFF), (short)(c.x >> 16), (short)(c.y & 0xFFFF)};
+            int v[3];
 #pragma unroll
-            for (int ch = 0; ch < 3; ch++) {
-                e[k][ch] = av[ch] + 6 * bv[ch] + cv[ch];
-                o[k][ch] = 4 * (bv[ch] + cv[ch]);
-            }
+            for (int r = 0; r < 3; r++)
+                v[r] = ch == 0 ? (int)(short)f.v[r][k].x : (ch == 2 ? (int)f.v[r][k].x >> 16 : (int)(short)f.v[r][k].y);
+            e[k] = v[0] + 6 * v[1] + v[2];
+            o[k] = v[1] + v[2];
         }
+        n[0][ch] += ((e[0] + 6 * e[1] + e[2] + 32) >> 6) - kCBias;
+        n[1][ch] += ((e[1] + e[2] + 8) >> 4) - kCBias;
+        n[2][ch] += ((o[0] + 6 * o[1] + o[2] + 8) >> 4) - kCBias;
+        n[3][ch] += ((o[1] + o[2] + 2) >> 2) - kCBias;
+    }
+}
+
+// The block's collapsed level (j >= 1) from its four pixels' words.
+__device__ __forceinline__ void storeC(const UnitGeo& G, int x, int y, const uint2* v)
+{
+    const long long cext = (long long)G.pitch * G.h * 8;
 #pragma unroll
-        for (int ch = 0; ch < 3; ch++) {
-            n[0][ch] += (e[0][ch] + 6 * e[1][ch] + e[2][ch] + 32) >> 6;
-            n[1][ch] += (4 * (e[1][ch] + e[2][ch]) + 32) >> 6;
-            n[2][ch] += (o[0][ch] + 6 * o[1][ch] + o[2][ch] + 32) >> 6;
-            n[3][ch] += (4 * (o[1][ch] + o[2][ch]) + 32) >> 6;
+    for (int r = 0; r < 2; r++) {
+        if (y + r >= G.h) break;
+        uint2* Cj = reinterpret_cast<uint2*>(G.C) + (size_t)(y + r) * G.pitch + x;
+        if (x + 1 < G.w) {
+            if (inside(reinterpret_cast<uint4*>(Cj), G.C, cext))
+                *reinterpret_cast<uint4*>(Cj) = make_uint4(v[2 * r].x, v[2 * r].y, v[2 * r + 1].x, v[2 * r + 1].y);
+        } else if (x < G.w && inside(Cj, G.C, cext)) {
+            Cj[0] = v[2 * r];
         }
     }
-    if (j > 0) {
-        const long long cext = (long long)G.pitch * G.h * 8;
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            if (y + r >= G.h) break;
-            short4* Cj = G.C + (size_t)(y + r) * G.pitch + x;
-            const int* a = n[2 * r];
-            const int* b = n[2 * r + 1];
-            if (x + 1 < G.w) {
-                if (inside(reinterpret_cast<int4*>(Cj), G.C, cext))
-                    *reinterpret_cast<int4*>(Cj) =
-                        make_int4((int)((uint32_t)(uint16_t)a[0] | ((uint32_t)(uint16_t)a[1] << 16)),
-                                  (int)(uint32_t)(uint16_t)a[2],
-                                  (int)((uint32_t)(uint16_t)b[0] | ((uint32_t)(uint16_t)b[1] << 16)),
-                                  (int)(uint32_t)(uint16_t)b[2]);
-            } else if (x < G.w && inside(Cj, G.C, cext)) {
-                Cj[0] = make_short4((short)a[0], (short)a[1], (short)a[2], 0);
-            }
-        }
-        return;
-    }
-    // level 0 (the render's canvas is even in both directions, the blender's need not be)
-    if (y >= G.h || x >= G.w) return;
+}
+
+// The block's output pixels (level 0), o[2 * row + column] = B | G << 8 | R << 16;
+// the render's canvas is even in both directions, the blender's need not be.
+__device__ __forceinline__ void storeOut(const UnitGeo& G, int x, int y, const uint32_t* o)
+{
     const int rows = y + 1 < G.h ? 2 : 1, cols = x + 1 < G.w ? 2 : 1;
-    uint32_t o[4] = {0, 0, 0, 0};
-    if (cls != 0) {
-#pragma unroll
-        for (int p = 0; p < 4; p++)
-            o[p] = packSatBgr(n[p][0], n[p][1], n[p][2]);
-        if (cls == 2) {
-            const long long uext = (long long)G.pitch * G.h;
-            for (int r = 0; r < rows; r++) {
-                const uint8_t* um = G.um + (size_t)(y + r) * G.pitch + x;
-                if (!(inside(um, G.um, uext) ? um[0] : 0)) o[2 * r] = 0;
-                if (cols == 2 && !(inside(um + 1, G.um, uext) ? um[1] : 0)) o[2 * r + 1] = 0;
-            }
-        }
-    }
     if (G.outFmt == PS_FMT_YUV420P || G.outFmt == PS_FMT_NV12) {  // even sizes only (checked at the API)
         storeYuv(G, x, y, o);
         return;
@@ -1582,6 +1518,172 @@ __device__ __forceinline__ void computeUnit(const Stage& S, const UnitGeo& G, co
     }
 }
 
+// The Laplacian L = G - U of one pixel, B and R in the two 16-bit lanes of one
+// word, each biased by 256 so that neither the lane sums nor the subtraction
+// carry or borrow across lanes (one PRMT puts a byte and the 1 of the bias into
+// a lane).
+__device__ __forceinline__ uint32_t biasedBR(uint32_t px) { return __byte_perm(px, 0x01010101u, 0x4240); }
+__device__ __forceinline__ uint32_t biasedG(uint32_t px) { return __byte_perm(px, 0x01010101u, 0x4341); }
+
+// Accumulate one unit from its stage; at a tile's last unit normalise,
+// collapse and store.  Threads 0..kConsumers-1.
+//
+// A uniform tile (one camera, weight 256 everywhere: 80% of level 0 of the
+// six-camera rig) is G - U + pyrUp(C) with both upsamples, the sum and the
+// saturation two channels per word: half the instructions of the general path,
+// which such a tile takes only where C leaves the packed range.
+template <class Stage>
+__device__ __forceinline__ void computeUnit(const Stage& S, const UnitGeo& G, const uint4& raw, int chunk, BlendAcc& acc)
+{
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int lx = 2 * lane, ly = 2 * wp;
+    const int j = raw.x & 0xFF, cls = (raw.x >> 8) & 0xFF, camCnt = (raw.x >> 16) & 0xFF;
+    const bool uni = ((raw.x >> 24) & kTileUniform) != 0;  // weights are not read
+    const int tx = raw.y & 0xFFFF, ty = raw.y >> 16;
+    const bool hasUp = G.hasUp != 0;
+    const int x = tx * kBlendTW + lx, y = ty * kBlendTH + ly;
+    const bool active = !(j == 0 && cls == 0);
+    constexpr int NC = Stage::kCams;
+    const int c0 = chunk * NC;
+    const int nc = max(0, min(NC, camCnt - c0));
+    const bool first = chunk == 0, last = chunk == unitChunks<NC>(raw) - 1;
+    if (uni && hasUp) {
+        const CFootprint cf = loadC(&S.cf[wp][1 + lane]);
+        if (__all_sync(0xffffffffu, cInRange(cf))) {
+            uint32_t ulo[4], uhi[4], clo[4], chi[4];
+            upsampleG(&S.fpw[0][wp * kFpW + 3 + lane], ulo, uhi);
+            upsampleC(cf, clo, chi);
+            const uint2 gt = *reinterpret_cast<const uint2*>(&S.gj[0][ly][lx]);
+            const uint2 gb = *reinterpret_cast<const uint2*>(&S.gj[0][ly + 1][lx]);
+            const uint32_t gp[4] = {gt.x, gt.y, gb.x, gb.y};
+            // lanes: (256 + G - U) + (256 + C), at least 1
+            uint32_t br[4], gg[4];
+#pragma unroll
+            for (int p = 0; p < 4; p++) {
+                br[p] = biasedBR(gp[p]) - ulo[p] + clo[p];
+                gg[p] = biasedG(gp[p]) - uhi[p] + chi[p];
+            }
+            if (j > 0) {
+                uint2 v[4];
+#pragma unroll
+                for (int p = 0; p < 4; p++)  // back to one bias, as signed lanes (the fourth channel 0)
+                    v[p] = make_uint2(__viaddmax_s16x2(br[p], 0xFF00FF00u, 0x80008000u),
+                                      __viaddmax_s16x2(gg[p], 0xFF00FF00u, 0x80008000u));
+                storeC(G, x, y, v);
+                return;
+            }
+            if (y >= G.h || x >= G.w) return;
+            uint32_t o[4];
+#pragma unroll
+            for (int p = 0; p < 4; p++)  // min(max(lane - 512, 0), 255)
+                o[p] = __viaddmin_s16x2_relu(br[p], 0xFE00FE00u, 0x00FF00FFu) +
+                       (__viaddmin_s16x2_relu(gg[p], 0xFE00FE00u, 0x00FF00FFu) << 8);
+            storeOut(G, x, y, o);
+            return;
+        }
+    }
+    if (first) {
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+            acc.r[p][0] = acc.r[p][1] = acc.r[p][2] = 0;
+            acc.wsum[p] = 0;
+        }
+    }
+    if (active) {
+        for (int q = 0; q < nc; q++) {
+            uint32_t ulo[4] = {0, 0, 0, 0}, uhi[4] = {0, 0, 0, 0};
+            if (hasUp) upsampleG(&S.fpw[q][wp * kFpW + 3 + lane], ulo, uhi);
+            const uint2 gt = *reinterpret_cast<const uint2*>(&S.gj[q][ly][lx]);
+            const uint2 gb = *reinterpret_cast<const uint2*>(&S.gj[q][ly + 1][lx]);
+            const uint32_t gp[4] = {gt.x, gt.y, gb.x, gb.y};
+            uint32_t wq[2] = {0x01000100u, 0x01000100u};
+            if (!uni) {
+                wq[0] = *reinterpret_cast<const uint32_t*>(&S.w[q][ly][lx]);
+                wq[1] = *reinterpret_cast<const uint32_t*>(&S.w[q][ly + 1][lx]);
+            }
+#pragma unroll
+            for (int p = 0; p < 4; p++) {
+                // w * (256 + L); the 256 * sum(w) comes off at normalisation
+                const uint32_t br = biasedBR(gp[p]) - ulo[p];
+                const int g = (int)(biasedG(gp[p]) & 0xFFFFu) - (int)uhi[p];
+                const int w = (int)((wq[p >> 1] >> (16 * (p & 1))) & 0xFFFFu);
+                acc.r[p][0] += w * (int)(br & 0xFFFFu);
+                acc.r[p][1] += w * g;
+                acc.r[p][2] += w * (int)(br >> 16);
+                acc.wsum[p] += w;
+            }
+        }
+    }
+    if (!last) return;
+    int n[4][3];
+#pragma unroll
+    for (int p = 0; p < 4; p++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) acc.r[p][c] -= acc.wsum[p] << 8;
+    if (G.full) {
+#pragma unroll
+        for (int p = 0; p < 4; p++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) n[p][c] = (acc.r[p][c] + 128) >> 8;
+    } else if (j == 0 && __all_sync(0xffffffffu, ((acc.wsum[0] | acc.wsum[1] | acc.wsum[2] | acc.wsum[3]) & ~256) == 0)) {
+        // Level-0 weights are the 0/256 seam masks.  Where each pixel's sum is 0 or 256 (one camera at
+        // most: always, unless custom masks overlap), R = 256 L exactly, and R / W truncated is the shift.
+#pragma unroll
+        for (int p = 0; p < 4; p++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) n[p][c] = acc.r[p][c] >> 8;
+    } else {
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+            const int d = acc.wsum[p] ? acc.wsum[p] : 1;
+            const float inv = __frcp_rn((float)d);
+#pragma unroll
+            for (int c = 0; c < 3; c++) n[p][c] = divTrunc(acc.r[p][c], d, inv);
+        }
+    }
+    // collapse: + pyrUp32(C_{j+1})
+    if (hasUp && active) addUpsampledC(loadC(&S.cf[wp][1 + lane]), n);
+    if (j > 0) {
+        uint2 v[4];
+#pragma unroll
+        for (int p = 0; p < 4; p++) v[p] = packC(n[p][0], n[p][1], n[p][2]);
+        storeC(G, x, y, v);
+        return;
+    }
+    if (y >= G.h || x >= G.w) return;
+    uint32_t o[4] = {0, 0, 0, 0};
+    if (cls != 0) {
+#pragma unroll
+        for (int p = 0; p < 4; p++)
+            o[p] = packSatBgr(n[p][0], n[p][1], n[p][2]);
+        if (cls == 2) {
+            const long long uext = (long long)G.pitch * G.h;
+            const int rows = y + 1 < G.h ? 2 : 1, cols = x + 1 < G.w ? 2 : 1;
+            for (int r = 0; r < rows; r++) {
+                const uint8_t* um = G.um + (size_t)(y + r) * G.pitch + x;
+                if (!(inside(um, G.um, uext) ? um[0] : 0)) o[2 * r] = 0;
+                if (cols == 2 && !(inside(um + 1, G.um, uext) ? um[1] : 0)) o[2 * r + 1] = 0;
+            }
+        }
+    }
+    storeOut(G, x, y, o);
+}
+
+// The Laplacian of one pixel in half tiles: U unrounded, scaled by 64.
+struct Lap {
+    uint32_t br;  // (256 + L_B) | (256 + L_R) << 16
+    int g;        // L_G
+};
+
+__device__ __forceinline__ Lap laplacian(uint32_t gpx, uint32_t ulo, uint32_t uhi)
+{
+    const uint32_t ubr = ((ulo + 0x00200020u) >> 6) & 0x03FF03FFu;  // round(U) of B and R, per lane
+    Lap l;
+    l.br = biasedBR(gpx) - ubr;
+    l.g = (int)__byte_perm(gpx, 0, 0x4441) - (int)(((uhi & 0xFFFFu) + 32u) >> 6);
+    return l;
+}
+
 // The tail kernel's variant for levels above 0: one 64x8 half of a tile
 // (rows 8*half ..), consumer thread t owning pixels (2*(t%32), t/32) and the
 // one to its right, so all eight warps share the few tiles of these levels.
@@ -1605,8 +1707,7 @@ __device__ __forceinline__ void computeUnitRows(const HalfStage& S, const UnitGe
     const bool hasUp = G.hasUp != 0;
     const int x = tx * kBlendTW + lx, y = ty * kBlendTH + kHalfRows * half + ly;
     constexpr int NC = HalfStage::kCams;
-    const int c0 = chunk * NC;
-    const int nc = max(0, min(NC, camCnt - c0));
+    const int nc = max(0, min(NC, camCnt - chunk * NC));
     const bool first = chunk == 0, last = chunk == unitChunks<NC>(raw) - 1;
     if (first) {
         acc.r0[0] = acc.r0[1] = acc.r0[2] = acc.r1[0] = acc.r1[1] = acc.r1[2] = 0;
@@ -1671,13 +1772,13 @@ __device__ __forceinline__ void computeUnitRows(const HalfStage& S, const UnitGe
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             const uint2 a = cf[vr0 * kCfW + fc + k], b = cf[(vr0 + 1) * kCfW + fc + k];
-            const int ax = (short)(a.x & 0xFFFF), ay = (short)(a.x >> 16), az = (short)(a.y & 0xFFFF);
-            const int bx = (short)(b.x & 0xFFFF), by = (short)(b.x >> 16), bz = (short)(b.y & 0xFFFF);
+            const int ax = (short)a.x, ay = (short)a.y, az = (int)a.x >> 16;  // B, G, R
+            const int bx = (short)b.x, by = (short)b.y, bz = (int)b.x >> 16;
             if (evenRow) {
                 const uint2 c = cf[(vr0 + 2) * kCfW + fc + k];
-                v[k][0] = ax + 6 * bx + (short)(c.x & 0xFFFF);
-                v[k][1] = ay + 6 * by + (short)(c.x >> 16);
-                v[k][2] = az + 6 * bz + (short)(c.y & 0xFFFF);
+                v[k][0] = ax + 6 * bx + (short)c.x;
+                v[k][1] = ay + 6 * by + (short)c.y;
+                v[k][2] = az + 6 * bz + ((int)c.x >> 16);
             } else {
                 v[k][0] = 4 * (ax + bx);
                 v[k][1] = 4 * (ay + by);
@@ -1686,22 +1787,19 @@ __device__ __forceinline__ void computeUnitRows(const HalfStage& S, const UnitGe
         }
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            n0[c] += (v[0][c] + 6 * v[1][c] + v[2][c] + 32) >> 6;
-            n1[c] += (4 * (v[1][c] + v[2][c]) + 32) >> 6;
+            n0[c] += ((v[0][c] + 6 * v[1][c] + v[2][c] + 32) >> 6) - kCBias;
+            n1[c] += ((4 * (v[1][c] + v[2][c]) + 32) >> 6) - kCBias;
         }
     }
     if (y >= G.h || j == 0) return;  // level 0 goes through computeUnit
-    short4* Cj = G.C + (size_t)y * G.pitch + x;
+    uint2* Cj = reinterpret_cast<uint2*>(G.C) + (size_t)y * G.pitch + x;
     const long long cext = (long long)G.pitch * G.h * 8;
+    const uint2 c0 = packC(n0[0], n0[1], n0[2]), c1 = packC(n1[0], n1[1], n1[2]);
     if (x + 1 < G.w) {
-        if (inside(reinterpret_cast<int4*>(Cj), G.C, cext))
-            *reinterpret_cast<int4*>(Cj) =
-                make_int4((int)((uint32_t)(uint16_t)n0[0] | ((uint32_t)(uint16_t)n0[1] << 16)),
-                          (int)(uint32_t)(uint16_t)n0[2],
-                          (int)((uint32_t)(uint16_t)n1[0] | ((uint32_t)(uint16_t)n1[1] << 16)),
-                          (int)(uint32_t)(uint16_t)n1[2]);
+        if (inside(reinterpret_cast<uint4*>(Cj), G.C, cext))
+            *reinterpret_cast<uint4*>(Cj) = make_uint4(c0.x, c0.y, c1.x, c1.y);
     } else if (x < G.w && inside(Cj, G.C, cext)) {
-        Cj[0] = make_short4((short)n0[0], (short)n0[1], (short)n0[2], 0);
+        Cj[0] = c0;
     }
 }
 
@@ -1734,7 +1832,10 @@ __global__ void __launch_bounds__(kBlendThreads, 4) k_blend(const Segment* __res
         mbarInit(&never, 1);
         s_timeout = 0;
     }
-    if (threadIdx.x < kBStages) info[threadIdx.x].valid = 0;  // a stage read after a wait ran out ends the loop
+    if (threadIdx.x < kBStages) {
+        info[threadIdx.x].valid = 0;  // a stage read after a wait ran out ends the loop
+        info[threadIdx.x].seg = -1;   // its geometry is not filled in
+    }
     __syncthreads();
     const int lane = threadIdx.x & 31;
 
@@ -1749,153 +1850,125 @@ __global__ void __launch_bounds__(kBlendThreads, 4) k_blend(const Segment* __res
         // G_{j+1} footprint, written by launches that have completed, are
         // copied (through L2, by the tensor copies) while it finishes.
         bool waited = false;
-        auto nextItem = [&] {
-            int v = 0;
-            if (lane == 0) v = atomicAdd(counter, 1);
-            return __shfl_sync(0xffffffffu, v, 0);
-        };
-        int it = nextItem(), chunk = 0, seg = 0;
+        // Tiles are taken in runs, a lane holding a tile's descriptor; the next
+        // run is fetched once the first unit of the one in use is on its way.
+        int seg = -1, chunk = 0;
         uint4 raw = make_uint4(0, 0, 0, 0);
-        bool valid = it < total;
-        if (valid) {
-            seg = findSegment(segs, nsegs, it, 0);
-            raw = __ldg(static_cast<const uint4*>(segs[seg].items) + (it - segs[seg].prefix));
-        }
+        bool valid = false;
+        uint4 laneRaw = raw, nextRaw = raw;
+        int laneSeg = 0, nextSeg = 0, len = 0, nextLen = 0, at = 0, pos = 0;
+        bool ahead = false;  // the next run is fetched
+        auto fetchRun = [&] {
+            const int want = max(1, min(kBlendRun, (total - pos) / (kBlendShare * (int)gridDim.x)));
+            int it = 0;
+            if (lane == 0) it = atomicAdd(counter, want);
+            it = pos = __shfl_sync(0xffffffffu, it, 0);
+            nextLen = max(0, min(want, total - it));
+            if (lane < nextLen) {
+                nextSeg = findSegment(segs, nsegs, it + lane, nextSeg);
+                nextRaw = __ldg(static_cast<const uint4*>(segs[nextSeg].items) + (it + lane - segs[nextSeg].prefix));
+            }
+            ahead = true;
+        };
+        // of the segment (one level of one rig)
+        int h = 0, uw = 0, uh = 0;
+        bool hasUp = false;
+        const uint8_t *tmJ = nullptr, *tmU = nullptr;  // tensor maps of the level and of the one above
+        const uint8_t* camLists = nullptr;
+        auto takeNext = [&] {
+            if (at == len) {
+                laneRaw = nextRaw;
+                laneSeg = nextSeg;
+                len = nextLen;
+                at = 0;
+                ahead = false;
+            }
+            valid = len > 0;
+            if (!valid) return;
+            raw.x = __shfl_sync(0xffffffffu, laneRaw.x, at);
+            raw.y = __shfl_sync(0xffffffffu, laneRaw.y, at);
+            raw.z = __shfl_sync(0xffffffffu, laneRaw.z, at);
+            raw.w = __shfl_sync(0xffffffffu, laneRaw.w, at);
+            const int s = __shfl_sync(0xffffffffu, laneSeg, at);
+            at++;
+            if (s != seg) {
+                seg = s;
+                const RigDev& R = *segs[seg].rig;
+                const int j = raw.x & 0xFF;
+                hasUp = j < R.L;
+                h = R.lv[j].h;
+                uw = R.lv[hasUp ? j + 1 : j].w;
+                uh = R.lv[hasUp ? j + 1 : j].h;
+                tmJ = R.tmaps ? static_cast<const uint8_t*>(R.tmaps) + (size_t)j * kTmapsPerLevel * 128 : nullptr;
+                tmU = tmJ + kTmapsPerLevel * 128;
+                camLists = R.camLists;
+            }
+        };
+        fetchRun();
+        takeNext();
         for (int u = 0;; u++) {
             const int stg = u % kBStages;
             if (u >= kBStages && !mbarWait(&empty[stg], ((u / kBStages) - 1) & 1)) s_timeout = 1;
-            UnitInfo ui;
-            ui.raw = raw;
-            ui.seg = seg;
-            ui.chunk = chunk;
-            ui.valid = valid;
-            ui.staged = 0;
-            int nc = 0, cb = 8, j = 0, tx = 0, ty = 0, nCopies = 0;
-            bool hasUp = false, last = false, uni = false;
-            const RigDev* R = nullptr;
-            if (valid) {
-                R = segs[seg].rig;
-                j = raw.x & 0xFF;
-                if (lane == 0) fillGeo(ui.geo, *R, *segs[seg].frame, j);
-                const int cls = (raw.x >> 8) & 0xFF, camCnt = (raw.x >> 16) & 0xFF;
-                uni = ((raw.x >> 24) & kTileUniform) != 0;
-                tx = raw.y & 0xFFFF;
-                ty = raw.y >> 16;
-                hasUp = j < R->L;
-                const LevelDev& Lj = R->lv[j];
-                const LevelDev& Lu = R->lv[hasUp ? j + 1 : j];
-                nc = max(0, min(kCamsPerUnit, camCnt - chunk * kCamsPerUnit));
-                last = chunk == unitChunks(raw) - 1;
-                const int fx0 = tx * (kBlendTW / 2) - 1, fy0 = ty * (kBlendTH / 2) - 1;
-                const bool rowsIn = (ty + 1) * kBlendTH <= Lj.h;
-                const bool fpIn = !hasUp || (fx0 - 3 >= 0 && fx0 - 3 + kFpW <= Lu.w && fy0 >= 0 && fy0 + kFH <= Lu.h);
-                const bool active = !(j == 0 && cls == 0);
-                if (active && rowsIn && fpIn && (nc > 0 || (hasUp && last))) {
-                    ui.staged = 1;
-                    cb = kBlendTH + (uni ? 0 : kBlendTH) + (hasUp ? kFH : 0);
-                    nCopies = nc * cb + (hasUp && last ? kFH : 0);
+            const int tx = raw.y & 0xFFFF, ty = raw.y >> 16;
+            const int fx0 = tx * (kBlendTW / 2) - 1, fy0 = ty * (kBlendTH / 2) - 1;
+            const int nc = max(0, min(kCamsPerUnit, (int)((raw.x >> 16) & 0xFF) - chunk * kCamsPerUnit));
+            const bool last = chunk == unitChunks(raw) - 1, uni = ((raw.x >> 24) & kTileUniform) != 0;
+            bool staged = false;  // by tensor copies; else the consumers stage the unit
+#ifndef PS_CHECK_BOUNDS
+            staged = valid && tmJ && !((raw.x & 0xFFFF) == 0) && (ty + 1) * kBlendTH <= h && (nc > 0 || (hasUp && last)) &&
+                     (!hasUp || (fx0 - 3 >= 0 && fx0 - 3 + kFpW <= uw && fy0 >= 0 && fy0 + kFH <= uh));
+#endif
+            fenceProxyAsync();
+            if (lane == 0) {
+                UnitInfo& I = info[stg];
+                I.raw = raw;
+                I.chunk = chunk;
+                I.valid = valid;
+                I.staged = staged;
+                if (valid && I.seg != seg) {
+                    I.seg = seg;
+                    fillGeo(I.geo, *segs[seg].rig, *segs[seg].frame, raw.x & 0xFF);
                 }
             }
-            fenceProxyAsync();
-            if (lane == 0) info[stg] = ui;
-            bool tma = false;
-#ifndef PS_CHECK_BOUNDS
-            tma = ui.staged && R->tmaps;
-#endif
-            if (!waited && !(early && tma)) {
+            if (!waited && !(early && staged)) {
                 waitPrevGrid();
                 allowNextGrid();
                 waited = true;
             }
-            if (ui.staged) {
-                const LevelDev& Lj = R->lv[j];
-                const LevelDev& Lu = R->lv[hasUp ? j + 1 : j];
+            if (staged) {
+                // one bulk tensor copy per camera and array: the G_j tile,
+                // its weights, its G_{j+1} footprint; then the C_{j+1} footprint
                 if (lane == 0) {
-                    const uint32_t bytes = nc * (kBlendTH * kBlendTW * 4 + (uni ? 0 : kBlendTH * kBlendTW * 2) +
-                                                 (hasUp ? kFH * kFpW * 4 : 0)) +
-                                           (hasUp && last ? kFH * kCfW * 8 : 0);
-                    mbarArriveExpectTx(&full[stg], bytes);
-                }
-                __syncwarp();
-                const int fx0 = tx * (kBlendTW / 2) - 1, fy0 = ty * (kBlendTH / 2) - 1;
-#ifndef PS_CHECK_BOUNDS
-                if (R->tmaps) {
-                    // one bulk tensor copy per camera and array: the G_j tile,
-                    // its weights, its G_{j+1} footprint; then the C_{j+1} footprint
-                    if (lane == 0) {
-                        const uint8_t* tm = static_cast<const uint8_t*>(R->tmaps);
-                        const uint8_t* tmJ = tm + (size_t)j * kTmapsPerLevel * 128;
-                        const uint8_t* tmU = tm + (size_t)(j + 1) * kTmapsPerLevel * 128;
-                        for (int q = 0; q < nc; q++) {
-                            const int cam = tileCam(raw, R->camLists, chunk * kCamsPerUnit + q);
-                            tmaLoad3d(&st[stg].gj[q][0][0], tmJ + kTmG * 128, tx * kBlendTW, ty * kBlendTH, cam,
-                                      &full[stg]);
-                            if (!uni)
-                                tmaLoad3d(&st[stg].w[q][0][0], tmJ + kTmW * 128, tx * kBlendTW, ty * kBlendTH, cam,
-                                          &full[stg]);
-                            if (hasUp) tmaLoad3d(&st[stg].fpw[q][0], tmU + kTmGfp * 128, fx0 - 3, fy0, cam, &full[stg]);
-                        }
-                    }
-                    if (!waited) {  // C_{j+1} is the previous launch's output
-                        __syncwarp();
-                        waitPrevGrid();
-                        allowNextGrid();
-                        waited = true;
-                    }
-                    if (lane == 0 && hasUp && last) {
-                        const uint8_t* tmU = static_cast<const uint8_t*>(R->tmaps) + (size_t)(j + 1) * kTmapsPerLevel * 128;
-                        tmaLoad2d(&st[stg].cf[0][0], tmU + kTmC * 128, fx0 - 1, fy0, &full[stg]);
-                    }
-                    nCopies = 0;
-                }
-#endif
-                for (int k = lane; k < nCopies; k += 32) {
-                    if (k < nc * cb) {
-                        const int q = k / cb;
-                        int r = k - q * cb;
-                        const int cam = tileCam(raw, R->camLists, chunk * kCamsPerUnit + q);
-                        if (r < kBlendTH) {
-                            bulkCopyChecked(&st[stg].gj[q][r][0],
-                                            Lj.G + (size_t)cam * Lj.camStride + (size_t)(ty * kBlendTH + r) * Lj.pitch +
-                                                tx * kBlendTW,
-                                            kBlendTW * 4, &full[stg], Lj.G, gBytes(*R, Lj));
-                            continue;
-                        }
-                        r -= kBlendTH;
-                        if (!uni) {
-                            if (r < kBlendTH) {
-                                bulkCopyChecked(&st[stg].w[q][r][0],
-                                                Lj.Wt + (size_t)cam * Lj.camStride +
-                                                    (size_t)(ty * kBlendTH + r) * Lj.pitch + tx * kBlendTW,
-                                                kBlendTW * 2, &full[stg], Lj.Wt, wBytes(*R, Lj));
-                                continue;
-                            }
-                            r -= kBlendTH;
-                        }
-                        bulkCopyChecked(&st[stg].fpw[q][r * kFpW],
-                                        Lu.G + (size_t)cam * Lu.camStride + (size_t)(fy0 + r) * Lu.pitch + (fx0 - 3),
-                                        kFpW * 4, &full[stg], Lu.G, gBytes(*R, Lu));
-                    } else {
-                        const int r = k - nc * cb;
-                        bulkCopyChecked(&st[stg].cf[r][0], Lu.C + (size_t)(fy0 + r) * Lu.pitch + (fx0 - 1), kCfW * 8,
-                                        &full[stg], Lu.C, cBytes(Lu));
+                    mbarArriveExpectTx(&full[stg], nc * (kBlendTH * kBlendTW * 4 + (uni ? 0 : kBlendTH * kBlendTW * 2) +
+                                                         (hasUp ? kFH * kFpW * 4 : 0)) +
+                                                       (hasUp && last ? kFH * kCfW * 8 : 0));
+                    for (int q = 0; q < nc; q++) {
+                        const int cam = tileCam(raw, camLists, chunk * kCamsPerUnit + q);
+                        tmaLoad3d(&st[stg].gj[q][0][0], tmJ + kTmG * 128, tx * kBlendTW, ty * kBlendTH, cam, &full[stg]);
+                        if (!uni)
+                            tmaLoad3d(&st[stg].w[q][0][0], tmJ + kTmW * 128, tx * kBlendTW, ty * kBlendTH, cam, &full[stg]);
+                        if (hasUp) tmaLoad3d(&st[stg].fpw[q][0], tmU + kTmGfp * 128, fx0 - 3, fy0, cam, &full[stg]);
                     }
                 }
+                if (!waited) {  // C_{j+1} is the previous launch's output
+                    __syncwarp();
+                    waitPrevGrid();
+                    allowNextGrid();
+                    waited = true;
+                }
+                if (lane == 0 && hasUp && last) tmaLoad2d(&st[stg].cf[0][0], tmU + kTmC * 128, fx0 - 1, fy0, &full[stg]);
             } else if (lane == 0) {
                 mbarArrive(&full[stg]);
             }
             if (!valid) break;  // the terminal unit is out
+            if (!ahead) fetchRun();
             if (chunk + 1 < unitChunks(raw)) {
                 chunk++;
             } else {
                 chunk = 0;
-                it = nextItem();
-                valid = it < total;
-                if (valid) {
-                    seg = findSegment(segs, nsegs, it, seg);
-                    raw = __ldg(static_cast<const uint4*>(segs[seg].items) + (it - segs[seg].prefix));
-                }
+                takeNext();
             }
+            __syncwarp();
         }
         return;
     }
@@ -1919,7 +1992,7 @@ __global__ void __launch_bounds__(kBlendThreads, 4) k_blend(const Segment* __res
                                    [] { namedBarrier(1, kConsumers); });
             namedBarrier(1, kConsumers);
         }
-        computeUnit(st[stg], ui.geo, raw, chunk, staged, acc);
+        computeUnit(st[stg], ui.geo, raw, chunk, acc);
         if (active && !staged) fenceProxyAsync();  // our stage writes precede later bulk copies into it
         __syncwarp();
         if (lane == 0) mbarArrive(&empty[stg]);  // this warp is done with the stage
@@ -2034,7 +2107,7 @@ __global__ void __launch_bounds__(kThreads) k_tail(const Segment* __restrict__ s
                     __syncthreads();
                     if (active) stageUnitDirect<true>(st.whole, R, raw, chunk, sm.fRow, sm.fCol, [] { __syncthreads(); });
                     __syncthreads();
-                    computeUnit(st.whole, geo, raw, chunk, false, acc);
+                    computeUnit(st.whole, geo, raw, chunk, acc);
                 }
             }
         }

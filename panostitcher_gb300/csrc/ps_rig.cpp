@@ -1130,6 +1130,14 @@ void Rig::exportCollapsed(int level, int16_t* host, long long bytes, cudaStream_
     PS_CUDA(cudaMemcpy2DAsync(host, (size_t)g.w * 8, lv_[level].C[lastSlot_].get(), (size_t)g.pitch * 8, (size_t)g.w * 8, g.h,
                               cudaMemcpyDeviceToHost, st));
     PS_CUDA(cudaStreamSynchronize(st));
+    // the kernels keep B, R, G, 0, the first three biased (packC)
+    for (size_t i = 0; i < (size_t)g.w * g.h; i++) {
+        int16_t* p = host + 4 * i;
+        const int16_t b = p[0], r = p[1], gr = p[2];
+        p[0] = (int16_t)(b - kCBias);
+        p[1] = (int16_t)(gr - kCBias);
+        p[2] = (int16_t)(r - kCBias);
+    }
 }
 
 double Rig::stepBytes(int kind, int level) const
