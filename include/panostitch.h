@@ -338,7 +338,8 @@ typedef struct ps_launch_shape {
                              one-wave grids; 0 = as many as fit (default 0) */
     int small_blend_max_items; /* blend levels above 0 (below the tail) with at
                              most this many tiles run as 64x8 half tiles, up to
-                             eight cameras staged at once; 0 = none (default 0) */
+                             eight cameras staged at once; 0 = the library's
+                             choice, 128 (default 0) */
     int remap_defer_ties; /* 0 or 1, kept for its callers: the remap recomputes
                              near-tie pixels itself after each run of tiles,
                              with either value (default 1) */

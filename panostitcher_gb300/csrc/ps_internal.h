@@ -169,7 +169,14 @@ struct LaunchShape {
     int tailCluster = 0;           // CTAs per rig in the tail kernel: 8, 16, or 0 = the widest co-schedulable
     int tailHalf = 1;              // the tail blends levels above 0 in 64x8 half tiles
     int ctasPerSm[3] = {0, 0, 0};  // k_remap, k_pyrdown, k_blend; 0 = as many as fit
-    int smallBlendMaxItems = 0;    // blend levels above 0 with at most this many tiles run in k_blend_small
+    int smallBlendMaxItems = 0;    // blend levels above 0 with at most this many tiles run in k_blend_small (0: kSmallBlendTiles)
+    // Where k_blend_small takes over from k_blend by default: with 128 tiles
+    // (two CTAs each) a level is one short wave, and each level of 8 to 128
+    // tiles is 2 - 4 us shorter (6 x 1920x1080 to 4096x2048: 189 against 183 us
+    // a frame); with 512 tiles k_blend's larger blocks win (190 us).  With
+    // eight frames in flight the two are equal (949 against 945 us for eight).
+    static constexpr int kSmallBlendTiles = 128;
+    int smallBlend() const { return smallBlendMaxItems > 0 ? smallBlendMaxItems : kSmallBlendTiles; }
     int remapDefer = 1;            // kept for its callers: both values run the same launch
     bool operator==(const LaunchShape& o) const
     {

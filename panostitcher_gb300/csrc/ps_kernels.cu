@@ -2125,7 +2125,7 @@ __global__ void __launch_bounds__(kThreads) k_tail(const Segment* __restrict__ s
 // a chain of load-and-compute rounds that these levels cannot hide behind
 // other tiles; here each CTA has one short chain and all its warps busy.
 // ============================================================================
-__global__ void __launch_bounds__(kThreads) k_blend_small(const Segment* __restrict__ segs, int nsegs, int total,
+__global__ void __launch_bounds__(kThreads, 4) k_blend_small(const Segment* __restrict__ segs, int nsegs, int total,
                                                           int early)
 {
     __shared__ HalfStage st;

@@ -1407,7 +1407,7 @@ void Plan::bind(const std::vector<Rig*>& rigs)
             const int j = rigs[r]->tailBlend() - 1 - s;
             if (j < 0) continue;
             const int cnt = rigs[r]->numBlendItems(j);
-            if (j > 0 && cnt <= rigs[r]->shape().smallBlendMaxItems) small.push_back({r, {rigs[r]->blendItems(j), 2 * cnt}});
+            if (j > 0 && cnt <= rigs[r]->shape().smallBlend()) small.push_back({r, {rigs[r]->blendItems(j), 2 * cnt}});
             else parts.push_back({r, {rigs[r]->blendItems(j), cnt}});
         }
         const size_t before = steps_.size();

@@ -170,7 +170,7 @@ std::vector<LaunchShape> neighbours(const Rig& rig, const LaunchShape& cur, int 
             // k_blend_small (each knob alone can measure slower than the pair)
             int most = 0;
             for (int j = std::max(1, b); j < curBlend; j++) most = std::max(most, rig.numBlendItems(j));
-            if (most > cur.smallBlendMaxItems && most <= 512) {
+            if (most > cur.smallBlend() && most <= 512) {
                 s.smallBlendMaxItems = most;
                 out.push_back(s);
             }
@@ -197,8 +197,8 @@ std::vector<LaunchShape> neighbours(const Rig& rig, const LaunchShape& cur, int 
             for (int j = 1; j < curBlend; j++) c += rig.numBlendItems(j) <= v;
             return c;
         };
-        std::vector<int> seen{smallLevels(cur.smallBlendMaxItems)};
-        for (int v : {0, 32, 64, 128, 256, 512, 1024, 2048, 4096}) {
+        std::vector<int> seen{smallLevels(cur.smallBlend())};
+        for (int v : {1, 32, 64, 128, 256, 512, 1024, 2048, 4096}) {
             const int c = smallLevels(v);
             if (std::find(seen.begin(), seen.end(), c) != seen.end()) continue;
             seen.push_back(c);
@@ -277,7 +277,7 @@ LaunchShape autotune(Rig& rig, Plan& plan, int framesPerTrial, int inflight, boo
             std::vector<LaunchShape> seen{best};
             const int L = rig.numLevels();
             for (int tail : {0, 2, 16})
-                for (int small : {0, 32, 128})
+                for (int small : {0, 1, 32})
                     for (int ctas : {0, 1, 2}) {
                         LaunchShape s;
                         s.tailMaxItems = tail;
@@ -287,13 +287,13 @@ LaunchShape autotune(Rig& rig, Plan& plan, int framesPerTrial, int inflight, boo
                         int d = 0, b = 0;
                         rig.tailSplit(tail, &d, &b);
                         int smallLevels = 0;
-                        for (int j = 1; j < b && j <= L; j++) smallLevels += rig.numBlendItems(j) <= small;
+                        for (int j = 1; j < b && j <= L; j++) smallLevels += rig.numBlendItems(j) <= s.smallBlend();
                         bool dup = false;
                         for (const LaunchShape& o : seen) {
                             int od = 0, ob = 0;
                             rig.tailSplit(o.tailMaxItems, &od, &ob);
                             int os = 0;
-                            for (int j = 1; j < ob && j <= L; j++) os += rig.numBlendItems(j) <= o.smallBlendMaxItems;
+                            for (int j = 1; j < ob && j <= L; j++) os += rig.numBlendItems(j) <= o.smallBlend();
                             if (od == d && ob == b && os == smallLevels && o.ctasPerSm[2] == ctas) dup = true;
                         }
                         if (dup) continue;
