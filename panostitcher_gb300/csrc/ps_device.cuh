@@ -143,7 +143,6 @@ struct YuvFrame {
     uint8_t* dst;
     long long dstPitch;
     int fmt;
-    int vec;  // w % 8 == 0 and every plane aligned for 8-pixel-wide vector access
 };
 struct YuvFrames {
     YuvFrame frame[PS_MAX_CAMS];

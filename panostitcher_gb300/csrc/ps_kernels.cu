@@ -1028,6 +1028,7 @@ constexpr int kConsumers = kThreads;          // 8 warps
 // descriptor's load per tile held the consumers up (7680x3840 level 0: 94 us,
 // 84 with runs of 4); larger shares leave CTAs unequal at the end.
 constexpr int kBlendRun = 4, kBlendShare = 4;
+constexpr int kYuvThreads = 128;  // of the eight-pixel conversions
 constexpr int kBlendThreads = kConsumers + 32;  // + the producer warp
 
 // One unit's shared-memory stage: NC cameras of one tile (k_blend stages
@@ -2172,9 +2173,58 @@ __global__ void __launch_bounds__(kThreads, 4) k_blend_small(const Segment* __re
 
 // ============================================================================
 // k_cvt_yuv: standalone BGR32 -> YUV420P / NV12 of a device image
-// (cvtBGR32ToYUV420P / cvtBGR32ToNV12, ImageProc.cu:97-160).  One thread per
-// 2x2 block, consecutive threads on consecutive blocks of a block row.
+// (cvtBGR32ToYUV420P / cvtBGR32ToNV12, ImageProc.cu:97-160).  Where the image
+// and its planes allow 16- and 8-byte accesses (cvtVector), a thread converts
+// eight pixels of a row pair: four 16-byte loads, 8-byte luma stores, the four
+// blocks' chroma in one store (YUV420P: two of 4 bytes).  Otherwise one thread
+// per 2x2 block, byte by byte.  4096x2048 NV12: 14.4 us before (byte stores
+// for every image), 10.7 us now.
 // ============================================================================
+__device__ __forceinline__ uint32_t packBytes(uint32_t lo, uint32_t hi) { return lo | (hi << 16); }
+
+__global__ void __launch_bounds__(kYuvThreads) k_cvt_yuv8(const uint8_t* __restrict__ src, long long srcPitch, int w,
+                                                          int h, int fmt, uint8_t* __restrict__ py, long long yPitch,
+                                                          uint8_t* __restrict__ pu, long long uPitch,
+                                                          uint8_t* __restrict__ pv, long long vPitch)
+{
+    const int x = 8 * (blockIdx.x * kYuvThreads + threadIdx.x);
+    if (x >= w) return;
+    for (int by = blockIdx.y; by < h / 2; by += gridDim.y) {
+        uint4 q[2][2];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const uint4* p = reinterpret_cast<const uint4*>(src + (size_t)(2 * by + r) * srcPitch) + x / 4;
+            q[r][0] = __ldg(p);
+            q[r][1] = __ldg(p + 1);
+        }
+        uint32_t us = 0, vs = 0;
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const uint32_t* o = &q[r][0].x;
+            uint32_t y4[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) y4[k] = packSat2(yuvLumaRaw(o[2 * k]), yuvLumaRaw(o[2 * k + 1]));
+            *reinterpret_cast<uint2*>(py + (size_t)(2 * by + r) * yPitch + x) =
+                make_uint2(packBytes(y4[0], y4[1]), packBytes(y4[2], y4[3]));
+        }
+        uint32_t uv[4];  // U | V << 8 of the four blocks, from their left columns
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int2 c = yuvChromaSums((&q[0][0].x)[2 * k]), d = yuvChromaSums((&q[1][0].x)[2 * k]);
+            uv[k] = packSat2((c.x + d.x) >> (kYuvShift + 1), (c.y + d.y) >> (kYuvShift + 1));
+        }
+        if (fmt == PS_FMT_NV12) {
+            *reinterpret_cast<uint2*>(pu + (size_t)by * uPitch + x) =
+                make_uint2(packBytes(uv[0], uv[1]), packBytes(uv[2], uv[3]));
+        } else {
+            us = __byte_perm(packBytes(uv[0], uv[1]), packBytes(uv[2], uv[3]), 0x6420);
+            vs = __byte_perm(packBytes(uv[0], uv[1]), packBytes(uv[2], uv[3]), 0x7531);
+            *reinterpret_cast<uint32_t*>(pu + (size_t)by * uPitch + x / 2) = us;
+            *reinterpret_cast<uint32_t*>(pv + (size_t)by * vPitch + x / 2) = vs;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(kThreads) k_cvt_yuv(const uint8_t* __restrict__ src, long long srcPitch, int w,
                                                       int h, int fmt, uint8_t* __restrict__ py, long long yPitch,
                                                       uint8_t* __restrict__ pu, long long uPitch,
@@ -2228,7 +2278,6 @@ __device__ __forceinline__ uint32_t yuvPixel(int yv, int ruv, int guv, int buv)
 
 // Eight pixels of a row pair (four 2x2 blocks) per thread: 8-byte luma
 // loads, the blocks' chroma in one load, 16-byte stores.
-constexpr int kYuvChunks = 2;  // chunks a thread has in flight (4 measured slower)
 
 struct YuvChunk {
     uint2 yt, yb;     // luma of the top and bottom rows
@@ -2276,31 +2325,25 @@ __device__ __forceinline__ void yuvStore(const YuvFrame& F, int cx, int by, cons
     b[1] = make_uint4(ob[4], ob[5], ob[6], ob[7]);
 }
 
+// The frames the vector path takes (all of them, or none): a thread has one
+// chunk of eight pixels by two rows, blockIdx.y being the row pair and blockIdx.z
+// the frame, so that no index needs a division and every load is in flight at
+// once; two or four chunks a thread measured slower.  4096x2048 NV12: 13.8 us
+// before (a grid of one wave), 12.7 us now; 6 x 1920x1080 22.3 and 19.1 us.
+__global__ void __launch_bounds__(kYuvThreads, 8) k_yuv_to_bgr32_8(YuvFrames f)
+{
+    const int cx = blockIdx.x * kYuvThreads + threadIdx.x;
+    if (8 * cx >= f.w) return;
+    const YuvFrame& F = f.frame[blockIdx.z];
+    for (int by = blockIdx.y; by < f.h >> 1; by += gridDim.y) yuvStore(F, cx, by, yuvLoad(F, cx, by));
+}
+
 __global__ void __launch_bounds__(kThreads) k_yuv_to_bgr32(YuvFrames f)
 {
     const int cam = blockIdx.y;
     const int bw = f.w >> 1, bh = f.h >> 1;
     const YuvFrame& F = f.frame[cam];
     // the launcher takes frames below 2^32 pixels, so 32-bit indices cover the work
-    if (F.vec) {
-        // kYuvChunks chunks per step, all loaded before any is converted
-        const unsigned cw = (unsigned)f.w >> 3;
-        const unsigned chunks = cw * (unsigned)bh, stride = gridDim.x * blockDim.x;
-        for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < chunks; c += kYuvChunks * stride) {
-            YuvChunk v[kYuvChunks];
-#pragma unroll
-            for (int k = 0; k < kYuvChunks; k++) {
-                const unsigned ck = c + k * stride, by = ck / cw;
-                if (ck < chunks) v[k] = yuvLoad(F, (int)(ck - by * cw), (int)by);
-            }
-#pragma unroll
-            for (int k = 0; k < kYuvChunks; k++) {
-                const unsigned ck = c + k * stride, by = ck / cw;
-                if (ck < chunks) yuvStore(F, (int)(ck - by * cw), (int)by, v[k]);
-            }
-        }
-        return;
-    }
     const unsigned total = (unsigned)bw * (unsigned)bh;
     for (unsigned b = blockIdx.x * blockDim.x + threadIdx.x; b < total; b += gridDim.x * blockDim.x) {
         const int by = (int)(b / (unsigned)bw), bx = (int)(b - (unsigned)by * (unsigned)bw);
@@ -2528,11 +2571,24 @@ cudaError_t launchTail(const Segment* segs, int nsegs, int cluster, cudaStream_t
     return cudaLaunchKernelEx(&cfg, k_tail, segs, nsegs, cluster);
 }
 
+// A plane whose rows all start on a multiple of `to` bytes.
+static bool aligned(const void* p, long long pitch, int to)
+{
+    return reinterpret_cast<uintptr_t>(p) % to == 0 && pitch % to == 0;
+}
+
 cudaError_t launchCvtYuv(const uint8_t* src, long long srcPitch, int w, int h, int fmt, uint8_t* y, long long yPitch,
                          uint8_t* u, long long uPitch, uint8_t* v, long long vPitch, cudaStream_t st)
 {
     const long long blocks = (long long)(w / 2) * (h / 2);
     if (blocks <= 0) return cudaSuccess;
+    const bool nv12 = fmt == PS_FMT_NV12;
+    if (w % 8 == 0 && aligned(src, srcPitch, 16) && aligned(y, yPitch, 8) && aligned(u, uPitch, nv12 ? 8 : 4) &&
+        (nv12 || aligned(v, vPitch, 4))) {
+        const dim3 grid8((w / 8 + kYuvThreads - 1) / kYuvThreads, std::min(h / 2, 65535));
+        k_cvt_yuv8<<<grid8, kYuvThreads, 0, st>>>(src, srcPitch, w, h, fmt, y, yPitch, u, uPitch, v, vPitch);
+        return cudaGetLastError();
+    }
     const int grid = (int)std::min<long long>((blocks + kThreads - 1) / kThreads, (long long)smCount() * 8);
     k_cvt_yuv<<<grid, kThreads, 0, st>>>(src, srcPitch, w, h, fmt, y, yPitch, u, uPitch, v, vPitch);
     return cudaGetLastError();
@@ -2541,28 +2597,25 @@ cudaError_t launchCvtYuv(const uint8_t* src, long long srcPitch, int w, int h, i
 // Frames whose width and planes allow the 8-pixel path.
 static bool yuvVector(const YuvFrame& F, int w)
 {
-    auto al = [](const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; };
-    if (w % 8 || !al(F.y, 8) || F.yPitch % 8) return false;
-    if (F.fmt == PS_FMT_NV12) {
-        if (!al(F.u, 8) || F.uPitch % 8) return false;
-    } else if (!al(F.u, 4) || F.uPitch % 4 || !al(F.v, 4) || F.vPitch % 4) {
-        return false;
-    }
-    return al(F.dst, 16) && F.dstPitch % 16 == 0;
+    if (w % 8 || !aligned(F.y, F.yPitch, 8) || !aligned(F.dst, F.dstPitch, 16)) return false;
+    if (F.fmt == PS_FMT_NV12) return aligned(F.u, F.uPitch, 8);
+    return aligned(F.u, F.uPitch, 4) && aligned(F.v, F.vPitch, 4);
 }
 
 cudaError_t launchYuvToBgr32(const YuvFrames& frames, cudaStream_t st)
 {
-    if (frames.n <= 0 || frames.w <= 0 || frames.h <= 0) return cudaSuccess;
-    if ((long long)frames.w * frames.h >= (1LL << 32)) return cudaErrorInvalidValue;
-    YuvFrames f = frames;
-    for (int i = 0; i < f.n; i++) f.frame[i].vec = yuvVector(f.frame[i], f.w) ? 1 : 0;
-    // work items per frame: 2x2 blocks, or 8x2 chunks (kYuvChunks per thread) on the vector path
+    const YuvFrames& f = frames;
+    if (f.n <= 0 || f.w <= 0 || f.h <= 0) return cudaSuccess;
+    if ((long long)f.w * f.h >= (1LL << 32)) return cudaErrorInvalidValue;
     bool vec = true;
-    for (int i = 0; i < f.n; i++) vec = vec && f.frame[i].vec;
-    const long long items = vec ? ((long long)(f.w / 8) * (f.h / 2) + kYuvChunks - 1) / kYuvChunks
-                                : (long long)(f.w / 2) * (f.h / 2);
+    for (int i = 0; i < f.n; i++) vec = vec && yuvVector(f.frame[i], f.w);
+    if (vec) {
+        const dim3 grid((f.w / 8 + kYuvThreads - 1) / kYuvThreads, std::min(f.h / 2, 65535), f.n);
+        k_yuv_to_bgr32_8<<<grid, kYuvThreads, 0, st>>>(f);
+        return cudaGetLastError();
+    }
     // one wave of 8 CTAs per SM across all frames, or fewer CTAs if the work is smaller
+    const long long items = (long long)(f.w / 2) * (f.h / 2);
     const long long want = std::max<long long>(1, (long long)smCount() * 8 / f.n);
     const int gx = (int)std::min<long long>((items + kThreads - 1) / kThreads, want);
     k_yuv_to_bgr32<<<dim3(gx, f.n), kThreads, 0, st>>>(f);
