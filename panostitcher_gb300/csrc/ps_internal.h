@@ -153,10 +153,15 @@ cudaError_t launchCovTiles(const uint8_t* cov, int W, int H, long long maskStrid
 RemapParamF remapParamF(const RemapDev& r);
 cudaError_t launchCompactMaps(const float* xmap, const float* ymap, int W, int H, long long maskStride,
                               const RemapItem* items, int nitems, float2* maps, cudaStream_t st);
-// int16x4 / uint8x4 images -> uchar4 level 0, checking range and zero outside coverage
-cudaError_t launchImagesToLevel0(const void* const* images, const long long* pitches, int fmt, int n, int W,
-                                 int H, const uint8_t* cov, long long maskStride, uchar4* g0, int pitch,
-                                 long long camStride, int* status, cudaStream_t st);
+// int16x4 (fmt 16) / uint8x4 (8) images -> uchar4 level 0.  flags (two ints,
+// pinned host memory will do; only ever set): a value out of range, a pixel
+// that is not zero outside the coverage.
+struct ImageArgs {
+    const uint8_t* image[PS_MAX_CAMS];
+    long long pitch[PS_MAX_CAMS];
+};
+cudaError_t launchImagesToLevel0(const ImageArgs& args, int fmt, int n, int W, int H, const uint8_t* cov, uchar4* g0,
+                                 int pitch, long long camStride, int* flags, cudaStream_t st);
 
 // ---- launch shapes ----------------------------------------------------------------
 // The launch choices that can change after prepare.  Tile sizes are fixed

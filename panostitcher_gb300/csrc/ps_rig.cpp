@@ -126,7 +126,7 @@ void Rig::clear()
     nextSlot_ = lastSlot_ = 0;
     maps_.reset(); union_.reset(); inputs_.reset(); output_.reset(); covDev_.reset(); status_.reset(); planar_.reset();
     camsF_.reset(); covTiles_.reset();
-    imgArgs_.reset(); dDesc_.reset(); dRemap_.reset(); dDown_.reset(); dBlend_.reset(); dCams_.reset();
+    dDesc_.reset(); dRemap_.reset(); dDown_.reset(); dBlend_.reset(); dCams_.reset();
     tmaps_.reset();
     hRemap_.clear();
     hDown_.clear();
@@ -186,7 +186,7 @@ long long Rig::residentBytes() const
         b += l.Wt.bytes() + l.Am.bytes();
     }
     b += maps_.bytes() + union_.bytes() + inputs_.bytes() + output_.bytes() + covDev_.bytes() + status_.bytes();
-    b += imgArgs_.bytes() + dDesc_.bytes() + dRemap_.bytes() + dDown_.bytes() + dBlend_.bytes() + dCams_.bytes();
+    b += dDesc_.bytes() + dRemap_.bytes() + dDown_.bytes() + dBlend_.bytes() + dCams_.bytes();
     b += tmaps_.bytes();
     b += dLinear_.bytes() + linW_.bytes() + planar_.bytes() + camsF_.bytes() + covTiles_.bytes();
     return b;
@@ -405,7 +405,7 @@ void Rig::prepareFromMasks(const uint8_t* const* masks, const uint8_t* const* se
         // CudaMultibandBlend.cpp:570-571
         if (!seams) distanceSeams(covDev_.as<uint8_t>(), n, W, H, seam.as<uint8_t>(), st);
         output_.alloc(npx * 4 * slots_);
-        imgArgs_.alloc((sizeof(void*) + sizeof(long long)) * n);
+        if (!imgFlags_.bytes()) imgFlags_.alloc(2 * sizeof(int));
         preparePyramids(covDev_.as<uint8_t>(), seam.as<uint8_t>(), nullptr, nullptr, st);
         PS_CUDA(cudaStreamSynchronize(st));
     } catch (...) {
@@ -1023,22 +1023,22 @@ void Rig::zeroLevel0(int cam, int slot, cudaStream_t st)
 void Rig::toLevel0(const void* const* images, const long long* pitches, int fmt, int cam0, int count, int slot,
                    cudaStream_t st)
 {
-    const size_t n = count;
-    std::vector<uint8_t> args((sizeof(void*) + sizeof(long long)) * n);
-    std::memcpy(args.data(), images, sizeof(void*) * n);
-    std::memcpy(args.data() + sizeof(void*) * n, pitches, sizeof(long long) * n);
-    PS_CUDA(cudaMemcpyAsync(imgArgs_.get(), args.data(), args.size(), cudaMemcpyHostToDevice, st));
-    PS_CUDA(cudaMemsetAsync(status_.get(), 0, sizeof(int), st));
     const LevelGeom& g = geom_[0];
-    const size_t npx = (size_t)W_ * H_;
-    PS_CUDA(launchImagesToLevel0(imgArgs_.as<const void* const>(),
-                                 reinterpret_cast<const long long*>(imgArgs_.as<uint8_t>() + sizeof(void*) * n), fmt,
-                                 count, W_, H_, covDev_.as<uint8_t>() + cam0 * npx, (long long)npx,
+    ImageArgs args{};
+    for (int i = 0; i < count; i++) {
+        args.image[i] = static_cast<const uint8_t*>(images[i]);
+        args.pitch[i] = pitches[i];
+    }
+    // the kernel flags bad input in pinned host memory: nothing to clear or to
+    // read back on the stream
+    volatile int* flags = imgFlags_.as<int>();
+    flags[0] = flags[1] = 0;
+    PS_CUDA(launchImagesToLevel0(args, fmt, count, W_, H_, covDev_.as<uint8_t>() + cam0 * ((size_t)W_ * H_),
                                  lv_[0].G[slot].as<uchar4>() + (size_t)cam0 * g.pitch * g.h, g.pitch,
-                                 (long long)g.pitch * g.h, status_.as<int>(), st));
-    int status = 0;
-    PS_CUDA(cudaMemcpyAsync(&status, status_.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
+                                 (long long)g.pitch * g.h, imgFlags_.as<int>(), st));
     PS_CUDA(cudaStreamSynchronize(st));
+    const int status = (flags[0] ? 1 : 0) | (flags[1] ? 2 : 0);
+    if (status) PS_CUDA(cudaMemcpy(status_.get(), &status, sizeof status, cudaMemcpyHostToDevice));
     if (status & 1) fail(PS_EINVAL, "an int16 input value lies outside 0..255");
     if (status & 2) fail(PS_EINVAL, "an input image is non-zero where its coverage mask is zero");
 }

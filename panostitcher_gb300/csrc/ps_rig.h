@@ -204,7 +204,8 @@ private:
     uint64_t gen_ = 0;
     std::vector<LevelGeom> geom_;
     LevelBufs lv_[PS_MAX_LEVELS + 1];
-    DevBuf maps_, union_, inputs_, output_, covDev_, status_, imgArgs_, planar_;
+    DevBuf maps_, union_, inputs_, output_, covDev_, status_, planar_;
+    HostBuf imgFlags_;  // what k_images_to_level0 found wrong
     long long inPitch_ = 0, budget_ = 0;
     DevBuf dDesc_, dRemap_, dDown_, dBlend_, dCams_;
     DevBuf tmaps_;  // slots x (L + 1) x kTmapsPerLevel CUtensorMap
