@@ -302,7 +302,7 @@ int ps_render_export_collapsed(const ps_render* r, int level, int16_t* host_out,
    renders launch step by step with a CUDA event pair around every launch
    (no graph); ps_render_profile_read aggregates the finished launches of
    one kernel kind (0 remap, 1 pyrDown, 2 blend, 3 the tail kernel that runs
-   the few-tile top levels, reported at its lowest blend level, 4 the
+   the smallest levels, reported at its lowest, 4 the
    linear-blend render, 5 the conversion of decoder frames, at level 0, 6
    the blend of few-tile levels in half tiles, 7 nothing any more) at
    one level (-1 = all levels): launch count, summed device milliseconds
@@ -327,13 +327,15 @@ double ps_render_algorithmic_bytes(const ps_render* r, int bytes_in_per_px, int 
    (32x16 remap and pyrDown tiles, 64x16 blend tiles); every shape gives the
    same output bytes. */
 typedef struct ps_launch_shape {
-    int tail_max_items;   /* pyramid levels (from the top) with at most this many
-                             tiles run in the one-cluster tail kernel; 0 = no tail
+    int tail_max_items;   /* pyramid levels (from the top) of at most 32x16 pixels
+                             and this many tiles run in the one-cluster tail
+                             kernel (rigs of up to 16 cameras); 0 = no tail
                              (default 16) */
-    int tail_cluster;     /* CTAs per rig in the tail kernel: 8, 16, or 0 = the
-                             widest the GPU co-schedules (default 0) */
-    int tail_half_tiles;  /* 1: the tail blends levels above 0 in 64x8 half tiles,
-                             two pixels per thread; 0: whole tiles (default 1) */
+    int tail_cluster;     /* CTAs per rig in the tail kernel: 8, 16, or 0 = 8 for up
+                             to 8 cameras, else 16 (at most the widest the GPU
+                             co-schedules; default 0) */
+    int tail_half_tiles;  /* 0 or 1, kept for its callers: the tail has no tiles,
+                             with either value (default 1) */
     int ctas_per_sm[3];   /* CTAs per SM of the remap, pyrDown and blend kernels'
                              one-wave grids; 0 = as many as fit (default 0) */
     int small_blend_max_items; /* blend levels above 0 (below the tail) with at

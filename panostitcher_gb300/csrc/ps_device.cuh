@@ -31,6 +31,7 @@ constexpr int kRemapTW = 32, kRemapTH = 16;    // level-0 remap tile (two pixels
 constexpr int kDownTW = 32, kDownTH = 16;      // pyrDown output tile (two pixels per thread)
 constexpr int kBlendTW = 64, kBlendTH = 16;    // blend tile (a 2x2 pixel block per thread)
 constexpr int kThreads = 256;
+constexpr int kTailW = 32, kTailH = 16, kTailCams = 16;  // largest level and most cameras of k_tail
 constexpr int kCBias = 256;  // of the collapsed levels' values
 
 // Pixel i of a remap tile (its map, its linear weight): the tile is 16 blocks
@@ -103,15 +104,10 @@ struct RigDev {
     // NULL when they could not be encoded (k_blend then copies row by row)
     const void* tmaps;
     LevelDev lv[PS_MAX_LEVELS + 1];
-    // work items of every level (used by the tail kernel)
-    const DownItem* downItems;
-    const BlendItem* blendItems;
-    int downOff[PS_MAX_LEVELS + 1], downCnt[PS_MAX_LEVELS + 1];
-    int blendOff[PS_MAX_LEVELS + 1], blendCnt[PS_MAX_LEVELS + 1];
-    // the small top of the pyramid runs in one launch: pyrDown levels
-    // tailDown..L, then blend levels L..tailBlend (L + 1 = none); with
-    // tailHalf the blend levels above 0 go in 64x8 half tiles
-    int tailDown, tailBlend, tailHalf;
+    // the top of the pyramid in one launch (k_tail): pyrDown and blend levels
+    // tailStart..L (L + 1 = none), and of each the cameras with a pyrDown tile
+    int tailStart;
+    uint32_t tailCams[PS_MAX_LEVELS + 1];
     // linear-blend mode: the remap items (tile-major) and their weights,
     // 512 floats per item in the layout of the maps
     const RemapItem* remapItems;

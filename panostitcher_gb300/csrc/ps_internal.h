@@ -170,9 +170,9 @@ cudaError_t launchImagesToLevel0(const ImageArgs& args, int fmt, int n, int W, i
 // width and tile split, and the CTAs per SM of the persistent kernels.
 // Set by hand or chosen by the autotuner (ps_tune.cpp).
 struct LaunchShape {
-    int tailMaxItems = 16;         // levels with at most this many tiles run in the tail kernel (0: none)
-    int tailCluster = 0;           // CTAs per rig in the tail kernel: 8, 16, or 0 = the widest co-schedulable
-    int tailHalf = 1;              // the tail blends levels above 0 in 64x8 half tiles
+    int tailMaxItems = 16;         // levels with at most this many tiles may run in the tail kernel (0: none)
+    int tailCluster = 0;           // CTAs per rig in the tail kernel: 8, 16, or 0 = by the number of cameras
+    int tailHalf = 1;              // kept for its callers: both values run the same launches
     int ctasPerSm[3] = {0, 0, 0};  // k_remap, k_pyrdown, k_blend; 0 = as many as fit
     int smallBlendMaxItems = 0;    // blend levels above 0 with at most this many tiles run in k_blend_small (0: kSmallBlendTiles)
     // Where k_blend_small takes over from k_blend by default: with 128 tiles
@@ -219,10 +219,10 @@ cudaError_t launchBlend(const Segment* segs, int nsegs, int total, int perSm, in
                         bool early, cudaStream_t st);
 // blend of few-tile levels above 0: two work items (the 64x8 halves) per tile
 cudaError_t launchBlendSmall(const Segment* segs, int nsegs, int total, bool early, cudaStream_t st);
-// one cluster per segment: the rig's pyrDown levels tailDown..L and blend
-// levels L..tailBlend; cluster 8 or 16 CTAs (0 or more than the GPU
-// co-schedules: the widest it does)
-cudaError_t launchTail(const Segment* segs, int nsegs, int cluster, cudaStream_t st);
+// one cluster per segment: the rig's pyrDown levels tailStart..L and blend
+// levels L..tailStart; cams: the most cameras of any rig; cluster 8 or 16 CTAs
+// (0: by cams; at most the widest the GPU co-schedules)
+cudaError_t launchTail(const Segment* segs, int nsegs, int cluster, int cams, cudaStream_t st);
 // CTAs of k_remap (kind 0), k_pyrdown (1), k_blend (2) resident per SM;
 // the widest tail cluster the GPU co-schedules (8 or 16)
 int residentCtasPerSm(int kind);

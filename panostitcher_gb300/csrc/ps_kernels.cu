@@ -781,9 +781,9 @@ __device__ __forceinline__ void initMagic(uint32_t* magic)
     for (int m = threadIdx.x; m < 257; m += blockDim.x) magic[m] = m ? (uint32_t)((16777216u + m - 1) / m) : 0u;
 }
 
-// Loads of pyramid levels.  A level written earlier in the same launch (the
-// tail kernel's levels) is read through L2 (ld.global.cg); one written by an
-// earlier launch may use the read-only path.
+// Loads of pyramid levels.  What may have been written by a launch that ends
+// only while this one runs is read through L2 (ld.global.cg); the rest may use
+// the read-only path.
 template <bool kFresh, class T>
 __device__ __forceinline__ T ldLevel(const T* p)
 {
@@ -810,7 +810,6 @@ __device__ __forceinline__ bool downInterior(const RigDev& R, const DownItem& it
 // the first input column is even and rows are 256-byte aligned); tiles whose
 // input crosses the level's border map every row and column with the
 // reference's reflect-101 / wrap rules.
-template <bool kFresh>
 __device__ __forceinline__ void downLoad(const RigDev& R, const DownItem& item, DownRegs& g)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -833,10 +832,10 @@ __device__ __forceinline__ void downLoad(const RigDev& R, const DownItem& item, 
 #pragma unroll
         for (int r = 0; r < kDRows; r++, row += Ls.pitch) {
             const uint2* q = reinterpret_cast<const uint2*>(row) + lane;
-            const uint2 v = inside(q, Ls.G, ext) ? ldLevel<kFresh>(q) : make_uint2(0, 0);
+            const uint2 v = inside(q, Ls.G, ext) ? __ldg(q) : make_uint2(0, 0);
             g.a[r] = v.x;
             g.b[r] = v.y;
-            g.c[r] = extra && inside(row + 64 + lane, Ls.G, ext) ? ldLevel<kFresh>(row + 64 + lane) : 0u;
+            g.c[r] = extra && inside(row + 64 + lane, Ls.G, ext) ? __ldg(row + 64 + lane) : 0u;
         }
         return;
     }
@@ -845,9 +844,9 @@ __device__ __forceinline__ void downLoad(const RigDev& R, const DownItem& item, 
 #pragma unroll
     for (int r = 0; r < kDRows; r++) {
         const uint32_t* row = G + (size_t)rowMap(iy0 + r, Ls.h) * Ls.pitch;
-        g.a[r] = inside(row + c0, Ls.G, ext) ? ldLevel<kFresh>(row + c0) : 0u;
-        g.b[r] = inside(row + c1, Ls.G, ext) ? ldLevel<kFresh>(row + c1) : 0u;
-        g.c[r] = extra && inside(row + c2, Ls.G, ext) ? ldLevel<kFresh>(row + c2) : 0u;
+        g.a[r] = inside(row + c0, Ls.G, ext) ? __ldg(row + c0) : 0u;
+        g.b[r] = inside(row + c1, Ls.G, ext) ? __ldg(row + c1) : 0u;
+        g.c[r] = extra && inside(row + c2, Ls.G, ext) ? __ldg(row + c2) : 0u;
     }
 }
 
@@ -929,17 +928,6 @@ __device__ __forceinline__ void downHorizontal(const RigDev& R, const DownItem& 
     }
 }
 
-// One 32x16 output tile of one camera (all warps of the CTA; the magic table
-// is ready), without overlap (the tail kernel's few tiles).
-template <bool kFresh>
-__device__ __forceinline__ void pyrDownTile(const RigDev& R, const DownItem item, DownSmem& sm)
-{
-    DownRegs g;
-    downLoad<kFresh>(R, item, g);
-    downVertical(g, sm);
-    downHorizontal(R, item, g.m, sm);
-}
-
 // One CTA walks a contiguous run of tiles; the next tile's loads are issued
 // before the current tile's horizontal pass, so their latency overlaps it.
 __global__ void __launch_bounds__(kThreads, 5) k_pyrdown(const Segment* __restrict__ segs, int nsegs, int total)
@@ -962,7 +950,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_pyrdown(const Segment* __restri
     if (begin >= end) return;
     __syncthreads();  // the magic table
     DownRegs g;
-    downLoad<false>(*R, item, g);
+    downLoad(*R, item, g);
     for (int it = begin; it < end; it++) {
         const bool more = it + 1 < end;
         int sn = s;
@@ -973,7 +961,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_pyrdown(const Segment* __restri
         }
         downVertical(g, sm);
         const uint32_t m = g.m;
-        if (more) downLoad<false>(*segs[sn].rig, next, g);
+        if (more) downLoad(*segs[sn].rig, next, g);
         downHorizontal(*R, item, m, sm);
         s = sn;
         R = segs[s].rig;
@@ -1054,7 +1042,6 @@ static_assert(offsetof(BlendStage, w) % 128 == 0 && offsetof(BlendStage, fpw) % 
               "every bulk tensor copy destination starts on a 128-byte boundary");
 constexpr int kHalfRows = kBlendTH / 2;
 using HalfStage = BlendStageT<8, kHalfRows>;  // half tiles of the few-tile levels
-using WholeStage = BlendStageT<4>;            // whole tiles in the tail kernel
 
 // What the consumers need of a unit besides its stage: the level geometry
 // and the frame's output, resolved once per unit (in k_blend by the
@@ -1204,11 +1191,10 @@ struct BlendAcc {
     int wsum[4];
 };
 
-// Stage one unit with index-mapped loads (border tiles; every tile of the
-// tail kernel).  Threads 0..kConsumers-1; the caller synchronises.
+// Stage one unit with index-mapped loads (border tiles).  Threads 0..kConsumers-1; the caller synchronises.
 // fRow / fCol: footprint index tables (kFH / kFW ints) filled here; sync is
 // the barrier over the calling threads.
-template <bool kFresh, class Stage, class Sync>
+template <class Stage, class Sync>
 __device__ __forceinline__ void stageUnitDirect(Stage& S, const RigDev& R, const uint4& raw, int chunk, int* fRow,
                                                 int* fCol, Sync sync)
 {
@@ -1233,7 +1219,7 @@ __device__ __forceinline__ void stageUnitDirect(Stage& S, const RigDev& R, const
                 const size_t o = (size_t)cam * Lj.camStride + (size_t)(y + r) * Lj.pitch + x;
                 const uint2* gp = reinterpret_cast<const uint2*>(Lj.G + o);
                 const uint32_t* wp = reinterpret_cast<const uint32_t*>(Lj.Wt + o);
-                if (inside(gp, Lj.G, gBytes(R, Lj))) g = ldLevel<kFresh>(gp);
+                if (inside(gp, Lj.G, gBytes(R, Lj))) g = __ldg(gp);
                 if (inside(wp, Lj.Wt, wBytes(R, Lj))) w = __ldg(wp);
             }
             *reinterpret_cast<uint2*>(&S.gj[q][ly + r][lx]) = g;
@@ -1251,13 +1237,13 @@ __device__ __forceinline__ void stageUnitDirect(Stage& S, const RigDev& R, const
             const int cam = tileCam(raw, R.camLists, c0 + q);
             const uint32_t* gp = reinterpret_cast<const uint32_t*>(Lu.G) + (size_t)cam * Lu.camStride +
                                  (size_t)fRow[r] * Lu.pitch + fCol[c];
-            S.fpw[q][r * kFpW + c + 3] = inside(gp, Lu.G, gBytes(R, Lu)) ? ldLevel<kFresh>(gp) : 0u;
+            S.fpw[q][r * kFpW + c + 3] = inside(gp, Lu.G, gBytes(R, Lu)) ? __ldg(gp) : 0u;
         }
         if (last)
             for (int k = threadIdx.x; k < elems; k += kConsumers) {
                 const int r = k / kFW, c = k % kFW;
                 const uint2* cp = reinterpret_cast<const uint2*>(Lu.C + (size_t)fRow[r] * Lu.pitch + fCol[c]);
-                S.cf[r][c + 1] = inside(cp, Lu.C, cBytes(Lu)) ? ldLevel<kFresh>(cp) : make_uint2(0, 0);
+                S.cf[r][c + 1] = inside(cp, Lu.C, cBytes(Lu)) ? __ldg(cp) : make_uint2(0, 0);
             }
     }
 }
@@ -1685,7 +1671,7 @@ __device__ __forceinline__ Lap laplacian(uint32_t gpx, uint32_t ulo, uint32_t uh
     return l;
 }
 
-// The tail kernel's variant for levels above 0: one 64x8 half of a tile
+// k_blend_small's variant, for levels above 0: one 64x8 half of a tile
 // (rows 8*half ..), consumer thread t owning pixels (2*(t%32), t/32) and the
 // one to its right, so all eight warps share the few tiles of these levels.
 // Same arithmetic as computeUnit; output is the collapsed level C_j.
@@ -1989,7 +1975,7 @@ __global__ void __launch_bounds__(kBlendThreads, 4) k_blend(const Segment* __res
         const bool staged = ui.staged != 0;
         const bool active = !((raw.x & 0xFF) == 0 && ((raw.x >> 8) & 0xFF) == 0);
         if (active && !staged) {
-            stageUnitDirect<false>(st[stg], *segs[ui.seg].rig, raw, chunk, fRow, fCol,
+            stageUnitDirect(st[stg], *segs[ui.seg].rig, raw, chunk, fRow, fCol,
                                    [] { namedBarrier(1, kConsumers); });
             namedBarrier(1, kConsumers);
         }
@@ -2008,114 +1994,289 @@ __global__ void __launch_bounds__(kBlendThreads, 4) k_blend(const Segment* __res
 }
 
 // ============================================================================
-// k_tail: the small top of the pyramid of each rig in one launch.  A cluster
-// of 16 CTAs (8 where 16 cannot be co-scheduled) owns one rig: it runs pyrDown levels tailDown..L and
-// then blend levels L..tailBlend, spreading each level's tiles over its
-// CTAs, with a cluster barrier (release / acquire, so the level's global
-// writes are visible to the whole cluster) between levels.  These levels
-// hold few tiles, so separate launches would cost mostly launch latency.
-// A level is a chain of latencies: its data from L2 (0.7 us), the arithmetic
-// (1 - 2 us, two warps a scheduler), the barrier (0.5 us of release, 0.4 us of
-// wait).  Descriptors and first items wait in shared memory, a level's G part
-// is staged during the barrier above it, no division maps an index.  Seven
-// levels of 6 x 1920x1080 to 4096x2048 take 25 us, 46 us before that; the nine
-// of a 256x128 canvas 24 us, 36 us before.
+// k_tail: the levels of at most 32x16 pixels (one pyrDown tile a camera, one
+// blend tile) of rigs of up to 16 cameras in one launch.  A launch a level is
+// 3 us of release, loads and stores around some hundred nanoseconds of
+// arithmetic.  Here a cluster owns a rig.  The levels' pyrDown needs no other
+// camera, so a CTA takes a camera (two in small clusters) down all of them in
+// its own shared memory and pushes every level into that of the cluster's last
+// CTA, which blends them all from there: between two levels lie a CTA's barrier
+// and a few shared loads, and one cluster barrier is left.  What does not
+// depend on the frame (alpha divisors, weights, index maps with the reference's
+// borders) is fetched while the launch before finishes.  The levels' buffers in
+// memory are written as everywhere, for the levels below and the state export.
+// A tail that also took the levels of up to 16 tiles, each spread over 16 CTAs
+// with a cluster barrier between levels, cost as much as a launch a level did.
+// Five levels of 6 x 1920x1080 to 4096x2048: 6.4 us from its release, and a
+// frame of 172.5 us (177.5 with a launch a level, 183.8 with that wider tail);
+// 256x128: 33.7 us a frame against 40.6 and 42.4.
 // ============================================================================
 constexpr int kTailCluster = 8;       // portable cluster size
-constexpr int kTailClusterWide = 16;  // used when the GPU can co-schedule it
+constexpr int kTailClusterWide = 16;  // used for more cameras where the GPU can co-schedule it
+constexpr int kTailThreads = 512;     // a pixel of the largest level each
+// of all levels of a plane: 512 + 128 + 32 + 8 + 2 + 1 + 1 ...
+constexpr int kTailPx = 704;
+static_assert(kTailThreads == kTailW * kTailH && kTailW == 32 && kTailH == 16, "tailLevel and tailPixel");
+static_assert(PS_MAX_LEVELS <= 24, "levels of one pixel fit behind the others");
 
 __device__ __forceinline__ void clusterArrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void clusterWait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// The address of a shared variable of this CTA in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t clusterAddr(const void* p, int rank)
+{
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void clusterStore(uint32_t addr, uint32_t v)
+{
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void clusterStore(uint32_t addr, uint16_t v)
+{
+    asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
+}
 
-// The rig's descriptor and the CTA's first item of every level are copied to
-// shared memory while the launch before finishes, so that a level's chain is
-// one round trip to L2 (its data), the arithmetic, the stores and the barrier.
 struct TailSmem {
     RigDev rig;
-    DownItem down[PS_MAX_LEVELS + 1];
-    uint4 blend[PS_MAX_LEVELS + 1];
-    int fRow[kFH], fCol[kFW];
-    union Stage {
-        DownSmem down;
-        HalfStage half[2];
-        WholeStage whole;
-    };
-    alignas(128) unsigned char stage[sizeof(Stage)];
+    alignas(16) uint32_t in[2 * kTailH][2 * kTailW];  // the camera's level above the first
+    uint32_t plane[kTailPx];              // the camera's levels
+    uint16_t am[kTailPx];                 // their alpha divisors
+    uint32_t magic[257];
+    // the pixels that the borders' rules give a filter's columns and rows:
+    // pyrDown column 2X - 2 + i at [2X + i], upsample column x / 2 - 1 + i at
+    // [x / 2 + i], rows the same
+    uint8_t downCol[PS_MAX_LEVELS + 1][72], downRow[PS_MAX_LEVELS + 1][40];
+    uint8_t upCol[PS_MAX_LEVELS + 1][20], upRow[PS_MAX_LEVELS + 1][12];
+    uint2 c[kTailPx];  // the collapsed levels (the last CTA's)
+    // behind it in the last CTA: every camera's levels, then their weights
 };
-static_assert(sizeof(RigDev) % 4 == 0 && sizeof(DownItem) % 4 == 0 && sizeof(BlendItem) == 16, "copied word by word");
+constexpr int kTailTables = 72 + 40 + 20 + 12;
+size_t tailSmemBytes(int cams) { return sizeof(TailSmem) + (size_t)cams * kTailPx * 6; }
 
-__global__ void __launch_bounds__(kThreads) k_tail(const Segment* __restrict__ segs, int nsegs, int cluster)
+// Level k of the tail in a plane of kTailPx pixels: its row pitch is the least
+// power of two that fits any such level, its place what lies before it.
+struct TailLevel {
+    int shift, rows, off;
+};
+__device__ __forceinline__ TailLevel tailLevel(int k)
 {
-    extern __shared__ __align__(128) uint8_t tailSmem[];  // a TailSmem (dynamic: above the 48 KB static limit)
-    TailSmem& sm = *reinterpret_cast<TailSmem*>(tailSmem);
-    TailSmem::Stage& st = *reinterpret_cast<TailSmem::Stage*>(sm.stage);
-    const int rig = blockIdx.x / cluster, rank = blockIdx.x % cluster;
-    const Segment& sg = segs[min(rig, nsegs - 1)];  // the grid is nsegs clusters
-    const RigDev& R = sm.rig;
-    for (int k = threadIdx.x; k < (int)sizeof(RigDev) / 4; k += kThreads)
-        reinterpret_cast<uint32_t*>(&sm.rig)[k] = __ldg(reinterpret_cast<const uint32_t*>(sg.rig) + k);
-    initMagic(st.down.magic);
-    __syncthreads();
-    // blend levels above 0 (with tailHalf) go as half tiles with two pixels
-    // per thread, so the few tiles of these levels keep twice the CTAs and all
-    // warps busy; otherwise whole tiles, 2x2 blocks
-    auto parts = [&](int j) { return j > 0 && R.tailHalf ? 2 : 1; };
-    if (threadIdx.x <= R.L) {
-        const int j = threadIdx.x;
-        if (j >= R.tailDown && rank < R.downCnt[j]) sm.down[j] = R.downItems[R.downOff[j] + rank];
-        if (j >= R.tailBlend && rank < parts(j) * R.blendCnt[j])
-            sm.blend[j] = *reinterpret_cast<const uint4*>(R.blendItems + R.blendOff[j] + rank / parts(j));
+    if (k < 5) return {5 - k, max(1, kTailH >> k), (2048 - (2048 >> 2 * k)) / 3};
+    return {0, 1, 682 + k - 5};
+}
+// Pixel i of a plane; false where no level has it.
+__device__ __forceinline__ bool tailPixel(const RigDev& R, int i, int& j, int& x, int& y)
+{
+    const int k = i < 512 ? 0 : (i < 640 ? 1 : (i < 672 ? 2 : (i < 680 ? 3 : (i < 682 ? 4 : i - 677))));
+    const TailLevel t = tailLevel(k);
+    j = R.tailStart + k;
+    x = (i - t.off) & ((1 << t.shift) - 1);
+    y = (i - t.off) >> t.shift;
+    return j <= R.L && x < R.lv[j].w && y < R.lv[j].h;
+}
+
+// The alpha divisors or the weights of a camera, a value at a time through f(pixel, value).
+template <class F>
+__device__ __forceinline__ void tailConstants(const RigDev& R, bool weights, int cam, F f)
+{
+    uint16_t v[2];
+    bool ok[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const int i = threadIdx.x + q * kTailThreads;
+        int j, x, y;
+        ok[q] = i < kTailPx && tailPixel(R, i, j, x, y);
+        if (!ok[q]) continue;
+        const LevelDev& lv = R.lv[j];
+        const uint16_t* base = weights ? lv.Wt : lv.Am;
+        v[q] = ldChecked(base + cam * lv.camStride + (size_t)y * lv.pitch + x, base, wBytes(R, lv));
     }
-    __syncthreads();
-    waitPrevGrid();
-    allowNextGrid();
-    for (int J = R.tailDown; J <= R.L; J++) {
-        for (int k = rank; k < R.downCnt[J]; k += cluster)
-            pyrDownTile<true>(R, k == rank ? sm.down[J] : R.downItems[R.downOff[J] + k], st.down);
-        clusterArrive();
-        clusterWait();
-    }
-    BlendAcc acc;
-    PairAcc pacc;
-    // With half tiles, the level's first unit is staged but for its C_{j+1}
-    // footprint while the CTA waits for the level above (two buffers in turn).
-    auto stageAhead = [&](int j) {
-        if (j >= R.tailBlend && parts(j) == 2 && rank < 2 * R.blendCnt[j])
-            stageHalfG<true>(st.half[j & 1], R, sm.blend[j], 0, rank & 1);
-    };
-    __syncthreads();  // the stages overlay the pyrDown's shared memory
-    stageAhead(R.L);
-    for (int j = R.L; j >= R.tailBlend; j--) {
-        const BlendItem* items = R.blendItems + R.blendOff[j];
-        UnitGeo geo;
-        fillGeo(geo, R, *sg.frame, j);
-        for (int k = rank; k < parts(j) * R.blendCnt[j]; k += cluster) {
-            const uint4 raw = k == rank ? sm.blend[j] : *reinterpret_cast<const uint4*>(items + k / parts(j));
-            if (parts(j) == 2) {
-                HalfStage& h = st.half[j & 1];
-                for (int chunk = 0; chunk < unitChunks<HalfStage::kCams>(raw); chunk++) {
-                    if (k != rank || chunk > 0) {
-                        __syncthreads();  // readers of the previous unit are done
-                        stageHalfG<true>(h, R, raw, chunk, k & 1);
-                    }
-                    stageHalfC<true>(h, R, raw, chunk, k & 1);
-                    __syncthreads();
-                    computeUnitRows(h, geo, raw, chunk, pacc, k & 1);
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+        if (ok[q]) f((int)threadIdx.x + q * kTailThreads, v[q]);
+}
+
+// A camera through its pyrDown levels; to: its levels in the last CTA.
+__device__ __forceinline__ void tailDown(TailSmem& S, int cam, uint32_t to)
+{
+    const RigDev& R = S.rig;
+    const uint32_t* src = &S.in[0][0];
+    int pitch = 2 * kTailW;
+    for (int j = R.tailStart; j <= R.L; j++) {
+        __syncthreads();
+        const TailLevel t = tailLevel(j - R.tailStart);
+        const LevelDev& Ld = R.lv[j];
+        const int p = threadIdx.x, X = p & ((1 << t.shift) - 1), Y = p >> t.shift;
+        if (p < t.rows << t.shift && X < Ld.w && Y < Ld.h) {
+            uint32_t v = 0;
+            if (R.tailCams[j] >> cam & 1) {
+                const uint8_t *cols = &S.downCol[j][2 * X], *rows = &S.downRow[j][2 * Y];
+                int col[5];
+                uint32_t lo[5], hi[5];
+#pragma unroll
+                for (int i = 0; i < 5; i++) col[i] = cols[i];
+#pragma unroll
+                for (int r = 0; r < 5; r++) {
+                    const uint32_t* row = src + rows[r] * pitch;
+                    uint2 u[5];
+#pragma unroll
+                    for (int i = 0; i < 5; i++) u[i] = unpackBytes(row[col[i]]);
+                    lo[r] = k5(u[0].x, u[1].x, u[2].x, u[3].x, u[4].x);
+                    hi[r] = k5(u[0].y, u[1].y, u[2].y, u[3].y, u[4].y);
                 }
-            } else {
-                const bool active = !(j == 0 && ((raw.x >> 8) & 0xFF) == 0);
-                for (int chunk = 0; chunk < unitChunks<WholeStage::kCams>(raw); chunk++) {
-                    __syncthreads();
-                    if (active) stageUnitDirect<true>(st.whole, R, raw, chunk, sm.fRow, sm.fCol, [] { __syncthreads(); });
-                    __syncthreads();
-                    computeUnit(st.whole, geo, raw, chunk, acc);
+                v = downDivide(k5(lo[0], lo[1], lo[2], lo[3], lo[4]), k5(hi[0], hi[1], hi[2], hi[3], hi[4]),
+                               S.am[t.off + p], S.magic);
+                uint32_t* d = reinterpret_cast<uint32_t*>(Ld.G) + cam * Ld.camStride + (size_t)Y * Ld.pitch + X;
+                if (inside(d, Ld.G, gBytes(R, Ld))) *d = v;
+            }
+            S.plane[t.off + p] = v;
+            clusterStore(to + 4 * (t.off + p), v);
+        }
+        src = S.plane + t.off;
+        pitch = 1 << t.shift;
+    }
+}
+
+// Blend levels L .. tailStart from the shared memory of this CTA: the cameras'
+// levels g and weights w.  A level of few pixels has its cameras spread over
+// lanes of a pixel.
+__device__ __forceinline__ void tailBlend(TailSmem& S, const uint32_t* g, const uint16_t* w)
+{
+    const RigDev& R = S.rig;
+    const int most = R.n <= 1 ? 1 : 1 << (32 - __clz(R.n - 1));  // lanes with a camera of their own
+    for (int j = R.L; j >= R.tailStart; j--) {
+        const TailLevel t = tailLevel(j - R.tailStart), tu = tailLevel(j - R.tailStart + 1);
+        const LevelDev& Lj = R.lv[j];
+        const bool hasUp = j < R.L;
+        const int slots = t.rows << t.shift;
+        const int lanes = min(most, kTailThreads / slots);
+        const int p = threadIdx.x / lanes, sub = threadIdx.x & (lanes - 1);
+        if (((int)threadIdx.x & ~31) < slots * lanes) {  // whole warps
+            const int x = p & ((1 << t.shift) - 1), y = p >> t.shift;
+            const bool in = p < slots && x < Lj.w && y < Lj.h;
+            int at[3][3], wt[3][3];
+            if (in && hasUp) {
+                const int wx[3] = {x & 1 ? 0 : 1, x & 1 ? 4 : 6, x & 1 ? 4 : 1};
+                const int wy[3] = {y & 1 ? 0 : 1, y & 1 ? 4 : 6, y & 1 ? 4 : 1};
+#pragma unroll
+                for (int r = 0; r < 3; r++) {
+                    const int row = tu.off + (S.upRow[j][(y >> 1) + r] << tu.shift);
+#pragma unroll
+                    for (int i = 0; i < 3; i++) {
+                        at[r][i] = row + S.upCol[j][(x >> 1) + i];
+                        wt[r][i] = wy[r] * wx[i];
+                    }
                 }
             }
+            int acc[4] = {0, 0, 0, 0};  // weighted B, G, R and the weights
+            for (int cam = sub; in && cam < R.n; cam += lanes) {
+                const int wq = w[cam * kTailPx + t.off + p];
+                if (!wq) continue;
+                const uint32_t* gc = g + cam * kTailPx;
+                uint32_t lo = 0, hi = 0;
+                if (hasUp) {
+#pragma unroll
+                    for (int r = 0; r < 3; r++)
+#pragma unroll
+                        for (int i = 0; i < 3; i++) {
+                            const uint2 u = unpackBytes(gc[at[r][i]]);
+                            lo += wt[r][i] * u.x;
+                            hi += wt[r][i] * u.y;
+                        }
+                }
+                const Lap l = laplacian(gc[t.off + p], lo, hi);
+                acc[0] += wq * ((int)(l.br & 0xFFFFu) - 256);
+                acc[1] += wq * l.g;
+                acc[2] += wq * ((int)(l.br >> 16) - 256);
+                acc[3] += wq;
+            }
+            for (int o = lanes / 2; o > 0; o >>= 1)
+#pragma unroll
+                for (int c = 0; c < 4; c++) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+            if (in && !sub) {
+                int n[3];
+                const int d = acc[3] ? acc[3] : 1;
+                const float rcp = __frcp_rn((float)d);
+#pragma unroll
+                for (int c = 0; c < 3; c++) n[c] = R.full ? (acc[c] + 128) >> 8 : divTrunc(acc[c], d, rcp);
+                if (hasUp) {
+                    int v[3] = {32, 32, 32};
+#pragma unroll
+                    for (int r = 0; r < 3; r++)
+#pragma unroll
+                        for (int i = 0; i < 3; i++) {
+                            const uint2 q = S.c[at[r][i]];
+                            v[0] += wt[r][i] * (short)q.x;
+                            v[1] += wt[r][i] * (short)q.y;
+                            v[2] += wt[r][i] * ((int)q.x >> 16);
+                        }
+#pragma unroll
+                    for (int c = 0; c < 3; c++) n[c] += (v[c] >> 6) - kCBias;
+                }
+                const uint2 out = packC(n[0], n[1], n[2]);
+                S.c[t.off + p] = out;
+                uint2* q = reinterpret_cast<uint2*>(Lj.C) + (size_t)y * Lj.pitch + x;
+                if (inside(q, Lj.C, cBytes(Lj))) *q = out;
+            }
         }
-        clusterArrive();
-        stageAhead(j - 1);
-        clusterWait();
+        __syncthreads();
     }
+}
+
+// cluster CTAs a segment; cams: the most cameras of any
+__global__ void __launch_bounds__(kTailThreads) k_tail(const Segment* __restrict__ segs, int cluster, int cams)
+{
+    extern __shared__ __align__(128) uint8_t tailSmem[];
+    TailSmem& S = *reinterpret_cast<TailSmem*>(tailSmem);
+    uint32_t* g = reinterpret_cast<uint32_t*>(tailSmem + sizeof(TailSmem));
+    uint16_t* w = reinterpret_cast<uint16_t*>(g + cams * kTailPx);
+    const int rank = blockIdx.x % cluster, last = cluster - 1;
+    clusterArrive();  // every CTA has started before any writes another's shared memory
+    const uint32_t* desc = reinterpret_cast<const uint32_t*>(segs[blockIdx.x / cluster].rig);
+    for (int k = threadIdx.x; k < (int)sizeof(RigDev) / 4; k += kTailThreads)
+        reinterpret_cast<uint32_t*>(&S.rig)[k] = __ldg(desc + k);
+    initMagic(S.magic);
+    __syncthreads();
+    const RigDev& R = S.rig;
+    const int T = R.tailStart;
+    if (rank < R.n) tailConstants(R, false, rank, [&](int i, uint16_t v) { S.am[i] = v; });
+    for (int k = threadIdx.x; k < (R.L - T + 1) * kTailTables; k += kTailThreads) {
+        const int j = T + k / kTailTables, e = k % kTailTables;
+        const LevelDev &Ls = R.lv[j - 1], &Ld = R.lv[j], &Lu = R.lv[min(j + 1, R.L)];
+        if (e < 72) {
+            if (e < 2 * Ld.w + 3) S.downCol[j][e] = (uint8_t)colMap(e - 2, Ls.w);
+        } else if (e < 112) {
+            if (e - 72 < 2 * Ld.h + 3) S.downRow[j][e - 72] = (uint8_t)rowMap(e - 74, Ls.h);
+        } else if (e < 132) {
+            if (e - 112 < Ld.w / 2 + 3) S.upCol[j][e - 112] = (uint8_t)colMap(e - 113, Lu.w);
+        } else if (e - 132 < Ld.h / 2 + 3) {
+            S.upRow[j][e - 132] = (uint8_t)rowMap(e - 133, Lu.h);
+        }
+    }
+    clusterWait();
+    for (int cam = rank; cam < R.n; cam += cluster) {
+        const uint32_t to = clusterAddr(w + cam * kTailPx, last);
+        tailConstants(R, true, cam, [&](int i, uint16_t v) { clusterStore(to + 2 * i, v); });
+    }
+    waitPrevGrid();
+    allowNextGrid();
+    const LevelDev& Li = R.lv[T - 1];
+    for (int cam = rank; cam < R.n; cam += cluster) {
+        if (cam != rank) {
+            __syncthreads();  // readers of the camera before are done
+            tailConstants(R, false, cam, [&](int i, uint16_t v) { S.am[i] = v; });
+        }
+        // at most 64x32; its rows are 64 pixels at least
+        const int x = threadIdx.x % (kTailW / 2) * 4, y = threadIdx.x / (kTailW / 2);
+        if (y < Li.h) {
+            const uint4* p = reinterpret_cast<const uint4*>(Li.G + cam * Li.camStride + (size_t)y * Li.pitch + x);
+            *reinterpret_cast<uint4*>(&S.in[y][x]) = inside(p, Li.G, gBytes(R, Li)) ? __ldg(p) : make_uint4(0, 0, 0, 0);
+        }
+        tailDown(S, cam, clusterAddr(g + cam * kTailPx, last));
+    }
+    clusterArrive();
+    clusterWait();
+    if (rank == last) tailBlend(S, g, w);
 }
 
 // ============================================================================
@@ -2525,12 +2686,13 @@ int tailClusterMax()
 {
     static const int widest = [] {  // the attributes are set before any launch can see the width
         int size = kTailCluster;
-        cudaFuncSetAttribute(k_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TailSmem));
+        const int smem = (int)tailSmemBytes(kTailCams);
+        cudaFuncSetAttribute(k_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (cudaFuncSetAttribute(k_tail, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(kTailClusterWide);
-            cfg.blockDim = dim3(kThreads);
-            cfg.dynamicSmemBytes = sizeof(TailSmem);
+            cfg.blockDim = dim3(kTailThreads);
+            cfg.dynamicSmemBytes = smem;
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = kTailClusterWide;
@@ -2548,16 +2710,16 @@ int tailClusterMax()
     return widest;
 }
 
-cudaError_t launchTail(const Segment* segs, int nsegs, int cluster, cudaStream_t st)
+cudaError_t launchTail(const Segment* segs, int nsegs, int cluster, int cams, cudaStream_t st)
 {
     if (nsegs <= 0) return cudaSuccess;
     const int widest = tailClusterMax();
-    if (cluster <= 0 || cluster > widest) cluster = widest;
-    else cluster = cluster >= kTailClusterWide ? kTailClusterWide : kTailCluster;
+    if (cluster <= 0) cluster = cams <= kTailCluster ? kTailCluster : kTailClusterWide;
+    cluster = std::min(cluster >= kTailClusterWide ? kTailClusterWide : kTailCluster, widest);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nsegs * cluster);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = sizeof(TailSmem);
+    cfg.blockDim = dim3(kTailThreads);
+    cfg.dynamicSmemBytes = tailSmemBytes(cams);
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -2568,7 +2730,7 @@ cudaError_t launchTail(const Segment* segs, int nsegs, int cluster, cudaStream_t
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, k_tail, segs, nsegs, cluster);
+    return cudaLaunchKernelEx(&cfg, k_tail, segs, cluster, cams);
 }
 
 // A plane whose rows all start on a multiple of `to` bytes.

@@ -132,7 +132,7 @@ void Rig::clear()
     hDown_.clear();
     hBlend_.clear();
     hCams_.clear();
-    tailDown_ = tailBlend_ = 1;
+    tailStart_ = 1;
     for (int j = 0; j <= PS_MAX_LEVELS; j++) downOff_[j] = downCnt_[j] = blendOff_[j] = blendCnt_[j] = 0;
     covCount_ = weightCount_ = alphaCount_ = 0;
     covBits_.clear();
@@ -539,8 +539,8 @@ void Rig::preparePyramids(const uint8_t* cov, const uint8_t* seam, const float* 
     hDown_ = down;
     // the weights' part: union coverage, fullMask, blend items
     buildBlendState(cov, false, st);
-    // levels with few tiles (from the top down) go to the tail kernel
-    tailSplit(shape_.tailMaxItems, &tailDown_, &tailBlend_);
+    // the smallest levels go to the tail kernel
+    tailStart_ = tailStart(shape_.tailMaxItems);
     dRemap_.alloc(std::max<size_t>(1, hRemap_.size()) * sizeof(RemapItem));
     dDown_.alloc(std::max<size_t>(1, down.size()) * sizeof(DownItem));
     if (!hRemap_.empty())
@@ -582,17 +582,9 @@ void Rig::preparePyramids(const uint8_t* cov, const uint8_t* seam, const float* 
     d.covTiles = covTiles_.as<uint32_t>();
     d.unionMask = union_.as<uint8_t>();
     d.camLists = dCams_.as<uint8_t>();
-    d.downItems = dDown_.as<DownItem>();
-    d.blendItems = dBlend_.as<BlendItem>();
-    for (int j = 0; j <= L; j++) {
-        d.downOff[j] = downOff_[j];
-        d.downCnt[j] = downCnt_[j];
-        d.blendOff[j] = blendOff_[j];
-        d.blendCnt[j] = blendCnt_[j];
-    }
-    d.tailDown = tailDown_;
-    d.tailBlend = tailBlend_;
-    d.tailHalf = shape_.tailHalf;
+    d.tailStart = tailStart_;
+    if (n <= kTailCams)
+        for (const DownItem& it : hDown_) d.tailCams[it.level] |= 1u << it.cam;
     for (int j = 0; j <= L; j++) {
         const LevelGeom& g = geom_[j];
         d.lv[j].w = g.w;
@@ -749,16 +741,10 @@ void Rig::setCustomMasks(const uint8_t* const* masks, cudaStream_t st)
     }
     buildBlendState(masks ? wm.as<uint8_t>() : um.as<uint8_t>(), masks != nullptr, st);
     custom_ = masks != nullptr;
-    tailSplit(shape_.tailMaxItems, &tailDown_, &tailBlend_);
+    tailStart_ = tailStart(shape_.tailMaxItems);
     hDesc_.full = full_;
     hDesc_.camLists = dCams_.as<uint8_t>();
-    hDesc_.blendItems = dBlend_.as<BlendItem>();
-    for (int j = 0; j <= L; j++) {
-        hDesc_.blendOff[j] = blendOff_[j];
-        hDesc_.blendCnt[j] = blendCnt_[j];
-    }
-    hDesc_.tailDown = tailDown_;
-    hDesc_.tailBlend = tailBlend_;
+    hDesc_.tailStart = tailStart_;
     writeDescriptors(st);  // synchronises
     gen_ = g_generation++;
 }
@@ -875,13 +861,14 @@ void Rig::waitIdleQuiet() noexcept
             if (es[k] && cudaEventSynchronize(es[k]) != cudaSuccess) cudaGetLastError();
 }
 
-void Rig::tailSplit(int maxItems, int* down, int* blend) const
+int Rig::tailStart(int maxItems) const
 {
-    int d = L_ + 1, b = L_ + 1;
-    while (d > 1 && downCnt_[d - 1] <= maxItems) d--;
-    while (b > 0 && blendCnt_[b - 1] <= maxItems) b--;
-    *down = d;
-    *blend = b;
+    int j = L_ + 1;
+    if (n_ <= kTailCams)
+        while (j > 1 && geom_[j - 1].w <= kTailW && geom_[j - 1].h <= kTailH && downCnt_[j - 1] <= maxItems &&
+               blendCnt_[j - 1] <= maxItems)
+            j--;
+    return j;
 }
 
 void Rig::setShape(const LaunchShape& s)
@@ -903,10 +890,8 @@ void Rig::setShape(const LaunchShape& s)
     // the descriptors change under no run: launch lists follow the new
     // generation (plans rebind), and no kernel may read the old split
     waitIdle();
-    tailSplit(shape_.tailMaxItems, &tailDown_, &tailBlend_);
-    hDesc_.tailDown = tailDown_;
-    hDesc_.tailBlend = tailBlend_;
-    hDesc_.tailHalf = shape_.tailHalf;
+    tailStart_ = tailStart(shape_.tailMaxItems);
+    hDesc_.tailStart = tailStart_;
     writeDescriptors(nullptr);
     gen_ = g_generation++;
 }
@@ -989,7 +974,7 @@ void Rig::prepareLinear(const uint8_t* cov, const uint8_t* seam, const float* xm
     d.remapItems = dRemap_.as<RemapItem>();
     d.numRemapItems = (int)hRemap_.size();
     d.linWeights = linW_.as<float>();
-    d.tailDown = d.tailBlend = 1;
+    d.tailStart = 1;
     d.lv[0].w = W;
     d.lv[0].h = H;
     d.lv[0].pitch = geom_[0].pitch;
@@ -998,7 +983,7 @@ void Rig::prepareLinear(const uint8_t* cov, const uint8_t* seam, const float* xm
     dDesc_.alloc(sizeof(RigDev) * slots_);
     PS_CUDA(cudaMemcpyAsync(dDesc_.get(), ds, sizeof(RigDev) * slots_, cudaMemcpyHostToDevice, st));
     PS_CUDA(cudaStreamSynchronize(st));
-    tailDown_ = tailBlend_ = 1;  // no pyramid
+    tailStart_ = 1;  // no pyramid
     gen_ = g_generation++;
 }
 
@@ -1156,8 +1141,7 @@ double Rig::stepBytes(int kind, int level) const
         return b + (double)W_ * H_ * 4;
     }
     if (kind == 3) {
-        for (int J = tailDown_; J <= L_; J++) b += stepBytes(1, J);
-        for (int j = tailBlend_; j <= L_; j++) b += stepBytes(2, j);
+        for (int j = tailStart_; j <= L_; j++) b += stepBytes(1, j) + stepBytes(2, j);
         return b;
     }
     if (kind == 0) {
@@ -1344,6 +1328,9 @@ void Plan::bind(const std::vector<Rig*>& rigs)
         return v < 0 ? 0 : v;
     };
     tailCluster_ = widest([](const LaunchShape& s) { return s.tailCluster; });
+    tailCams_ = 0;
+    for (Rig* r : rigs)
+        if (!r->linear() && r->hasTail()) tailCams_ = std::max(tailCams_, r->numImages());
     for (int k = 0; k < 3; k++) perSm_[k] = widest([k](const LaunchShape& s) { return s.ctasPerSm[k]; });
     maps_ = true;
     for (Rig* r : rigs) maps_ = maps_ && !r->mapFree();
@@ -1359,7 +1346,7 @@ void Plan::bind(const std::vector<Rig*>& rigs)
                              reinterpret_cast<const FrameDev*>(sizeof(FrameDev) * p.first), p.second.second, s.total});
             s.total += p.second.second;
             const Rig* rg = rigs[p.first];
-            const int lvl = kind == 0 || kind == 4 ? 0 : (kind == 1 ? step : rg->tailBlend() - 1 - step);
+            const int lvl = kind == 0 || kind == 4 ? 0 : (kind == 1 ? step : rg->tailStart() - 1 - step);
             if (s.level < 0) s.level = lvl;
             s.bytes += rg->stepBytes(kind == 6 ? 2 : kind, lvl);
         }
@@ -1377,7 +1364,7 @@ void Plan::bind(const std::vector<Rig*>& rigs)
     for (int J = 1; J <= maxL; J++) {
         parts.clear();
         for (int r = 0; r < nr; r++)
-            if (J < rigs[r]->tailDown()) parts.push_back({r, {rigs[r]->downItems(J), rigs[r]->numDownItems(J)}});
+            if (J < rigs[r]->tailStart()) parts.push_back({r, {rigs[r]->downItems(J), rigs[r]->numDownItems(J)}});
         addStep(1, parts, J);
     }
     {
@@ -1389,7 +1376,7 @@ void Plan::bind(const std::vector<Rig*>& rigs)
             segs_.push_back({nullptr, rigs[r]->deviceDesc(), reinterpret_cast<const FrameDev*>(sizeof(FrameDev) * r), 1,
                              s.total});
             s.total += 1;
-            if (s.level < 0) s.level = rigs[r]->tailBlend();
+            if (s.level < 0) s.level = rigs[r]->tailStart();
             s.bytes += rigs[r]->stepBytes(3, 0);
         }
         s.nsegs = (int)segs_.size() - s.segOff;
@@ -1397,14 +1384,14 @@ void Plan::bind(const std::vector<Rig*>& rigs)
     }
     int maxB = 0;
     for (Rig* r : rigs)
-        if (!r->linear()) maxB = std::max(maxB, r->tailBlend());
+        if (!r->linear()) maxB = std::max(maxB, r->tailStart());
     for (int s = 0; s < maxB; s++) {
         // levels above 0 with few tiles go to k_blend_small (two halves per tile)
         std::vector<std::pair<int, std::pair<const void*, int>>> small;
         parts.clear();
         for (int r = 0; r < nr; r++) {
             if (rigs[r]->linear()) continue;
-            const int j = rigs[r]->tailBlend() - 1 - s;
+            const int j = rigs[r]->tailStart() - 1 - s;
             if (j < 0) continue;
             const int cnt = rigs[r]->numBlendItems(j);
             if (j > 0 && cnt <= rigs[r]->shape().smallBlend()) small.push_back({r, {rigs[r]->blendItems(j), 2 * cnt}});
@@ -1473,7 +1460,7 @@ void Plan::launchAll(const IoSlot& slot, cudaStream_t st, int srcFmt, Profiler* 
         if (s.kind == 0) PS_CUDA(launchRemap(p, s.nsegs, s.total, perSm_[0], counters + si, srcFmt, maps_, st));
         else if (s.kind == 1) PS_CUDA(launchPyrDown(p, s.nsegs, s.total, perSm_[1], st));
         else if (s.kind == 2) PS_CUDA(launchBlend(p, s.nsegs, s.total, perSm_[2], counters + si, probe_, s.early, st));
-        else if (s.kind == 3) PS_CUDA(launchTail(p, s.nsegs, tailCluster_, st));
+        else if (s.kind == 3) PS_CUDA(launchTail(p, s.nsegs, tailCluster_, tailCams_, st));
         else if (s.kind == 6) PS_CUDA(launchBlendSmall(p, s.nsegs, s.total, s.early, st));
         else PS_CUDA(launchLinear(p, s.nsegs, s.total, maxCams_, srcFmt, st));
         if (prof) {

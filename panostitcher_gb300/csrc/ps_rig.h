@@ -150,12 +150,10 @@ public:
     // new generation.
     void setShape(const LaunchShape& s);
     const LaunchShape& shape() const { return shape_; }
-    // the tail levels a tail_max_items value gives: pyrDown down..L, blend L..blend
-    void tailSplit(int maxItems, int* down, int* blend) const;
-    // pyrDown levels tailDown()..L and blend levels L..tailBlend() run in the tail kernel
-    int tailDown() const { return tailDown_; }
-    int tailBlend() const { return tailBlend_; }
-    bool hasTail() const { return tailDown_ <= L_ || tailBlend_ <= L_; }
+    // the tail a tail_max_items value gives: levels tailStart..L (L + 1 = none)
+    int tailStart(int maxItems) const;
+    int tailStart() const { return tailStart_; }
+    bool hasTail() const { return tailStart_ <= L_; }
 
     // blender input: int16x4 / uint8x4 device images -> level 0 of a slot (checks)
     void imagesToLevel0(const void* const* images, const long long* pitches, int fmt, int slot, cudaStream_t st);
@@ -212,7 +210,7 @@ private:
     std::vector<RemapItem> hRemap_;
     int downOff_[PS_MAX_LEVELS + 1] = {}, downCnt_[PS_MAX_LEVELS + 1] = {};
     int blendOff_[PS_MAX_LEVELS + 1] = {}, blendCnt_[PS_MAX_LEVELS + 1] = {};
-    int tailDown_ = 1, tailBlend_ = 1;
+    int tailStart_ = 1;
     LaunchShape shape_;
     RigDev hDesc_ = {};  // slot-independent part of the descriptors
     std::vector<uint8_t> covBits_, seamBits_;  // host copies for exports (1 bit / pixel)
@@ -302,7 +300,7 @@ private:
     std::vector<size_t> lutOff_;
     size_t segOff_ = 0, counterOff_ = 0, stageBytes_ = 0;
     int maxCams_ = 0;
-    int tailCluster_ = 0, perSm_[3] = {0, 0, 0};  // launch widths (from the rigs' shapes)
+    int tailCluster_ = 0, tailCams_ = 0, perSm_[3] = {0, 0, 0};  // launch widths (from the rigs' shapes)
     bool maps_ = true;                             // every rig has resident maps
     int probe_ = 0;                                // wait probe of k_blend (Rig::setWaitProbe)
     IoSlot io_[Rig::kIoSlots];

@@ -151,50 +151,31 @@ std::vector<LaunchShape> neighbours(const Rig& rig, const LaunchShape& cur, int 
 {
     std::vector<LaunchShape> out;
     const int L = rig.numLevels();
-    int curDown = 0, curBlend = 0;
-    rig.tailSplit(cur.tailMaxItems, &curDown, &curBlend);
-    const bool tail = curDown <= L || curBlend <= L;
+    const int curTail = rig.tailStart(cur.tailMaxItems);
     switch (knob) {
-    case 0: {  // the tail split: one value per distinct split
-        std::vector<std::pair<int, int>> seen{{curDown, curBlend}};
-        for (int v : {0, 2, 4, 8, 16, 32, 64, 128, 256}) {
-            int d = 0, b = 0;
-            rig.tailSplit(v, &d, &b);
-            if (std::find(seen.begin(), seen.end(), std::make_pair(d, b)) != seen.end()) continue;
-            seen.push_back({d, b});
+    case 0: {  // the tail's levels: one value per distinct set
+        std::vector<int> seen{curTail};
+        for (int v : {0, 1, 2, 4, 8, 16}) {
+            const int t = rig.tailStart(v);
+            if (std::find(seen.begin(), seen.end(), t) != seen.end()) continue;
+            seen.push_back(t);
             LaunchShape s = cur;
             s.tailMaxItems = v;
             out.push_back(s);
-            // the blend levels a smaller tail hands back run best as half tiles
-            // together with it, so the split is also tried with those levels in
-            // k_blend_small (each knob alone can measure slower than the pair)
-            int most = 0;
-            for (int j = std::max(1, b); j < curBlend; j++) most = std::max(most, rig.numBlendItems(j));
-            if (most > cur.smallBlend() && most <= 512) {
-                s.smallBlendMaxItems = most;
-                out.push_back(s);
-            }
         }
         break;
     }
-    case 1:  // whole or half tiles for the tail's blend levels above 0
-        if (tail && curBlend <= L && L >= 1) {
-            LaunchShape s = cur;
-            s.tailHalf = 1 - cur.tailHalf;
-            out.push_back(s);
-        }
-        break;
     case 2:  // tail cluster width
-        if (tail && tailClusterMax() > 8) {
+        if (curTail <= L && tailClusterMax() > 8) {
             LaunchShape s = cur;
-            s.tailCluster = cur.tailCluster == 8 ? 0 : 8;
+            s.tailCluster = cur.tailCluster == 8 ? 16 : 8;
             out.push_back(s);
         }
         break;
     case 6: {  // the blend levels run as half tiles by k_blend_small: one value per distinct set
         auto smallLevels = [&](int v) {
             int c = 0;
-            for (int j = 1; j < curBlend; j++) c += rig.numBlendItems(j) <= v;
+            for (int j = 1; j < curTail; j++) c += rig.numBlendItems(j) <= v;
             return c;
         };
         std::vector<int> seen{smallLevels(cur.smallBlend())};
@@ -276,7 +257,7 @@ LaunchShape autotune(Rig& rig, Plan& plan, int framesPerTrial, int inflight, boo
         {
             std::vector<LaunchShape> seen{best};
             const int L = rig.numLevels();
-            for (int tail : {0, 2, 16})
+            for (int tail : {0, 16})
                 for (int small : {0, 1, 32})
                     for (int ctas : {0, 1, 2}) {
                         LaunchShape s;
@@ -284,17 +265,15 @@ LaunchShape autotune(Rig& rig, Plan& plan, int framesPerTrial, int inflight, boo
                         s.smallBlendMaxItems = small;
                         s.ctasPerSm[2] = ctas;
                         // shapes that launch the same work the same way are timed once
-                        int d = 0, b = 0;
-                        rig.tailSplit(tail, &d, &b);
+                        const int t0 = rig.tailStart(tail);
                         int smallLevels = 0;
-                        for (int j = 1; j < b && j <= L; j++) smallLevels += rig.numBlendItems(j) <= s.smallBlend();
+                        for (int j = 1; j < t0 && j <= L; j++) smallLevels += rig.numBlendItems(j) <= s.smallBlend();
                         bool dup = false;
                         for (const LaunchShape& o : seen) {
-                            int od = 0, ob = 0;
-                            rig.tailSplit(o.tailMaxItems, &od, &ob);
+                            const int ot = rig.tailStart(o.tailMaxItems);
                             int os = 0;
-                            for (int j = 1; j < ob && j <= L; j++) os += rig.numBlendItems(j) <= o.smallBlend();
-                            if (od == d && ob == b && os == smallLevels && o.ctasPerSm[2] == ctas) dup = true;
+                            for (int j = 1; j < ot && j <= L; j++) os += rig.numBlendItems(j) <= o.smallBlend();
+                            if (ot == t0 && os == smallLevels && o.ctasPerSm[2] == ctas) dup = true;
                         }
                         if (dup) continue;
                         seen.push_back(s);
@@ -309,7 +288,7 @@ LaunchShape autotune(Rig& rig, Plan& plan, int framesPerTrial, int inflight, boo
         // coordinate descent, two passes; a move must gain 1%
         for (int pass = 0; pass < 2; pass++) {
             bool moved = false;
-            for (int knob : {0, 6, 1, 2, 3, 4, 5})
+            for (int knob : {0, 6, 2, 3, 4, 5})
                 for (const LaunchShape& s : neighbours(rig, best, knob)) {
                     const double t = trials.time(s);
                     report.trials++;
