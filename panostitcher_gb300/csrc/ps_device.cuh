@@ -28,7 +28,7 @@ namespace ps {
 
 // ---- tiles ------------------------------------------------------------------
 constexpr int kRemapTW = 32, kRemapTH = 16;    // level-0 remap tile (two pixels per thread)
-constexpr int kDownTW = 32, kDownTH = 16;      // pyrDown output tile (two pixels per thread)
+constexpr int kDownTW = 32, kDownTH = 16;      // pyrDown output tile (four pixels per thread)
 constexpr int kBlendTW = 64, kBlendTH = 16;    // blend tile (a 2x2 pixel block per thread)
 constexpr int kThreads = 256;
 constexpr int kTailW = 32, kTailH = 16, kTailCams = 16;  // largest level and most cameras of k_tail
@@ -54,7 +54,8 @@ struct LevelDev {
 // Work items (one per tile), resident per rig and built at prepare time.
 struct RemapItem { uint16_t cam, pad; uint16_t tx, ty; uint32_t mapTile; };
 
-struct DownItem { uint8_t cam, level; uint16_t tx, ty; uint16_t pad; };   // level = output level
+// level: the output's; whole: every alpha of the tile is 256 (m == 256)
+struct DownItem { uint8_t cam, level; uint16_t tx, ty; uint16_t whole; };
 // A blend tile lists the cameras whose weight touches it: up to 8 inline,
 // more through RigDev::camLists (cams[0..3] then hold the uint32 offset).
 struct alignas(16) BlendItem { uint8_t level, cls, camCnt, flags; uint16_t tx, ty; uint8_t cams[8]; };

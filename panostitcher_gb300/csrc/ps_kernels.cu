@@ -756,25 +756,38 @@ __global__ void __launch_bounds__(kThreads) k_reproject16s(RemapSrc src, const f
 // With alpha = 256*m this is floor(S / m), evaluated exactly as
 // (S * ceil(2^24 / m)) >> 24 (exact for S < 65793; S <= 65280 here).
 // One CTA produces a 32x16 output tile of one camera from its 67x35 input
-// tile.  Warp w owns output rows 2w and 2w + 1, i.e. input rows 4w .. 4w+6:
-// lane l loads input columns 2l and 2l + 1 of those seven rows (lanes 0..2
-// also column 64 + l), forms the vertical sums of both output rows in
-// registers, two channels per 32-bit word, and hands them to the warp
-// through the warp's own rows of shared memory; lane l then filters output
-// columns 2(l % 16) and 2(l % 16) + 1 of output row 2w + l / 16.  No step
-// waits for another warp.
+// tile; warp w owns output rows 4w .. 4w + 3, i.e. input rows 8w .. 8w + 10.
+// Lane l loads input columns 2l and 2l + 1 of those rows, all before the first
+// is used, and forms the four output rows' vertical sums in registers, B and R
+// in one word a column, G of both columns in another; lanes 0..11 form those of
+// the three columns beyond.  They go to the warp through its own rows of shared
+// memory, and lane l filters output columns 2(l % 16) and 2(l % 16) + 1 of two
+// output rows.  No step waits for another warp.  Tiles whose every alpha is 256
+// (DownItem::whole, nearly all) read no divisors: S / 256 is a byte of S.
+// Two output rows a warp, four words a column pair and a division for every
+// pixel were 274 instructions a warp for 64 pixels, 60% of the issue slots.  Now
+// level 1 of 6 x 1920x1080 to 4096x2048 takes 11.7 us (17.3 before), of 8 x
+// 3840x2160 to 7680x3840 41 us (71), where memory alone would take about 10 and
+// 38 us.  The item's level descriptions wait in shared memory, a level of few
+// tiles is one trip to L2 long: 2.3 us against 3.2 us with them read from L2.
 // ============================================================================
 constexpr int kDInW = 2 * kDownTW + 3;   // 67 input columns
-constexpr int kDVP = kDInW + 1;          // 68: row stride of the vertical sums (16-byte aligned rows)
-constexpr int kDWarps = kThreads / 32;   // 8
-constexpr int kDRows = 7;                // input rows of a warp's two output rows
-static_assert(kDownTH == 2 * kDWarps, "a warp owns two output rows");
-static_assert(kDownTW == 32 && kDInW - 64 <= 32, "lanes cover the input columns as 2 x 32 + 3");
+constexpr int kDVP = kDInW + 1;          // 68: row stride of the vertical sums
+constexpr int kDownThreads = 128;
+constexpr int kDWarps = kDownThreads / 32;
+constexpr int kDOut = kDownTH / kDWarps;  // 4 output rows of a warp
+constexpr int kDRows = 2 * kDOut + 3;     // 11 input rows
+constexpr int kDHalo = kDInW - 64;        // 3 input columns beyond the lanes' pairs
+static_assert(kDownTW == 32 && kDOut % 2 == 0 && kDHalo * kDOut <= 32, "the lanes' columns, rows and halo sums");
 
 struct alignas(16) DownSmem {
-    uint2 v[kDWarps][2][kDVP];  // vertical sums (B|R, G|X lanes) of each warp's two output rows
+    uint32_t br[kDWarps][kDOut][kDVP];  // vertical sums, B | R << 16
+    uint16_t g[kDWarps][kDOut][kDVP];   // G
     uint32_t magic[257];
+    alignas(16) LevelDev lv[kDWarps][2];  // the item's input and output level, a copy a warp
 };
+static_assert(sizeof(LevelDev) % 4 == 0 && 2 * sizeof(LevelDev) / 4 <= 32, "a word a lane");
+static_assert(kDVP * 4 % 16 == 0 && kDVP * 2 % 8 == 0, "16- and 8-byte loads of rows");
 
 __device__ __forceinline__ void initMagic(uint32_t* magic)
 {
@@ -791,100 +804,11 @@ __device__ __forceinline__ T ldLevel(const T* p)
     else return __ldg(p);
 }
 
-// A lane's part of its warp's input rows, and the alpha divisors of the
-// lane's two outputs (low half: the left one).
-struct DownRegs {
-    uint32_t a[kDRows], b[kDRows];  // input columns 2*lane, 2*lane + 1
-    uint32_t c[kDRows];             // input column 64 + lane (lanes 0..2)
-    uint32_t m;
-};
-
-__device__ __forceinline__ bool downInterior(const RigDev& R, const DownItem& item)
-{
-    const LevelDev& Ls = R.lv[item.level - 1];
-    const int ix0 = 2 * item.tx * kDownTW - 2, iy0 = 2 * item.ty * kDownTH - 2;
-    return ix0 >= 0 && iy0 >= 0 && ix0 + kDInW <= Ls.w && iy0 + 2 * kDownTH + 3 <= Ls.h;
-}
-
-// The lane's loads for a tile.  Interior tiles read whole rows (8-byte loads:
-// the first input column is even and rows are 256-byte aligned); tiles whose
-// input crosses the level's border map every row and column with the
-// reference's reflect-101 / wrap rules.
-__device__ __forceinline__ void downLoad(const RigDev& R, const DownItem& item, DownRegs& g)
-{
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const LevelDev& Ls = R.lv[item.level - 1];
-    const LevelDev& Ld = R.lv[item.level];
-    const int ox0 = item.tx * kDownTW, oy0 = item.ty * kDownTH;
-    const int ix0 = 2 * ox0 - 2, iy0 = 2 * oy0 - 2 + 4 * w;  // the warp's first input row
-    const uint32_t* G = reinterpret_cast<const uint32_t*>(Ls.G) + (size_t)item.cam * Ls.camStride;
-    // the lane's outputs (X, Y), (X + 1, Y): X is even, so both divisors are
-    // one aligned 4-byte load (X + 1 stays inside the row pitch)
-    const int X = ox0 + 2 * (lane & 15), Y = oy0 + 2 * w + (lane >> 4);
-    g.m = X < Ld.w && Y < Ld.h ? ldChecked(reinterpret_cast<const uint32_t*>(Ld.Am + (size_t)item.cam * Ld.camStride +
-                                                                           (size_t)Y * Ld.pitch + X),
-                                           Ld.Am, wBytes(R, Ld))
-                               : 0u;
-    const bool extra = lane < kDInW - 64;
-    const long long ext = gBytes(R, Ls);
-    if (downInterior(R, item)) {
-        const uint32_t* row = G + (size_t)iy0 * Ls.pitch + ix0;
-#pragma unroll
-        for (int r = 0; r < kDRows; r++, row += Ls.pitch) {
-            const uint2* q = reinterpret_cast<const uint2*>(row) + lane;
-            const uint2 v = inside(q, Ls.G, ext) ? __ldg(q) : make_uint2(0, 0);
-            g.a[r] = v.x;
-            g.b[r] = v.y;
-            g.c[r] = extra && inside(row + 64 + lane, Ls.G, ext) ? __ldg(row + 64 + lane) : 0u;
-        }
-        return;
-    }
-    const int c0 = colMap(ix0 + 2 * lane, Ls.w), c1 = colMap(ix0 + 2 * lane + 1, Ls.w);
-    const int c2 = extra ? colMap(ix0 + 64 + lane, Ls.w) : 0;
-#pragma unroll
-    for (int r = 0; r < kDRows; r++) {
-        const uint32_t* row = G + (size_t)rowMap(iy0 + r, Ls.h) * Ls.pitch;
-        g.a[r] = inside(row + c0, Ls.G, ext) ? __ldg(row + c0) : 0u;
-        g.b[r] = inside(row + c1, Ls.G, ext) ? __ldg(row + c1) : 0u;
-        g.c[r] = extra && inside(row + c2, Ls.G, ext) ? __ldg(row + c2) : 0u;
-    }
-}
-
 // [1 4 6 4 1] over five 16-bit-lane words (sums of up to 16 * 4080 stay in
 // the lanes).
 __device__ __forceinline__ uint32_t k5(uint32_t p0, uint32_t p1, uint32_t p2, uint32_t p3, uint32_t p4)
 {
     return p0 + p4 + 4 * (p1 + p3) + 6 * p2;
-}
-
-// Vertical sums of one input column: the even output row from input rows
-// 0..4, the odd one from rows 2..6.
-__device__ __forceinline__ void downColumn(const uint32_t* p, uint2& e, uint2& o)
-{
-    uint2 u[kDRows];
-#pragma unroll
-    for (int r = 0; r < kDRows; r++) u[r] = unpackBytes(p[r]);
-    e = make_uint2(k5(u[0].x, u[1].x, u[2].x, u[3].x, u[4].x), k5(u[0].y, u[1].y, u[2].y, u[3].y, u[4].y));
-    o = make_uint2(k5(u[2].x, u[3].x, u[4].x, u[5].x, u[6].x), k5(u[2].y, u[3].y, u[4].y, u[5].y, u[6].y));
-}
-
-// The lane's vertical sums into the warp's rows.
-__device__ __forceinline__ void downVertical(const DownRegs& g, DownSmem& sm)
-{
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    uint2 ea, oa, eb, ob;
-    downColumn(g.a, ea, oa);
-    downColumn(g.b, eb, ob);
-    __syncwarp();  // the warp's reads of its previous tile are done
-    *reinterpret_cast<uint4*>(&sm.v[w][0][2 * lane]) = make_uint4(ea.x, ea.y, eb.x, eb.y);
-    *reinterpret_cast<uint4*>(&sm.v[w][1][2 * lane]) = make_uint4(oa.x, oa.y, ob.x, ob.y);
-    if (lane < kDInW - 64) {
-        uint2 ec, oc;
-        downColumn(g.c, ec, oc);
-        sm.v[w][0][64 + lane] = ec;
-        sm.v[w][1][64 + lane] = oc;
-    }
-    __syncwarp();
 }
 
 // floor(S / m) of the B, G, R sums (lo = B | R << 16, hi = G | X << 16):
@@ -899,38 +823,129 @@ __device__ __forceinline__ uint32_t downDivide(uint32_t lo, uint32_t hi, uint32_
     return b | (gg << 8) | (r << 16);
 }
 
-// Horizontal pass of the lane's two outputs from the warp's rows, and the
-// stores.  m: the divisors loaded with the tile.
-__device__ __forceinline__ void downHorizontal(const RigDev& R, const DownItem& item, uint32_t m, const DownSmem& sm)
+// The warp's four output rows of one tile.
+__device__ __forceinline__ void downRows(const RigDev& R, const DownItem& item, DownSmem& sm)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const LevelDev &Ls = sm.lv[w][0], &Ld = sm.lv[w][1];
+    const int ox0 = item.tx * kDownTW, oy0 = item.ty * kDownTH + kDOut * w;
+    if (oy0 >= Ld.h) return;
+    const int ix0 = 2 * ox0 - 2, iy0 = 2 * oy0 - 2;  // the warp's first input pixel
+    const uint32_t* G = reinterpret_cast<const uint32_t*>(Ls.G) + (size_t)item.cam * Ls.camStride;
+    const long long ext = gBytes(R, Ls);
+    // the lane's halo sum: column 64 + hc of output row hr
+    const bool halo = lane < kDHalo * kDOut;
+    const int hc = lane % kDHalo, hr = lane / kDHalo;
+    uint32_t a[kDRows], b[kDRows], h[5];
+    // Tiles inside the level read whole rows (8-byte loads: the first input
+    // column is even and rows are 256-byte aligned); where the input crosses the
+    // border every row and column is mapped by the reference's rules.
+    if (ix0 >= 0 && iy0 >= 0 && ix0 + kDInW <= Ls.w && iy0 + kDRows <= Ls.h) {
+        const uint32_t* row = G + (size_t)iy0 * Ls.pitch + ix0;
+        const uint2* q = reinterpret_cast<const uint2*>(row) + lane;
+        const uint32_t* p = row + 2 * hr * Ls.pitch + 64 + hc;
+#pragma unroll
+        for (int r = 0; r < kDRows; r++, q += Ls.pitch / 2) {
+            const uint2 v = inside(q, Ls.G, ext) ? __ldg(q) : make_uint2(0, 0);
+            a[r] = v.x;
+            b[r] = v.y;
+        }
+#pragma unroll
+        for (int r = 0; r < 5; r++, p += Ls.pitch) h[r] = halo && inside(p, Ls.G, ext) ? __ldg(p) : 0u;
+    } else {
+        const int c0 = colMap(ix0 + 2 * lane, Ls.w), c1 = colMap(ix0 + 2 * lane + 1, Ls.w);
+        const int c2 = colMap(ix0 + 64 + hc, Ls.w);
+#pragma unroll
+        for (int r = 0; r < kDRows; r++) {
+            const uint32_t* row = G + (size_t)rowMap(iy0 + r, Ls.h) * Ls.pitch;
+            a[r] = inside(row + c0, Ls.G, ext) ? __ldg(row + c0) : 0u;
+            b[r] = inside(row + c1, Ls.G, ext) ? __ldg(row + c1) : 0u;
+        }
+#pragma unroll
+        for (int r = 0; r < 5; r++) {
+            const uint32_t* p = G + (size_t)rowMap(iy0 + 2 * hr + r, Ls.h) * Ls.pitch + c2;
+            h[r] = halo && inside(p, Ls.G, ext) ? __ldg(p) : 0u;
+        }
+    }
+    // the lane's outputs (X, y), (X + 1, y) for y = oy0 + rsel and two below: X
+    // is even, so both divisors are one aligned 4-byte load (X + 1 stays inside
+    // the row pitch)
     const int k = lane & 15, rsel = lane >> 4;
-    // output columns 2k and 2k + 1 read vertical sums 4k .. 4k + 4 and 4k + 2 .. 4k + 6
-    const uint2* vr = &sm.v[w][rsel][4 * k];
-    const uint4 q01 = *reinterpret_cast<const uint4*>(vr);
-    const uint4 q23 = *reinterpret_cast<const uint4*>(vr + 2);
-    const uint4 q45 = *reinterpret_cast<const uint4*>(vr + 4);
-    const uint2 q6 = vr[6];
-    const uint32_t lo0 = k5(q01.x, q01.z, q23.x, q23.z, q45.x), hi0 = k5(q01.y, q01.w, q23.y, q23.w, q45.y);
-    const uint32_t lo1 = k5(q23.x, q23.z, q45.x, q45.z, q6.x), hi1 = k5(q23.y, q23.w, q45.y, q45.w, q6.y);
-    const uint32_t out0 = downDivide(lo0, hi0, m & 0xFFFFu, sm.magic);
-    const uint32_t out1 = downDivide(lo1, hi1, m >> 16, sm.magic);
-    const LevelDev& Ld = R.lv[item.level];
-    const int X = item.tx * kDownTW + 2 * k, Y = item.ty * kDownTH + 2 * w + rsel;
-    if (X < Ld.w && Y < Ld.h) {
-        uint32_t* dst = reinterpret_cast<uint32_t*>(Ld.G) + (size_t)item.cam * Ld.camStride + (size_t)Y * Ld.pitch + X;
-        const long long ext = gBytes(R, Ld);
+    const int X = ox0 + 2 * k;
+    const size_t at = (size_t)item.cam * Ld.camStride + (size_t)(oy0 + rsel) * Ld.pitch + X;
+    uint32_t m[kDOut / 2];
+    if (!item.whole) {
+#pragma unroll
+        for (int i = 0; i < kDOut / 2; i++)
+            m[i] = X < Ld.w && oy0 + rsel + 2 * i < Ld.h
+                       ? ldChecked(reinterpret_cast<const uint32_t*>(Ld.Am + at + 2 * i * Ld.pitch), Ld.Am, wBytes(R, Ld))
+                       : 0u;
+    }
+    uint32_t ba[kDRows], bb[kDRows], gg[kDRows];  // B | R << 16 of either column, G of both (the fourth byte is 0)
+#pragma unroll
+    for (int r = 0; r < kDRows; r++) {
+        ba[r] = a[r] & 0x00FF00FFu;
+        bb[r] = b[r] & 0x00FF00FFu;
+        gg[r] = __byte_perm(a[r], b[r], 0x7531);
+    }
+    __syncwarp();  // the warp's reads of its previous tile are done
+#pragma unroll
+    for (int o = 0; o < kDOut; o++) {
+        const int r = 2 * o;
+        *reinterpret_cast<uint2*>(&sm.br[w][o][2 * lane]) =
+            make_uint2(k5(ba[r], ba[r + 1], ba[r + 2], ba[r + 3], ba[r + 4]),
+                       k5(bb[r], bb[r + 1], bb[r + 2], bb[r + 3], bb[r + 4]));
+        *reinterpret_cast<uint32_t*>(&sm.g[w][o][2 * lane]) = k5(gg[r], gg[r + 1], gg[r + 2], gg[r + 3], gg[r + 4]);
+    }
+    if (halo) {
+        uint2 u[5];
+#pragma unroll
+        for (int r = 0; r < 5; r++) u[r] = unpackBytes(h[r]);
+        sm.br[w][hr][64 + hc] = k5(u[0].x, u[1].x, u[2].x, u[3].x, u[4].x);
+        sm.g[w][hr][64 + hc] = (uint16_t)k5(u[0].y, u[1].y, u[2].y, u[3].y, u[4].y);
+    }
+    __syncwarp();
+    uint32_t* dst = reinterpret_cast<uint32_t*>(Ld.G) + at;
+    const long long oext = gBytes(R, Ld);
+#pragma unroll
+    for (int i = 0; i < kDOut / 2; i++, dst += 2 * Ld.pitch) {
+        // output columns 2k and 2k + 1 read vertical sums 4k .. 4k + 4 and 4k + 2 .. 4k + 6
+        const uint32_t* vb = &sm.br[w][rsel + 2 * i][4 * k];
+        const uint16_t* vg = &sm.g[w][rsel + 2 * i][4 * k];
+        const uint4 p = *reinterpret_cast<const uint4*>(vb), q = *reinterpret_cast<const uint4*>(vb + 4);
+        const uint2 gp = *reinterpret_cast<const uint2*>(vg), gq = *reinterpret_cast<const uint2*>(vg + 4);
+        const uint32_t br0 = k5(p.x, p.y, p.z, p.w, q.x), br1 = k5(p.z, p.w, q.x, q.y, q.z);
+        const uint32_t g0 = __dp2a_lo(gp.x, 0x0401u, __dp2a_lo(gp.y, 0x0406u, gq.x & 0xFFFFu));
+        const uint32_t g1 = __dp2a_lo(gp.y, 0x0401u, __dp2a_lo(gq.x, 0x0406u, gq.y & 0xFFFFu));
+        uint32_t out0, out1;
+        if (item.whole) {
+            out0 = __byte_perm(br0, g0, 0x7351);
+            out1 = __byte_perm(br1, g1, 0x7351);
+        } else {
+            out0 = downDivide(br0, g0, m[i] & 0xFFFFu, sm.magic);
+            out1 = downDivide(br1, g1, m[i] >> 16, sm.magic);
+        }
+        if (X >= Ld.w || oy0 + rsel + 2 * i >= Ld.h) continue;
         if (X + 1 < Ld.w) {
-            if (inside(reinterpret_cast<uint2*>(dst), Ld.G, ext)) *reinterpret_cast<uint2*>(dst) = make_uint2(out0, out1);
-        } else if (inside(dst, Ld.G, ext)) {
+            if (inside(reinterpret_cast<uint2*>(dst), Ld.G, oext)) *reinterpret_cast<uint2*>(dst) = make_uint2(out0, out1);
+        } else if (inside(dst, Ld.G, oext)) {
             dst[0] = out0;
         }
     }
 }
 
-// One CTA walks a contiguous run of tiles; the next tile's loads are issued
-// before the current tile's horizontal pass, so their latency overlaps it.
-__global__ void __launch_bounds__(kThreads, 5) k_pyrdown(const Segment* __restrict__ segs, int nsegs, int total)
+// The levels of an item into the warp's copy.
+__device__ __forceinline__ void downLevels(const RigDev& R, int level, DownSmem& sm)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __syncwarp();
+    if (lane < 2 * (int)sizeof(LevelDev) / 4)
+        reinterpret_cast<uint32_t*>(sm.lv[w])[lane] = __ldg(reinterpret_cast<const uint32_t*>(&R.lv[level - 1]) + lane);
+    __syncwarp();
+}
+
+// One CTA walks a contiguous run of tiles, each warp for itself.
+__global__ void __launch_bounds__(kDownThreads, 8) k_pyrdown(const Segment* __restrict__ segs, int nsegs, int total)
 {
     __shared__ DownSmem sm;
     initMagic(sm.magic);
@@ -938,34 +953,24 @@ __global__ void __launch_bounds__(kThreads, 5) k_pyrdown(const Segment* __restri
     itemRange(total, begin, end);
     // Items and descriptors are written before the launch sequence, not by
     // a kernel: the first tile's are read while the previous kernel finishes.
-    const RigDev* R = nullptr;
     DownItem item{};
     if (begin < end) {
         s = findSegment(segs, nsegs, begin, s);
-        R = segs[s].rig;
         item = static_cast<const DownItem*>(segs[s].items)[begin - segs[s].prefix];
+        downLevels(*segs[s].rig, item.level, sm);
     }
+    __syncthreads();  // the magic table
     waitPrevGrid();
     allowNextGrid();
-    if (begin >= end) return;
-    __syncthreads();  // the magic table
-    DownRegs g;
-    downLoad(*R, item, g);
-    for (int it = begin; it < end; it++) {
-        const bool more = it + 1 < end;
-        int sn = s;
-        DownItem next = item;
-        if (more) {
-            sn = findSegment(segs, nsegs, it + 1, s);
-            next = static_cast<const DownItem*>(segs[sn].items)[it + 1 - segs[sn].prefix];
+    for (int it = begin; it < end;) {
+        const DownItem now = item;
+        const int sn = s;
+        if (++it < end) {
+            s = findSegment(segs, nsegs, it, s);
+            item = static_cast<const DownItem*>(segs[s].items)[it - segs[s].prefix];
         }
-        downVertical(g, sm);
-        const uint32_t m = g.m;
-        if (more) downLoad(*segs[sn].rig, next, g);
-        downHorizontal(*R, item, m, sm);
-        s = sn;
-        R = segs[s].rig;
-        item = next;
+        downRows(*segs[sn].rig, now, sm);
+        if (s != sn) downLevels(*segs[s].rig, item.level, sm);
     }
 }
 
@@ -2603,7 +2608,7 @@ int residentCtasPerSm(int kind)
     case 0:
         return std::min({residentPerSm<k_remap<0, true>>(kRemapThreads), residentPerSm<k_remap<PS_FMT_BGR24, true>>(kRemapThreads),
                          residentPerSm<k_remap<PS_FMT_BGR32, true>>(kRemapThreads)});
-    case 1: return residentPerSm<k_pyrdown>(kThreads);
+    case 1: return residentPerSm<k_pyrdown>(kDownThreads);
     case 2: return residentPerSm<k_blend>(kBlendThreads);
     default: return 1;
     }
@@ -2637,7 +2642,7 @@ cudaError_t launchRemap(const Segment* segs, int nsegs, int total, int perSm, in
 cudaError_t launchPyrDown(const Segment* segs, int nsegs, int total, int perSm, cudaStream_t st)
 {
     if (total <= 0) return cudaSuccess;
-    return launchPdl(k_pyrdown, gridFor(total, residentPerSm<k_pyrdown>(kThreads), perSm), kThreads, st, segs, nsegs,
+    return launchPdl(k_pyrdown, gridFor(total, residentPerSm<k_pyrdown>(kDownThreads), perSm), kDownThreads, st, segs, nsegs,
                      total);
 }
 

@@ -480,7 +480,7 @@ void Rig::preparePyramids(const uint8_t* cov, const uint8_t* seam, const float* 
         rflags.zero(st);
         PS_CUDA(launchTileFlags8(cov, W, H, W, (long long)npx, n, kRemapTW, kRemapTH, rX, rY, rflags.as<uint8_t>(), st));
     }
-    std::vector<DevBuf> dflags(L + 1);
+    std::vector<DevBuf> dflags(L + 1), pflags(L + 1);  // any alpha, an alpha below 256
     DevBuf counts(sizeof(unsigned long long));
     counts.zero(st);
     for (int j = 1; j <= L; j++) {
@@ -491,17 +491,23 @@ void Rig::preparePyramids(const uint8_t* cov, const uint8_t* seam, const float* 
         dflags[j].zero(st);
         PS_CUDA(launchTileFlags16(lv_[j].Am.as<uint16_t>(), g.w, g.h, g.pitch, stride, n, kDownTW, kDownTH, dX, dY,
                                   dflags[j].as<uint8_t>(), st));
+        pflags[j].alloc(dflags[j].bytes());
+        pflags[j].zero(st);
+        PS_CUDA(launchTileNot256(lv_[j].Am.as<uint16_t>(), g.w, g.h, g.pitch, stride, n, kDownTW, kDownTH, dX, dY,
+                                 pflags[j].as<uint8_t>(), st));
         PS_CUDA(launchCountNonzero16(lv_[j].Am.as<uint16_t>(), g.w, g.h, g.pitch, stride, n,
                                      counts.as<unsigned long long>(), st));
     }
     unsigned long long hAlpha = 0;
     std::vector<uint8_t> hR(xmap ? rflags.bytes() : 0);
-    std::vector<std::vector<uint8_t>> hD(L + 1);
+    std::vector<std::vector<uint8_t>> hD(L + 1), hP(L + 1);
     PS_CUDA(cudaMemcpyAsync(&hAlpha, counts.get(), sizeof hAlpha, cudaMemcpyDeviceToHost, st));
     if (xmap) PS_CUDA(cudaMemcpyAsync(hR.data(), rflags.get(), hR.size(), cudaMemcpyDeviceToHost, st));
     for (int j = 1; j <= L; j++) {
         hD[j].resize(dflags[j].bytes());
         PS_CUDA(cudaMemcpyAsync(hD[j].data(), dflags[j].get(), hD[j].size(), cudaMemcpyDeviceToHost, st));
+        hP[j].resize(pflags[j].bytes());
+        PS_CUDA(cudaMemcpyAsync(hP[j].data(), pflags[j].get(), hP[j].size(), cudaMemcpyDeviceToHost, st));
     }
     std::vector<uint8_t> hCov(n * npx), hSeam(n * npx);
     PS_CUDA(cudaMemcpyAsync(hCov.data(), cov, n * npx, cudaMemcpyDeviceToHost, st));
@@ -531,9 +537,11 @@ void Rig::preparePyramids(const uint8_t* cov, const uint8_t* seam, const float* 
         downOff_[j] = (int)down.size();
         for (int c = 0; c < n; c++)
             for (int ty = 0; ty < dY; ty++)
-                for (int tx = 0; tx < dX; tx++)
-                    if (hD[j][((size_t)c * dY + ty) * dX + tx])
-                        down.push_back({(uint8_t)c, (uint8_t)j, (uint16_t)tx, (uint16_t)ty, 0});
+                for (int tx = 0; tx < dX; tx++) {
+                    const size_t t = ((size_t)c * dY + ty) * dX + tx;
+                    if (hD[j][t])
+                        down.push_back({(uint8_t)c, (uint8_t)j, (uint16_t)tx, (uint16_t)ty, (uint16_t)!hP[j][t]});
+                }
         downCnt_[j] = (int)down.size() - downOff_[j];
     }
     hDown_ = down;
