@@ -404,9 +404,12 @@ struct RemapChunk {
     alignas(256) uint8_t lut[3 * 256];
 };
 
-// The producer warp's state: the run of tiles it has taken.
+// The producer warp's state: the run of tiles it has taken.  The first run is
+// the CTA's by its number, the counter hands out what lies behind all of them:
+// a frame starts with nothing to hide an atomic's trip to L2 behind.
 struct RemapRun {
     int it, end, pos, seg;
+    int first;  // tiles of all first runs; 0 before this CTA's
 };
 
 // The next chunk (all lanes of the producer warp); false after the last one.
@@ -416,9 +419,14 @@ __device__ __forceinline__ bool remapProduce(RemapRun& r, RemapChunk& c, const S
     const int lane = threadIdx.x & 31;
     if (r.it >= r.end) {  // a new run: a quarter of a CTA's share of what is left
         const int want = max(1, min(kRemapRun, (total - r.pos) / (4 * (int)gridDim.x)));
-        int v = 0;
-        if (lane == 0) v = atomicAdd(counter, want);
-        r.it = r.pos = __shfl_sync(0xffffffffu, v, 0);
+        if (r.first == 0) {
+            r.it = r.pos = blockIdx.x * want;
+            r.first = gridDim.x * want;
+        } else {
+            int v = 0;
+            if (lane == 0) v = atomicAdd(counter, want);
+            r.it = r.pos = r.first + __shfl_sync(0xffffffffu, v, 0);
+        }
         r.end = min(r.it + want, total);
     }
     if (r.it >= total) {
@@ -430,24 +438,29 @@ __device__ __forceinline__ bool remapProduce(RemapRun& r, RemapChunk& c, const S
     const int last = min(r.end, sg.prefix + sg.count);  // the run's tiles in this segment
     RemapItem item{};
     if (r.it + lane < last) item = static_cast<const RemapItem*>(sg.items)[r.it - sg.prefix + lane];
+    // what does not depend on the item is on its way with it
+    const FrameDev& F = *sg.frame;
+    const RigDev& R = *sg.rig;
+    const LevelDev L = R.lv[0];
+    const float2* const maps = R.maps;
+    const uint32_t* const covTiles = R.covTiles;
+    const uint8_t* const luts = F.luts;
+    const int H = R.H, srcW = R.srcW, srcH = R.srcH, srcFmt = F.srcFmt;
     const int cam = __shfl_sync(0xffffffffu, (int)item.cam, 0);
     const uint32_t other = __ballot_sync(0xffffffffu, r.it + lane >= last || item.cam != cam);
     const int n = other ? __ffs(other) - 1 : 32;  // the leading tiles of that camera
-    const FrameDev& F = *sg.frame;
-    const RigDev& R = *sg.rig;
-    const LevelDev& L = R.lv[0];
     if (lane < n) {
         c.item[lane] = item;
-        c.tile[lane] = {R.maps ? static_cast<const void*>(R.maps + (size_t)item.mapTile * (kRemapTW * kRemapTH))
-                               : static_cast<const void*>(R.covTiles + (size_t)item.mapTile * kRemapTH),
+        c.tile[lane] = {maps ? static_cast<const void*>(maps + (size_t)item.mapTile * (kRemapTW * kRemapTH))
+                             : static_cast<const void*>(covTiles + (size_t)item.mapTile * kRemapTH),
                         reinterpret_cast<uint64_t>(reinterpret_cast<uint32_t*>(L.G) + (size_t)cam * L.camStride +
                                                    (size_t)item.ty * kRemapTH * L.pitch + item.tx * kRemapTW) +
-                            (uint32_t)min(kRemapTH, R.H - item.ty * kRemapTH)};
+                            (uint32_t)min(kRemapTH, H - item.ty * kRemapTH)};
     }
-    const uint4* t = reinterpret_cast<const uint4*>(F.luts + cam * 768);
+    const uint4* t = reinterpret_cast<const uint4*>(luts + cam * 768);
     for (int k = lane; k < 48; k += 32) reinterpret_cast<uint4*>(c.lut)[k] = __ldg(t + k);
     if (lane == 0) {
-        c.src = {F.src[cam], F.srcPitch[cam], F.srcFmt, R.srcW, R.srcH};
+        c.src = {F.src[cam], F.srcPitch[cam], srcFmt, srcW, srcH};
         c.R = &R;
         c.n = n;
         c.gpitch = L.pitch;
@@ -480,7 +493,7 @@ __global__ void __launch_bounds__(kRemapThreads, kRemapCtas) k_remap(const Segme
         // The hand-out counter, items, descriptors and LUTs are written before
         // the launch sequence, not by a kernel: the first chunks are resolved
         // while the previous kernel finishes.
-        RemapRun r{0, 0, 0, 0};
+        RemapRun r{0, 0, 0, 0, 0};
         bool more = true;
         for (int k = 0; more; k++) {
             const int s = k % kRemapRing;
