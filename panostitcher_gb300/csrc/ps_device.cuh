@@ -31,6 +31,11 @@ constexpr int kRemapTW = 32, kRemapTH = 16;    // level-0 remap tile (two pixels
 constexpr int kDownTW = 32, kDownTH = 16;      // pyrDown output tile (four pixels per thread)
 constexpr int kBlendTW = 64, kBlendTH = 16;    // blend tile (a 2x2 pixel block per thread)
 constexpr int kThreads = 256;
+// k_pyrdown_pair takes two levels whose lower one has this many tiles at most
+// (a CTA an SM): 40% of a tile's work is done twice, which levels of 380 tiles
+// do not hide (a launch of 5.7 - 6.3 us, as long as two of k_pyrdown; eight
+// frames in flight 918 us instead of 872).
+constexpr int kPairTiles = 152;
 constexpr int kTailW = 32, kTailH = 16, kTailCams = 16;  // largest level and most cameras of k_tail
 constexpr int kCBias = 256;  // of the collapsed levels' values
 

@@ -207,6 +207,8 @@ cudaError_t launchRemap(const Segment* segs, int nsegs, int total, int perSm, in
 // pitches of 4 GB or more, which their 32-bit row step cannot hold.
 int remapSourceFormat(int fmt, int sw, int sh, long long pitch);
 cudaError_t launchPyrDown(const Segment* segs, int nsegs, int total, int perSm, cudaStream_t st);
+// two levels at once; items: 32x16 tiles of the lower level (Rig::pairItems)
+cudaError_t launchPyrDownPair(const Segment* segs, int nsegs, int total, cudaStream_t st);
 // counter: a zeroed int the launch hands its tiles out through
 // Accesses the checked build's kernels refused since the last reset
 // (waits for the device); -1 in the normal build, -2 on a CUDA error.

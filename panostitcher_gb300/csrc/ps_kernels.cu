@@ -988,6 +988,157 @@ __global__ void __launch_bounds__(kDownThreads, 8) k_pyrdown(const Segment* __re
 }
 
 // ============================================================================
+// k_pyrdown_pair: two levels J and J + 1 of few tiles in one launch.  A level of
+// few tiles is a chain of latencies (its release, a trip to L2, the arithmetic,
+// the stores), 3 us whatever it holds.  A CTA takes a 32x16 tile of level J and
+// the 16x8 pixels of level J + 1 under it: it stages the 73x41 input pixels,
+// makes the 35x19 pixels of level J that its part of level J + 1 reads (the
+// halo a second time: each belongs to a neighbour's tile) and filters those.
+// Columns wrap as the input does, which is the reference's rule as long as the
+// input is twice level J wide (Rig::downPairs); rows beyond the level are mapped
+// when level J + 1 reads them.
+// 512 threads: with 256 a launch is 3.8 us, with 704 no shorter.  256x128: 31.2 us
+// a frame, 33.5 with a launch a level; 2048x1024: 78.8 against 80.3; 6 x
+// 1920x1080 to 4096x2048: 161.2 against 163.5.
+// ============================================================================
+constexpr int kPairThreads = 512;
+constexpr int kPairInW = 74, kPairInH = 41;    // staged input (an even number of columns)
+constexpr int kPairInP = 76;
+constexpr int kPairMidW = 35, kPairMidH = 19;  // staged level J
+constexpr int kPairMidP = 36;
+
+struct alignas(16) PairSmem {
+    uint32_t in[kPairInH][kPairInP];
+    uint32_t mid[kPairMidH][kPairMidP];
+    uint32_t magic[257];
+    alignas(16) LevelDev lv[3];  // J - 1, J, J + 1
+};
+
+// The 5x5 filter on five rows from their first tap.
+__device__ __forceinline__ uint32_t pairFilter(const uint32_t* const (&rows)[5], uint32_t m, const uint32_t* magic)
+{
+    uint32_t lo[5], hi[5];
+#pragma unroll
+    for (int r = 0; r < 5; r++) {
+        uint2 u[5];
+#pragma unroll
+        for (int i = 0; i < 5; i++) u[i] = unpackBytes(rows[r][i]);
+        lo[r] = k5(u[0].x, u[1].x, u[2].x, u[3].x, u[4].x);
+        hi[r] = k5(u[0].y, u[1].y, u[2].y, u[3].y, u[4].y);
+    }
+    return downDivide(k5(lo[0], lo[1], lo[2], lo[3], lo[4]), k5(hi[0], hi[1], hi[2], hi[3], hi[4]), m, magic);
+}
+
+__device__ __forceinline__ void pairStore(const RigDev& R, const LevelDev& L, int cam, int x, int y, uint32_t v)
+{
+    uint32_t* d = reinterpret_cast<uint32_t*>(L.G) + (size_t)cam * L.camStride + (size_t)y * L.pitch + x;
+    if (inside(d, L.G, gBytes(R, L))) *d = v;
+}
+
+__device__ __forceinline__ uint32_t pairAlpha(const RigDev& R, const LevelDev& L, int cam, int x, int y)
+{
+    return ldChecked(L.Am + (size_t)cam * L.camStride + (size_t)y * L.pitch + x, L.Am, wBytes(R, L));
+}
+
+__device__ __forceinline__ void pairTile(const RigDev& R, const DownItem& item, PairSmem& sm)
+{
+    const LevelDev &Li = sm.lv[0], &Lm = sm.lv[1], &Lo = sm.lv[2];
+    const int t = threadIdx.x, cam = item.cam;
+    const int mx0 = item.tx * kDownTW - 2, my0 = item.ty * kDownTH - 2;  // first pixel of mid
+    const int ix0 = 2 * mx0 - 2, iy0 = 2 * my0 - 2;                      // of in
+    const uint32_t* G = reinterpret_cast<const uint32_t*>(Li.G) + (size_t)cam * Li.camStride;
+    const long long ext = gBytes(R, Li);
+    // every load before any store
+    constexpr int kPieces = kPairInH * (kPairInW / 2), kIn = (kPieces + kPairThreads - 1) / kPairThreads;
+    constexpr int kMid = (kPairMidH * kPairMidP + kPairThreads - 1) / kPairThreads;
+    const bool whole = ix0 >= 0 && iy0 >= 0 && ix0 + kPairInW <= Li.w && iy0 + kPairInH <= Li.h;
+    uint2 v[kIn];
+#pragma unroll
+    for (int k = 0; k < kIn; k++) {
+        const int e = t + k * kPairThreads, r = e / (kPairInW / 2), c = 2 * (e % (kPairInW / 2));
+        v[k] = make_uint2(0, 0);
+        if (e >= kPieces) continue;
+        if (whole) {
+            const uint2* p = reinterpret_cast<const uint2*>(G + (size_t)(iy0 + r) * Li.pitch + ix0 + c);
+            if (inside(p, Li.G, ext)) v[k] = __ldg(p);
+        } else {
+            const uint32_t* row = G + (size_t)rowMap(iy0 + r, Li.h) * Li.pitch;
+            const uint32_t *p = row + colMap(ix0 + c, Li.w), *q = row + colMap(ix0 + c + 1, Li.w);
+            v[k] = make_uint2(inside(p, Li.G, ext) ? __ldg(p) : 0u, inside(q, Li.G, ext) ? __ldg(q) : 0u);
+        }
+    }
+    uint32_t m[kMid];
+    int mx[kMid];
+#pragma unroll
+    for (int k = 0; k < kMid; k++) {
+        const int e = t + k * kPairThreads, r = e / kPairMidP, c = e % kPairMidP;
+        mx[k] = -1;
+        m[k] = 0;
+        if (r < kPairMidH && c < kPairMidW && my0 + r >= 0 && my0 + r < Lm.h) {
+            mx[k] = colMap(mx0 + c, Lm.w);
+            m[k] = pairAlpha(R, Lm, cam, mx[k], my0 + r);
+        }
+    }
+    const int ox = item.tx * (kDownTW / 2) + (t & 15), oy = item.ty * (kDownTH / 2) + (t >> 4);
+    const bool out = t < 128 && ox < Lo.w && oy < Lo.h;
+    const uint32_t mo = out ? pairAlpha(R, Lo, cam, ox, oy) : 0u;
+    __syncthreads();  // readers of the tile before are done
+#pragma unroll
+    for (int k = 0; k < kIn; k++) {
+        const int e = t + k * kPairThreads, r = e / (kPairInW / 2), c = 2 * (e % (kPairInW / 2));
+        if (e < kPieces) *reinterpret_cast<uint2*>(&sm.in[r][c]) = v[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kMid; k++) {
+        if (mx[k] < 0) continue;
+        const int e = t + k * kPairThreads, r = e / kPairMidP, c = e % kPairMidP;
+        const uint32_t* p = &sm.in[2 * r][2 * c];
+        const uint32_t* const rows[5] = {p, p + kPairInP, p + 2 * kPairInP, p + 3 * kPairInP, p + 4 * kPairInP};
+        const uint32_t o = pairFilter(rows, m[k], sm.magic);
+        sm.mid[r][c] = o;
+        // the tile's own pixels
+        if (r >= 2 && r < 2 + kDownTH && c >= 2 && c < 2 + kDownTW && mx0 + c < Lm.w) pairStore(R, Lm, cam, mx[k], my0 + r, o);
+    }
+    __syncthreads();
+    if (out) {
+        const uint32_t* rows[5];
+#pragma unroll
+        for (int r = 0; r < 5; r++) rows[r] = &sm.mid[rowMap(2 * oy - 2 + r, Lm.h) - my0][2 * (t & 15)];
+        pairStore(R, Lo, cam, ox, oy, pairFilter(rows, mo, sm.magic));
+    }
+}
+
+__global__ void __launch_bounds__(kPairThreads) k_pyrdown_pair(const Segment* __restrict__ segs, int nsegs, int total)
+{
+    __shared__ PairSmem sm;
+    initMagic(sm.magic);
+    int s = -1;
+    for (int it = blockIdx.x; it < total; it += gridDim.x) {
+        const int sn = findSegment(segs, nsegs, it, max(s, 0));
+        const DownItem item = static_cast<const DownItem*>(segs[sn].items)[it - segs[sn].prefix];
+        const RigDev& R = *segs[sn].rig;
+        if (sn != s) {  // the first one's while the previous kernel finishes
+            __syncthreads();
+            if (threadIdx.x < 3 * sizeof(LevelDev) / 4)
+                reinterpret_cast<uint32_t*>(sm.lv)[threadIdx.x] =
+                    __ldg(reinterpret_cast<const uint32_t*>(&R.lv[item.level - 1]) + threadIdx.x);
+            __syncthreads();
+            if (s < 0) {
+                waitPrevGrid();
+                allowNextGrid();
+            }
+            s = sn;
+        }
+        pairTile(R, item, sm);
+    }
+    if (s < 0) {
+        waitPrevGrid();
+        allowNextGrid();
+    }
+}
+
+// ============================================================================
 // k_blend: one canvas level of the blend, all cameras at once.
 //   For each camera i whose weight touches the tile:
 //     U = pyrUp(G_{i,j+1})            pyrUp16SC4To16SC4, CudaPyramid2.cu:628-710
@@ -2657,6 +2808,13 @@ cudaError_t launchPyrDown(const Segment* segs, int nsegs, int total, int perSm, 
     if (total <= 0) return cudaSuccess;
     return launchPdl(k_pyrdown, gridFor(total, residentPerSm<k_pyrdown>(kDownThreads), perSm), kDownThreads, st, segs, nsegs,
                      total);
+}
+
+cudaError_t launchPyrDownPair(const Segment* segs, int nsegs, int total, cudaStream_t st)
+{
+    if (total <= 0) return cudaSuccess;
+    return launchPdl(k_pyrdown_pair, gridFor(total, residentPerSm<k_pyrdown_pair>(kPairThreads)), kPairThreads, st, segs,
+                     nsegs, total);
 }
 
 template <int kFmt>

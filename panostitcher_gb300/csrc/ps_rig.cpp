@@ -133,7 +133,7 @@ void Rig::clear()
     hBlend_.clear();
     hCams_.clear();
     tailStart_ = 1;
-    for (int j = 0; j <= PS_MAX_LEVELS; j++) downOff_[j] = downCnt_[j] = blendOff_[j] = blendCnt_[j] = 0;
+    for (int j = 0; j <= PS_MAX_LEVELS; j++) downOff_[j] = downCnt_[j] = pairOff_[j] = pairCnt_[j] = blendOff_[j] = blendCnt_[j] = 0;
     covCount_ = weightCount_ = alphaCount_ = 0;
     covBits_.clear();
     seamBits_.clear();
@@ -217,7 +217,7 @@ static long long listBytes(int W, int H, int n, int L, int slots)
     for (int j = 0; j <= L; j++) {
         const long long down = (long long)divUp(w, kDownTW) * divUp(h, kDownTH) * n;
         const long long blend = (long long)divUp(w, kBlendTW) * divUp(h, kBlendTH);
-        b += (j ? down * (long long)sizeof(DownItem) : 0) + blend * ((long long)sizeof(BlendItem) + n);
+        b += (j ? (down + std::min<long long>(down, kPairTiles)) * (long long)sizeof(DownItem) : 0) + blend * ((long long)sizeof(BlendItem) + n);
         w = (w + 1) / 2;
         h = (h + 1) / 2;
     }
@@ -480,7 +480,8 @@ void Rig::preparePyramids(const uint8_t* cov, const uint8_t* seam, const float* 
         rflags.zero(st);
         PS_CUDA(launchTileFlags8(cov, W, H, W, (long long)npx, n, kRemapTW, kRemapTH, rX, rY, rflags.as<uint8_t>(), st));
     }
-    std::vector<DevBuf> dflags(L + 1), pflags(L + 1);  // any alpha, an alpha below 256
+    // of a level's tiles: any alpha, an alpha below 256; of its 16x8 quarters: any alpha
+    std::vector<DevBuf> dflags(L + 1), pflags(L + 1), qflags(L + 1);
     DevBuf counts(sizeof(unsigned long long));
     counts.zero(st);
     for (int j = 1; j <= L; j++) {
@@ -495,12 +496,17 @@ void Rig::preparePyramids(const uint8_t* cov, const uint8_t* seam, const float* 
         pflags[j].zero(st);
         PS_CUDA(launchTileNot256(lv_[j].Am.as<uint16_t>(), g.w, g.h, g.pitch, stride, n, kDownTW, kDownTH, dX, dY,
                                  pflags[j].as<uint8_t>(), st));
+        const int qX = divUp(g.w, kDownTW / 2), qY = divUp(g.h, kDownTH / 2);
+        qflags[j].alloc((size_t)n * qX * qY);
+        qflags[j].zero(st);
+        PS_CUDA(launchTileFlags16(lv_[j].Am.as<uint16_t>(), g.w, g.h, g.pitch, stride, n, kDownTW / 2, kDownTH / 2, qX, qY,
+                                  qflags[j].as<uint8_t>(), st));
         PS_CUDA(launchCountNonzero16(lv_[j].Am.as<uint16_t>(), g.w, g.h, g.pitch, stride, n,
                                      counts.as<unsigned long long>(), st));
     }
     unsigned long long hAlpha = 0;
     std::vector<uint8_t> hR(xmap ? rflags.bytes() : 0);
-    std::vector<std::vector<uint8_t>> hD(L + 1), hP(L + 1);
+    std::vector<std::vector<uint8_t>> hD(L + 1), hP(L + 1), hQ(L + 1);
     PS_CUDA(cudaMemcpyAsync(&hAlpha, counts.get(), sizeof hAlpha, cudaMemcpyDeviceToHost, st));
     if (xmap) PS_CUDA(cudaMemcpyAsync(hR.data(), rflags.get(), hR.size(), cudaMemcpyDeviceToHost, st));
     for (int j = 1; j <= L; j++) {
@@ -508,6 +514,8 @@ void Rig::preparePyramids(const uint8_t* cov, const uint8_t* seam, const float* 
         PS_CUDA(cudaMemcpyAsync(hD[j].data(), dflags[j].get(), hD[j].size(), cudaMemcpyDeviceToHost, st));
         hP[j].resize(pflags[j].bytes());
         PS_CUDA(cudaMemcpyAsync(hP[j].data(), pflags[j].get(), hP[j].size(), cudaMemcpyDeviceToHost, st));
+        hQ[j].resize(qflags[j].bytes());
+        PS_CUDA(cudaMemcpyAsync(hQ[j].data(), qflags[j].get(), hQ[j].size(), cudaMemcpyDeviceToHost, st));
     }
     std::vector<uint8_t> hCov(n * npx), hSeam(n * npx);
     PS_CUDA(cudaMemcpyAsync(hCov.data(), cov, n * npx, cudaMemcpyDeviceToHost, st));
@@ -543,6 +551,25 @@ void Rig::preparePyramids(const uint8_t* cov, const uint8_t* seam, const float* 
                         down.push_back({(uint8_t)c, (uint8_t)j, (uint16_t)tx, (uint16_t)ty, (uint16_t)!hP[j][t]});
                 }
         downCnt_[j] = (int)down.size() - downOff_[j];
+    }
+    // the same for pairs of levels: a tile of the lower one is listed for any
+    // alpha of its own or of the quarter of the upper one under it
+    for (int j = 1; j < L; j++) {
+        const LevelGeom &gi = geom_[j - 1], &g = geom_[j];
+        pairOff_[j] = (int)down.size();
+        // the wrapped columns and the reflected rows of a tile's neighbourhood
+        // lie within one turn and inside the tile's own rows
+        if (gi.w != 2 * g.w || g.w < 2 * kDownTW || g.h < 2 * kDownTH) continue;
+        const int dX = divUp(g.w, kDownTW), dY = divUp(g.h, kDownTH);
+        const int qX = divUp(geom_[j + 1].w, kDownTW / 2), qY = divUp(geom_[j + 1].h, kDownTH / 2);
+        for (int c = 0; c < n; c++)
+            for (int ty = 0; ty < dY; ty++)
+                for (int tx = 0; tx < dX; tx++)
+                    if (hD[j][((size_t)c * dY + ty) * dX + tx] ||
+                        (tx < qX && ty < qY && hQ[j + 1][((size_t)c * qY + ty) * qX + tx]))
+                        down.push_back({(uint8_t)c, (uint8_t)j, (uint16_t)tx, (uint16_t)ty, 0});
+        if ((int)down.size() - pairOff_[j] > kPairTiles) down.resize(pairOff_[j]);
+        pairCnt_[j] = (int)down.size() - pairOff_[j];
     }
     hDown_ = down;
     // the weights' part: union coverage, fullMask, blend items
@@ -867,6 +894,16 @@ void Rig::waitIdleQuiet() noexcept
     for (cudaEvent_t* es : {slotComputed_, slotDownloaded_})
         for (int k = 0; k < kIoSlots; k++)
             if (es[k] && cudaEventSynchronize(es[k]) != cudaSuccess) cudaGetLastError();
+}
+
+std::vector<int> Rig::downSteps(bool pairs) const
+{
+    std::vector<int> steps;  // from the tail down
+    for (int j = std::min(tailStart_, L_ + 1) - 1; j >= 1; j--) {
+        if (pairs && j > 1 && pairCnt_[j - 1] > 0) steps.push_back(-(--j));
+        else steps.push_back(j);
+    }
+    return {steps.rbegin(), steps.rend()};
 }
 
 int Rig::tailStart(int maxItems) const
@@ -1301,10 +1338,8 @@ void Plan::quiesce()
 void Plan::bind(const std::vector<Rig*>& rigs)
 {
     const int nr = (int)rigs.size();
-    int maxL = 0;
     for (Rig* r : rigs) {
         if (!r || !r->ready()) fail(PS_ESTATE, "render not prepared");
-        maxL = std::max(maxL, r->numLevels());
     }
     quiesce();
     dropGraph();
@@ -1344,6 +1379,7 @@ void Plan::bind(const std::vector<Rig*>& rigs)
     for (Rig* r : rigs) maps_ = maps_ && !r->mapFree();
     probe_ = 0;
     for (Rig* r : rigs) probe_ = std::max(probe_, r->waitProbe());
+    std::vector<std::vector<int>> downSteps;  // of every rig
     auto addStep = [&](int kind, const std::vector<std::pair<int, std::pair<const void*, int>>>& parts, int step) {
         Step s{kind, (int)segs_.size(), 0, 0, -1, 0.0};
         for (const auto& p : parts) {
@@ -1354,9 +1390,12 @@ void Plan::bind(const std::vector<Rig*>& rigs)
                              reinterpret_cast<const FrameDev*>(sizeof(FrameDev) * p.first), p.second.second, s.total});
             s.total += p.second.second;
             const Rig* rg = rigs[p.first];
-            const int lvl = kind == 0 || kind == 4 ? 0 : (kind == 1 ? step : rg->tailStart() - 1 - step);
+            const int lvl = kind == 0 || kind == 4 ? 0
+                            : kind == 1 || kind == 8 ? std::abs(downSteps[p.first][downSteps[p.first].size() - step])
+                                                     : rg->tailStart() - 1 - step;
             if (s.level < 0) s.level = lvl;
-            s.bytes += rg->stepBytes(kind == 6 ? 2 : kind, lvl);
+            if (kind == 8) s.bytes += rg->stepBytes(1, lvl) + rg->stepBytes(1, lvl + 1);
+            else s.bytes += rg->stepBytes(kind == 6 ? 2 : kind, lvl);
         }
         s.nsegs = (int)segs_.size() - s.segOff;
         if (s.total > 0) steps_.push_back(s);
@@ -1369,11 +1408,37 @@ void Plan::bind(const std::vector<Rig*>& rigs)
     for (int r = 0; r < nr; r++)
         if (!rigs[r]->linear()) parts.push_back({r, {rigs[r]->remapItems(), rigs[r]->numRemapItems()}});
     addStep(0, parts, 0);
-    for (int J = 1; J <= maxL; J++) {
+    // pyrDown: every rig's levels in order, one or two of them a launch, the
+    // rigs' last ones together; pairs where they make the launches fewer (the
+    // pairs of one rig are a launch apart from the single levels of another)
+    std::vector<std::vector<int>> steps[2];
+    size_t slots[2] = {0, 0}, launches[2] = {0, 0};
+    for (int pairs = 0; pairs < 2; pairs++) {
+        for (Rig* r : rigs) {
+            steps[pairs].push_back(r->linear() ? std::vector<int>() : r->downSteps(pairs != 0));
+            slots[pairs] = std::max(slots[pairs], steps[pairs].back().size());
+        }
+        for (size_t k = 0; k < slots[pairs]; k++) {
+            bool one = false, two = false;
+            for (const std::vector<int>& v : steps[pairs])
+                if (k + v.size() >= slots[pairs]) (v[k + v.size() - slots[pairs]] > 0 ? one : two) = true;
+            launches[pairs] += one + two;
+        }
+    }
+    const int use = launches[1] < launches[0];
+    downSteps = steps[use];
+    for (size_t k = 0; k < slots[use]; k++) {
+        std::vector<std::pair<int, std::pair<const void*, int>>> pairs;
         parts.clear();
-        for (int r = 0; r < nr; r++)
-            if (J < rigs[r]->tailStart()) parts.push_back({r, {rigs[r]->downItems(J), rigs[r]->numDownItems(J)}});
-        addStep(1, parts, J);
+        for (int r = 0; r < nr; r++) {
+            const std::vector<int>& v = downSteps[r];
+            if (k + v.size() < slots[use]) continue;
+            const int j = v[k + v.size() - slots[use]];
+            if (j > 0) parts.push_back({r, {rigs[r]->downItems(j), rigs[r]->numDownItems(j)}});
+            else pairs.push_back({r, {rigs[r]->pairItems(-j), rigs[r]->numPairItems(-j)}});
+        }
+        addStep(1, parts, (int)(slots[use] - k));
+        addStep(8, pairs, (int)(slots[use] - k));
     }
     {
         // the tail: one cluster per rig that has one (segment count 1)
@@ -1458,7 +1523,7 @@ void Plan::launchAll(const IoSlot& slot, cudaStream_t st, int srcFmt, Profiler* 
         const Segment* p = segs + s.segOff;
         static const char* const kRangeName[] = {"ps.remap", "ps.pyrdown", "ps.blend", "ps.tail",
                                                  "ps.linear", "ps.cvt", "ps.blend_small"};
-        NvtxRange range(kRangeName[s.kind >= 0 && s.kind <= 6 ? s.kind : 5]);
+        NvtxRange range(kRangeName[s.kind == 8 ? 1 : s.kind]);
         cudaEvent_t a = nullptr, b = nullptr;
         if (prof) {
             a = prof->event();
@@ -1467,13 +1532,14 @@ void Plan::launchAll(const IoSlot& slot, cudaStream_t st, int srcFmt, Profiler* 
         }
         if (s.kind == 0) PS_CUDA(launchRemap(p, s.nsegs, s.total, perSm_[0], counters + si, srcFmt, maps_, st));
         else if (s.kind == 1) PS_CUDA(launchPyrDown(p, s.nsegs, s.total, perSm_[1], st));
+        else if (s.kind == 8) PS_CUDA(launchPyrDownPair(p, s.nsegs, s.total, st));
         else if (s.kind == 2) PS_CUDA(launchBlend(p, s.nsegs, s.total, perSm_[2], counters + si, probe_, s.early, st));
         else if (s.kind == 3) PS_CUDA(launchTail(p, s.nsegs, tailCluster_, tailCams_, st));
         else if (s.kind == 6) PS_CUDA(launchBlendSmall(p, s.nsegs, s.total, s.early, st));
         else PS_CUDA(launchLinear(p, s.nsegs, s.total, maxCams_, srcFmt, st));
         if (prof) {
             PS_CUDA(cudaEventRecord(b, st));
-            prof->record(s.kind, s.level, s.bytes, a, b);
+            prof->record(s.kind == 8 ? 1 : s.kind, s.level, s.bytes, a, b);
         }
     }
 }

@@ -142,6 +142,13 @@ public:
     int numRemapItems() const { return (int)hRemap_.size(); }
     const DownItem* downItems(int level) const { return dDown_.as<DownItem>() + downOff_[level]; }
     int numDownItems(int level) const { return downCnt_[level]; }
+    // tiles of levels `level` and level + 1 at once (k_pyrdown_pair); none where
+    // that kernel does not take them
+    const DownItem* pairItems(int level) const { return dDown_.as<DownItem>() + pairOff_[level]; }
+    int numPairItems(int level) const { return pairCnt_[level]; }
+    // the launches of the pyrDown levels below the tail: a level, or (with
+    // pairs) the lower level of a pair, negated
+    std::vector<int> downSteps(bool pairs) const;
     const BlendItem* blendItems(int level) const { return dBlend_.as<BlendItem>() + blendOff_[level]; }
     int numBlendItems(int level) const { return blendCnt_[level]; }
     // Launch shape (tail split, tail cluster and tile split, CTAs per SM).
@@ -209,6 +216,7 @@ private:
     DevBuf tmaps_;  // slots x (L + 1) x kTmapsPerLevel CUtensorMap
     std::vector<RemapItem> hRemap_;
     int downOff_[PS_MAX_LEVELS + 1] = {}, downCnt_[PS_MAX_LEVELS + 1] = {};
+    int pairOff_[PS_MAX_LEVELS + 1] = {}, pairCnt_[PS_MAX_LEVELS + 1] = {};
     int blendOff_[PS_MAX_LEVELS + 1] = {}, blendCnt_[PS_MAX_LEVELS + 1] = {};
     int tailStart_ = 1;
     LaunchShape shape_;
@@ -270,7 +278,7 @@ public:
 
 private:
     struct Step {
-        int kind;  // 0 remap, 1 pyrDown, 2 blend, 3 tail, 4 linear-blend render, 6 few-tile blend
+        int kind;  // 0 remap, 1 pyrDown, 2 blend, 3 tail, 4 linear-blend render, 6 few-tile blend, 8 pyrDown pair
         int segOff, nsegs, total;
         int level;      // level of the first rig in the step
         double bytes;   // algorithmic bytes of the step (all rigs)
