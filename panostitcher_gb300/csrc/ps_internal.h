@@ -214,13 +214,14 @@ cudaError_t launchPyrDownPair(const Segment* segs, int nsegs, int total, cudaStr
 // (waits for the device); -1 in the normal build, -2 on a CUDA error.
 long long boundsViolations(bool reset);
 // probePolls > 0: the failure-path test of the bounded waits (k_blend).
-// early: the launch before this one wrote only C levels (a blend step after
+// early: 2, the launch before this one wrote only C levels (a blend step after
 // the first), so the G_j, weight and G_{j+1} reads of each CTA's first unit
-// may be issued before the wait for it (k_blend, k_blend_small)
+// may be issued before the wait for it (k_blend, k_blend_small); 1, it is the
+// tail: the G_j reads may (k_blend_small)
 cudaError_t launchBlend(const Segment* segs, int nsegs, int total, int perSm, int* counter, int probePolls,
-                        bool early, cudaStream_t st);
+                        int early, cudaStream_t st);
 // blend of few-tile levels above 0: two work items (the 64x8 halves) per tile
-cudaError_t launchBlendSmall(const Segment* segs, int nsegs, int total, bool early, cudaStream_t st);
+cudaError_t launchBlendSmall(const Segment* segs, int nsegs, int total, int early, cudaStream_t st);
 // one cluster per segment: the rig's pyrDown levels tailStart..L and blend
 // levels L..tailStart; cams: the most cameras of any rig; cluster 8 or 16 CTAs
 // (0: by cams; at most the widest the GPU co-schedules)

@@ -807,16 +807,6 @@ __device__ __forceinline__ void initMagic(uint32_t* magic)
     for (int m = threadIdx.x; m < 257; m += blockDim.x) magic[m] = m ? (uint32_t)((16777216u + m - 1) / m) : 0u;
 }
 
-// Loads of pyramid levels.  What may have been written by a launch that ends
-// only while this one runs is read through L2 (ld.global.cg); the rest may use
-// the read-only path.
-template <bool kFresh, class T>
-__device__ __forceinline__ T ldLevel(const T* p)
-{
-    if constexpr (kFresh) return __ldcg(p);
-    else return __ldg(p);
-}
-
 // [1 4 6 4 1] over five 16-bit-lane words (sums of up to 16 * 4080 stay in
 // the lanes).
 __device__ __forceinline__ uint32_t k5(uint32_t p0, uint32_t p1, uint32_t p2, uint32_t p3, uint32_t p4)
@@ -1424,10 +1414,12 @@ __device__ __forceinline__ void stageUnitDirect(Stage& S, const RigDev& R, const
 // and up to eight of its cameras.  Threads 0..kConsumers-1; the caller
 // synchronises before the stage is read.
 //
-// stageHalfG: the cameras' G_j rows, weights and G_{j+1} footprints.
+// stageHalfG: of the cameras' G_j rows, weights and G_{j+1} footprints the
+// parts asked for, through L2 (what another launch wrote while this one began).
 // stageHalfC: the C_{j+1} footprint, with a tile's last unit -- the only part
 // the level above's blend writes, so the rest may be staged before it.
 static_assert(HalfStage::kFpRows * kFW <= kConsumers, "a footprint element a thread");
+constexpr int kPartW = 1, kPartG = 2, kPartUp = 4, kPartsAll = 7;
 
 // Element (r, c) of a half tile's footprint in a plane of level Lu.  Elements
 // that no pixel of level Lj needs (the tile reaches beyond the level) map to 0.
@@ -1439,8 +1431,8 @@ __device__ __forceinline__ size_t halfFpOffset(const LevelDev& Lu, const LevelDe
     return (size_t)rowMap(y / 2 - 1 + r, Lu.h) * Lu.pitch + colMap(x / 2 - 1 + c, Lu.w);
 }
 
-template <bool kFresh>
-__device__ __forceinline__ void stageHalfG(HalfStage& S, const RigDev& R, const uint4& raw, int chunk, int half)
+__device__ __forceinline__ void stageHalfG(HalfStage& S, const RigDev& R, const uint4& raw, int chunk, int half,
+                                           int parts)
 {
     constexpr int NC = HalfStage::kCams;
     const int j = raw.x & 0xFF, camCnt = (raw.x >> 16) & 0xFF;
@@ -1458,7 +1450,7 @@ __device__ __forceinline__ void stageHalfG(HalfStage& S, const RigDev& R, const 
     const int gc = (t & 15) * 4, gr = t >> 4 & 7, gy = ty * kBlendTH + kHalfRows * half + gr;
     const int wc = (t & 7) * 8, wr = t >> 3 & 7, wy = ty * kBlendTH + kHalfRows * half + wr;
     const int fr = t / kFW, fc = t % kFW;
-    const bool hasF = j < R.L && fr < HalfStage::kFpRows;
+    const bool hasF = (parts & kPartUp) && j < R.L && fr < HalfStage::kFpRows;
     const LevelDev& Lu = R.lv[j < R.L ? j + 1 : j];
     const size_t fo = hasF ? halfFpOffset(Lu, Lj, tx, ty, half, fr, fc) : 0;
 #pragma unroll
@@ -1466,24 +1458,24 @@ __device__ __forceinline__ void stageHalfG(HalfStage& S, const RigDev& R, const 
         f[q] = 0;
         if (q < nc && hasF) {
             const uint32_t* p = reinterpret_cast<const uint32_t*>(Lu.G) + camAt(q) * Lu.camStride + fo;
-            if (inside(p, Lu.G, gBytes(R, Lu))) f[q] = ldLevel<kFresh>(p);
+            if (inside(p, Lu.G, gBytes(R, Lu))) f[q] = __ldcg(p);
         }
     }
 #pragma unroll
     for (int i = 0; i < NC / 2; i++) {
         const int q = (t >> 7) + 2 * i;
         g[i] = make_uint4(0, 0, 0, 0);
-        if (q < nc && gy < Lj.h) {
+        if ((parts & kPartG) && q < nc && gy < Lj.h) {
             const uint4* p = reinterpret_cast<const uint4*>(Lj.G + camAt(q) * Lj.camStride + (size_t)gy * Lj.pitch +
                                                             tx * kBlendTW + gc);
-            if (inside(p, Lj.G, gBytes(R, Lj))) g[i] = ldLevel<kFresh>(p);
+            if (inside(p, Lj.G, gBytes(R, Lj))) g[i] = __ldcg(p);
         }
     }
 #pragma unroll
     for (int i = 0; i < NC / 4; i++) {
         const int q = (t >> 6) + 4 * i;
         w[i] = make_uint4(0, 0, 0, 0);
-        if (q < nc && wy < Lj.h) {
+        if ((parts & kPartW) && q < nc && wy < Lj.h) {
             const uint4* p = reinterpret_cast<const uint4*>(Lj.Wt + camAt(q) * Lj.camStride + (size_t)wy * Lj.pitch +
                                                             tx * kBlendTW + wc);
             if (inside(p, Lj.Wt, wBytes(R, Lj))) w[i] = __ldg(p);
@@ -1494,13 +1486,12 @@ __device__ __forceinline__ void stageHalfG(HalfStage& S, const RigDev& R, const 
         if (q < nc && hasF) S.fpw[q][fr * kFpW + fc + 3] = f[q];
 #pragma unroll
     for (int i = 0; i < NC / 2; i++)
-        if ((t >> 7) + 2 * i < nc) *reinterpret_cast<uint4*>(&S.gj[(t >> 7) + 2 * i][gr][gc]) = g[i];
+        if ((parts & kPartG) && (t >> 7) + 2 * i < nc) *reinterpret_cast<uint4*>(&S.gj[(t >> 7) + 2 * i][gr][gc]) = g[i];
 #pragma unroll
     for (int i = 0; i < NC / 4; i++)
-        if ((t >> 6) + 4 * i < nc) *reinterpret_cast<uint4*>(&S.w[(t >> 6) + 4 * i][wr][wc]) = w[i];
+        if ((parts & kPartW) && (t >> 6) + 4 * i < nc) *reinterpret_cast<uint4*>(&S.w[(t >> 6) + 4 * i][wr][wc]) = w[i];
 }
 
-template <bool kFresh>
 __device__ __forceinline__ void stageHalfC(HalfStage& S, const RigDev& R, const uint4& raw, int chunk, int half)
 {
     const int j = raw.x & 0xFF;
@@ -1510,7 +1501,7 @@ __device__ __forceinline__ void stageHalfC(HalfStage& S, const RigDev& R, const 
     const int r = threadIdx.x / kFW, c = threadIdx.x % kFW;
     if (r >= HalfStage::kFpRows) return;
     const uint2* p = reinterpret_cast<const uint2*>(Lu.C + halfFpOffset(Lu, R.lv[j], tx, ty, half, r, c));
-    S.cf[r][c + 1] = inside(p, Lu.C, cBytes(Lu)) ? ldLevel<kFresh>(p) : make_uint2(0, 0);
+    S.cf[r][c + 1] = inside(p, Lu.C, cBytes(Lu)) ? __ldg(p) : make_uint2(0, 0);
 }
 
 // ---- the zero-inserted upsample of a 2x2 block ----------------------------------
@@ -2461,22 +2452,21 @@ __global__ void __launch_bounds__(kThreads, 4) k_blend_small(const Segment* __re
 {
     __shared__ HalfStage st;
 
-    // Items and descriptors are written before the launch sequence, not by
-    // a kernel: the first item's are read while the previous kernel finishes.
-    // With early set (every blend step after the first: the launch before
-    // this one wrote only C levels), the first unit's G_j, weights and G_{j+1}
-    // footprints, written by launches that have completed, are staged then
-    // too, through L2; only its C_{j+1} footprint waits.
+    // Items, descriptors and weights are written before the launch sequence,
+    // not by a kernel: the first item's are fetched while the previous kernel
+    // finishes.  So are its G_j rows where that kernel is the tail (early 1: the
+    // level was complete before the tail began) and its G_{j+1} footprints where
+    // it wrote only C levels (early 2: every blend step after the first).
     int s = 0;
     uint4 raw = make_uint4(0, 0, 0, 0);
     UnitGeo geo;
     const int first = blockIdx.x;
-    const bool pre = early && first < total;
+    const int pre = kPartW | (early >= 1 ? kPartG : 0) | (early >= 2 ? kPartUp : 0);
     if (first < total) {
         s = findSegment(segs, nsegs, first, s);
         raw = __ldg(static_cast<const uint4*>(segs[s].items) + ((first - segs[s].prefix) >> 1));
         fillGeo(geo, *segs[s].rig, *segs[s].frame, raw.x & 0xFF);
-        if (pre) stageHalfG<true>(st, *segs[s].rig, raw, 0, (first - segs[s].prefix) & 1);
+        stageHalfG(st, *segs[s].rig, raw, 0, (first - segs[s].prefix) & 1, pre);
     }
     waitPrevGrid();
     allowNextGrid();
@@ -2492,9 +2482,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_blend_small(const Segment* __re
         const int half = (it - sg.prefix) & 1;
         for (int chunk = 0; chunk < unitChunks<HalfStage::kCams>(raw); chunk++) {
             __syncthreads();  // readers of the previous unit are done
-            // the first unit's G part was staged before the wait
-            if (!(pre && it == first && chunk == 0)) stageHalfG<false>(st, R, raw, chunk, half);
-            stageHalfC<false>(st, R, raw, chunk, half);
+            const int parts = it == first && chunk == 0 ? kPartsAll & ~pre : kPartsAll;
+            if (parts) stageHalfG(st, R, raw, chunk, half, parts);
+            stageHalfC(st, R, raw, chunk, half);
             __syncthreads();
             computeUnitRows(st, geo, raw, chunk, acc, half);
         }
@@ -2844,18 +2834,18 @@ cudaError_t launchLinear(const Segment* segs, int nsegs, int total, int maxCams,
 }
 
 cudaError_t launchBlend(const Segment* segs, int nsegs, int total, int perSm, int* counter, int probePolls,
-                        bool early, cudaStream_t st)
+                        int early, cudaStream_t st)
 {
     if (total <= 0) return cudaSuccess;
     return launchPdl(k_blend, gridFor(total, residentPerSm<k_blend>(kBlendThreads), perSm), kBlendThreads, st, segs,
-                     nsegs, total, counter, probePolls, (int)early);
+                     nsegs, total, counter, probePolls, (int)(early == 2));
 }
 
-cudaError_t launchBlendSmall(const Segment* segs, int nsegs, int total, bool early, cudaStream_t st)
+cudaError_t launchBlendSmall(const Segment* segs, int nsegs, int total, int early, cudaStream_t st)
 {
     if (total <= 0) return cudaSuccess;
     return launchPdl(k_blend_small, gridFor(total, residentPerSm<k_blend_small>(kThreads)), kThreads, st, segs, nsegs,
-                     total, (int)early);
+                     total, early);
 }
 
 int tailClusterMax()

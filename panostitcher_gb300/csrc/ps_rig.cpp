@@ -1440,6 +1440,7 @@ void Plan::bind(const std::vector<Rig*>& rigs)
         addStep(1, parts, (int)(slots[use] - k));
         addStep(8, pairs, (int)(slots[use] - k));
     }
+    bool tail = false;
     {
         // the tail: one cluster per rig that has one (segment count 1)
         Step s{3, (int)segs_.size(), 0, 0, -1, 0.0};
@@ -1454,6 +1455,7 @@ void Plan::bind(const std::vector<Rig*>& rigs)
         }
         s.nsegs = (int)segs_.size() - s.segOff;
         if (s.total > 0) steps_.push_back(s);
+        tail = s.total > 0;
     }
     int maxB = 0;
     for (Rig* r : rigs)
@@ -1473,7 +1475,7 @@ void Plan::bind(const std::vector<Rig*>& rigs)
         const size_t before = steps_.size();
         addStep(6, small, s);
         addStep(2, parts, s);
-        for (size_t k = before; k < steps_.size(); k++) steps_[k].early = s > 0;
+        for (size_t k = before; k < steps_.size(); k++) steps_[k].early = s > 0 ? 2 : (tail ? 1 : 0);
     }
     // one work counter per step after the segments, zeroed in every run's staged copy
     counterOff_ = (segOff_ + segs_.size() * sizeof(Segment) + 15) / 16 * 16;
