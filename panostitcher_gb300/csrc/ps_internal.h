@@ -218,7 +218,8 @@ long long boundsViolations(bool reset);
 // the first), so the G_j, weight and G_{j+1} reads of each CTA's first unit
 // may be issued before the wait for it (k_blend, k_blend_small); 1, it is the
 // tail: the G_j reads may (k_blend_small)
-cudaError_t launchBlend(const Segment* segs, int nsegs, int total, int perSm, int* counter, int probePolls,
+// work: the tiles' cameras, counted over all tiles (an uncovered one as one)
+cudaError_t launchBlend(const Segment* segs, int nsegs, int total, int work, int perSm, int* counter, int probePolls,
                         int early, cudaStream_t st);
 // blend of few-tile levels above 0: two work items (the 64x8 halves) per tile
 cudaError_t launchBlendSmall(const Segment* segs, int nsegs, int total, int early, cudaStream_t st);

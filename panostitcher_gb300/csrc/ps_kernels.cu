@@ -1528,21 +1528,26 @@ __device__ __forceinline__ void upsampleBlock(const ColumnSums* s, uint32_t one,
     out[3] = (s[1].o + s[2].o + 2 * one) >> 2;
 }
 
-// U = pyrUp(G_{j+1}) of the block from the camera's footprint g (row pitch
-// kFpW): B | R << 16 in lo, G in hi, 0..255 each.
-__device__ __forceinline__ void upsampleG(const uint32_t* g, uint32_t* lo, uint32_t* hi)
+// U = pyrUp(G_{j+1}) of the block from three columns of three footprint rows:
+// B | R << 16 in lo, G in hi, 0..255 each.
+__device__ __forceinline__ void upsampleG(const uint32_t* a, const uint32_t* b, const uint32_t* c, uint32_t* lo,
+                                          uint32_t* hi)
 {
     ColumnSums sl[3], sh[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        const uint32_t a = g[k], b = g[kFpW + k], c = g[2 * kFpW + k];
-        sl[k] = columnSums(__byte_perm(a, 0, 0x4240), __byte_perm(b, 0, 0x4240), __byte_perm(c, 0, 0x4240));
-        sh[k] = columnSums(__byte_perm(a, 0, 0x4341), __byte_perm(b, 0, 0x4341), __byte_perm(c, 0, 0x4341));
+        sl[k] = columnSums(__byte_perm(a[k], 0, 0x4240), __byte_perm(b[k], 0, 0x4240), __byte_perm(c[k], 0, 0x4240));
+        sh[k] = columnSums(__byte_perm(a[k], 0, 0x4341), __byte_perm(b[k], 0, 0x4341), __byte_perm(c[k], 0, 0x4341));
     }
     upsampleBlock(sl, 0x00010001u, lo);
     upsampleBlock(sh, 1u, hi);  // the fourth channel is 0
 #pragma unroll
     for (int p = 0; p < 4; p++) lo[p] &= 0x00FF00FFu;
+}
+// The same from a staged footprint (row pitch kFpW).
+__device__ __forceinline__ void upsampleG(const uint32_t* g, uint32_t* lo, uint32_t* hi)
+{
+    upsampleG(g, g + kFpW, g + 2 * kFpW, lo, hi);
 }
 
 // ---- the collapsed levels C_j ---------------------------------------------------
@@ -1672,96 +1677,61 @@ __device__ __forceinline__ void storeOut(const UnitGeo& G, int x, int y, const u
 __device__ __forceinline__ uint32_t biasedBR(uint32_t px) { return __byte_perm(px, 0x01010101u, 0x4240); }
 __device__ __forceinline__ uint32_t biasedG(uint32_t px) { return __byte_perm(px, 0x01010101u, 0x4341); }
 
-// Accumulate one unit from its stage; at a tile's last unit normalise,
-// collapse and store.  Threads 0..kConsumers-1.
-//
-// A uniform tile (one camera, weight 256 everywhere: 80% of level 0 of the
-// six-camera rig) is G - U + pyrUp(C) with both upsamples, the sum and the
-// saturation two channels per word: half the instructions of the general path,
-// which such a tile takes only where C leaves the packed range.
-template <class Stage>
-__device__ __forceinline__ void computeUnit(const Stage& S, const UnitGeo& G, const uint4& raw, int chunk, BlendAcc& acc)
+// A 2x2 block of a uniform tile (one camera, weight 256 everywhere: 80% of
+// level 0 of the six-camera rig) is G - U + pyrUp(C), both upsamples, the sum
+// and the saturation two channels per word: half the instructions of the
+// general path, which such a block takes only where C leaves the packed range.
+// px: the block's pixels of G; ulo .. chi: upsampleG's and upsampleC's.
+__device__ __forceinline__ void finishUniform(const UnitGeo& G, int j, int x, int y, const uint32_t* px, const uint32_t* ulo,
+                                              const uint32_t* uhi, const uint32_t* clo, const uint32_t* chi)
 {
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    const int lx = 2 * lane, ly = 2 * wp;
-    const int j = raw.x & 0xFF, cls = (raw.x >> 8) & 0xFF, camCnt = (raw.x >> 16) & 0xFF;
-    const bool uni = ((raw.x >> 24) & kTileUniform) != 0;  // weights are not read
-    const int tx = raw.y & 0xFFFF, ty = raw.y >> 16;
-    const bool hasUp = G.hasUp != 0;
-    const int x = tx * kBlendTW + lx, y = ty * kBlendTH + ly;
-    const bool active = !(j == 0 && cls == 0);
-    constexpr int NC = Stage::kCams;
-    const int c0 = chunk * NC;
-    const int nc = max(0, min(NC, camCnt - c0));
-    const bool first = chunk == 0, last = chunk == unitChunks<NC>(raw) - 1;
-    if (uni && hasUp) {
-        const CFootprint cf = loadC(&S.cf[wp][1 + lane]);
-        if (__all_sync(0xffffffffu, cInRange(cf))) {
-            uint32_t ulo[4], uhi[4], clo[4], chi[4];
-            upsampleG(&S.fpw[0][wp * kFpW + 3 + lane], ulo, uhi);
-            upsampleC(cf, clo, chi);
-            const uint2 gt = *reinterpret_cast<const uint2*>(&S.gj[0][ly][lx]);
-            const uint2 gb = *reinterpret_cast<const uint2*>(&S.gj[0][ly + 1][lx]);
-            const uint32_t gp[4] = {gt.x, gt.y, gb.x, gb.y};
-            // lanes: (256 + G - U) + (256 + C), at least 1
-            uint32_t br[4], gg[4];
+    // lanes: (256 + G - U) + (256 + C), at least 1
+    uint32_t br[4], gg[4];
 #pragma unroll
-            for (int p = 0; p < 4; p++) {
-                br[p] = biasedBR(gp[p]) - ulo[p] + clo[p];
-                gg[p] = biasedG(gp[p]) - uhi[p] + chi[p];
-            }
-            if (j > 0) {
-                uint2 v[4];
-#pragma unroll
-                for (int p = 0; p < 4; p++)  // back to one bias, as signed lanes (the fourth channel 0)
-                    v[p] = make_uint2(__viaddmax_s16x2(br[p], 0xFF00FF00u, 0x80008000u),
-                                      __viaddmax_s16x2(gg[p], 0xFF00FF00u, 0x80008000u));
-                storeC(G, x, y, v);
-                return;
-            }
-            if (y >= G.h || x >= G.w) return;
-            uint32_t o[4];
-#pragma unroll
-            for (int p = 0; p < 4; p++)  // min(max(lane - 512, 0), 255)
-                o[p] = __viaddmin_s16x2_relu(br[p], 0xFE00FE00u, 0x00FF00FFu) +
-                       (__viaddmin_s16x2_relu(gg[p], 0xFE00FE00u, 0x00FF00FFu) << 8);
-            storeOut(G, x, y, o);
-            return;
-        }
+    for (int p = 0; p < 4; p++) {
+        br[p] = biasedBR(px[p]) - ulo[p] + clo[p];
+        gg[p] = biasedG(px[p]) - uhi[p] + chi[p];
     }
-    if (first) {
+    if (j > 0) {
+        uint2 v[4];
 #pragma unroll
-        for (int p = 0; p < 4; p++) {
-            acc.r[p][0] = acc.r[p][1] = acc.r[p][2] = 0;
-            acc.wsum[p] = 0;
-        }
+        for (int p = 0; p < 4; p++)  // back to one bias, as signed lanes (the fourth channel 0)
+            v[p] = make_uint2(__viaddmax_s16x2(br[p], 0xFF00FF00u, 0x80008000u),
+                              __viaddmax_s16x2(gg[p], 0xFF00FF00u, 0x80008000u));
+        storeC(G, x, y, v);
+        return;
     }
-    if (active) {
-        for (int q = 0; q < nc; q++) {
-            uint32_t ulo[4] = {0, 0, 0, 0}, uhi[4] = {0, 0, 0, 0};
-            if (hasUp) upsampleG(&S.fpw[q][wp * kFpW + 3 + lane], ulo, uhi);
-            const uint2 gt = *reinterpret_cast<const uint2*>(&S.gj[q][ly][lx]);
-            const uint2 gb = *reinterpret_cast<const uint2*>(&S.gj[q][ly + 1][lx]);
-            const uint32_t gp[4] = {gt.x, gt.y, gb.x, gb.y};
-            uint32_t wq[2] = {0x01000100u, 0x01000100u};
-            if (!uni) {
-                wq[0] = *reinterpret_cast<const uint32_t*>(&S.w[q][ly][lx]);
-                wq[1] = *reinterpret_cast<const uint32_t*>(&S.w[q][ly + 1][lx]);
-            }
+    if (y >= G.h || x >= G.w) return;
+    uint32_t o[4];
 #pragma unroll
-            for (int p = 0; p < 4; p++) {
-                // w * (256 + L); the 256 * sum(w) comes off at normalisation
-                const uint32_t br = biasedBR(gp[p]) - ulo[p];
-                const int g = (int)(biasedG(gp[p]) & 0xFFFFu) - (int)uhi[p];
-                const int w = (int)((wq[p >> 1] >> (16 * (p & 1))) & 0xFFFFu);
-                acc.r[p][0] += w * (int)(br & 0xFFFFu);
-                acc.r[p][1] += w * g;
-                acc.r[p][2] += w * (int)(br >> 16);
-                acc.wsum[p] += w;
-            }
-        }
+    for (int p = 0; p < 4; p++)  // min(max(lane - 512, 0), 255)
+        o[p] = __viaddmin_s16x2_relu(br[p], 0xFE00FE00u, 0x00FF00FFu) +
+               (__viaddmin_s16x2_relu(gg[p], 0xFE00FE00u, 0x00FF00FFu) << 8);
+    storeOut(G, x, y, o);
+}
+
+// One camera's part of the general path: w * L, and w.
+__device__ __forceinline__ void accumulateBlock(BlendAcc& acc, const uint32_t* px, const uint32_t* ulo, const uint32_t* uhi,
+                                                const uint32_t* wq)
+{
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+        // w * (256 + L); the 256 * sum(w) comes off at normalisation
+        const uint32_t br = biasedBR(px[p]) - ulo[p];
+        const int g = (int)(biasedG(px[p]) & 0xFFFFu) - (int)uhi[p];
+        const int w = (int)((wq[p >> 1] >> (16 * (p & 1))) & 0xFFFFu);
+        acc.r[p][0] += w * (int)(br & 0xFFFFu);
+        acc.r[p][1] += w * g;
+        acc.r[p][2] += w * (int)(br >> 16);
+        acc.wsum[p] += w;
     }
-    if (!last) return;
+}
+
+// Normalise, collapse (loadUp: the C_{j+1} footprint, called where there is one)
+// and store.
+template <class LoadUp>
+__device__ __forceinline__ void finishBlock(const UnitGeo& G, int j, int cls, int x, int y, BlendAcc& acc, LoadUp loadUp)
+{
     int n[4][3];
 #pragma unroll
     for (int p = 0; p < 4; p++)
@@ -1789,7 +1759,7 @@ __device__ __forceinline__ void computeUnit(const Stage& S, const UnitGeo& G, co
         }
     }
     // collapse: + pyrUp32(C_{j+1})
-    if (hasUp && active) addUpsampledC(loadC(&S.cf[wp][1 + lane]), n);
+    if (G.hasUp != 0 && !(j == 0 && cls == 0)) addUpsampledC(loadUp(), n);
     if (j > 0) {
         uint2 v[4];
 #pragma unroll
@@ -1814,6 +1784,56 @@ __device__ __forceinline__ void computeUnit(const Stage& S, const UnitGeo& G, co
         }
     }
     storeOut(G, x, y, o);
+}
+
+// Accumulate one unit from its stage; at a tile's last unit normalise,
+// collapse and store.  Threads 0..kConsumers-1.
+template <class Stage>
+__device__ __forceinline__ void computeUnit(const Stage& S, const UnitGeo& G, const uint4& raw, int chunk, BlendAcc& acc)
+{
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int lx = 2 * lane, ly = 2 * wp;
+    const int j = raw.x & 0xFF, cls = (raw.x >> 8) & 0xFF, camCnt = (raw.x >> 16) & 0xFF;
+    const bool uni = ((raw.x >> 24) & kTileUniform) != 0;  // weights are not read
+    const int tx = raw.y & 0xFFFF, ty = raw.y >> 16;
+    const bool hasUp = G.hasUp != 0;
+    const int x = tx * kBlendTW + lx, y = ty * kBlendTH + ly;
+    constexpr int NC = Stage::kCams;
+    const int nc = max(0, min(NC, camCnt - chunk * NC));
+    auto pixels = [&](int q, uint32_t* px) {
+        const uint2 gt = *reinterpret_cast<const uint2*>(&S.gj[q][ly][lx]);
+        const uint2 gb = *reinterpret_cast<const uint2*>(&S.gj[q][ly + 1][lx]);
+        px[0] = gt.x;
+        px[1] = gt.y;
+        px[2] = gb.x;
+        px[3] = gb.y;
+    };
+    if (uni && hasUp) {
+        const CFootprint cf = loadC(&S.cf[wp][1 + lane]);
+        if (__all_sync(0xffffffffu, cInRange(cf))) {
+            uint32_t ulo[4], uhi[4], clo[4], chi[4], px[4];
+            upsampleG(&S.fpw[0][wp * kFpW + 3 + lane], ulo, uhi);
+            upsampleC(cf, clo, chi);
+            pixels(0, px);
+            finishUniform(G, j, x, y, px, ulo, uhi, clo, chi);
+            return;
+        }
+    }
+    if (chunk == 0) acc = BlendAcc{};
+    if (!(j == 0 && cls == 0)) {
+        for (int q = 0; q < nc; q++) {
+            uint32_t ulo[4] = {0, 0, 0, 0}, uhi[4] = {0, 0, 0, 0}, px[4];
+            if (hasUp) upsampleG(&S.fpw[q][wp * kFpW + 3 + lane], ulo, uhi);
+            pixels(q, px);
+            uint32_t wq[2] = {0x01000100u, 0x01000100u};
+            if (!uni) {
+                wq[0] = *reinterpret_cast<const uint32_t*>(&S.w[q][ly][lx]);
+                wq[1] = *reinterpret_cast<const uint32_t*>(&S.w[q][ly + 1][lx]);
+            }
+            accumulateBlock(acc, px, ulo, uhi, wq);
+        }
+    }
+    if (chunk == unitChunks<NC>(raw) - 1) finishBlock(G, j, cls, x, y, acc, [&] { return loadC(&S.cf[wp][1 + lane]); });
 }
 
 // The Laplacian of one pixel in half tiles: U unrounded, scaled by 64.
@@ -2151,6 +2171,189 @@ __global__ void __launch_bounds__(kBlendThreads, 4) k_blend(const Segment* __res
     if (s_timeout && threadIdx.x == 0)
         for (int k = 0; k < nsegs; k++)
             if (segs[k].frame->status) atomicOr(segs[k].frame->status, 4);
+}
+
+// ============================================================================
+// k_blend_rows: k_blend's levels of few tiles (kRowsWork), without the ring: a
+// warp takes kPairs row pairs of a tile and loads what they need straight into
+// registers.  A uniform tile's footprint rows go from one pair to the next.  The
+// ring's warm-up (a producer's trips before the first copy, the copies, a CTA's
+// eight warps on one tile) is what a launch of few tiles consists of; on larger
+// levels the ring's bulk copies move more (level 0 of 4096x2048: 45 us by rows,
+// 40 us by the ring; of 7680x3840: 107 and 83 us).  256x128: 28.5 us a frame,
+// 31.0 with the ring; 2048x1024: 74.0 against 78.4; 4096x2048: 158.4 against 160.0.
+// ============================================================================
+// The line between the two: the tiles' cameras, counted over the level's tiles.
+// 2048 mostly uniform tiles (level 0 of 2048x1024) are 4.3 us shorter here, 1800
+// tiles of two cameras (level 2 of the 8K ring) as long, 2048 tiles and 2500
+// cameras (level 1 of 6 x 1920x1080 to 4096x2048) 0.8 us longer, eight frames
+// in flight 8 us.
+constexpr int kRowsWork = 2200;
+constexpr int kRowsCtas = 3;  // CTAs per SM: 80 registers (64 spill, 2 us more)
+
+// The levels of a unit's segment and its output, a copy a warp.
+struct RowsGeo {
+    LevelDev j, u;
+    UnitGeo g;
+    const uint8_t* camLists;
+    int n;
+};
+static_assert(sizeof(LevelDev) / 4 <= 16, "two descriptions a warp, a word a lane");
+
+__device__ __forceinline__ void fillRowsGeo(RowsGeo& b, const RigDev& R, const FrameDev& F, int j)
+{
+    const int lane = threadIdx.x & 31, k = lane & 15;
+    __syncwarp();
+    if (k < (int)sizeof(LevelDev) / 4)
+        reinterpret_cast<uint32_t*>(lane < 16 ? &b.j : &b.u)[k] =
+            __ldg(reinterpret_cast<const uint32_t*>(&R.lv[lane < 16 ? j : min(j + 1, R.L)]) + k);
+    if (lane == 0) {
+        fillGeo(b.g, R, F, j);
+        b.camLists = R.camLists;
+        b.n = R.n;
+    }
+    __syncwarp();
+}
+
+// Pixel (x, y) of camera cam at the unit's level, rows y and y + 1.
+__device__ __forceinline__ void rowsPixels(const RowsGeo& B, int cam, int x, int y, uint32_t* px)
+{
+    const uint2* p = reinterpret_cast<const uint2*>(B.j.G + (size_t)cam * B.j.camStride + (size_t)y * B.j.pitch + x);
+    const uint2* q = p + B.j.pitch / 2;
+    const long long ext = (long long)B.n * B.j.camStride * 4;
+    const uint2 t = inside(p, B.j.G, ext) ? __ldg(p) : make_uint2(0, 0);
+    const uint2 b = y + 1 < B.j.h && inside(q, B.j.G, ext) ? __ldg(q) : make_uint2(0, 0);
+    px[0] = t.x;
+    px[1] = t.y;
+    px[2] = b.x;
+    px[3] = b.y;
+}
+// Three columns of a row of the level above: a camera's G, and C.
+__device__ __forceinline__ void rowsFootprint(const RowsGeo& B, const uint32_t* row, const int* col, uint32_t* f)
+{
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        f[k] = inside(row + col[k], B.u.G, (long long)B.n * B.u.camStride * 4) ? __ldg(row + col[k]) : 0u;
+}
+__device__ __forceinline__ void rowsFootprint(const RowsGeo& B, const uint2* row, const int* col, uint2* f)
+{
+#pragma unroll
+    for (int k = 0; k < 3; k++) f[k] = inside(row + col[k], B.u.C, cBytes(B.u)) ? __ldg(row + col[k]) : make_uint2(0, 0);
+}
+__device__ __forceinline__ int rowsOffset(const RowsGeo& B, int y, int r)
+{
+    return rowMap(y / 2 - 1 + r, B.u.h) * B.u.pitch;
+}
+
+// One row pair, any cameras, any values.
+__device__ __forceinline__ void rowsPair(const RowsGeo& B, const uint4& raw, int x, int y, const int* col)
+{
+    const int j = raw.x & 0xFF, cls = (raw.x >> 8) & 0xFF, camCnt = (raw.x >> 16) & 0xFF;
+    const bool uni = ((raw.x >> 24) & kTileUniform) != 0, hasUp = B.g.hasUp != 0;
+    BlendAcc acc{};
+    if (!(j == 0 && cls == 0)) {
+        for (int q = 0; q < camCnt; q++) {
+            const int cam = tileCam(raw, B.camLists, q);
+            uint32_t ulo[4] = {0, 0, 0, 0}, uhi[4] = {0, 0, 0, 0}, px[4], f[3][3];
+            rowsPixels(B, cam, x, y, px);
+            uint32_t wq[2] = {0x01000100u, 0x01000100u};
+            if (!uni) {
+                const uint32_t* p =
+                    reinterpret_cast<const uint32_t*>(B.j.Wt + (size_t)cam * B.j.camStride + (size_t)y * B.j.pitch + x);
+                const uint32_t* p1 = p + B.j.pitch / 2;
+                const long long ext = (long long)B.n * B.j.camStride * 2;
+                wq[0] = inside(p, B.j.Wt, ext) ? __ldg(p) : 0u;
+                wq[1] = y + 1 < B.j.h && inside(p1, B.j.Wt, ext) ? __ldg(p1) : 0u;
+            }
+            if (hasUp) {
+                const uint32_t* U = reinterpret_cast<const uint32_t*>(B.u.G) + (size_t)cam * B.u.camStride;
+#pragma unroll
+                for (int r = 0; r < 3; r++) rowsFootprint(B, U + rowsOffset(B, y, r), col, f[r]);
+                upsampleG(f[0], f[1], f[2], ulo, uhi);
+            }
+            accumulateBlock(acc, px, ulo, uhi, wq);
+        }
+    }
+    finishBlock(B.g, j, cls, x, y, acc, [&] {
+        CFootprint c;
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+            rowsFootprint(B, reinterpret_cast<const uint2*>(B.u.C) + rowsOffset(B, y, r), col, c.v[r]);
+        return c;
+    });
+}
+
+template <int kPairs>
+__global__ void __launch_bounds__(kThreads, kRowsCtas) k_blend_rows(const Segment* __restrict__ segs, int nsegs, int total,
+                                                                    int probePolls)
+{
+    __shared__ RowsGeo s_geo[kThreads / 32];
+    __shared__ uint64_t never;
+    constexpr int kParts = kBlendTH / 2 / kPairs;  // units of a tile
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) mbarInit(&never, 1);
+    __syncthreads();
+    RowsGeo& B = s_geo[warp];
+    const int units = total * kParts, first = blockIdx.x * (kThreads / 32) + warp;
+    int seg = 0, filled = -1;
+    for (int u = first; u < units; u += gridDim.x * (kThreads / 32)) {
+        seg = findSegment(segs, nsegs, u / kParts, seg);
+        const uint4 raw = __ldg(static_cast<const uint4*>(segs[seg].items) + (u / kParts - segs[seg].prefix));
+        const int j = raw.x & 0xFF, cls = (raw.x >> 8) & 0xFF;
+        if (seg != filled) fillRowsGeo(B, *segs[seg].rig, *segs[seg].frame, j);
+        if (filled < 0) {  // items and descriptors are written before the launch sequence, not by a kernel
+            waitPrevGrid();
+            allowNextGrid();
+            if (probePolls > 0 && threadIdx.x == 0 && !mbarWait(&never, 0, probePolls)) flagTimeout(segs, nsegs);
+        }
+        filled = seg;
+        const int tx = raw.y & 0xFFFF, ty = raw.y >> 16;
+        const int x = tx * kBlendTW + 2 * lane, y0 = ty * kBlendTH + u % kParts * (2 * kPairs);
+        const int rows = (B.g.h - y0 + 1) / 2;                     // row pairs inside the level
+        int todo = rows <= 0 ? 0 : (1 << min(kPairs, rows)) - 1;  // left for the general path
+        int col[3] = {0, 0, 0};
+        if (B.g.hasUp) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) col[k] = colMap(tx * (kBlendTW / 2) - 1 + lane + k, B.u.w);
+        }
+        if ((raw.x >> 24 & kTileUniform) && B.g.hasUp && rows >= kPairs && (j | cls)) {
+            const int cam = tileCam(raw, B.camLists, 0);
+            const uint32_t* U = reinterpret_cast<const uint32_t*>(B.u.G) + (size_t)cam * B.u.camStride;
+            const uint2* C = reinterpret_cast<const uint2*>(B.u.C);
+            uint32_t f[kPairs + 2][3], px[kPairs][4];
+            uint2 c[kPairs + 2][3];
+#pragma unroll
+            for (int r = 0; r < kPairs + 2; r++) {
+                const int o = rowsOffset(B, y0, r);
+                rowsFootprint(B, U + o, col, f[r]);
+                rowsFootprint(B, C + o, col, c[r]);
+            }
+#pragma unroll
+            for (int p = 0; p < kPairs; p++) rowsPixels(B, cam, x, y0 + 2 * p, px[p]);
+            todo = 0;
+#pragma unroll
+            for (int p = 0; p < kPairs; p++) {
+                CFootprint cf;
+#pragma unroll
+                for (int r = 0; r < 3; r++)
+#pragma unroll
+                    for (int k = 0; k < 3; k++) cf.v[r][k] = c[p + r][k];
+                if (!__all_sync(0xffffffffu, cInRange(cf))) {
+                    todo |= 1 << p;
+                    continue;
+                }
+                uint32_t ulo[4], uhi[4], clo[4], chi[4];
+                upsampleG(f[p], f[p + 1], f[p + 2], ulo, uhi);
+                upsampleC(cf, clo, chi);
+                finishUniform(B.g, j, x, y0 + 2 * p, px[p], ulo, uhi, clo, chi);
+            }
+        }
+        for (; todo; todo &= todo - 1) rowsPair(B, raw, x, y0 + 2 * (__ffs(todo) - 1), col);
+    }
+    if (filled < 0) {
+        waitPrevGrid();
+        allowNextGrid();
+    }
 }
 
 // ============================================================================
@@ -2833,10 +3036,17 @@ cudaError_t launchLinear(const Segment* segs, int nsegs, int total, int maxCams,
     }
 }
 
-cudaError_t launchBlend(const Segment* segs, int nsegs, int total, int perSm, int* counter, int probePolls,
+cudaError_t launchBlend(const Segment* segs, int nsegs, int total, int work, int perSm, int* counter, int probePolls,
                         int early, cudaStream_t st)
 {
     if (total <= 0) return cudaSuccess;
+    if (work <= kRowsWork) {
+        // a row pair a warp, two where the warps would take more than one
+        const bool two = total * (kBlendTH / 4) >= smCount() * kRowsCtas * (kThreads / 32);
+        const int ctas = (total * (kBlendTH / (two ? 4 : 2)) + kThreads / 32 - 1) / (kThreads / 32);
+        auto* kernel = two ? k_blend_rows<2> : k_blend_rows<1>;
+        return launchPdl(kernel, gridFor(ctas, kRowsCtas, perSm), kThreads, st, segs, nsegs, total, probePolls);
+    }
     return launchPdl(k_blend, gridFor(total, residentPerSm<k_blend>(kBlendThreads), perSm), kBlendThreads, st, segs,
                      nsegs, total, counter, probePolls, (int)(early == 2));
 }

@@ -480,43 +480,42 @@ void Rig::preparePyramids(const uint8_t* cov, const uint8_t* seam, const float* 
         rflags.zero(st);
         PS_CUDA(launchTileFlags8(cov, W, H, W, (long long)npx, n, kRemapTW, kRemapTH, rX, rY, rflags.as<uint8_t>(), st));
     }
-    // of a level's tiles: any alpha, an alpha below 256; of its 16x8 quarters: any alpha
-    std::vector<DevBuf> dflags(L + 1), pflags(L + 1), qflags(L + 1);
+    // of a level's tiles: any alpha, an alpha below 256; of its 16x8 quarters:
+    // any alpha (one buffer for all levels)
+    std::vector<size_t> dOff(L + 2), pOff(L + 2), qOff(L + 2);
+    size_t flagBytes = 0;
+    for (int j = 1; j <= L; j++) {
+        const LevelGeom& g = geom_[j];
+        const size_t tiles = (size_t)n * divUp(g.w, kDownTW) * divUp(g.h, kDownTH);
+        dOff[j] = flagBytes;
+        pOff[j] = dOff[j] + tiles;
+        qOff[j] = pOff[j] + tiles;
+        flagBytes = qOff[j] + (size_t)n * divUp(g.w, kDownTW / 2) * divUp(g.h, kDownTH / 2);
+    }
+    DevBuf flags(std::max<size_t>(1, flagBytes));
+    flags.zero(st);
     DevBuf counts(sizeof(unsigned long long));
     counts.zero(st);
     for (int j = 1; j <= L; j++) {
         const LevelGeom& g = geom_[j];
         const long long stride = (long long)g.pitch * g.h;
+        const uint16_t* am = lv_[j].Am.as<uint16_t>();
         const int dX = divUp(g.w, kDownTW), dY = divUp(g.h, kDownTH);
-        dflags[j].alloc((size_t)n * dX * dY);
-        dflags[j].zero(st);
-        PS_CUDA(launchTileFlags16(lv_[j].Am.as<uint16_t>(), g.w, g.h, g.pitch, stride, n, kDownTW, kDownTH, dX, dY,
-                                  dflags[j].as<uint8_t>(), st));
-        pflags[j].alloc(dflags[j].bytes());
-        pflags[j].zero(st);
-        PS_CUDA(launchTileNot256(lv_[j].Am.as<uint16_t>(), g.w, g.h, g.pitch, stride, n, kDownTW, kDownTH, dX, dY,
-                                 pflags[j].as<uint8_t>(), st));
         const int qX = divUp(g.w, kDownTW / 2), qY = divUp(g.h, kDownTH / 2);
-        qflags[j].alloc((size_t)n * qX * qY);
-        qflags[j].zero(st);
-        PS_CUDA(launchTileFlags16(lv_[j].Am.as<uint16_t>(), g.w, g.h, g.pitch, stride, n, kDownTW / 2, kDownTH / 2, qX, qY,
-                                  qflags[j].as<uint8_t>(), st));
-        PS_CUDA(launchCountNonzero16(lv_[j].Am.as<uint16_t>(), g.w, g.h, g.pitch, stride, n,
-                                     counts.as<unsigned long long>(), st));
+        PS_CUDA(launchTileFlags16(am, g.w, g.h, g.pitch, stride, n, kDownTW, kDownTH, dX, dY,
+                                  flags.as<uint8_t>() + dOff[j], st));
+        PS_CUDA(launchTileNot256(am, g.w, g.h, g.pitch, stride, n, kDownTW, kDownTH, dX, dY,
+                                 flags.as<uint8_t>() + pOff[j], st));
+        PS_CUDA(launchTileFlags16(am, g.w, g.h, g.pitch, stride, n, kDownTW / 2, kDownTH / 2, qX, qY,
+                                  flags.as<uint8_t>() + qOff[j], st));
+        PS_CUDA(launchCountNonzero16(am, g.w, g.h, g.pitch, stride, n, counts.as<unsigned long long>(), st));
     }
     unsigned long long hAlpha = 0;
     std::vector<uint8_t> hR(xmap ? rflags.bytes() : 0);
-    std::vector<std::vector<uint8_t>> hD(L + 1), hP(L + 1), hQ(L + 1);
+    std::vector<uint8_t> hFlags(flagBytes);
     PS_CUDA(cudaMemcpyAsync(&hAlpha, counts.get(), sizeof hAlpha, cudaMemcpyDeviceToHost, st));
     if (xmap) PS_CUDA(cudaMemcpyAsync(hR.data(), rflags.get(), hR.size(), cudaMemcpyDeviceToHost, st));
-    for (int j = 1; j <= L; j++) {
-        hD[j].resize(dflags[j].bytes());
-        PS_CUDA(cudaMemcpyAsync(hD[j].data(), dflags[j].get(), hD[j].size(), cudaMemcpyDeviceToHost, st));
-        hP[j].resize(pflags[j].bytes());
-        PS_CUDA(cudaMemcpyAsync(hP[j].data(), pflags[j].get(), hP[j].size(), cudaMemcpyDeviceToHost, st));
-        hQ[j].resize(qflags[j].bytes());
-        PS_CUDA(cudaMemcpyAsync(hQ[j].data(), qflags[j].get(), hQ[j].size(), cudaMemcpyDeviceToHost, st));
-    }
+    if (flagBytes) PS_CUDA(cudaMemcpyAsync(hFlags.data(), flags.get(), flagBytes, cudaMemcpyDeviceToHost, st));
     std::vector<uint8_t> hCov(n * npx), hSeam(n * npx);
     PS_CUDA(cudaMemcpyAsync(hCov.data(), cov, n * npx, cudaMemcpyDeviceToHost, st));
     PS_CUDA(cudaMemcpyAsync(hSeam.data(), seam, n * npx, cudaMemcpyDeviceToHost, st));
@@ -547,8 +546,8 @@ void Rig::preparePyramids(const uint8_t* cov, const uint8_t* seam, const float* 
             for (int ty = 0; ty < dY; ty++)
                 for (int tx = 0; tx < dX; tx++) {
                     const size_t t = ((size_t)c * dY + ty) * dX + tx;
-                    if (hD[j][t])
-                        down.push_back({(uint8_t)c, (uint8_t)j, (uint16_t)tx, (uint16_t)ty, (uint16_t)!hP[j][t]});
+                    if (hFlags[dOff[j] + t])
+                        down.push_back({(uint8_t)c, (uint8_t)j, (uint16_t)tx, (uint16_t)ty, (uint16_t)!hFlags[pOff[j] + t]});
                 }
         downCnt_[j] = (int)down.size() - downOff_[j];
     }
@@ -565,8 +564,8 @@ void Rig::preparePyramids(const uint8_t* cov, const uint8_t* seam, const float* 
         for (int c = 0; c < n; c++)
             for (int ty = 0; ty < dY; ty++)
                 for (int tx = 0; tx < dX; tx++)
-                    if (hD[j][((size_t)c * dY + ty) * dX + tx] ||
-                        (tx < qX && ty < qY && hQ[j + 1][((size_t)c * qY + ty) * qX + tx]))
+                    if (hFlags[dOff[j] + ((size_t)c * dY + ty) * dX + tx] ||
+                        (tx < qX && ty < qY && hFlags[qOff[j + 1] + ((size_t)c * qY + ty) * qX + tx]))
                         down.push_back({(uint8_t)c, (uint8_t)j, (uint16_t)tx, (uint16_t)ty, 0});
         if ((int)down.size() - pairOff_[j] > kPairTiles) down.resize(pairOff_[j]);
         pairCnt_[j] = (int)down.size() - pairOff_[j];
@@ -695,6 +694,7 @@ void Rig::buildBlendState(const uint8_t* uniSrc, bool custom, cudaStream_t st)
         const LevelGeom& g = geom_[j];
         const int bX = divUp(g.w, kBlendTW), bY = divUp(g.h, kBlendTH);
         blendOff_[j] = (int)blend.size();
+        blendWork_[j] = 0;
         for (int ty = 0; ty < bY; ty++)
             for (int tx = 0; tx < bX; tx++) {
                 std::vector<uint8_t> list;
@@ -722,6 +722,7 @@ void Rig::buildBlendState(const uint8_t* uniSrc, bool custom, cudaStream_t st)
                     cams.insert(cams.end(), list.begin(), list.end());
                 }
                 blend.push_back(it);
+                blendWork_[j] += std::max<int>(1, it.camCnt);
             }
         blendCnt_[j] = (int)blend.size() - blendOff_[j];
     }
@@ -1394,6 +1395,7 @@ void Plan::bind(const std::vector<Rig*>& rigs)
                             : kind == 1 || kind == 8 ? std::abs(downSteps[p.first][downSteps[p.first].size() - step])
                                                      : rg->tailStart() - 1 - step;
             if (s.level < 0) s.level = lvl;
+            if (kind == 2) s.work += rg->blendWork(lvl);
             if (kind == 8) s.bytes += rg->stepBytes(1, lvl) + rg->stepBytes(1, lvl + 1);
             else s.bytes += rg->stepBytes(kind == 6 ? 2 : kind, lvl);
         }
@@ -1535,7 +1537,7 @@ void Plan::launchAll(const IoSlot& slot, cudaStream_t st, int srcFmt, Profiler* 
         if (s.kind == 0) PS_CUDA(launchRemap(p, s.nsegs, s.total, perSm_[0], counters + si, srcFmt, maps_, st));
         else if (s.kind == 1) PS_CUDA(launchPyrDown(p, s.nsegs, s.total, perSm_[1], st));
         else if (s.kind == 8) PS_CUDA(launchPyrDownPair(p, s.nsegs, s.total, st));
-        else if (s.kind == 2) PS_CUDA(launchBlend(p, s.nsegs, s.total, perSm_[2], counters + si, probe_, s.early, st));
+        else if (s.kind == 2) PS_CUDA(launchBlend(p, s.nsegs, s.total, s.work, perSm_[2], counters + si, probe_, s.early, st));
         else if (s.kind == 3) PS_CUDA(launchTail(p, s.nsegs, tailCluster_, tailCams_, st));
         else if (s.kind == 6) PS_CUDA(launchBlendSmall(p, s.nsegs, s.total, s.early, st));
         else PS_CUDA(launchLinear(p, s.nsegs, s.total, maxCams_, srcFmt, st));

@@ -151,6 +151,7 @@ public:
     std::vector<int> downSteps(bool pairs) const;
     const BlendItem* blendItems(int level) const { return dBlend_.as<BlendItem>() + blendOff_[level]; }
     int numBlendItems(int level) const { return blendCnt_[level]; }
+    int blendWork(int level) const { return blendWork_[level]; }  // the tiles' cameras
     // Launch shape (tail split, tail cluster and tile split, CTAs per SM).
     // Set before prepare, it applies at prepare; set after, it waits for the
     // rig's runs to finish (waitIdle), rewrites the descriptors and starts a
@@ -217,7 +218,7 @@ private:
     std::vector<RemapItem> hRemap_;
     int downOff_[PS_MAX_LEVELS + 1] = {}, downCnt_[PS_MAX_LEVELS + 1] = {};
     int pairOff_[PS_MAX_LEVELS + 1] = {}, pairCnt_[PS_MAX_LEVELS + 1] = {};
-    int blendOff_[PS_MAX_LEVELS + 1] = {}, blendCnt_[PS_MAX_LEVELS + 1] = {};
+    int blendOff_[PS_MAX_LEVELS + 1] = {}, blendCnt_[PS_MAX_LEVELS + 1] = {}, blendWork_[PS_MAX_LEVELS + 1] = {};
     int tailStart_ = 1;
     LaunchShape shape_;
     RigDev hDesc_ = {};  // slot-independent part of the descriptors
@@ -282,6 +283,7 @@ private:
         int segOff, nsegs, total;
         int level;      // level of the first rig in the step
         double bytes;   // algorithmic bytes of the step (all rigs)
+        int work = 0;   // of a blend step: its tiles' cameras
         int early = 0;  // of a blend step, the launch before: 2 wrote only C levels, 1 is the tail
     };
     // Per-run state in kIoSlots copies: run k uses slot k % kIoSlots, so while
