@@ -214,10 +214,11 @@ cudaError_t launchPyrDownPair(const Segment* segs, int nsegs, int total, cudaStr
 // (waits for the device); -1 in the normal build, -2 on a CUDA error.
 long long boundsViolations(bool reset);
 // probePolls > 0: the failure-path test of the bounded waits (k_blend).
-// early: 2, the launch before this one wrote only C levels (a blend step after
-// the first), so the G_j, weight and G_{j+1} reads of each CTA's first unit
-// may be issued before the wait for it (k_blend, k_blend_small); 1, it is the
-// tail: the G_j reads may (k_blend_small)
+// early: what of a launch's first units may precede its wait for the launch
+// before: their G_j reads (that launch is the tail), those and the G_{j+1} reads
+// too (it wrote only C levels: a blend step after the first); and of few-tile
+// launches: this one begins when that one does; the next one does with this one
+constexpr int kEarlyG = 1, kEarlyUp = 2, kEarlyBegin = 4, kEarlyNext = 8;
 // work: the tiles' cameras, counted over all tiles (an uncovered one as one)
 cudaError_t launchBlend(const Segment* segs, int nsegs, int total, int work, int perSm, int* counter, int probePolls,
                         int early, cudaStream_t st);

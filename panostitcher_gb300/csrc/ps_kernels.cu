@@ -1416,8 +1416,6 @@ __device__ __forceinline__ void stageUnitDirect(Stage& S, const RigDev& R, const
 //
 // stageHalfG: of the cameras' G_j rows, weights and G_{j+1} footprints the
 // parts asked for, through L2 (what another launch wrote while this one began).
-// stageHalfC: the C_{j+1} footprint, with a tile's last unit -- the only part
-// the level above's blend writes, so the rest may be staged before it.
 static_assert(HalfStage::kFpRows * kFW <= kConsumers, "a footprint element a thread");
 constexpr int kPartW = 1, kPartG = 2, kPartUp = 4, kPartsAll = 7;
 
@@ -1490,18 +1488,6 @@ __device__ __forceinline__ void stageHalfG(HalfStage& S, const RigDev& R, const 
 #pragma unroll
     for (int i = 0; i < NC / 4; i++)
         if ((parts & kPartW) && (t >> 6) + 4 * i < nc) *reinterpret_cast<uint4*>(&S.w[(t >> 6) + 4 * i][wr][wc]) = w[i];
-}
-
-__device__ __forceinline__ void stageHalfC(HalfStage& S, const RigDev& R, const uint4& raw, int chunk, int half)
-{
-    const int j = raw.x & 0xFF;
-    const int tx = raw.y & 0xFFFF, ty = raw.y >> 16;
-    if (j >= R.L || chunk != unitChunks<HalfStage::kCams>(raw) - 1) return;
-    const LevelDev& Lu = R.lv[j + 1];
-    const int r = threadIdx.x / kFW, c = threadIdx.x % kFW;
-    if (r >= HalfStage::kFpRows) return;
-    const uint2* p = reinterpret_cast<const uint2*>(Lu.C + halfFpOffset(Lu, R.lv[j], tx, ty, half, r, c));
-    S.cf[r][c + 1] = inside(p, Lu.C, cBytes(Lu)) ? __ldg(p) : make_uint2(0, 0);
 }
 
 // ---- the zero-inserted upsample of a 2x2 block ----------------------------------
@@ -1860,8 +1846,25 @@ struct PairAcc {
     int wsum0, wsum1;
 };
 
-__device__ __forceinline__ void computeUnitRows(const HalfStage& S, const UnitGeo& G, const uint4& raw, int chunk,
-                                                PairAcc& acc, int half)
+// The thread's element of the C_{j+1} footprint.
+__device__ __forceinline__ size_t halfCOffset(const RigDev& R, const uint4& raw, int half)
+{
+    const int j = raw.x & 0xFF, r = threadIdx.x / kFW, c = threadIdx.x % kFW;
+    if (j >= R.L || r >= HalfStage::kFpRows) return 0;
+    return halfFpOffset(R.lv[j + 1], R.lv[j], raw.y & 0xFFFF, raw.y >> 16, half, r, c);
+}
+__device__ __forceinline__ void stageHalfC(HalfStage& S, const RigDev& R, int j, size_t offset)
+{
+    const int r = threadIdx.x / kFW, c = threadIdx.x % kFW;
+    if (j >= R.L || r >= HalfStage::kFpRows) return;
+    const LevelDev& Lu = R.lv[j + 1];
+    const uint2* p = reinterpret_cast<const uint2*>(Lu.C + offset);
+    S.cf[r][c + 1] = inside(p, Lu.C, cBytes(Lu)) ? __ldg(p) : make_uint2(0, 0);
+}
+
+// Accumulate one unit's cameras.
+__device__ __forceinline__ void accumulateRows(const HalfStage& S, const UnitGeo& G, const uint4& raw, int chunk,
+                                               PairAcc& acc)
 {
     const int lx = (threadIdx.x & 31) * 2, ly = threadIdx.x >> 5;  // row in the half tile
     // vertical taps: even rows footprint rows ly/2 .. ly/2+2 (1 6 1), odd rows
@@ -1869,17 +1872,11 @@ __device__ __forceinline__ void computeUnitRows(const HalfStage& S, const UnitGe
     const bool evenRow = (ly & 1) == 0;
     const int vr0 = evenRow ? ly / 2 : (ly + 1) / 2;
     const int fc = lx / 2;
-    const int j = raw.x & 0xFF, camCnt = (raw.x >> 16) & 0xFF;
-    const int tx = raw.y & 0xFFFF, ty = raw.y >> 16;
+    const int camCnt = (raw.x >> 16) & 0xFF;
     const bool hasUp = G.hasUp != 0;
-    const int x = tx * kBlendTW + lx, y = ty * kBlendTH + kHalfRows * half + ly;
     constexpr int NC = HalfStage::kCams;
     const int nc = max(0, min(NC, camCnt - chunk * NC));
-    const bool first = chunk == 0, last = chunk == unitChunks<NC>(raw) - 1;
-    if (first) {
-        acc.r0[0] = acc.r0[1] = acc.r0[2] = acc.r1[0] = acc.r1[1] = acc.r1[2] = 0;
-        acc.wsum0 = acc.wsum1 = 0;
-    }
+    if (chunk == 0) acc = PairAcc{};
 #pragma unroll 2
     for (int q = 0; q < nc; q++) {
         uint32_t u0lo = 0, u0hi = 0, u1lo = 0, u1hi = 0;
@@ -1918,12 +1915,15 @@ __device__ __forceinline__ void computeUnitRows(const HalfStage& S, const UnitGe
         acc.wsum0 += w0;
         acc.wsum1 += w1;
     }
-    if (!last) return;
+}
+
+// The two pixels' normalised values.
+__device__ __forceinline__ void normaliseRows(const UnitGeo& G, PairAcc& acc, int* n0, int* n1)
+{
     acc.r0[0] -= acc.wsum0 << 8;
     acc.r0[2] -= acc.wsum0 << 8;
     acc.r1[0] -= acc.wsum1 << 8;
     acc.r1[2] -= acc.wsum1 << 8;
-    int n0[3], n1[3];
     if (G.full) {
 #pragma unroll
         for (int c = 0; c < 3; c++) { n0[c] = (acc.r0[c] + 128) >> 8; n1[c] = (acc.r1[c] + 128) >> 8; }
@@ -1933,7 +1933,15 @@ __device__ __forceinline__ void computeUnitRows(const HalfStage& S, const UnitGe
 #pragma unroll
         for (int c = 0; c < 3; c++) { n0[c] = divTrunc(acc.r0[c], d0, i0); n1[c] = divTrunc(acc.r1[c], d1, i1); }
     }
-    if (hasUp) {
+}
+
+// Collapse (the staged C_{j+1} footprint) and store.
+__device__ __forceinline__ void collapseRows(const HalfStage& S, const UnitGeo& G, int x, int y, int* n0, int* n1)
+{
+    if (G.hasUp) {
+        const int ly = threadIdx.x >> 5, fc = threadIdx.x & 31;
+        const bool evenRow = (ly & 1) == 0;
+        const int vr0 = evenRow ? ly / 2 : (ly + 1) / 2;
         const uint2* cf = &S.cf[0][0] + 1;
         int v[3][3];
 #pragma unroll
@@ -1958,7 +1966,6 @@ __device__ __forceinline__ void computeUnitRows(const HalfStage& S, const UnitGe
             n1[c] += ((4 * (v[1][c] + v[2][c]) + 32) >> 6) - kCBias;
         }
     }
-    if (y >= G.h || j == 0) return;  // level 0 goes through computeUnit
     uint2* Cj = reinterpret_cast<uint2*>(G.C) + (size_t)y * G.pitch + x;
     const long long cext = (long long)G.pitch * G.h * 8;
     const uint2 c0 = packC(n0[0], n0[1], n0[2]), c1 = packC(n1[0], n1[1], n1[2]);
@@ -2643,8 +2650,8 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(const Segment* __restrict
 }
 
 // ============================================================================
-// k_blend_small: blend levels above 0 with few tiles, below the tail.  The
-// tail kernel's per-unit code on a plain grid: one 64x8 half tile per work
+// k_blend_small: blend levels above 0 with few tiles, below the tail, on a
+// plain grid: one 64x8 half tile per work
 // item (items 2t and 2t + 1 are the halves of tile t), up to eight cameras
 // staged per unit.  In k_blend a CTA walks a tile's cameras two at a time,
 // a chain of load-and-compute rounds that these levels cannot hide behind
@@ -2657,41 +2664,64 @@ __global__ void __launch_bounds__(kThreads, 4) k_blend_small(const Segment* __re
 
     // Items, descriptors and weights are written before the launch sequence,
     // not by a kernel: the first item's are fetched while the previous kernel
-    // finishes.  So are its G_j rows where that kernel is the tail (early 1: the
+    // finishes.  So are its G_j rows where that kernel is the tail (kEarlyG: the
     // level was complete before the tail began) and its G_{j+1} footprints where
-    // it wrote only C levels (early 2: every blend step after the first).
-    int s = 0;
-    uint4 raw = make_uint4(0, 0, 0, 0);
+    // it wrote only C levels (kEarlyUp: every blend step after the first); only
+    // the C_{j+1} footprint waits.  A launch that begins with the one before it
+    // (kEarlyBegin) has the time to normalise its first item ahead of the wait
+    // too.  It may: all G levels were complete before the first blend step let
+    // its successor begin.
+    const int pre = kPartW | (early & kEarlyG ? kPartG : 0) | (early & kEarlyUp ? kPartUp : 0);
+    const bool begun = (early & kEarlyBegin) != 0;
+    if (early & kEarlyNext) allowNextGrid();
+    bool waited = false;
+    auto wait = [&] {
+        waitPrevGrid();
+        if (!(early & kEarlyNext)) allowNextGrid();
+        waited = true;
+    };
+    int s = 0, filled = -1;
     UnitGeo geo;
-    const int first = blockIdx.x;
-    const int pre = kPartW | (early >= 1 ? kPartG : 0) | (early >= 2 ? kPartUp : 0);
-    if (first < total) {
-        s = findSegment(segs, nsegs, first, s);
-        raw = __ldg(static_cast<const uint4*>(segs[s].items) + ((first - segs[s].prefix) >> 1));
-        fillGeo(geo, *segs[s].rig, *segs[s].frame, raw.x & 0xFF);
-        stageHalfG(st, *segs[s].rig, raw, 0, (first - segs[s].prefix) & 1, pre);
-    }
-    waitPrevGrid();
-    allowNextGrid();
     PairAcc acc;
-    for (int it = first; it < total; it += gridDim.x) {
-        if (it != first) {
-            s = findSegment(segs, nsegs, it, s);
-            raw = __ldg(static_cast<const uint4*>(segs[s].items) + ((it - segs[s].prefix) >> 1));
-            fillGeo(geo, *segs[s].rig, *segs[s].frame, raw.x & 0xFF);
-        }
+    for (int it = blockIdx.x; it < total; it += gridDim.x) {
+        s = findSegment(segs, nsegs, it, s);
         const Segment& sg = segs[s];
         const RigDev& R = *sg.rig;
+        const uint4 raw = __ldg(static_cast<const uint4*>(sg.items) + ((it - sg.prefix) >> 1));
+        if (s != filled) fillGeo(geo, R, *sg.frame, raw.x & 0xFF);
+        filled = s;
         const int half = (it - sg.prefix) & 1;
-        for (int chunk = 0; chunk < unitChunks<HalfStage::kCams>(raw); chunk++) {
+        const size_t up = halfCOffset(R, raw, half);
+        const int chunks = unitChunks<HalfStage::kCams>(raw);
+        bool staged = false;  // the C_{j+1} footprint
+        for (int chunk = 0; chunk < chunks; chunk++) {
             __syncthreads();  // readers of the previous unit are done
-            const int parts = it == first && chunk == 0 ? kPartsAll & ~pre : kPartsAll;
+            int parts = kPartsAll;
+            if (!waited && !begun) {
+                stageHalfG(st, R, raw, chunk, half, pre);
+                wait();
+                parts &= ~pre;
+            }
             if (parts) stageHalfG(st, R, raw, chunk, half, parts);
-            stageHalfC(st, R, raw, chunk, half);
+            if (waited && chunk == chunks - 1) {
+                stageHalfC(st, R, raw.x & 0xFF, up);
+                staged = true;
+            }
             __syncthreads();
-            computeUnitRows(st, geo, raw, chunk, acc, half);
+            accumulateRows(st, geo, raw, chunk, acc);
         }
+        int n0[3], n1[3];
+        normaliseRows(geo, acc, n0, n1);
+        if (!staged) {
+            wait();
+            stageHalfC(st, R, raw.x & 0xFF, up);
+            __syncthreads();
+        }
+        const int x = (int)(raw.y & 0xFFFF) * kBlendTW + (threadIdx.x & 31) * 2;
+        const int y = (int)(raw.y >> 16) * kBlendTH + kHalfRows * half + (threadIdx.x >> 5);
+        if (y < geo.h) collapseRows(st, geo, x, y, n0, n1);
     }
+    if (!waited) wait();
 }
 
 // ============================================================================
@@ -3048,7 +3078,7 @@ cudaError_t launchBlend(const Segment* segs, int nsegs, int total, int work, int
         return launchPdl(kernel, gridFor(ctas, kRowsCtas, perSm), kThreads, st, segs, nsegs, total, probePolls);
     }
     return launchPdl(k_blend, gridFor(total, residentPerSm<k_blend>(kBlendThreads), perSm), kBlendThreads, st, segs,
-                     nsegs, total, counter, probePolls, (int)(early == 2));
+                     nsegs, total, counter, probePolls, (int)((early & kEarlyUp) != 0));
 }
 
 cudaError_t launchBlendSmall(const Segment* segs, int nsegs, int total, int early, cudaStream_t st)

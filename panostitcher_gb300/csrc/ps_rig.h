@@ -284,7 +284,7 @@ private:
         int level;      // level of the first rig in the step
         double bytes;   // algorithmic bytes of the step (all rigs)
         int work = 0;   // of a blend step: its tiles' cameras
-        int early = 0;  // of a blend step, the launch before: 2 wrote only C levels, 1 is the tail
+        int early = 0;  // of a blend step (kEarlyG ...)
     };
     // Per-run state in kIoSlots copies: run k uses slot k % kIoSlots, so while
     // run k computes, run k + 1 uploads and run k - 1 downloads.
