@@ -2377,9 +2377,9 @@ __global__ void __launch_bounds__(kThreads, kRowsCtas) k_blend_rows(const Segmen
 // memory are written as everywhere, for the levels below and the state export.
 // A tail that also took the levels of up to 16 tiles, each spread over 16 CTAs
 // with a cluster barrier between levels, cost as much as a launch a level did.
-// Five levels of 6 x 1920x1080 to 4096x2048: 6.4 us from its release, and a
-// frame of 172.5 us (177.5 with a launch a level, 183.8 with that wider tail);
-// 256x128: 33.7 us a frame against 40.6 and 42.4.
+// The two levels of 6 x 1920x1080 to 4096x2048 (8 levels): 6.1 us from its
+// release, and a frame of 172.5 us when it came (177.5 with a launch a level,
+// 183.8 with that wider tail); 256x128: 33.7 us a frame against 40.6 and 42.4.
 // ============================================================================
 constexpr int kTailCluster = 8;       // portable cluster size
 constexpr int kTailClusterWide = 16;  // used for more cameras where the GPU can co-schedule it
