@@ -611,22 +611,27 @@ __device__ __forceinline__ uint32_t roundSaturate3(const float* a)
     return v;
 }
 
-// A CTA takes runs of four consecutive tiles and one pixel a thread (16x2 block
-// per warp); the map, weight and camera of the next (tile, camera) pair are
-// loaded before the current one's texels, the launch being bound by the latency
-// of that chain and by L1.  6 x 1920x1080 to 4096x2048: 109 us before (32x1
-// rows, two pixels a thread, no look-ahead, FP64 near ties), 87.5 us now; three
-// CTAs of 40 registers spill (135 us).
-constexpr int kLinearThreads = kRemapTW * kRemapTH;
-constexpr int kLinearCtas = 2;  // CTAs per SM
-constexpr int kLinearRun = 4;  // consecutive tiles of a CTA's step
+// A warp takes four 16x2 blocks of a tile through all of its cameras: the
+// descriptors of a (tile, camera) pair are read once for 128 pixels, and its
+// four map values and weights are in flight together.  A pixel at a time, 23
+// of the 35 wavefronts a block and camera took in L1 were descriptors' and
+// tables': 6 x 1920x1080 to 4096x2048 took 89.1 us a frame (109 us the launch
+// before 16x2 blocks and fixed point), 76.4 us now.  Two blocks a warp: 94 us;
+// eight: 88; two CTAs of 512 threads: 84.4, four of 256: 85.2.
+constexpr int kLinearThreads = 384;
+constexpr int kLinearCtas = 3;    // CTAs per SM: 36 warps of 56 registers
+constexpr int kLinearBlocks = 4;  // blocks of a warp
+constexpr int kLinearRun = kLinearThreads / 32 * kLinearBlocks / kRemapBlocks;  // tiles of a CTA's step
+static_assert(kLinearRun >= 1 && kRemapBlocks % kLinearBlocks == 0, "a tile is whole warps");
 
 template <int kFmt>
 __global__ void __launch_bounds__(kLinearThreads, kLinearCtas) k_linear(const Segment* __restrict__ segs, int nsegs,
-                                                                           int total)
+                                                                            int total)
 {
     extern __shared__ __align__(256) uint8_t luts[];  // 768 bytes per camera of the current rig
-    const int lx = mapTileX(threadIdx.x), ly = mapTileY(threadIdx.x);
+    constexpr int kWarps = kRemapBlocks / kLinearBlocks;  // of a tile
+    const int warp = threadIdx.x >> 5;
+    const int first = warp % kWarps * kLinearBlocks * 32 + (threadIdx.x & 31);  // the lane's first pixel of the tile
     int s = 0, loaded = -1;
     waitPrevGrid();
     allowNextGrid();
@@ -643,62 +648,62 @@ __global__ void __launch_bounds__(kLinearThreads, kLinearCtas) k_linear(const Se
                 __syncthreads();
                 loaded = s;
             }
+            if (it + warp / kWarps >= end) continue;
             const uint32_t lutAddr = smemAddr(luts);
-            const LinearItem* items = static_cast<const LinearItem*>(sg.items) + (it - sg.prefix);
+            const LinearItem item = static_cast<const LinearItem*>(sg.items)[it - sg.prefix + warp / kWarps];
             const long long tilePx = (long long)R.numRemapItems * kRemapTW * kRemapTH;
-            // The tiles' cameras are consecutive remap items (a remap item's
-            // tile number is its index), so the next one's map, weight and
-            // camera are loaded before the current one's texels.
-            float2 m = make_float2(-1.f, -1.f);
-            float w = 0.f;
-            int cam = 0;
-            const uint32_t last = items[end - it - 1].first + items[end - it - 1].count;
-            auto load = [&](uint32_t e, float2& mv, float& wv, int& cv) {
-                const size_t base = (size_t)e * (kRemapTW * kRemapTH) + threadIdx.x;
-                mv = ldChecked(R.maps + base, R.maps, tilePx * 8);
-                wv = ldChecked(R.linWeights + base, R.linWeights, tilePx * 4);
-                cv = R.remapItems[e].cam;
-            };
             auto add = [&](float* a, uint32_t v, float wv) {
 #pragma unroll
                 for (int c = 0; c < 3; c++) a[c] = __fadd_rn(a[c], __fmul_rn(byteToFloat((v >> (8 * c)) & 0xFF), wv));
             };
-            uint32_t e = items[0].first;
-            if (e < last) load(e, m, w, cam);
-            for (int k = 0; k < end - it; k++) {
-                const LinearItem item = items[k];
-                float a[3] = {0.f, 0.f, 0.f};
-                bool ties = false;
-                for (const uint32_t stop = item.first + item.count; e < stop; e++) {
-                    float2 nm = m;
-                    float nw = w;
-                    int ncam = cam;
-                    if (e + 1 < last) load(e + 1, nm, nw, ncam);
-                    const RemapSrc src{F.src[cam], F.srcPitch[cam], F.srcFmt, R.srcW, R.srcH};
+            auto store = [&](int q, const float* a) {
+                const int x = item.tx * kRemapTW + mapTileX(first + 32 * q), y = item.ty * kRemapTH + mapTileY(first + 32 * q);
+                if (x < R.W && y < R.H) storeBgr(F, x, y, R.H, roundSaturate3(a));
+            };
+            float a[kLinearBlocks][3];
+#pragma unroll
+            for (int q = 0; q < kLinearBlocks; q++) a[q][0] = a[q][1] = a[q][2] = 0.f;
+            uint32_t ties = 0;
+            for (uint32_t e = item.first; e < item.first + item.count; e++) {
+                // a remap item's tile number is its index
+                const float2* mp = R.maps + (size_t)e * (kRemapTW * kRemapTH) + first;
+                const float* wp = R.linWeights + (size_t)e * (kRemapTW * kRemapTH) + first;
+                const int cam = R.remapItems[e].cam;
+                float2 m[kLinearBlocks];
+                float w[kLinearBlocks];
+#pragma unroll
+                for (int q = 0; q < kLinearBlocks; q++) {
+                    m[q] = ldChecked(mp + 32 * q, R.maps, tilePx * 8);
+                    w[q] = ldChecked(wp + 32 * q, R.linWeights, tilePx * 4);
+                }
+                const RemapSrc src{F.src[cam], F.srcPitch[cam], F.srcFmt, R.srcW, R.srcH};
+#pragma unroll
+                for (int q = 0; q < kLinearBlocks; q++) {
                     RemapTap p;
-                    remapFetch<kFmt>(m, src, p);
+                    remapFetch<kFmt>(m[q], src, p);
                     bool tie;
                     const uint32_t v = remapFinish(p, lutAddr + cam * 768, tie);
-                    ties |= tie;
-                    add(a, v, w);
-                    m = nm;
-                    w = nw;
-                    cam = ncam;
+                    if (tie) ties |= 1u << q;
+                    add(a[q], v, w[q]);
                 }
-                if (ties) {  // near a rounding tie in some camera: the pixel again, exactly
-                    a[0] = a[1] = a[2] = 0.f;
-                    for (uint32_t q = item.first; q < item.first + item.count; q++) {
-                        float2 qm;
-                        float qw;
-                        int qcam;
-                        load(q, qm, qw, qcam);
-                        const RemapSrc src{F.src[qcam], F.srcPitch[qcam], F.srcFmt, R.srcW, R.srcH};
-                        const bool valid = qm.x >= 0.f && qm.y >= 0.f && qm.x < (float)src.sw && qm.y < (float)src.sh;
-                        add(a, valid ? remapExact(qm, src, luts + qcam * 768) : 0u, qw);
-                    }
+            }
+#pragma unroll
+            for (int q = 0; q < kLinearBlocks; q++) store(q, a[q]);
+#pragma unroll 1
+            for (; ties; ties &= ties - 1) {  // near a rounding tie in some camera: the pixel again, exactly
+                const int q = __ffs(ties) - 1;
+                float x[3] = {0.f, 0.f, 0.f};
+#pragma unroll 1
+                for (uint32_t e = item.first; e < item.first + item.count; e++) {
+                    const size_t at = (size_t)e * (kRemapTW * kRemapTH) + first + 32 * q;
+                    const float2 m = ldChecked(R.maps + at, R.maps, tilePx * 8);
+                    const float w = ldChecked(R.linWeights + at, R.linWeights, tilePx * 4);
+                    const int cam = R.remapItems[e].cam;
+                    const RemapSrc src{F.src[cam], F.srcPitch[cam], F.srcFmt, R.srcW, R.srcH};
+                    const bool valid = m.x >= 0.f && m.y >= 0.f && m.x < (float)src.sw && m.y < (float)src.sh;
+                    add(x, valid ? remapExact(m, src, luts + cam * 768) : 0u, w);
                 }
-                const int x = item.tx * kRemapTW + lx, y = item.ty * kRemapTH + ly;
-                if (x < R.W && y < R.H) storeBgr(F, x, y, R.H, roundSaturate3(a));
+                store(q, x);
             }
         }
     }
