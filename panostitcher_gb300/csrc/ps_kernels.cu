@@ -716,11 +716,16 @@ __global__ void __launch_bounds__(kLinearThreads, kLinearCtas) k_linear(const Se
 // canvas, for one camera) fetches nothing.  Near-tie pixels are recomputed at
 // the end, which keeps the call out of the blocks' code.  4096x2048 from
 // 1920x1080: 53.8 us before (one pixel a thread, FP64 behind a
-// test per channel), 29.2 us now.
+// test per channel), 27.1 us now.
 constexpr int kReprojectBlocks = 4;
+// Canvases of this many CTAs take the build of five CTAs a SM: 3872 of them
+// (2800x1400) are as fast either way, 5000 (3200x1600) 14.6 us against 16.4,
+// 8192 (4096x2048) 27.1 against 29.2, 28800 (7680x3840) 80 against 88; 2048
+// (2048x1024) 8.9 against 8.5.
+constexpr unsigned kReprojectMany = 3500;
 
-template <int kFmt>
-__global__ void __launch_bounds__(kThreads) k_reproject16s(RemapSrc src, const float* __restrict__ xmap,
+template <int kFmt, int kCtas>  // kCtas: CTAs per SM
+__global__ void __launch_bounds__(kThreads, kCtas) k_reproject16s(RemapSrc src, const float* __restrict__ xmap,
                                                            const float* __restrict__ ymap, long long mapPitch,
                                                            int W, int H, const uint8_t* __restrict__ glut,
                                                            short4* dst, long long dstPitch)
@@ -3202,14 +3207,16 @@ cudaError_t launchReprojectTo16S(const uint8_t* src, long long srcPitch, int src
     dim3 grid((dstW + 16 * kReprojectBlocks - 1) / (16 * kReprojectBlocks), (dstH + 15) / 16);
     const RemapSrc S{src, srcPitch, srcFmt, srcW, srcH};
     short4* const d = reinterpret_cast<short4*>(dst);
+    auto go = [&](auto* few, auto* many) {
+        // kReprojectMany CTAs and more: five a SM, at 48 registers and a few
+        // spills, where the others hide each other's trips to memory
+        auto* kernel = grid.x * grid.y >= kReprojectMany ? many : few;
+        kernel<<<grid, kThreads, 0, st>>>(S, xmap, ymap, mapPitch, dstW, dstH, lut, d, dstPitch);
+    };
     switch (remapSourceFormat(srcFmt, srcW, srcH, srcPitch)) {
-    case PS_FMT_BGR32:
-        k_reproject16s<PS_FMT_BGR32><<<grid, kThreads, 0, st>>>(S, xmap, ymap, mapPitch, dstW, dstH, lut, d, dstPitch);
-        break;
-    case PS_FMT_BGR24:
-        k_reproject16s<PS_FMT_BGR24><<<grid, kThreads, 0, st>>>(S, xmap, ymap, mapPitch, dstW, dstH, lut, d, dstPitch);
-        break;
-    default: k_reproject16s<0><<<grid, kThreads, 0, st>>>(S, xmap, ymap, mapPitch, dstW, dstH, lut, d, dstPitch);
+    case PS_FMT_BGR32: go(k_reproject16s<PS_FMT_BGR32, 1>, k_reproject16s<PS_FMT_BGR32, 5>); break;
+    case PS_FMT_BGR24: go(k_reproject16s<PS_FMT_BGR24, 1>, k_reproject16s<PS_FMT_BGR24, 5>); break;
+    default: go(k_reproject16s<0, 1>, k_reproject16s<0, 5>);
     }
     return cudaGetLastError();
 }
