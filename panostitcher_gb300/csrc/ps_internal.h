@@ -167,7 +167,8 @@ cudaError_t launchImagesToLevel0(const ImageArgs& args, int fmt, int n, int W, i
 // The launch choices that can change after prepare.  Tile sizes are fixed
 // at compile time (the tile-compact maps and the 2x2 blend layout depend on
 // them); what varies is which levels the tail kernel runs, its cluster
-// width and tile split, and the CTAs per SM of the persistent kernels.
+// width, the levels run as half tiles, and the CTAs per SM of the persistent
+// kernels.
 // Set by hand or chosen by the autotuner (ps_tune.cpp).
 struct LaunchShape {
     int tailMaxItems = 16;         // levels with at most this many tiles may run in the tail kernel (0: none)
@@ -175,7 +176,7 @@ struct LaunchShape {
     int tailHalf = 1;              // kept for its callers: both values run the same launches
     int ctasPerSm[3] = {0, 0, 0};  // k_remap, k_pyrdown, k_blend; 0 = as many as fit
     int smallBlendMaxItems = 0;    // blend levels above 0 with at most this many tiles run in k_blend_small (0: kSmallBlendTiles)
-    // Where k_blend_small takes over from k_blend by default: with 128 tiles
+    // Where k_blend_small takes over by default (measured against k_blend): with 128 tiles
     // (two CTAs each) a level is one short wave, and each level of 8 to 128
     // tiles is 2 - 4 us shorter (6 x 1920x1080 to 4096x2048: 189 against 183 us
     // a frame); with 512 tiles k_blend's larger blocks win (190 us).  With

@@ -1,19 +1,22 @@
 // ps_kernels.cu -- the per-frame stitch kernels (sm_103a).
 //
-// One frame of one or more rigs runs as about 2L+2 launches over prepared
+// One frame of one or more rigs runs as at most 2L+2 launches over prepared
 // work lists:
 //   k_remap        level 0: LUT gain + bilinear remap of every covered tile,
 //                  written as uchar4 G0 (cudaTransform + cudaReprojectTo16S);
 //   k_pyrdown      levels 1..L: masked 5x5 decimation G_j -> G_{j+1}
-//                  (pyrDown16SC4To16SC4 with alpha scale);
+//                  (pyrDown16SC4To16SC4 with alpha scale); k_pyrdown_pair, two
+//                  levels of few tiles at once;
 //   k_blend        levels L..0: for every canvas tile, the Laplacian of each
 //                  camera whose seam weight touches the tile
 //                  (G_j - pyrUp(G_{j+1})), its weighted accumulation, the
 //                  normalisation, and the collapse step pyrUp(C_{j+1}) + N_j,
 //                  all in registers; level 0 writes the 8-bit output with
 //                  the uncovered pixels zeroed;
-//   k_blend_small, k_tail  the same for the few-tile top levels (half tiles;
-//                  one thread-block cluster running several levels).
+//   k_blend_rows, k_blend_small  the same for levels of few tiles (row pairs
+//                  a warp; half tiles a CTA);
+//   k_tail         pyrDown and blend of the smallest levels, one thread-block
+//                  cluster a rig.
 // The reference runs the same arithmetic as ~35 launches per camera plus
 // ~36 per frame over full-canvas int16/int32 images
 // (source/CudaAccel/CudaMultibandBlend.cpp:785-823).
@@ -1165,12 +1168,13 @@ __global__ void __launch_bounds__(kPairThreads) k_pyrdown_pair(const Segment* __
 // (horizontal wrap, vertical reflect-101) are staged by the consumers with the
 // reference's index mapping.
 //
-// Level 0 of 6 x 1920x1080 to 4096x2048: 37 us, 42 before the uniform tiles'
-// packed path and the runs (24.4 M instead of 32.0 M warp instructions); of 8 x
-// 3840x2160 to 7680x3840: 80 us, 100 before.  Left: a unit's arithmetic (2300
-// cycles of eight warps a scheduler) and the producer's work on the next one
-// (2300 cycles too) take turns waiting for each other; a 4-stage ring, a
-// 3-stage one and one lane doing the producer's work measured no shorter.
+// Level 0 of 6 x 1920x1080 to 4096x2048 in a running frame: 30 us from its
+// release, 37.5 before the uniform tiles' packed path and the runs (24.3 M instead
+// of 32.0 M warp instructions); of 8 x 3840x2160 to 7680x3840: 77 us, 101 before.
+// Left: a unit's arithmetic (2300 cycles of eight warps a scheduler) and the
+// staging of the next take turns waiting for each other; a 4-stage ring, a
+// 3-stage one, one lane doing the producer's work, and copies issued ahead of
+// everything else in the producer's step measured no shorter.
 // ============================================================================
 constexpr int kFW = kBlendTW / 2 + 2;  // 34: footprint columns fx0 .. fx0+33
 constexpr int kFH = kBlendTH / 2 + 2;  // 10: footprint rows    fy0 .. fy0+9
