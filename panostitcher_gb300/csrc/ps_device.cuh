@@ -172,14 +172,15 @@ __device__ __forceinline__ int findSegment(const Segment* segs, int nsegs, int i
 }
 
 // Contiguous chunk of items for this CTA (k_pyrdown): neighbouring tiles of
-// one camera stay on one SM, and no item is handed out through an atomic.
+// one camera stay on one SM, and no item is handed out through an atomic.  The
+// CTAs' shares differ by one item at most: equal shares rounded up left the
+// last CTAs, and with them some SMs, idle (a frame of 8 x 3840x2160 to 7680x3840
+// 419.5 us, 417.3 us so; of 2048x1024 74.0 and 72.7).
 __device__ __forceinline__ void itemRange(int total, int& begin, int& end)
 {
-    const int chunk = (total + gridDim.x - 1) / gridDim.x;
-    begin = min(total, (int)blockIdx.x * chunk);
-    end = min(total, begin + chunk);
+    begin = (int)((long long)total * blockIdx.x / gridDim.x);
+    end = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
 }
-
 
 // ---- borders: source/CudaAccel/CudaUtil.cuh:6-98 ------------------------------
 // Vertical reflect-101 (BrdColReflect101) and horizontal wrap (BrdRowWrap),
