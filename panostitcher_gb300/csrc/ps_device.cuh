@@ -66,7 +66,8 @@ struct DownItem { uint8_t cam, level; uint16_t tx, ty; uint16_t whole; };
 struct alignas(16) BlendItem { uint8_t level, cls, camCnt, flags; uint16_t tx, ty; uint8_t cams[8]; };
 constexpr int kInlineCams = 8;
 // flags bit 0: one camera, weight 256 on every pixel of the tile, so the
-// normalised value is the Laplacian itself (R = 256 L, W = 256).
+// normalised value is the Laplacian itself (R = 256 L, W = 256); at level 0 the
+// tile is fully covered too (cls 1).
 constexpr int kTileUniform = 1;
 // cls of a level-0 blend tile: 0 uncovered (write zeros), 1 fully covered,
 // 2 partially covered (read the union mask).  Unused above level 0.

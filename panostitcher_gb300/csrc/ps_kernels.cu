@@ -2320,7 +2320,7 @@ __global__ void __launch_bounds__(kThreads, kRowsCtas) k_blend_rows(const Segmen
     for (int u = first; u < units; u += gridDim.x * (kThreads / 32)) {
         seg = findSegment(segs, nsegs, u / kParts, seg);
         const uint4 raw = __ldg(static_cast<const uint4*>(segs[seg].items) + (u / kParts - segs[seg].prefix));
-        const int j = raw.x & 0xFF, cls = (raw.x >> 8) & 0xFF;
+        const int j = raw.x & 0xFF;
         if (seg != filled) fillRowsGeo(B, *segs[seg].rig, *segs[seg].frame, j);
         if (filled < 0) {  // items and descriptors are written before the launch sequence, not by a kernel
             waitPrevGrid();
@@ -2337,7 +2337,7 @@ __global__ void __launch_bounds__(kThreads, kRowsCtas) k_blend_rows(const Segmen
 #pragma unroll
             for (int k = 0; k < 3; k++) col[k] = colMap(tx * (kBlendTW / 2) - 1 + lane + k, B.u.w);
         }
-        if ((raw.x >> 24 & kTileUniform) && B.g.hasUp && rows >= kPairs && (j | cls)) {
+        if ((raw.x >> 24 & kTileUniform) && B.g.hasUp && rows >= kPairs) {
             const int cam = tileCam(raw, B.camLists, 0);
             const uint32_t* U = reinterpret_cast<const uint32_t*>(B.u.G) + (size_t)cam * B.u.camStride;
             const uint2* C = reinterpret_cast<const uint2*>(B.u.C);

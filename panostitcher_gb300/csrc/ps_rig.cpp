@@ -711,7 +711,11 @@ void Rig::buildBlendState(const uint8_t* uniSrc, bool custom, cudaStream_t st)
                 it.level = (uint8_t)j;
                 it.cls = cls;
                 it.camCnt = (uint8_t)list.size();
-                if (list.size() == 1 && !hU[j][((size_t)list[0] * bY + ty) * bX + tx]) it.flags |= kTileUniform;
+                // Explicit seams may reach beyond the coverage, so a level-0 tile of one camera's
+                // weight 256 may hold pixels that no camera covers: the kernels' path of uniform
+                // tiles zeroes none, so only wholly covered ones are.
+                if (list.size() == 1 && !hU[j][((size_t)list[0] * bY + ty) * bX + tx] && (j > 0 || cls == 1))
+                    it.flags |= kTileUniform;
                 it.tx = (uint16_t)tx;
                 it.ty = (uint16_t)ty;
                 if (list.size() <= (size_t)kInlineCams) {
