@@ -2934,7 +2934,7 @@ __global__ void __launch_bounds__(kThreads) k_yuv_to_bgr32(YuvFrames f)
         uint32_t* o1 = reinterpret_cast<uint32_t*>(F.dst + (size_t)(y + 1) * F.dstPitch) + x;
         const uint32_t p00 = yuvPixel(y0[0], ruv, guv, buv), p01 = yuvPixel(y0[1], ruv, guv, buv);
         const uint32_t p10 = yuvPixel(y1[0], ruv, guv, buv), p11 = yuvPixel(y1[1], ruv, guv, buv);
-        if ((F.dstPitch & 7) == 0) {  // x is even, so 8-byte aligned
+        if (((reinterpret_cast<uintptr_t>(o0) | reinterpret_cast<uintptr_t>(o1)) & 7) == 0) {  // images are 4-byte aligned
             *reinterpret_cast<uint2*>(o0) = make_uint2(p00, p01);
             *reinterpret_cast<uint2*>(o1) = make_uint2(p10, p11);
         } else {
