@@ -1072,10 +1072,8 @@ void Rig::toLevel0(const void* const* images, const long long* pitches, int fmt,
                                  lv_[0].G[slot].as<uchar4>() + (size_t)cam0 * g.pitch * g.h, g.pitch,
                                  (long long)g.pitch * g.h, imgFlags_.as<int>(), st));
     PS_CUDA(cudaStreamSynchronize(st));
-    const int status = (flags[0] ? 1 : 0) | (flags[1] ? 2 : 0);
-    if (status) PS_CUDA(cudaMemcpy(status_.get(), &status, sizeof status, cudaMemcpyHostToDevice));
-    if (status & 1) fail(PS_EINVAL, "an int16 input value lies outside 0..255");
-    if (status & 2) fail(PS_EINVAL, "an input image is non-zero where its coverage mask is zero");
+    if (flags[0]) fail(PS_EINVAL, "an int16 input value lies outside 0..255");
+    if (flags[1]) fail(PS_EINVAL, "an input image is non-zero where its coverage mask is zero");
 }
 
 void Rig::exportState(int what, int cam, int level, void* host, long long bytes) const
