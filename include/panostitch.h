@@ -259,16 +259,16 @@ long long ps_render_estimate_memory(const ps_photo_param* params, int num_params
 
 /* Failure status of the render's kernels.  No reference counterpart (the
    reference's kernels have no waits that can run out).  Every wait of the
-   blend kernels on the bulk-copy ring is bounded; one that runs out sets a
-   status bit on every frame of its launch and the kernel carries on, so the
-   device stays usable.  ps_render_check waits for the render's frames in
+   remap on its ring of tiles and of the blend kernels on the bulk-copy ring is
+   bounded; one that runs out sets a status bit on every frame of its launch
+   and the kernel carries on, so the device stays usable.  ps_render_check waits for the render's frames in
    flight, reads and clears that status, and returns PS_ETIMEOUT if a wait ran
    out since the last check (those frames may be wrong), else PS_OK. */
 int ps_render_check(ps_render* r);
 /* Failure-path test hook, no reference counterpart: with polls > 0 every
-   blend launch of this render makes one wait of that many polls on a
-   barrier that nothing completes, so that wait runs out and
-   ps_render_check reports PS_ETIMEOUT.  0 (default) turns it off.  Waits
+   remap and blend launch of this render makes one wait of that many polls on
+   a barrier that nothing completes, so that wait runs out and
+   ps_render_check reports PS_ETIMEOUT, naming the kernels.  0 (default) turns it off.  Waits
    for the frames in flight; the next render re-records its launches. */
 int ps_render_set_wait_probe(ps_render* r, int polls);
 

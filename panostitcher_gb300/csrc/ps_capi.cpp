@@ -449,15 +449,24 @@ long long ps_render_estimate_memory(const ps_photo_param* params, int num_params
     return st == PS_OK ? v : -1;
 }
 
+namespace {
+
+void checkTimeouts(int status, const char* what)
+{
+    const bool remap = status & ps::kStatusRemap, blend = status & ps::kStatusBlend;
+    if (remap || blend)
+        fail(PS_ETIMEOUT, "a bounded wait of %s ran out: %s since the last check may be wrong",
+             remap && blend ? "the remap and of a blend kernel" : (remap ? "the remap" : "a blend kernel"), what);
+}
+
+}  // namespace
+
 int ps_render_check(ps_render* r)
 {
     return guarded([&] {
         if (!r) fail(PS_EINVAL, "render is NULL");
         if (!r->rig.ready()) return;
-        const int st = r->rig.takeStatus();
-        if (st & 4)
-            fail(PS_ETIMEOUT, "a bounded wait of a blend kernel ran out: frames rendered since the last check "
-                              "may be wrong");
+        checkTimeouts(r->rig.takeStatus(), "frames rendered");
     });
 }
 
@@ -782,9 +791,7 @@ int ps_blender_check(ps_blender* b)
     return guarded([&] {
         if (!b) fail(PS_EINVAL, "blender is NULL");
         if (!b->rig.ready()) return;
-        const int st = b->rig.takeStatus();
-        if (st & 4)
-            fail(PS_ETIMEOUT, "a bounded wait of a blend kernel ran out: blends since the last check may be wrong");
+        checkTimeouts(b->rig.takeStatus(), "blends");
     });
 }
 

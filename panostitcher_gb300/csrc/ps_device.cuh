@@ -94,6 +94,10 @@ struct RemapParamF {
 // weight tile (64 x 16 x 1 of uint16).
 constexpr int kTmG = 0, kTmGfp = 1, kTmC = 2, kTmW = 3, kTmapsPerLevel = 4;
 
+// Bits of a frame's error word: a bounded wait of a blend kernel, of the remap
+// ran out.
+constexpr int kStatusBlend = 4, kStatusRemap = 8;
+
 struct RigDev {
     int n, L, W, H;
     int full;                 // union of coverages == whole canvas
@@ -135,7 +139,7 @@ struct FrameDev {
     long long outCPitch;      // pitch of the U (or UV) plane
     long long outVPitch;      // pitch of the V plane
     const uint8_t* luts;      // n * 768 device bytes (B, G, R tables)
-    int* status;              // device error word (0 = ok)
+    int* status;              // device error word (0 = ok; kStatusBlend ...)
 };
 
 // Decoder frames to convert to BGR32 (k_yuv_to_bgr32): YUV420P (u, v

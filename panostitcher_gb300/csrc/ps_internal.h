@@ -200,8 +200,8 @@ struct LaunchShape {
 // srcFmt: the format of every source of the launch as remapSourceFormat
 // gives it, or 0 when they differ; maps: every rig of the launch has resident
 // maps
-cudaError_t launchRemap(const Segment* segs, int nsegs, int total, int perSm, int* counter, int srcFmt, bool maps,
-                        cudaStream_t st);
+cudaError_t launchRemap(const Segment* segs, int nsegs, int total, int perSm, int* counter, int probePolls, int srcFmt,
+                        bool maps, cudaStream_t st);
 // The format k_remap, k_linear and k_reproject16s may be specialised for: the
 // frame's own, or 0 (the general kernel) for frames of one column or row,
 // where the clamped left taps of the specialised ones would not exist, and for
@@ -214,7 +214,7 @@ cudaError_t launchPyrDownPair(const Segment* segs, int nsegs, int total, cudaStr
 // Accesses the checked build's kernels refused since the last reset
 // (waits for the device); -1 in the normal build, -2 on a CUDA error.
 long long boundsViolations(bool reset);
-// probePolls > 0: the failure-path test of the bounded waits (k_blend).
+// probePolls > 0: the failure-path test of the bounded waits (k_remap, k_blend, k_blend_rows).
 // early: what of a launch's first units may precede its wait for the launch
 // before: their G_j reads (that launch is the tail), those and the G_{j+1} reads
 // too (it wrote only C levels: a blend step after the first); and of few-tile

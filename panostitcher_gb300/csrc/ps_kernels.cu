@@ -472,25 +472,30 @@ __device__ __forceinline__ bool remapProduce(RemapRun& r, RemapChunk& c, const S
     return true;
 }
 
-// A wait of the launch ran out: every frame of it is flagged.
-__device__ __forceinline__ void flagTimeout(const Segment* segs, int nsegs)
+// A wait of the launch ran out: every frame of it is flagged (bit: kStatusBlend
+// or kStatusRemap).
+__device__ __forceinline__ void flagTimeout(const Segment* segs, int nsegs, int bit)
 {
     for (int k = 0; k < nsegs; k++)
-        if (segs[k].frame->status) atomicOr(segs[k].frame->status, 4);
+        if (segs[k].frame->status) atomicOr(segs[k].frame->status, bit);
 }
 
+// probePolls: as k_blend's.
 template <int kFmt, bool kMaps>
 __global__ void __launch_bounds__(kRemapThreads, kRemapCtas) k_remap(const Segment* __restrict__ segs, int nsegs,
-                                                                        int total, int* __restrict__ counter)
+                                                                        int total, int* __restrict__ counter,
+                                                                        int probePolls)
 {
     __shared__ RemapChunk s_chunk[kRemapRing];
-    __shared__ uint64_t full[kRemapRing], empty[kRemapRing];
+    __shared__ uint64_t full[kRemapRing], empty[kRemapRing], never;
     const int lane = threadIdx.x & 31;
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 0) {
         for (int k = 0; k < kRemapRing; k++) {
             mbarInit(&full[k], 1);
             mbarInit(&empty[k], kRemapWarps);
         }
+        mbarInit(&never, 1);
+    }
     __syncthreads();
     if (threadIdx.x >= kRemapWarps * 32) {
         // The hand-out counter, items, descriptors and LUTs are written before
@@ -501,7 +506,7 @@ __global__ void __launch_bounds__(kRemapThreads, kRemapCtas) k_remap(const Segme
         for (int k = 0; more; k++) {
             const int s = k % kRemapRing;
             if (k >= kRemapRing && !mbarWait(&empty[s], (k / kRemapRing - 1) & 1)) {
-                if (lane == 0) flagTimeout(segs, nsegs);
+                if (lane == 0) flagTimeout(segs, nsegs, kStatusRemap);
                 break;
             }
             more = remapProduce(r, s_chunk[s], segs, nsegs, total, counter);
@@ -513,11 +518,12 @@ __global__ void __launch_bounds__(kRemapThreads, kRemapCtas) k_remap(const Segme
         return;
     }
     const int warp = threadIdx.x >> 5;
+    if (probePolls > 0 && threadIdx.x == 0 && !mbarWait(&never, 0, probePolls)) flagTimeout(segs, nsegs, kStatusRemap);
     bool waited = false;
     for (int k = 0;; k++) {
         const int s = k % kRemapRing;
         if (!mbarWait(&full[s], (k / kRemapRing) & 1)) {
-            if (lane == 0) flagTimeout(segs, nsegs);
+            if (lane == 0) flagTimeout(segs, nsegs, kStatusRemap);
             break;
         }
         const RemapChunk& c = s_chunk[s];
@@ -1997,7 +2003,7 @@ __device__ __forceinline__ void collapseRows(const HalfStage& S, const UnitGeo& 
 // probePolls > 0 is the failure-path test of the bounded waits: consumer
 // thread 0 first waits that many polls on an mbarrier that nothing arrives
 // on, so the wait runs out, and the timeout is reported as any other
-// (status bit 4 of every frame in the launch).
+// (kStatusBlend in every frame of the launch).
 __global__ void __launch_bounds__(kBlendThreads, 4) k_blend(const Segment* __restrict__ gsegs, int nsegs, int total,
                                                             int* __restrict__ counter, int probePolls, int early)
 {
@@ -2189,9 +2195,7 @@ __global__ void __launch_bounds__(kBlendThreads, 4) k_blend(const Segment* __res
     // consumer has waited on; the consumers' own meet here.  A desynchronised
     // ring can have corrupted any unit, so every frame of the launch is flagged.
     namedBarrier(1, kConsumers);
-    if (s_timeout && threadIdx.x == 0)
-        for (int k = 0; k < nsegs; k++)
-            if (segs[k].frame->status) atomicOr(segs[k].frame->status, 4);
+    if (s_timeout && threadIdx.x == 0) flagTimeout(segs, nsegs, kStatusBlend);
 }
 
 // ============================================================================
@@ -2325,7 +2329,8 @@ __global__ void __launch_bounds__(kThreads, kRowsCtas) k_blend_rows(const Segmen
         if (filled < 0) {  // items and descriptors are written before the launch sequence, not by a kernel
             waitPrevGrid();
             allowNextGrid();
-            if (probePolls > 0 && threadIdx.x == 0 && !mbarWait(&never, 0, probePolls)) flagTimeout(segs, nsegs);
+            if (probePolls > 0 && threadIdx.x == 0 && !mbarWait(&never, 0, probePolls))
+                flagTimeout(segs, nsegs, kStatusBlend);
         }
         filled = seg;
         const int tx = raw.y & 0xFFFF, ty = raw.y >> 16;
@@ -3022,21 +3027,22 @@ int remapSourceFormat(int fmt, int sw, int sh, long long pitch)
 }
 
 template <int kFmt, bool kMaps>
-static cudaError_t launchRemapAs(const Segment* segs, int nsegs, int total, int perSm, int* counter, cudaStream_t st)
+static cudaError_t launchRemapAs(const Segment* segs, int nsegs, int total, int perSm, int* counter, int probePolls,
+                                 cudaStream_t st)
 {
     return launchPdl(k_remap<kFmt, kMaps>, gridFor(total, residentPerSm<k_remap<kFmt, kMaps>>(kRemapThreads), perSm),
-                     kRemapThreads, st, segs, nsegs, total, counter);
+                     kRemapThreads, st, segs, nsegs, total, counter, probePolls);
 }
 
-cudaError_t launchRemap(const Segment* segs, int nsegs, int total, int perSm, int* counter, int srcFmt, bool maps,
-                        cudaStream_t st)
+cudaError_t launchRemap(const Segment* segs, int nsegs, int total, int perSm, int* counter, int probePolls, int srcFmt,
+                        bool maps, cudaStream_t st)
 {
     if (total <= 0) return cudaSuccess;
-    if (!maps) return launchRemapAs<0, false>(segs, nsegs, total, perSm, counter, st);
+    if (!maps) return launchRemapAs<0, false>(segs, nsegs, total, perSm, counter, probePolls, st);
     switch (srcFmt) {
-    case PS_FMT_BGR32: return launchRemapAs<PS_FMT_BGR32, true>(segs, nsegs, total, perSm, counter, st);
-    case PS_FMT_BGR24: return launchRemapAs<PS_FMT_BGR24, true>(segs, nsegs, total, perSm, counter, st);
-    default: return launchRemapAs<0, true>(segs, nsegs, total, perSm, counter, st);
+    case PS_FMT_BGR32: return launchRemapAs<PS_FMT_BGR32, true>(segs, nsegs, total, perSm, counter, probePolls, st);
+    case PS_FMT_BGR24: return launchRemapAs<PS_FMT_BGR24, true>(segs, nsegs, total, perSm, counter, probePolls, st);
+    default: return launchRemapAs<0, true>(segs, nsegs, total, perSm, counter, probePolls, st);
     }
 }
 

@@ -1548,7 +1548,7 @@ void Plan::launchAll(const IoSlot& slot, cudaStream_t st, int srcFmt, Profiler* 
             b = prof->event();
             PS_CUDA(cudaEventRecord(a, st));
         }
-        if (s.kind == 0) PS_CUDA(launchRemap(p, s.nsegs, s.total, perSm_[0], counters + si, srcFmt, maps_, st));
+        if (s.kind == 0) PS_CUDA(launchRemap(p, s.nsegs, s.total, perSm_[0], counters + si, probe_, srcFmt, maps_, st));
         else if (s.kind == 1) PS_CUDA(launchPyrDown(p, s.nsegs, s.total, perSm_[1], st));
         else if (s.kind == 8) PS_CUDA(launchPyrDownPair(p, s.nsegs, s.total, st));
         else if (s.kind == 2) PS_CUDA(launchBlend(p, s.nsegs, s.total, s.work, perSm_[2], counters + si, probe_, s.early, st));

@@ -98,13 +98,12 @@ public:
     }
     uint8_t* outputBuffer(int slot = 0) const { return output_.as<uint8_t>() + (size_t)slot * W_ * H_ * 4; }
     int* statusWord() const { return status_.as<int>(); }
-    // The status bits the kernels set since the last call (bit 4: a bounded
-    // wait of a blend kernel ran out), read and cleared after the rig's runs
-    // have finished.
+    // The status bits the kernels set since the last call (kStatusBlend,
+    // kStatusRemap), read and cleared after the rig's runs have finished.
     int takeStatus();
-    // Failure-path test of the bounded waits: with polls > 0 every blend
-    // launch of this rig makes one wait of that many polls on a barrier that
-    // nothing completes, which therefore runs out.  0 (the default) is off.
+    // Failure-path test of the bounded waits: with polls > 0 every remap
+    // and blend launch of this rig (k_remap, k_blend, k_blend_rows) makes one
+    // wait of that many polls on a barrier that nothing completes, which therefore runs out.  0 (the default) is off.
     // Waits for the rig's runs; the next run re-records its launches.
     void setWaitProbe(int polls);
     int waitProbe() const { return probe_; }
@@ -312,7 +311,7 @@ private:
     int maxCams_ = 0;
     int tailCluster_ = 0, tailCams_ = 0, perSm_[3] = {0, 0, 0};  // launch widths (from the rigs' shapes)
     bool maps_ = true;                             // every rig has resident maps
-    int probe_ = 0;                                // wait probe of k_blend (Rig::setWaitProbe)
+    int probe_ = 0;                                // wait probe (Rig::setWaitProbe)
     IoSlot io_[Rig::kIoSlots];
     int nextIo_ = 0;
     // copy-in, compute and copy-out streams (non-blocking), the capture stream

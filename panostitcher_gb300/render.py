@@ -262,7 +262,7 @@ class CudaPanoramaRender2:
         return self._status(lib().ps_render_check(self._h), check)
 
     def set_wait_probe(self, polls: int) -> None:
-        """Failure-path test hook: every blend launch makes one wait of `polls` polls that runs out."""
+        """Failure-path test hook: every remap and blend launch makes one wait of `polls` polls that runs out."""
         check(lib().ps_render_set_wait_probe(self._h, int(polls)))
 
     def clear(self) -> None:
