@@ -336,16 +336,17 @@ typedef struct ps_launch_shape {
                              to 8 cameras, else 16 (at most the widest the GPU
                              co-schedules; default 0) */
     int tail_half_tiles;  /* 0 or 1, kept for its callers: the tail has no tiles,
-                             with either value (default 1) */
+                             with either value, and a change of it alone costs
+                             nothing (default 1) */
     int ctas_per_sm[3];   /* CTAs per SM of the remap, pyrDown and blend kernels'
                              one-wave grids; 0 = as many as fit (default 0) */
     int small_blend_max_items; /* blend levels above 0 (below the tail) with at
                              most this many tiles run as 64x8 half tiles, up to
-                             eight cameras staged at once; 0 = the library's
-                             choice, 128 (default 0) */
-    int remap_defer_ties; /* 0 or 1, kept for its callers: the remap recomputes
-                             near-tie pixels itself after each run of tiles,
-                             with either value (default 1) */
+                             eight cameras staged at once; 0 = none
+                             (default 128) */
+    int remap_defer_ties; /* 0 or 1, kept for its callers in the same way: the
+                             remap recomputes near-tie pixels itself after each
+                             run of tiles, with either value (default 1) */
 } ps_launch_shape;
 typedef struct ps_tune_report {
     double ms_per_frame_default;  /* device ms per frame of the default shape */

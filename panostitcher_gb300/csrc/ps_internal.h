@@ -175,22 +175,21 @@ struct LaunchShape {
     int tailCluster = 0;           // CTAs per rig in the tail kernel: 8, 16, or 0 = by the number of cameras
     int tailHalf = 1;              // kept for its callers: both values run the same launches
     int ctasPerSm[3] = {0, 0, 0};  // k_remap, k_pyrdown, k_blend; 0 = as many as fit
-    int smallBlendMaxItems = 0;    // blend levels above 0 with at most this many tiles run in k_blend_small (0: kSmallBlendTiles)
-    // Where k_blend_small takes over by default (measured against k_blend): with 128 tiles
+    // Blend levels above 0 with at most this many tiles run in k_blend_small (0:
+    // none).  The default, measured against k_blend: with 128 tiles
     // (two CTAs each) a level is one short wave, and each level of 8 to 128
     // tiles is 2 - 4 us shorter (6 x 1920x1080 to 4096x2048: 189 against 183 us
     // a frame); with 512 tiles k_blend's larger blocks win (190 us).  With
     // eight frames in flight the two are equal (949 against 945 us for eight).
-    static constexpr int kSmallBlendTiles = 128;
-    int smallBlend() const { return smallBlendMaxItems > 0 ? smallBlendMaxItems : kSmallBlendTiles; }
+    int smallBlendMaxItems = 128;
     int remapDefer = 1;            // kept for its callers: both values run the same launch
-    bool operator==(const LaunchShape& o) const
+    // Both shapes give the same launches (tailHalf and remapDefer choose none).
+    bool sameLaunches(const LaunchShape& o) const
     {
-        return tailMaxItems == o.tailMaxItems && tailCluster == o.tailCluster && tailHalf == o.tailHalf &&
-               ctasPerSm[0] == o.ctasPerSm[0] && ctasPerSm[1] == o.ctasPerSm[1] && ctasPerSm[2] == o.ctasPerSm[2] &&
-               smallBlendMaxItems == o.smallBlendMaxItems && remapDefer == o.remapDefer;
+        return tailMaxItems == o.tailMaxItems && tailCluster == o.tailCluster && ctasPerSm[0] == o.ctasPerSm[0] &&
+               ctasPerSm[1] == o.ctasPerSm[1] && ctasPerSm[2] == o.ctasPerSm[2] &&
+               smallBlendMaxItems == o.smallBlendMaxItems;
     }
-    bool operator!=(const LaunchShape& o) const { return !(*this == o); }
 };
 
 // ---- per-frame kernels ------------------------------------------------------------

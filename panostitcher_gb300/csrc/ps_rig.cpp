@@ -934,9 +934,9 @@ void Rig::setShape(const LaunchShape& s)
     for (int k = 0; k < 3; k++)
         if (s.ctasPerSm[k] < 0 || s.ctasPerSm[k] > 64)
             fail(PS_EINVAL, "ctas_per_sm[%d] = %d out of range 0..64", k, s.ctasPerSm[k]);
-    if (s == shape_) return;
+    const bool same = s.sameLaunches(shape_);
     shape_ = s;
-    if (!ready() || linear_) return;
+    if (same || !ready() || linear_) return;
     // the descriptors change under no run: launch lists follow the new
     // generation (plans rebind), and no kernel may read the old split
     waitIdle();
@@ -1473,7 +1473,7 @@ void Plan::bind(const std::vector<Rig*>& rigs)
             const int j = rigs[r]->tailStart() - 1 - s;
             if (j < 0) continue;
             const int cnt = rigs[r]->numBlendItems(j);
-            if (j > 0 && cnt <= rigs[r]->shape().smallBlend()) small.push_back({r, {rigs[r]->blendItems(j), 2 * cnt}});
+            if (j > 0 && cnt <= rigs[r]->shape().smallBlendMaxItems) small.push_back({r, {rigs[r]->blendItems(j), 2 * cnt}});
             else parts.push_back({r, {rigs[r]->blendItems(j), cnt}});
         }
         const size_t before = steps_.size();

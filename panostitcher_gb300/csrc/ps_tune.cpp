@@ -178,8 +178,8 @@ std::vector<LaunchShape> neighbours(const Rig& rig, const LaunchShape& cur, int 
             for (int j = 1; j < curTail; j++) c += rig.numBlendItems(j) <= v;
             return c;
         };
-        std::vector<int> seen{smallLevels(cur.smallBlend())};
-        for (int v : {1, 32, 64, 128, 256, 512, 1024, 2048, 4096}) {
+        std::vector<int> seen{smallLevels(cur.smallBlendMaxItems)};
+        for (int v : {0, 32, 64, 128, 256, 512, 1024, 2048, 4096}) {
             const int c = smallLevels(v);
             if (std::find(seen.begin(), seen.end(), c) != seen.end()) continue;
             seen.push_back(c);
@@ -258,7 +258,7 @@ LaunchShape autotune(Rig& rig, Plan& plan, int framesPerTrial, int inflight, boo
             std::vector<LaunchShape> seen{best};
             const int L = rig.numLevels();
             for (int tail : {0, 16})
-                for (int small : {0, 1, 32})
+                for (int small : {128, 0, 32})
                     for (int ctas : {0, 1, 2}) {
                         LaunchShape s;
                         s.tailMaxItems = tail;
@@ -267,12 +267,12 @@ LaunchShape autotune(Rig& rig, Plan& plan, int framesPerTrial, int inflight, boo
                         // shapes that launch the same work the same way are timed once
                         const int t0 = rig.tailStart(tail);
                         int smallLevels = 0;
-                        for (int j = 1; j < t0 && j <= L; j++) smallLevels += rig.numBlendItems(j) <= s.smallBlend();
+                        for (int j = 1; j < t0 && j <= L; j++) smallLevels += rig.numBlendItems(j) <= s.smallBlendMaxItems;
                         bool dup = false;
                         for (const LaunchShape& o : seen) {
                             const int ot = rig.tailStart(o.tailMaxItems);
                             int os = 0;
-                            for (int j = 1; j < ot && j <= L; j++) os += rig.numBlendItems(j) <= o.smallBlend();
+                            for (int j = 1; j < ot && j <= L; j++) os += rig.numBlendItems(j) <= o.smallBlendMaxItems;
                             if (ot == t0 && os == smallLevels && o.ctasPerSm[2] == ctas) dup = true;
                         }
                         if (dup) continue;

@@ -307,7 +307,7 @@ class CudaPanoramaRender2:
         return lib().ps_render_algorithmic_bytes(self._h, bytes_in_per_px, bytes_out_per_px)
 
     SHAPE_DEFAULT = {"tail_max_items": 16, "tail_cluster": 0, "tail_half_tiles": 1, "ctas_per_sm": (0, 0, 0),
-                     "small_blend_max_items": 0, "remap_defer_ties": 1}
+                     "small_blend_max_items": 128, "remap_defer_ties": 1}
 
     @staticmethod
     def _shape_dict(s: "L.LaunchShape") -> dict:
