@@ -224,6 +224,21 @@ cudaError_t launchBlend(const Segment* segs, int nsegs, int total, int work, int
                         int early, cudaStream_t st);
 // blend of few-tile levels above 0: two work items (the 64x8 halves) per tile
 cudaError_t launchBlendSmall(const Segment* segs, int nsegs, int total, int early, cudaStream_t st);
+// The tail's cluster: 8 CTAs (the portable size) for up to 8 cameras, 16 for
+// more where the GPU co-schedules that (widest), or the width a shape asks for.
+constexpr int kTailCluster = 8, kTailClusterWide = 16;
+constexpr int tailClusterWidth(int asked, int cams, int widest)
+{
+    const int w = asked > 0 ? (asked >= kTailClusterWide ? kTailClusterWide : kTailCluster)
+                            : (cams <= kTailCluster ? kTailCluster : kTailClusterWide);
+    return w < widest ? w : widest;
+}
+// The width that this is not, as a value to ask for; 0 where there is no other.
+constexpr int tailClusterOther(int asked, int cams, int widest)
+{
+    const int other = kTailCluster + kTailClusterWide - tailClusterWidth(asked, cams, widest);
+    return other <= widest ? other : 0;
+}
 // one cluster per segment: the rig's pyrDown levels tailStart..L and blend
 // levels L..tailStart; cams: the most cameras of any rig; cluster 8 or 16 CTAs
 // (0: by cams; at most the widest the GPU co-schedules)

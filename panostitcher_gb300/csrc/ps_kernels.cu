@@ -2400,8 +2400,6 @@ __global__ void __launch_bounds__(kThreads, kRowsCtas) k_blend_rows(const Segmen
 // release, and a frame of 172.5 us when it came (177.5 with a launch a level,
 // 183.8 with that wider tail); 256x128: 33.7 us a frame against 40.6 and 42.4.
 // ============================================================================
-constexpr int kTailCluster = 8;       // portable cluster size
-constexpr int kTailClusterWide = 16;  // used for more cameras where the GPU can co-schedule it
 constexpr int kTailThreads = 512;     // a pixel of the largest level each
 // of all levels of a plane: 512 + 128 + 32 + 8 + 2 + 1 + 1 ...
 constexpr int kTailPx = 704;
@@ -3139,9 +3137,7 @@ int tailClusterMax()
 cudaError_t launchTail(const Segment* segs, int nsegs, int cluster, int cams, cudaStream_t st)
 {
     if (nsegs <= 0) return cudaSuccess;
-    const int widest = tailClusterMax();
-    if (cluster <= 0) cluster = cams <= kTailCluster ? kTailCluster : kTailClusterWide;
-    cluster = std::min(cluster >= kTailClusterWide ? kTailClusterWide : kTailCluster, widest);
+    cluster = tailClusterWidth(cluster, cams, tailClusterMax());
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nsegs * cluster);
     cfg.blockDim = dim3(kTailThreads);

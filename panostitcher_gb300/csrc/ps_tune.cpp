@@ -166,9 +166,9 @@ std::vector<LaunchShape> neighbours(const Rig& rig, const LaunchShape& cur, int 
         break;
     }
     case 2:  // tail cluster width
-        if (curTail <= L && tailClusterMax() > 8) {
+        if (const int other = tailClusterOther(cur.tailCluster, rig.numImages(), tailClusterMax()); other && curTail <= L) {
             LaunchShape s = cur;
-            s.tailCluster = cur.tailCluster == 8 ? 16 : 8;
+            s.tailCluster = other;
             out.push_back(s);
         }
         break;
