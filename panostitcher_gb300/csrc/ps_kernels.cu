@@ -752,8 +752,8 @@ __global__ void __launch_bounds__(kThreads, kCtas) k_reproject16s(RemapSrc src, 
     }
     for (int k = threadIdx.x; k < 768; k += kThreads) lut[k] = glut ? glut[k] : (uint8_t)(k & 255);
     __syncthreads();
+    const uint32_t lanes = __ballot_sync(0xffffffffu, y < H);  // the warp's lanes inside the canvas
     if (y >= H) return;
-    const uint32_t lanes = __activemask();  // the warp's lanes inside the canvas
     short4* row = reinterpret_cast<short4*>(reinterpret_cast<uint8_t*>(dst) + (size_t)y * dstPitch) + x;
     auto store = [&](int k, uint32_t v) {
         row[16 * k] = make_short4((short)(v & 0xFF), (short)((v >> 8) & 0xFF), (short)((v >> 16) & 0xFF), 0);
