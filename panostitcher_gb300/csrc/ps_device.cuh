@@ -27,7 +27,7 @@
 namespace ps {
 
 // ---- tiles ------------------------------------------------------------------
-constexpr int kRemapTW = 32, kRemapTH = 16;    // level-0 remap tile (two pixels per thread)
+constexpr int kRemapTW = 32, kRemapTH = 16;    // level-0 remap tile (16x2 blocks, a pixel a lane)
 constexpr int kDownTW = 32, kDownTH = 16;      // pyrDown output tile (four pixels per thread)
 constexpr int kBlendTW = 64, kBlendTH = 16;    // blend tile (a 2x2 pixel block per thread)
 constexpr int kThreads = 256;
@@ -112,7 +112,8 @@ struct RigDev {
     const uint8_t* camLists;  // camera indices of blend tiles with more than 8 cameras
     // TMA tensor maps of this state slot (CUtensorMap, 128 bytes each, 64-byte
     // aligned in device memory), kTmapsPerLevel per level: see kTmG ... kTmW;
-    // NULL when they could not be encoded (k_blend then copies row by row)
+    // NULL when they could not be encoded (k_blend's consumers then stage the
+    // units themselves)
     const void* tmaps;
     LevelDev lv[PS_MAX_LEVELS + 1];
     // the top of the pyramid in one launch (k_tail): pyrDown and blend levels

@@ -209,7 +209,6 @@ int remapSourceFormat(int fmt, int sw, int sh, long long pitch);
 cudaError_t launchPyrDown(const Segment* segs, int nsegs, int total, int perSm, cudaStream_t st);
 // two levels at once; items: 32x16 tiles of the lower level (Rig::pairItems)
 cudaError_t launchPyrDownPair(const Segment* segs, int nsegs, int total, cudaStream_t st);
-// counter: a zeroed int the launch hands its tiles out through
 // Accesses the checked build's kernels refused since the last reset
 // (waits for the device); -1 in the normal build, -2 on a CUDA error.
 long long boundsViolations(bool reset);
@@ -219,7 +218,8 @@ long long boundsViolations(bool reset);
 // too (it wrote only C levels: a blend step after the first); and of few-tile
 // launches: this one begins when that one does; the next one does with this one
 constexpr int kEarlyG = 1, kEarlyUp = 2, kEarlyBegin = 4, kEarlyNext = 8;
-// work: the tiles' cameras, counted over all tiles (an uncovered one as one)
+// work: the tiles' cameras, counted over all tiles (an uncovered one as one);
+// counter: a zeroed int the launch hands its tiles out through
 cudaError_t launchBlend(const Segment* segs, int nsegs, int total, int work, int perSm, int* counter, int probePolls,
                         int early, cudaStream_t st);
 // blend of few-tile levels above 0: two work items (the 64x8 halves) per tile

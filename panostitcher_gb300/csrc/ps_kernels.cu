@@ -1004,7 +1004,7 @@ __global__ void __launch_bounds__(kDownThreads, 8) k_pyrdown(const Segment* __re
 // makes the 35x19 pixels of level J that its part of level J + 1 reads (the
 // halo a second time: each belongs to a neighbour's tile) and filters those.
 // Columns wrap as the input does, which is the reference's rule as long as the
-// input is twice level J wide (Rig::downPairs); rows beyond the level are mapped
+// input is twice level J wide (Rig::preparePyramids lists only such); rows beyond the level are mapped
 // when level J + 1 reads them.
 // 512 threads: with 256 a launch is 3.8 us, with 704 no shorter.  256x128: 31.2 us
 // a frame, 33.5 with a launch a level; 2048x1024: 78.8 against 80.3; 6 x
@@ -1997,8 +1997,9 @@ __device__ __forceinline__ void collapseRows(const HalfStage& S, const UnitGeo& 
     }
 }
 
-// Tiles are handed out one at a time through `counter` (zero at launch), so
-// a CTA that starts late, behind other frames' kernels, simply takes fewer.
+// Tiles are handed out in runs of up to kBlendRun through `counter` (zero at
+// launch), so a CTA that starts late, behind other frames' kernels, simply takes
+// fewer.
 //
 // probePolls > 0 is the failure-path test of the bounded waits: consumer
 // thread 0 first waits that many polls on an mbarrier that nothing arrives
