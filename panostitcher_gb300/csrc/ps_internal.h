@@ -131,6 +131,8 @@ cudaError_t launchAlphaDown(const uint16_t* aj, int sw, int sh, int spitch, long
 // weight chain: Wt_{j+1} = (pyrDown(Wt_j) + 128) >> 8
 cudaError_t launchWeightDown(const uint16_t* wj, int sw, int sh, int spitch, long long sstride, uint16_t* wn,
                              int dw, int dh, int dpitch, long long dstride, int n, cudaStream_t st);
+// a collapsed level of zeros (biased, see C[j] in ps_device.cuh); pixels: even
+cudaError_t launchZeroCollapsed(void* c, long long pixels, cudaStream_t st);
 // per-tile "any non-zero" flags of a 16-bit or 8-bit plane per camera
 cudaError_t launchTileFlags16(const uint16_t* p, int w, int h, int pitch, long long camStride, int n, int tw,
                               int th, int tilesX, int tilesY, uint8_t* flags, cudaStream_t st);

@@ -723,6 +723,21 @@ cudaError_t launchLinearWeights(const uint8_t* seam, const uint8_t* cov, int n, 
     return cudaGetLastError();
 }
 
+__global__ void k_zero_collapsed(uint4* c, long long n)
+{
+    constexpr uint32_t br = (uint32_t)kCBias << 16 | kCBias;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        c[i] = make_uint4(br, kCBias, br, kCBias);
+}
+
+cudaError_t launchZeroCollapsed(void* c, long long pixels, cudaStream_t st)
+{
+    const long long n = pixels / 2;  // 16 bytes each
+    if (n <= 0) return cudaSuccess;
+    k_zero_collapsed<<<(int)std::min<long long>((n + 255) / 256, 4096), 256, 0, st>>>(static_cast<uint4*>(c), n);
+    return cudaGetLastError();
+}
+
 // Blender input images -> uchar4 level 0.  flags[0]: a 16-bit value outside
 // 0..255; flags[1]: a non-zero pixel where the coverage mask is 0 (the
 // multiband blend needs zeros there, source/Warp/ZReproject.cpp:200-208).

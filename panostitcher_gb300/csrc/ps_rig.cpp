@@ -441,7 +441,7 @@ void Rig::preparePyramids(const uint8_t* cov, const uint8_t* seam, const float* 
             lv_[j].Am.zero(st);
             for (int k = 0; k < slots_; k++) {
                 lv_[j].C[k].alloc(plane * 8);
-                lv_[j].C[k].zero(st);
+                PS_CUDA(launchZeroCollapsed(lv_[j].C[k].get(), (long long)plane, st));
             }
         }
     }
